@@ -77,8 +77,8 @@ enum {
    * GPU can access pageable host memory directly (the default there). */
   LS_HOST_STAGING = 1u << 5,
   /* Run every FIM iteration of a time step in one cooperative (all CTAs
-   * resident) launch, the sweep, schedule and check passes separated by
-   * grid-wide barriers, instead of three launches per iteration.  Same
+   * resident) launch, the iterations separated by grid-wide barriers,
+   * instead of one launch per iteration.  Same
    * results.  Applies where the step's sweep kernel has a persistent form
    * (the two-copies-per-thread tet sweep; the one-copy sweep of up to 384
    * threads); elsewhere it is ignored.  A barrier wait that exceeds
@@ -133,7 +133,9 @@ typedef struct ls_stats {
   long long nb_patches;         /* sum over steps of |NB|                   */
   long long flagged_copies;     /* local solves repeated in FP64 (precision form) */
   double ms_total;              /* device time of ls_step / ls_solve calls  */
-  /* LS_PROFILE only: per-kernel device time (ms) and launches */
+  /* LS_PROFILE only: per-kernel device time (ms) and launches.  A FIM
+   * iteration is one launch (checks, visits and the next list), recorded as a
+   * sweep; there are no check and schedule launches. */
   double ms_sweep, ms_check, ms_schedule, ms_seed, ms_narrowband, ms_update;
   long long n_sweep, n_check, n_schedule, n_seed, n_narrowband, n_update;
   long long sweep_slab_bytes;   /* algorithmic bytes read+written by the FIM patch kernel (visits and checks) */
@@ -145,8 +147,8 @@ typedef struct ls_stats {
   long long moved_vertices;     /* warm vertices the FIM moved by more than 1e-3 h */
   long long learned_fallbacks;  /* steps redone as plain FIM after 16 support rounds */
   long long pairs_collected;    /* training pairs recorded (ls_learn_collect) */
-  long long early_visits;       /* patch visits run by the neighbour check that activated the patch
-                                   (fast build, tetrahedra; counted in patch_visits too) */
+  long long early_visits;       /* patch visits that continue the neighbour check that activated the patch
+                                   (two-copies-per-thread sweep, tetrahedra; counted in patch_visits too) */
 } ls_stats;
 
 typedef struct ls_handle ls_handle;
@@ -211,10 +213,10 @@ ls_status ls_get_stats(ls_handle* h, ls_stats* s);
 /* Zeroes the counters and drops profiled kernel times not yet read. */
 ls_status ls_reset_stats(ls_handle* h);
 /* Per-launch record of the FIM patch kernel (no counterpart in the
- * reference, whose host loop times nothing): for every sweep and check
+ * reference, whose host loop times nothing): for every FIM
  * launch of the profiled steps (LS_PROFILE / ls_set_profile) since the last
- * ls_reset_stats, oldest first, its kind (0 sweep, or the whole FIM loop of
- * a step with LS_PERSISTENT; 1 neighbour check), its device time in ms
+ * ls_reset_stats, oldest first, its kind (0: one FIM iteration, or the whole
+ * FIM loop of a step with LS_PERSISTENT), its device time in ms
  * (CUDA events on the handle's stream) and its algorithmic slab bytes (the
  * per-visit bytes of every patch visit and check it ran; -1 past 4,096
  * launches in one step).  Copies min(cap, available) records into the

@@ -65,31 +65,63 @@ struct PatchPar {
   float bw, scale, dt, cc;
 };
 
+// FIM distance of a vertex: two stamped values {v0, t0, v1, t1} (float bits
+// and iteration stamp).  A visit in iteration t writes its results with stamp
+// t over the older of the two, while every other patch of that iteration
+// reads the newest value with a stamp below t: the values of the previous
+// iteration stay readable until the next one, so that no copy-back pass
+// separates the iterations.  Stamps grow from step to step; a step's first
+// stamp (its base) marks its seeds, which are written to {v0, t0} and never
+// visited, and a vertex with no stamp of this step holds LARGENUM (no reset
+// pass either).
+typedef int4 DtCell;
+
+__device__ __forceinline__ float dt_before(const DtCell& c, int t, int base, float LN) {
+  const int a = c.y < t ? c.y : -1, b = c.w < t ? c.w : -1;
+  const bool second = b > a;
+  return (second ? b : a) >= base ? __int_as_float(second ? c.z : c.x) : LN;
+}
+__device__ __forceinline__ bool dt_is_seed(const DtCell& c, int base) { return c.y == base; }
+constexpr int kStampMax = 0x7fffffff;
+
+// Step control words (DevState::ctl, one int each).
+enum {
+  CTL_VISITS = 0,   // [3] patches to visit in list i (iteration t uses list t % 3)
+  CTL_NB = 3,       // narrowband patches
+  CTL_CANDS = 4,    // [3] candidates to check in list i
+  CTL_NB_PREV = 7,  // previous step's narrowband patches (0: the seed search takes every patch)
+  CTL_BODIES = 8,   // FIM loop bodies run this step
+  CTL_CAP = 9,      // the iteration cap was hit
+  CTL_NB_VALID = 10,  // the narrowband list belongs to the current phi
+  CTL_ERR = 11,     // a wait of a FIM kernel timed out and the launch was abandoned (1: grid
+                    // barrier of the persistent kernel, 2: geometry slab copy)
+  CTL_ITER = 12,    // stamp of the first iteration of the next loop body
+  CTL_BASE = 13,    // base stamp of the step
+  CTL_ITERS = 14,   // iterations of this step that visited a patch
+  CTL_LAST = 15,    // stamp of the last of them
+  CTL_WORDS = 16
+};
+// Stamps restart (every stamped array cleared) between steps once they pass
+// this limit; a new handle starts a few steps below it.
+constexpr int kStampLimit = 1 << 29;
+
 // Device step state.
 struct DevState {
   float* phi;
   float* phi_out;
-  float* DT;
-  float* DT_out;
-  uint8_t* seed;    // per vertex: 1 = seed point of this step
-  uint8_t* sign;    // per vertex: 1 = phi >= 0 before redistance
-  int* blabel;      // per patch: 0 far, 1 active (host FIM labels of the reference)
-  int* bcon;        // per patch: 1 = converged
-  float* bmin;      // per patch: min DT after the visit
-  int* list0;       // active list, even iterations
-  int* list1;       // active list, odd iterations
-  int* newlist;     // neighbour candidates of this iteration
+  DtCell* cell;     // per vertex: FIM distance
+  int* slot;        // per patch: the half of its vertices' cells that its last visit wrote
+  // per patch, stamps: 2t = in the list of iteration t and not done with it,
+  // 2t + 1 = done with iteration t and not in the next list
+  int* pend;
+  int* reach;       // per patch: last iteration that left it converged with its minimum inside the band
+  int* lists;       // [3][nparts]: visits from the front, candidates from the back
   int* nblist;      // narrowband patches
-  int* counts;      // [0] list0, [1] list1, [2] newlist, [3] nblist, [4] fim iters (step)
+  int* ctl;         // step control words (CTL_*)
   unsigned long long* stats;  // [0] visits [1] checks [2] nb verts [3] nb patch verts [4] nb patches [5] fim iters [6] flagged copies solved [7] FIM slab bytes [8] visits run by checks
-  int* ctl;         // step control: [0] FIM loop bodies run this step, [1] iteration cap hit,
-                    // [2] previous narrowband valid (seed search restricted to it), [3] a wait of a
-                    // FIM kernel timed out and the launch was abandoned (1: grid barrier of the
-                    // persistent kernel, 2: geometry slab copy); cleared at every step start
-  int* sched;       // dynamic patch assignment of the sweep kernels: [0] next list entry of a
-                    // sweep, [1] of a check; zero between launches (the launch's last draw
-                    // resets it)
-  unsigned* gbar;   // persistent FIM kernel (kGridBarrierWords, zeroed per launch): [0] grid-barrier
+  int* sched;       // dynamic patch assignment of the FIM kernels: next list entry; zero between
+                    // launches (the launch's last draw resets it)
+  unsigned* gbar;   // persistent FIM kernel (kGridBarrierWords, zeroed per step): [0] grid-barrier
                     // arrivals since the launch started, [2 + smid] CTAs on SM smid
 };
 constexpr int kGridBarrierWords = 2 + 1024;
@@ -135,13 +167,6 @@ __device__ __forceinline__ PatchPar patch_par(const DevMesh& m, const StepParams
   return PatchPar{sp.bandwidth, sp.scale, sp.dt, sp.curv_coeff};
 }
 
-
-enum { LS_FAR = 0, LS_ACTIVE = 1 };
-
-// Mark on an active-list entry: the patch was already visited by the
-// neighbour check that activated it (k_fim_pair); the sweep skips it and the
-// schedule masks the mark off.
-constexpr int kPrevisited = 1 << 30;
 
 template <typename R>
 __device__ __forceinline__ R rmin(R a, R b) { return fmin(a, b); }

@@ -4,23 +4,26 @@
 // order as the CPU oracle it reproduces the oracle bit for bit).
 //
 // One step (reference order, src/core3d/cuda/meshFIM3d.cu:639-678):
-//   k_reset        DT := LARGENUM, seed := 0, sign := (phi >= 0)     (whole mesh)
-//   k_seed         seed points and the first active patch list        (K9)
-//   FIM iterations, each:
-//     sweep        NITER sweeps on every active patch, fused per-patch
-//                  convergence AND and min (K11 + K13)
-//     k_schedule   copy-back, unconverged patches to the next list,
-//                  neighbours of converged patches with min < w to the
-//                  candidate list (the host loop of redistance3d.cu:139-181)
-//     check        one-sweep probe of the candidates; unconverged ones join
-//                  the next list (K12 + K13 + redistance3d.cu:188-222)
-//     The sweep and the check are one kernel with a runtime flag: k_fim
-//     (bit-exact build and triangles: one element copy per thread, the
-//     reference's solves in its order), k_fim_compact (fast build,
-//     tetrahedra: the solves that can lower a value listed and run densely,
-//     one copy per thread) and k_fim_pair (the same with two copies per
-//     thread, the default for patches of up to 384 copies; its checks also
-//     run the visits of the patches they activate on long check lists).
+//   k_begin        step control words: base stamp, empty lists
+//   k_seed         seed points and the first patch list               (K9)
+//   FIM iterations, one launch each (t: the iteration's stamp):
+//     candidates   a one-sweep probe of each neighbour that the previous
+//                  iteration put up (K12 + K13 + redistance3d.cu:188-222);
+//                  one that finds its patch unconverged goes on to visit it
+//     visits       NITER sweeps on the patches still unconverged, fused
+//                  per-patch convergence AND and min (K11 + K13)
+//     lists        each CTA ends a patch by putting up what the next
+//                  iteration has to look at: the patch itself if
+//                  unconverged, else its neighbours if its minimum lies
+//                  inside the band (the host loop of redistance3d.cu:139-181)
+//     The reference's iteration is sweep, schedule, check; the check of one
+//     iteration and the sweep of the next read the same values, so they are
+//     one launch here, and no pass copies values back (DtCell).
+//     Kernels: k_fim (bit-exact build and triangles: one element copy per
+//     thread, the reference's solves in its order), k_fim_compact (fast
+//     build, tetrahedra: the solves that can lower a value listed and run
+//     densely, one copy per thread) and k_fim_pair (the same with two copies
+//     per thread, the default for patches of up to 384 copies).
 //   k_narrowband   patch narrowband, phi := sign * DT, vertex-update count (K14 + K10b)
 //   k_update       advection (K16) or mean-curvature update on narrowband patches
 //                  (k_update_384: the same for patches of up to 384 copies,
@@ -41,24 +44,152 @@ __device__ __forceinline__ int warp_id_global() {
 }
 
 // ---------------------------------------------------------------------------
-__global__ void k_reset(DevState s, int nv, float LN) {
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
-    s.DT[v] = LN;
-    s.seed[v] = 0;
-    s.sign[v] = (s.phi[v] < 0.f) ? 0 : 1;
+// Start of a step: empty lists, a base stamp above every stamp in use, the
+// previous narrowband's size for the seed search (kept on a restart within
+// the step), zeroed draw counter and grid barrier (an abandoned launch can
+// leave them set).
+__global__ void k_begin(DevState s, int restart) {
+  int* c = s.ctl;
+  for (int i = threadIdx.x; i < kGridBarrierWords; i += blockDim.x) s.gbar[i] = 0u;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 3; ++i) c[CTL_VISITS + i] = c[CTL_CANDS + i] = 0;
+    if (!restart) {
+      c[CTL_NB_PREV] = c[CTL_NB_VALID] ? c[CTL_NB] : 0;
+      c[CTL_NB_VALID] = 1;
+    }
+    c[CTL_NB] = 0;
+    c[CTL_BODIES] = c[CTL_CAP] = c[CTL_ERR] = c[CTL_ITERS] = 0;
+    const int u = c[CTL_ITER];
+    c[CTL_BASE] = c[CTL_LAST] = u;  // u: seeds, u + 1: warm-start values
+    c[CTL_ITER] = u + 2;
+    s.sched[0] = 0;
   }
+}
+
+__device__ __forceinline__ int ld_relaxed(const int* p) { return *reinterpret_cast<const volatile int*>(p); }
+
+// One FIM iteration's view of the control words: its stamp, the step's base,
+// the sizes of its list (visits, then candidates).
+struct FimIter {
+  int t, base, nvis, count;
+  const int* list;  // visits from the front, candidates from the back
+  int* next;        // the next iteration's list
+  int* next_n;      // and its sizes: [0] visits, [CTL_CANDS - CTL_VISITS] candidates
+};
+
+__device__ __forceinline__ FimIter fim_iter(const DevMesh& m, const DevState& s, int t) {
+  FimIter f;
+  const int cur = t % 3, nxt = cur == 2 ? 0 : cur + 1;
+  f.t = t;
+  f.base = ld_relaxed(s.ctl + CTL_BASE);
+  f.nvis = ld_relaxed(s.ctl + CTL_VISITS + cur);
+  f.count = f.nvis + ld_relaxed(s.ctl + CTL_CANDS + cur);
+  f.list = s.lists + (size_t)cur * m.nparts;
+  f.next = s.lists + (size_t)nxt * m.nparts;
+  f.next_n = s.ctl + CTL_VISITS + nxt;
+  // the list after the next one was read by the previous iteration
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const int aft = nxt == 2 ? 0 : nxt + 1;
+    s.ctl[CTL_VISITS + aft] = 0;
+    s.ctl[CTL_CANDS + aft] = 0;
+  }
+  return f;
+}
+
+// Entry i of the list; *visit: a patch to visit (else a candidate to check).
+__device__ __forceinline__ int fim_entry(const DevMesh& m, const FimIter& f, int i, bool* visit) {
+  *visit = i < f.nvis;
+  return *visit ? f.list[i] : f.list[m.nparts - 1 - (i - f.nvis)];
+}
+
+// End of patch p in iteration t (one whole warp): what the next iteration has
+// to look at.  far: the patch converged (or its check found nothing); reach:
+// it was visited and its minimum lies inside the band.
+// An unconverged patch goes to the next list's visits.  A neighbour of a
+// patch that reached becomes a candidate unless it is unconverged itself,
+// and that is known only when it is done with its own entry.  So each patch
+// first publishes its state and then looks at its neighbours': of two
+// neighbours that end in the same iteration, at least one sees the other
+// done (sequentially consistent fences between the store and the loads on
+// both sides), and whichever moves the stamp of the candidate appends it.
+__device__ __forceinline__ void fim_publish(const DevMesh& m, const DevState& s, const FimIter& f, int p, bool far,
+                                            bool reach) {
+  const int lane = threadIdx.x & 31;
+  const int t = f.t, next = 2 * (t + 1);
+  if (!far) {
+    if (lane == 0) {
+      *reinterpret_cast<volatile int*>(s.pend + p) = next;
+      f.next[atomicAdd(f.next_n, 1)] = p;
+    }
+    return;
+  }
+  const int a = m.padj_off[p], b = m.padj_off[p + 1];
+  if (lane == 0) {
+    if (reach) *reinterpret_cast<volatile int*>(s.reach + p) = t;
+    *reinterpret_cast<volatile int*>(s.pend + p) = 2 * t + 1;
+  }
+  __syncwarp();
+  __threadfence();
+  bool self = false;
+  int* cands = f.next_n + (CTL_CANDS - CTL_VISITS);
+  for (int j0 = a; j0 < b; j0 += 32) {
+    const int j = j0 + lane;
+    bool take = false;
+    int q = -1;
+    if (j < b) {
+      q = m.padj[j];
+      self |= ld_relaxed(s.reach + q) == t;
+      if (reach) {
+        // not in this iteration's list (below 2t) or done with it: a
+        // candidate; pending (2t): it will see this patch's state itself
+        const int w = ld_relaxed(s.pend + q);
+        take = w != 2 * t && w < next && atomicCAS(s.pend + q, w, next) == w;
+      }
+    }
+    const unsigned mask = __ballot_sync(0xffffffffu, take);
+    if (mask) {
+      const int leader = __ffs(mask) - 1;
+      int pos = 0;
+      if (lane == leader) pos = atomicAdd(cands, __popc(mask));
+      pos = __shfl_sync(0xffffffffu, pos, leader);
+      if (take) f.next[m.nparts - 1 - (pos + __popc(mask & ((1u << lane) - 1u)))] = q;
+    }
+  }
+  if (__any_sync(0xffffffffu, self) && lane == 0 && atomicCAS(s.pend + p, 2 * t + 1, next) == 2 * t + 1)
+    f.next[m.nparts - 1 - atomicAdd(cands, 1)] = p;
+}
+
+// Work counters of a CTA's pass, kept by its thread 0 and added to the
+// step's once at the end.
+struct FimCount {
+  int visits, checks, early;
+  unsigned long long bytes;
+};
+__device__ __forceinline__ void fim_count_flush(const DevState& s, const FimIter& f, const FimCount& n) {
+  if (n.visits) {
+    atomicAdd(&s.stats[0], (unsigned long long)n.visits);
+    if (atomicMax(s.ctl + CTL_LAST, f.t) < f.t) {
+      atomicAdd(s.ctl + CTL_ITERS, 1);
+      atomicAdd(&s.stats[5], 1ull);
+    }
+  }
+  if (n.checks) atomicAdd(&s.stats[1], (unsigned long long)n.checks);
+  if (n.early) atomicAdd(&s.stats[8], (unsigned long long)n.early);
+  if (n.bytes) atomicAdd(&s.stats[7], n.bytes);
 }
 
 // Seed search (redistance_kernels3d.h:623-770): an element copy whose
 // vertex values include an exact zero or differ in sign marks those
 // vertices as seeds with DT = |phi|; the patch joins list0.
 template <int D1>
-__global__ void k_seed(DevMesh m, DevState s, int use_all, float scale, int warm) {
-  // use_all < 0: decided on the device from the step-control flag
-  if (use_all < 0) use_all = s.ctl[2] ? 0 : 1;
-  const int count = use_all ? m.nparts : s.counts[3];
+__global__ void k_seed(DevMesh m, DevState s, float scale, int warm) {
+  const int nprev = s.ctl[CTL_NB_PREV];
+  const int base = s.ctl[CTL_BASE], t0 = s.ctl[CTL_ITER];
+  int* list = s.lists + (size_t)(t0 % 3) * m.nparts;
+  int* list_n = s.ctl + CTL_VISITS + t0 % 3;
+  const int count = nprev ? nprev : m.nparts;
   for (int li = blockIdx.x; li < count; li += gridDim.x) {
-    const int p = use_all ? li : s.nblist[li];
+    const int p = nprev ? s.nblist[li] : li;
     const float sc = m.patch_mesh ? __ldg(&m.mesh_par[m.patch_mesh[p]]).y : scale;
     const int vs = m.vert_off[p], nvp = m.vert_off[p + 1] - vs;
     const int gs = m.ghost_off[p];
@@ -81,26 +212,24 @@ __global__ void k_seed(DevMesh m, DevState s, int use_all, float scale, int warm
 #pragma unroll
       for (int k = 0; k < D1; ++k) {
         if (cross || val[k] == 0.f) {
-          s.seed[gv[k]] = 1;
-          s.DT[gv[k]] = fabsf(val[k]) / sc;
+          *reinterpret_cast<int2*>(s.cell + gv[k]) = make_int2(__float_as_int(fabsf(val[k]) / sc), base);
           found = 1;
         }
       }
     }
     found = __syncthreads_or(found);
     if (threadIdx.x == 0 && (found || warm)) {
-      const int pos = atomicAdd(&s.counts[0], 1);
-      s.list0[pos] = p;
+      list[atomicAdd(list_n, 1)] = p;
+      s.pend[p] = 2 * t0;
     }
   }
 }
 
 // ---------------------------------------------------------------------------
-// FIM patch visit.  CHECK = false: NITER sweeps, writes DT_out and the patch
-// convergence / minimum / label (kernel_update_values + run_reduction_
-// bandwidth).  CHECK = true: one sweep, no value writes; unconverged
-// candidates are appended to the next list (kernel_run_check_neghbor +
-// run_reduction3d + redistance3d.cu:214-222).
+// FIM patch visit: NITER sweeps, then the patch's values, convergence and
+// minimum (kernel_update_values + run_reduction_bandwidth).  A candidate
+// first runs one sweep (kernel_run_check_neghbor + run_reduction3d +
+// redistance3d.cu:214-222) and is visited if that finds it unconverged.
 // Solves of one element copy (Jacobi: all from the values at sweep start).
 // With the precision form (tau > 0) a solve whose discriminant cancelled is
 // repeated in FP64; `nflag` counts those repeats.
@@ -230,49 +359,38 @@ __device__ __forceinline__ void copy_metric(const DevMesh& m, long long c, float
   }
 }
 
-// The neighbour check and the sweep are one kernel with a runtime flag: both
-// must evaluate a patch's first sweep with the same instructions, otherwise
-// differently contracted FMAs could make the check report a drop of more
-// than the tolerance that the following visit never applies, and two
+// A candidate's check is the first sweep of its visit, run by the same
+// instructions: with differently contracted FMAs the check could report a
+// drop of more than the tolerance that the visit never applies, and two
 // patches could re-activate each other without end.
-// vb: the CTA's index in the patch assignment (blockIdx.x, or the spread
-// index of the persistent kernel)
+// t: the iteration's stamp; vb: the CTA's index in the patch assignment
+// (blockIdx.x, or the spread index of the persistent kernel)
 template <int D1, bool XDIV, bool PREC>
-__device__ __forceinline__ void fim_copy_pass(const DevMesh& m, const DevState& s, const StepParams& sp, int cur,
-                                              int check, int vb) {
-  const bool CHECK = check != 0;
+__device__ __forceinline__ void fim_copy_pass(const DevMesh& m, const DevState& s, const StepParams& sp, int t,
+                                              int vb) {
   extern __shared__ float smem[];
   float* sT = smem;                       // owned + ghost values
   float* sOld = smem + sp.lvp + sp.lgp;   // owned values at the start of the last sweep
-  __shared__ unsigned s_min;
+  __shared__ unsigned s_min[2];           // patch minimum, by parity of the CTA's patches
   __shared__ int s_qn;  // deferred FP64 solves queued in this sweep (precision form)
   DeferredSolve* sQ = reinterpret_cast<DeferredSolve*>(smem + 2 * sp.lvp + sp.lgp);
   if (PREC && threadIdx.x == 0) s_qn = 0;
-  const int* list = CHECK ? s.newlist : (cur ? s.list1 : s.list0);
-  const int count = CHECK ? s.counts[2] : s.counts[cur];
-  const int nxt = cur ^ 1;
-  int* nlist = nxt ? s.list1 : s.list0;
-  if (!CHECK && blockIdx.x == 0 && threadIdx.x == 0) {
-    // the next list and the candidate list are filled by the following kernels
-    s.counts[nxt] = 0;
-    s.counts[2] = 0;
-    if (count > 0) {
-      s.counts[4] += 1;
-      atomicAdd(&s.stats[5], 1ull);
-    }
-    atomicAdd(&s.stats[0], (unsigned long long)count);
-  }
-  if (CHECK && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&s.stats[1], (unsigned long long)count);
-  const int niter = CHECK ? 1 : sp.niter;
+  const FimIter f = fim_iter(m, s, t);
   const int tid = threadIdx.x;
-  for (int li = vb; li < count; li += gridDim.x) {
-    const int p = list[li] & ~kPrevisited;  // re-visiting is harmless: same inputs, same results
+  FimCount cnt = {};
+  int par = 0;
+  for (int li = vb; li < f.count; li += gridDim.x, par ^= 1) {
+    bool visit;
+    const int p = fim_entry(m, f, li, &visit);
     const int vs = m.vert_off[p], nvp = m.vert_off[p + 1] - vs;
     const int gs = m.ghost_off[p], ngp = m.ghost_off[p + 1] - gs;
     const int es = m.ele_off[p], nep = m.ele_off[p + 1] - es;
+    const int slot = s.slot[p] ^ 1;
+    int niter = visit ? sp.niter : 1;
+    if (tid == 0) (visit ? cnt.visits : cnt.checks)++;
     for (int i = tid; i < nvp + ngp; i += blockDim.x)
-      sT[i] = s.DT[i < nvp ? vs + i : __ldg(m.ghost_ids + gs + i - nvp)];
-    if (tid == 0) s_min = 0x7f800000u;
+      sT[i] = dt_before(s.cell[i < nvp ? vs + i : __ldg(m.ghost_ids + gs + i - nvp)], t, f.base, sp.largenum);
+    if (tid == 0) s_min[par] = 0x7f800000u;
     __syncthreads();
     const bool act = tid < nep;
     int idx[4] = {0, 0, 0, 0};
@@ -363,60 +481,69 @@ __device__ __forceinline__ void fim_copy_pass(const DevMesh& m, const DevState& 
         for (int k = 0; k < D1; ++k)
           if ((shared_k >> k) & 1u) T[k] = sT[idx[k]];
       }
+      if (!visit) {
+        // the check's verdict: a drop of tol or more makes it a visit, whose
+        // first sweep this was
+        int c0 = 1;
+        for (int i = tid; i < nvp; i += blockDim.x)
+          if (!dt_is_seed(s.cell[vs + i], f.base)) c0 &= (sOld[i] - sT[i] < sp.tol) ? 1 : 0;
+        if (__syncthreads_and(c0)) break;
+        visit = true;
+        niter = sp.niter;
+        nflag *= 2;  // the visit's own repeats of this sweep, counted as run again
+        if (tid == 0) {
+          cnt.visits++;
+          cnt.bytes += (unsigned long long)(__ldg(m.patch_bytes + p) - 4 * nvp);
+        }
+      }
       __syncthreads();
     }
+    // a check that found nothing writes nothing
     int con = 1;
-    for (int i = tid; i < nvp; i += blockDim.x) {
-      const int v = vs + i;
-      const float nt = sT[i];
-      float outv;
-      if (!s.seed[v]) {
-        if (!CHECK) s.DT_out[v] = nt;
-        con &= (sOld[i] - nt < sp.tol) ? 1 : 0;
-        outv = nt;
-      } else {
-        outv = s.DT[v];
+    if (visit)
+      for (int i = tid; i < nvp; i += blockDim.x) {
+        const int v = vs + i;
+        const float nt = sT[i];
+        float outv;
+        const DtCell c = s.cell[v];
+        if (!dt_is_seed(c, f.base)) {
+          reinterpret_cast<int2*>(s.cell + v)[slot] = make_int2(__float_as_int(nt), t);
+          con &= (sOld[i] - nt < sp.tol) ? 1 : 0;
+          outv = nt;
+        } else {
+          outv = __int_as_float(c.x);
+        }
+        atomicMin(&s_min[par], __float_as_uint(outv));
       }
-      if (!CHECK) atomicMin(&s_min, __float_as_uint(outv));
-    }
     if (D1 == 4 && sp.tau > 0.f) {
       nflag = __reduce_add_sync(0xffffffffu, nflag);
       if ((tid & 31) == 0 && nflag) atomicAdd(&s.stats[6], (unsigned long long)nflag);
     }
     con = __syncthreads_and(con);
     if (tid == 0) {
-      if (!CHECK) {
-        atomicAdd(&s.stats[7], (unsigned long long)__ldg(m.patch_bytes + p));
-        s.bcon[p] = con;
-        s.bmin[p] = __uint_as_float(s_min);
-        s.blabel[p] = con ? LS_FAR : LS_ACTIVE;
-      } else {
-        // a check reads the visit's slab but writes no DT_out
-        atomicAdd(&s.stats[7], (unsigned long long)(__ldg(m.patch_bytes + p) - 4 * nvp));
-        if (!con) {
-          const int pos = atomicAdd(&s.counts[nxt], 1);
-          nlist[pos] = p;
-        } else {
-          s.blabel[p] = LS_FAR;
-        }
-      }
+      // a check reads the visit's slab but writes no values
+      cnt.bytes += (unsigned long long)(__ldg(m.patch_bytes + p) - (visit ? 0 : 4 * nvp));
+      if (visit) s.slot[p] = slot;
     }
+    if ((tid >> 5) == ((int)blockDim.x >> 5) - 1)
+      fim_publish(m, s, f, p, con != 0, visit && __uint_as_float(s_min[par]) < patch_par(m, sp, p).bw);
     __syncthreads();
   }
+  if (tid == 0) fim_count_flush(s, f, cnt);
 }
 
 template <int D1, int MAXT, bool XDIV, int MINB, bool PREC>
-__global__ void __launch_bounds__(MAXT, MINB) k_fim(DevMesh m, DevState s, StepParams sp, int cur, int check) {
-  fim_copy_pass<D1, XDIV, PREC>(m, s, sp, cur, check, blockIdx.x);
+__global__ void __launch_bounds__(MAXT, MINB) k_fim(DevMesh m, DevState s, StepParams sp, int off) {
+  fim_copy_pass<D1, XDIV, PREC>(m, s, sp, s.ctl[CTL_ITER] + off, blockIdx.x);
 }
 
 // Patch assignment of the sweep kernels: CTA b takes list entry b first
 // (consecutive CTA ids sit on different SMs, so a short list spreads over the
-// whole GPU), then draws entries gridDim.x, gridDim.x + 1, ... from the launch
-// kind's counter, so that CTAs that drew cheap patches take more.  Only CTAs
+// whole GPU), then draws entries gridDim.x, gridDim.x + 1, ... from a
+// counter, so that CTAs that drew cheap patches take more.  Only CTAs
 // that had a first entry draw, each until its first miss: the draws number
 // max(count - gridDim.x, 0) + min(count, gridDim.x), and the last of them
-// (value count - 1) resets the counter for the next launch of the kind.
+// (value count - 1) resets the counter for the next launch.
 __device__ __forceinline__ int draw_patch(int* next, int count) {
   const int v = atomicAdd(next, 1);
   if (v == count - 1) atomicExch(next, 0);
@@ -433,10 +560,10 @@ __device__ __forceinline__ int draw_patch(int* next, int count) {
 // then run the listed solves densely, one solve per thread at a time.
 // Shared memory per CTA (stride MAXT): metric [11], heights [4], copy
 // values at the sweep start [4], ghost results [4], connectivity, list.
+// A candidate found unconverged by its check runs its visit from the start
+// (the check's sweep left out the ghost targets).
 template <int MAXT, int MINB, bool PREC>
-__global__ void __launch_bounds__(MAXT, MINB) k_fim_compact(DevMesh m, DevState s, StepParams sp, int cur,
-                                                            int check) {
-  const bool CHECK = check != 0;
+__global__ void __launch_bounds__(MAXT, MINB) k_fim_compact(DevMesh m, DevState s, StepParams sp, int off) {
   extern __shared__ float smem[];
   float* sT = smem;                       // owned + ghost values
   float* sOld = smem + sp.lvp + sp.lgp;   // owned values at the start of the last sweep
@@ -448,27 +575,16 @@ __global__ void __launch_bounds__(MAXT, MINB) k_fim_compact(DevMesh m, DevState 
   int* sItem = reinterpret_cast<int*>(sC + MAXT);           // [4 * MAXT] listed solves (copy << 2 | k)
   int* sRep = sItem + 4 * MAXT;  // precision form: [4 * MAXT] solves to repeat in FP64
   __shared__ int s_rep;
-  __shared__ unsigned s_min;
+  __shared__ unsigned s_min[2];  // patch minimum, by parity of the CTA's patches
   __shared__ int s_n[2];  // listed solves, by sweep parity (reset one sweep ahead)
   __shared__ int s_li;    // list entry of the next patch
-  const int* list = CHECK ? s.newlist : (cur ? s.list1 : s.list0);
-  const int count = CHECK ? s.counts[2] : s.counts[cur];
-  const int nxt = cur ^ 1;
-  int* nlist = nxt ? s.list1 : s.list0;
-  if (!CHECK && blockIdx.x == 0 && threadIdx.x == 0) {
-    s.counts[nxt] = 0;
-    s.counts[2] = 0;
-    if (count > 0) {
-      s.counts[4] += 1;
-      atomicAdd(&s.stats[5], 1ull);
-    }
-    atomicAdd(&s.stats[0], (unsigned long long)count);
-  }
-  if (CHECK && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&s.stats[1], (unsigned long long)count);
-  const int niter = CHECK ? 1 : sp.niter;
+  const int t = s.ctl[CTL_ITER] + off;
+  const FimIter f = fim_iter(m, s, t);
+  FimCount cnt = {};
+  int par = 0;
   const int tid = threadIdx.x;
   // first entry by CTA index, later ones drawn from a counter (draw_patch)
-  int* next = s.sched + (CHECK ? 1 : 0);
+  int* next = s.sched;
   if (tid == 0) {
     s_n[0] = s_n[1] = 0;
     s_rep = 0;
@@ -476,14 +592,19 @@ __global__ void __launch_bounds__(MAXT, MINB) k_fim_compact(DevMesh m, DevState 
   }
   __syncthreads();
   int nflag = 0;
-  for (int li = s_li; li < count;) {
-    const int p = list[li] & ~kPrevisited;  // re-visiting is harmless: same inputs, same results
+  for (int li = s_li; li < f.count; par ^= 1) {
+    bool visit;
+    const int p = fim_entry(m, f, li, &visit);
     const int vs = m.vert_off[p], nvp = m.vert_off[p + 1] - vs;
     const int gs = m.ghost_off[p], ngp = m.ghost_off[p + 1] - gs;
     const int es = m.ele_off[p], nep = m.ele_off[p + 1] - es;
+    const int slot = s.slot[p] ^ 1;
+    if (tid == 0) (visit ? cnt.visits : cnt.checks)++;
+  again:
+    const int niter = visit ? sp.niter : 1;
     for (int i = tid; i < nvp + ngp; i += blockDim.x)
-      sT[i] = s.DT[i < nvp ? vs + i : __ldg(m.ghost_ids + gs + i - nvp)];
-    if (tid == 0) s_min = 0x7f800000u;
+      sT[i] = dt_before(s.cell[i < nvp ? vs + i : __ldg(m.ghost_ids + gs + i - nvp)], t, f.base, sp.largenum);
+    if (tid == 0) s_min[par] = 0x7f800000u;
     __syncthreads();
     const bool act = tid < nep;
     int idx[4] = {0, 0, 0, 0};
@@ -639,38 +760,35 @@ __global__ void __launch_bounds__(MAXT, MINB) k_fim_compact(DevMesh m, DevState 
       const int v = vs + i;
       const float nt = sT[i];
       float outv;
-      if (!s.seed[v]) {
-        if (!CHECK) s.DT_out[v] = nt;
+      const DtCell c = s.cell[v];
+      if (!dt_is_seed(c, f.base)) {
+        if (visit) reinterpret_cast<int2*>(s.cell + v)[slot] = make_int2(__float_as_int(nt), t);
         con &= (sOld[i] - nt < sp.tol) ? 1 : 0;
         outv = nt;
       } else {
-        outv = s.DT[v];
+        outv = __int_as_float(c.x);
       }
-      if (!CHECK) atomicMin(&s_min, __float_as_uint(outv));
+      if (visit) atomicMin(&s_min[par], __float_as_uint(outv));
     }
     con = __syncthreads_and(con);
     if (tid == 0) {
-      if (!CHECK) {
-        atomicAdd(&s.stats[7], (unsigned long long)__ldg(m.patch_bytes + p));
-        s.bcon[p] = con;
-        s.bmin[p] = __uint_as_float(s_min);
-        s.blabel[p] = con ? LS_FAR : LS_ACTIVE;
-      } else {
-        // a check reads the visit's slab but writes no DT_out
-        atomicAdd(&s.stats[7], (unsigned long long)(__ldg(m.patch_bytes + p) - 4 * nvp));
-        if (!con) {
-          const int pos = atomicAdd(&s.counts[nxt], 1);
-          nlist[pos] = p;
-        } else {
-          s.blabel[p] = LS_FAR;
-        }
-      }
+      // a check reads the visit's slab but writes no values
+      cnt.bytes += (unsigned long long)(__ldg(m.patch_bytes + p) - (visit ? 0 : 4 * nvp));
+      if (visit) s.slot[p] = slot;
     }
+    if (!visit && !con) {
+      visit = true;
+      if (tid == 0) cnt.visits++;
+      goto again;
+    }
+    if ((tid >> 5) == ((int)blockDim.x >> 5) - 1)
+      fim_publish(m, s, f, p, con != 0, visit && __uint_as_float(s_min[par]) < patch_par(m, sp, p).bw);
     __syncthreads();
-    if (tid == 0) s_li = draw_patch(next, count);
+    if (tid == 0) s_li = draw_patch(next, f.count);
     __syncthreads();
     li = s_li;
   }
+  if (tid == 0) fim_count_flush(s, f, cnt);
   if (PREC) {
     nflag = __reduce_add_sync(0xffffffffu, nflag);
     if ((tid & 31) == 0 && nflag) atomicAdd(&s.stats[6], (unsigned long long)nflag);
@@ -846,14 +964,12 @@ __device__ __forceinline__ bool slab_wait(unsigned bar, unsigned parity, bool gi
 // the copies in flight and ends the CTA's pass; the host then reports
 // LS_DEVICE_TIMEOUT.
 // Patches: the list entry of the CTA's index first, later ones from
-// draw_patch.  On a check launch of at least two patches per CTA, a check
-// that finds its patch unconverged goes on to run that patch's visit (the
-// next iteration's visit would read the same DT) and marks the patch's entry
-// in the next list with kPrevisited; the next sweep skips marked entries.
+// draw_patch.  A candidate's check is the first sweep of its visit without
+// the ghost targets; if it finds the patch unconverged, those are run from
+// the same sweep-start values and the visit goes on.
 template <int SOLVER>
-__device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& s, const StepParams& sp, int cur,
-                                              int check, int vb) {
-  const bool CHECK = check != 0;
+__device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& s, const StepParams& sp, int t,
+                                              int vb) {
   extern __shared__ float4 smem4[];
   float* sT = reinterpret_cast<float*>(smem4);  // owned + ghost values
   float* sOld = sT + sp.lvp + sp.lgp;          // owned values at the start of the last sweep
@@ -864,40 +980,22 @@ __device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& 
   float4* sR = sH + ncap;
   ushort4* sC = reinterpret_cast<ushort4*>(sR + ncap);
   unsigned short* sItem = reinterpret_cast<unsigned short*>(sC + ncap);
-  __shared__ unsigned s_min;
+  __shared__ unsigned s_min[2];  // patch minimum, by parity of the CTA's patches
   __shared__ int s_n[2];  // listed solves, by sweep parity (reset one sweep ahead)
   __shared__ int s_li;    // list entry of the next patch
   __shared__ int s_ng;    // ghost-target solves listed when a check becomes a visit
   __shared__ unsigned s_seed[kSeedMaskWords];  // seed flags of the owned vertices (bit i = vertex i)
   __shared__ __align__(8) unsigned long long s_bar;  // geometry slab copies of the current patch
   __shared__ int s_err;  // a slab wait ran out: the pass ends
-  const int* list = CHECK ? s.newlist : (cur ? s.list1 : s.list0);
-  const int count = CHECK ? s.counts[2] : s.counts[cur];
-  const int nxt = cur ^ 1;
-  int* nlist = nxt ? s.list1 : s.list0;
-  if (!CHECK && blockIdx.x == 0 && threadIdx.x == 0) {
-    s.counts[nxt] = 0;
-    s.counts[2] = 0;
-    if (count > 0) {
-      s.counts[4] += 1;
-      atomicAdd(&s.stats[5], 1ull);
-    }
-    atomicAdd(&s.stats[0], (unsigned long long)count);
-  }
-  if (CHECK && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&s.stats[1], (unsigned long long)count);
-  const int niter = CHECK ? 1 : sp.niter;
+  __shared__ FimCount s_cnt;  // thread 0's work counters (in shared memory for their registers)
+  const FimIter f = fim_iter(m, s, t);
   const int tid = threadIdx.x;
   const unsigned bar = smem_u32addr(&s_bar);
   unsigned phase = 0;      // thread 0: parity of the slab copies' current phase
   bool in_flight = false;  // thread 0: copies whose wait ran out twice
   // first entry by CTA index, later ones drawn from a counter (draw_patch)
-  int* next = s.sched + (CHECK ? 1 : 0);
-  // visits run by the checks that activate them only pay when the check
-  // launch is throughput bound (four checks or more per resident CTA, the
-  // best of 1, 2, 4 and 8 measured at 128^3): on fewer patches they add a
-  // visit's length to the iteration, while the next sweep launch still waits
-  // for the patches that stayed active
-  const bool early = CHECK && sp.niter > 1 && count >= 4 * (int)gridDim.x;
+  int* next = s.sched;
+  int par = 0;
   // the owned vertices' seed flags are kept in shared memory when every patch
   // fits the mask (read by the check's verdict and the copy-out)
   const bool seed_mask = sp.lvp <= 32 * kSeedMaskWords;
@@ -905,294 +1003,273 @@ __device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& 
     s_n[0] = s_n[1] = 0;
     s_li = vb;
     s_err = 0;
+    s_cnt = FimCount{};
     slab_bar_init(bar);
   }
   __syncthreads();
-  for (int li = s_li; li < count;) {
-    const int entry = list[li];
-    // an entry marked as visited ahead was visited by the check that activated
-    // it, from the inputs this sweep would read: nothing is left to do
-    if (!(entry & kPrevisited)) {
-      const int p = entry;
-      const int vs = m.vert_off[p], nvp = m.vert_off[p + 1] - vs;
-      const int gs = m.ghost_off[p], ngp = m.ghost_off[p + 1] - gs;
-      const int es = m.ele_off[p], nep = m.ele_off[p + 1] - es;
-      // the metric and height slabs: in flight while the values, seed flags
-      // and connectivity load (the previous patch's last reads of sM and sH
-      // came before its final barrier)
-      if (tid == 0) geo_issue(m, es, nep, sM, sH, bar);
-      // every load of the patch's own slab is issued before any of them is
-      // stored (values, seed flags, connectivity: independent round trips
-      // that overlap; a ghost value waits only for its id), then stored.
-      // First slab entry, seed flag and copies of each thread:
-      const int nslab = nvp + ngp;
-      const int gv0 = tid < nvp ? vs + tid : (tid < nslab ? __ldg(m.ghost_ids + gs + tid - nvp) : -1);
-      const bool sd0 = seed_mask && tid < nvp && s.seed[vs + tid] != 0;
-      ushort4 cvv[2];
-  #pragma unroll
+  for (int li = s_li; li < f.count; par ^= 1) {
+    bool visit;
+    const int p = fim_entry(m, f, li, &visit);
+    const bool check = !visit;
+    const int vs = m.vert_off[p], nvp = m.vert_off[p + 1] - vs;
+    const int gs = m.ghost_off[p], ngp = m.ghost_off[p + 1] - gs;
+    const int es = m.ele_off[p], nep = m.ele_off[p + 1] - es;
+    // the metric and height slabs: in flight while the values, seed flags
+    // and connectivity load (the previous patch's last reads of sM and sH
+    // came before its final barrier)
+    if (tid == 0) geo_issue(m, es, nep, sM, sH, bar);
+    // every load of the patch's own slab is issued before any of them is
+    // stored (values, seed flags, connectivity: independent round trips
+    // that overlap; a ghost value waits only for its id), then stored.
+    // First slab entry, seed flag and copies of each thread:
+    const int nslab = nvp + ngp;
+    const int gv0 = tid < nvp ? vs + tid : (tid < nslab ? __ldg(m.ghost_ids + gs + tid - nvp) : -1);
+    ushort4 cvv[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int c = tid + j * blockDim.x;
+      if (c < nep) cvv[j] = __ldcs(m.conn + es + c);  // streamed, like the geometry records (evict-first)
+    }
+    const DtCell c0 = gv0 >= 0 ? s.cell[gv0] : DtCell{};
+    const bool sd0 = tid < nvp && dt_is_seed(c0, f.base);
+    if (tid < nslab) sT[tid] = dt_before(c0, t, f.base, sp.largenum);
+    for (int i = tid + blockDim.x; i < nslab; i += blockDim.x)
+      sT[i] = dt_before(s.cell[i < nvp ? vs + i : __ldg(m.ghost_ids + gs + i - nvp)], t, f.base, sp.largenum);
+    // whole warps run each 32-vertex word (the block is whole warps and the
+    // bound a multiple of 32)
+    if (seed_mask)
+      for (int i = tid; i < ((nvp + 31) & ~31); i += blockDim.x) {
+        const bool sd = i == tid ? sd0 : (i < nvp && dt_is_seed(s.cell[vs + i], f.base));
+        const unsigned b = __ballot_sync(0xffffffffu, sd);
+        if ((i & 31) == 0) s_seed[i >> 5] = b;
+      }
+    // the copies' connectivity (the previous patch's last reads of sC came
+    // before its final barrier) and flags, which only this thread reads:
+    // bits 8j .. 8j+3 the vertices of copy j that changed in the previous
+    // sweep (all on the first), bits 8j+4 .. 8j+7 its ghost vertices
+    unsigned flags = 0u;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int c = tid + j * blockDim.x;
+      if (c < nep) {
+        const ushort4 cv = cvv[j];
+        sC[c] = cv;
+        const unsigned ghost = (cv.x >= nvp ? 1u : 0u) | (cv.y >= nvp ? 2u : 0u) | (cv.z >= nvp ? 4u : 0u) |
+                               (cv.w >= nvp ? 8u : 0u);
+        flags |= (0xFu | (ghost << 4)) << (8 * j);
+      }
+    }
+    if (tid == 0) {
+      s_min[par] = 0x7f800000u;
+      s_ng = 0;
+      if (!slab_wait(bar, phase, sp.spin_limit < 0)) {
+        // abandoned: the host reports a timeout; the copies are waited for
+        // once more so that none is in flight when the CTA leaves
+        atomicExch(s.ctl + CTL_ERR, 2);
+        in_flight = !slab_wait(bar, phase, false);
+        s_err = 1;
+      }
+      phase ^= 1u;
+    }
+    __syncthreads();
+    if (s_err) break;
+    auto is_seed = [&](int i) -> bool {
+      return seed_mask ? ((s_seed[i >> 5] >> (i & 31)) & 1u) != 0u : dt_is_seed(s.cell[vs + i], f.base);
+    };
+    // each thread's copies' values at the first sweep (read by the listing of
+    // the same thread, and by all solves after the listing's barrier)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int c = tid + j * blockDim.x;
+      if (c < nep) {
+        const ushort4 cv = cvv[j];
+        sTc[c] = make_float4(sT[cv.x], sT[cv.y], sT[cv.z], sT[cv.w]);
+      }
+    }
+    // a check that finds its patch unconverged turns into that patch's visit
+    int niter_p = visit ? sp.niter : 1;
+    unsigned need[2] = {0u, 0u};
+#pragma unroll 1
+    for (int it = 0; it < niter_p; ++it) {
+      // the owned values at the start of the last sweep (read back by the
+      // same thread only; this sweep's solves change sT only after the
+      // listing barrier below, so no barrier of its own)
+      if (it == niter_p - 1)
+        for (int i = tid; i < nvp; i += blockDim.x) sOld[i] = sT[i];
+      // list this thread's solves that can lower their target (the tests of
+      // k_fim_compact)
+      const unsigned allow_ghost = (it == niter_p - 1) ? 0u : 0xFu;
+#pragma unroll
       for (int j = 0; j < 2; ++j) {
         const int c = tid + j * blockDim.x;
-        if (c < nep) cvv[j] = __ldcs(m.conn + es + c);  // streamed, like the geometry records (evict-first)
-      }
-      const float dt0 = gv0 >= 0 ? s.DT[gv0] : 0.f;
-      if (tid < nslab) sT[tid] = dt0;
-      for (int i = tid + blockDim.x; i < nslab; i += blockDim.x)
-        sT[i] = s.DT[i < nvp ? vs + i : __ldg(m.ghost_ids + gs + i - nvp)];
-      // whole warps run each 32-vertex word (the block is whole warps and the
-      // bound a multiple of 32)
-      if (seed_mask)
-        for (int i = tid; i < ((nvp + 31) & ~31); i += blockDim.x) {
-          const bool sd = i == tid ? sd0 : (i < nvp && s.seed[vs + i] != 0);
-          const unsigned b = __ballot_sync(0xffffffffu, sd);
-          if ((i & 31) == 0) s_seed[i >> 5] = b;
-        }
-      // the copies' connectivity (the previous patch's last reads of sC came
-      // before its final barrier) and flags, which only this thread reads:
-      // bits 8j .. 8j+3 the vertices of copy j that changed in the previous
-      // sweep (all on the first), bits 8j+4 .. 8j+7 its ghost vertices
-      unsigned flags = 0u;
-  #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int c = tid + j * blockDim.x;
-        if (c < nep) {
-          const ushort4 cv = cvv[j];
-          sC[c] = cv;
-          const unsigned ghost = (cv.x >= nvp ? 1u : 0u) | (cv.y >= nvp ? 2u : 0u) | (cv.z >= nvp ? 4u : 0u) |
-                                 (cv.w >= nvp ? 8u : 0u);
-          flags |= (0xFu | (ghost << 4)) << (8 * j);
+        need[j] = 0u;
+        // a copy none of whose values changed in the previous sweep lists
+        // nothing: its flags are read first
+        const unsigned fl = (flags >> (8 * j)) & 0xFFu;  // zero past nep
+        if (fl & 0xFu) {
+          const float4 tv = sTc[c];
+          const float4 hv = sH[c];
+          const unsigned chg = fl & 0xFu, ghost = fl >> 4;
+          const float LN = sp.largenum;
+          const float m012 = fminf(fminf(tv.x, tv.y), tv.z), m013 = fminf(fminf(tv.x, tv.y), tv.w);
+          const float m023 = fminf(fminf(tv.x, tv.z), tv.w), m123 = fminf(fminf(tv.y, tv.z), tv.w);
+          unsigned cand = 0u;
+          if (chg & 0xEu) cand |= 1u;
+          if (chg & 0xDu) cand |= 2u;
+          if (chg & 0xBu) cand |= 4u;
+          if (chg & 0x7u) cand |= 8u;
+          cand &= (~ghost | allow_ghost) & 0xFu;
+          unsigned nd = 0u;
+          if (pair_may_lower<SOLVER>(cand & 1u, m123, hv.x, tv.x, LN)) nd |= 1u;
+          if (pair_may_lower<SOLVER>(cand & 2u, m023, hv.y, tv.y, LN)) nd |= 2u;
+          if (pair_may_lower<SOLVER>(cand & 4u, m013, hv.z, tv.z, LN)) nd |= 4u;
+          if (pair_may_lower<SOLVER>(cand & 8u, m012, hv.w, tv.w, LN)) nd |= 8u;
+          need[j] = nd;
         }
       }
-      if (tid == 0) {
-        s_min = 0x7f800000u;
-        s_ng = 0;
-        if (!slab_wait(bar, phase, sp.spin_limit < 0)) {
-          // abandoned: the host reports a timeout; the copies are waited for
-          // once more so that none is in flight when the CTA leaves
-          atomicExch(s.ctl + 3, 2);
-          in_flight = !slab_wait(bar, phase, false);
-          s_err = 1;
+      {
+        // list positions: one shared atomic per thread for both copies
+        const int nt = __popc(need[0]) + __popc(need[1]);
+        if (nt) {
+          int pos = atomicAdd(&s_n[it & 1], nt);
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const int c = tid + j * blockDim.x;
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              if (need[j] & (1u << k)) sItem[pos++] = (unsigned short)((c << 2) | k);
+          }
         }
-        phase ^= 1u;
       }
       __syncthreads();
-      if (s_err) break;
-      auto is_seed = [&](int i) -> bool {
-        return seed_mask ? ((s_seed[i >> 5] >> (i & 31)) & 1u) != 0u : s.seed[vs + i] != 0;
-      };
-      // each thread's copies' values at the first sweep (read by the listing of
-      // the same thread, and by all solves after the listing's barrier)
-  #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int c = tid + j * blockDim.x;
-        if (c < nep) {
-          const ushort4 cv = cvv[j];
-          sTc[c] = make_float4(sT[cv.x], sT[cv.y], sT[cv.z], sT[cv.w]);
-        }
+      const int nitems = s_n[it & 1];
+      // the other parity's counter is idle until the next sweep's listing,
+      // which starts after the barrier below
+      if (tid == 0) s_n[(it & 1) ^ 1] = 0;
+      // nothing listed in a visit's sweep before its last: no later sweep
+      // lists anything either (unchanged inputs), so the visit ends here
+      // with the bits the remaining empty sweeps would leave
+      if (nitems == 0 && visit && it < niter_p - 1) {
+        for (int i = tid; i < nvp; i += blockDim.x) sOld[i] = sT[i];
+        break;
       }
-      // a check that finds its patch unconverged turns into that patch's visit
-      int niter_p = niter;
-      bool visit = !CHECK;
-      int check_con = 1;  // the verdict of a check that stays a check
-      unsigned need[2] = {0u, 0u};
-  #pragma unroll 1
-      for (int it = 0; it < niter_p; ++it) {
-        // the owned values at the start of the last sweep (read back by the
-        // same thread only; this sweep's solves change sT only after the
-        // listing barrier below, so no barrier of its own)
-        if (it == niter_p - 1)
-          for (int i = tid; i < nvp; i += blockDim.x) sOld[i] = sT[i];
-        // list this thread's solves that can lower their target (the tests of
-        // k_fim_compact)
-        const unsigned allow_ghost = (it == niter_p - 1) ? 0u : 0xFu;
-  #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int c = tid + j * blockDim.x;
-          need[j] = 0u;
-          // a copy none of whose values changed in the previous sweep lists
-          // nothing: its flags are read first
-          const unsigned fl = (flags >> (8 * j)) & 0xFFu;  // zero past nep
-          if (fl & 0xFu) {
-            const float4 tv = sTc[c];
-            const float4 hv = sH[c];
-            const unsigned chg = fl & 0xFu, ghost = fl >> 4;
-            const float LN = sp.largenum;
-            const float m012 = fminf(fminf(tv.x, tv.y), tv.z), m013 = fminf(fminf(tv.x, tv.y), tv.w);
-            const float m023 = fminf(fminf(tv.x, tv.z), tv.w), m123 = fminf(fminf(tv.y, tv.z), tv.w);
-            unsigned cand = 0u;
-            if (chg & 0xEu) cand |= 1u;
-            if (chg & 0xDu) cand |= 2u;
-            if (chg & 0xBu) cand |= 4u;
-            if (chg & 0x7u) cand |= 8u;
-            cand &= (~ghost | allow_ghost) & 0xFu;
-            unsigned nd = 0u;
-            if (pair_may_lower<SOLVER>(cand & 1u, m123, hv.x, tv.x, LN)) nd |= 1u;
-            if (pair_may_lower<SOLVER>(cand & 2u, m023, hv.y, tv.y, LN)) nd |= 2u;
-            if (pair_may_lower<SOLVER>(cand & 4u, m013, hv.z, tv.z, LN)) nd |= 4u;
-            if (pair_may_lower<SOLVER>(cand & 8u, m012, hv.w, tv.w, LN)) nd |= 8u;
-            need[j] = nd;
-          }
-        }
-        {
-          // list positions: one shared atomic per thread for both copies
-          const int nt = __popc(need[0]) + __popc(need[1]);
-          if (nt) {
-            int pos = atomicAdd(&s_n[it & 1], nt);
-  #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-              const int c = tid + j * blockDim.x;
-  #pragma unroll
-              for (int k = 0; k < 4; ++k)
-                if (need[j] & (1u << k)) sItem[pos++] = (unsigned short)((c << 2) | k);
-            }
-          }
-        }
-        __syncthreads();
-        const int nitems = s_n[it & 1];
-        // the other parity's counter is idle until the next sweep's listing,
-        // which starts after the barrier below
-        if (tid == 0) s_n[(it & 1) ^ 1] = 0;
-        // nothing listed in a visit's sweep before its last: no later sweep
-        // lists anything either (unchanged inputs), so the visit ends here
-        // with the bits the remaining empty sweeps would leave
-        if (nitems == 0 && visit && it < niter_p - 1) {
-          for (int i = tid; i < nvp; i += blockDim.x) sOld[i] = sT[i];
-          break;
-        }
-        for (int i = tid; i < nitems; i += blockDim.x) pair_solve<SOLVER>(sItem[i], sTc, sM, sH, sC, sT, sR, nvp, sp);
-        __syncthreads();
-        if (CHECK && !visit) {
-          // the check's verdict (as at the end of a check): does an owned
-          // vertex drop by tol or more?
-          int c0 = 1;
-          for (int i = tid; i < nvp; i += blockDim.x)
-            if (!is_seed(i)) c0 &= (sOld[i] - sT[i] < sp.tol) ? 1 : 0;
-          check_con = __syncthreads_and(c0);
-          if (!check_con && early) {
-            // activated: the patch's visit in the next FIM iteration would read
-            // the same DT (DT changes only in the copy-back after the sweeps), so
-            // it runs here and the next sweep skips the patch.  This sweep was
-            // its first sweep minus the ghost targets (the check's last-sweep
-            // rule): list and run those from the same sweep-start values.
-            visit = true;
-            niter_p = sp.niter;
-  #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-              const int c = tid + j * blockDim.x;
-              if (c < nep) {
-                const float4 tv = sTc[c];
-                const float4 hv = sH[c];
-                const unsigned ghost = (flags >> (8 * j + 4)) & 0xFu;  // all four inputs count as changed
-                const float LN = sp.largenum;
-                const float m012 = fminf(fminf(tv.x, tv.y), tv.z), m013 = fminf(fminf(tv.x, tv.y), tv.w);
-                const float m023 = fminf(fminf(tv.x, tv.z), tv.w), m123 = fminf(fminf(tv.y, tv.z), tv.w);
-                unsigned nd = 0u;
-                if (pair_may_lower<SOLVER>(ghost & 1u, m123, hv.x, tv.x, LN)) nd |= 1u;
-                if (pair_may_lower<SOLVER>(ghost & 2u, m023, hv.y, tv.y, LN)) nd |= 2u;
-                if (pair_may_lower<SOLVER>(ghost & 4u, m013, hv.z, tv.z, LN)) nd |= 4u;
-                if (pair_may_lower<SOLVER>(ghost & 8u, m012, hv.w, tv.w, LN)) nd |= 8u;
-                need[j] |= nd;
-                const int n = __popc(nd);
-                if (n) {
-                  int pos = nitems + atomicAdd(&s_ng, n);
-  #pragma unroll
-                  for (int k = 0; k < 4; ++k)
-                    if (nd & (1u << k)) sItem[pos++] = (unsigned short)((c << 2) | k);
-                }
+      for (int i = tid; i < nitems; i += blockDim.x) pair_solve<SOLVER>(sItem[i], sTc, sM, sH, sC, sT, sR, nvp, sp);
+      __syncthreads();
+      if (!visit) {
+        // the check's verdict: does an owned vertex drop by tol or more?
+        int c0 = 1;
+        for (int i = tid; i < nvp; i += blockDim.x)
+          if (!is_seed(i)) c0 &= (sOld[i] - sT[i] < sp.tol) ? 1 : 0;
+        visit = !__syncthreads_and(c0);
+        niter_p = visit ? sp.niter : 1;
+        if (visit && sp.niter > 1) {
+          // this sweep was the visit's first minus the ghost targets (the
+          // last sweep's rule): list and run those from the same
+          // sweep-start values
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const int c = tid + j * blockDim.x;
+            if (c < nep) {
+              const float4 tv = sTc[c];
+              const float4 hv = sH[c];
+              const unsigned ghost = (flags >> (8 * j + 4)) & 0xFu;  // all four inputs count as changed
+              const float LN = sp.largenum;
+              const float m012 = fminf(fminf(tv.x, tv.y), tv.z), m013 = fminf(fminf(tv.x, tv.y), tv.w);
+              const float m023 = fminf(fminf(tv.x, tv.z), tv.w), m123 = fminf(fminf(tv.y, tv.z), tv.w);
+              unsigned nd = 0u;
+              if (pair_may_lower<SOLVER>(ghost & 1u, m123, hv.x, tv.x, LN)) nd |= 1u;
+              if (pair_may_lower<SOLVER>(ghost & 2u, m023, hv.y, tv.y, LN)) nd |= 2u;
+              if (pair_may_lower<SOLVER>(ghost & 4u, m013, hv.z, tv.z, LN)) nd |= 4u;
+              if (pair_may_lower<SOLVER>(ghost & 8u, m012, hv.w, tv.w, LN)) nd |= 8u;
+              need[j] |= nd;
+              const int n = __popc(nd);
+              if (n) {
+                int pos = nitems + atomicAdd(&s_ng, n);
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                  if (nd & (1u << k)) sItem[pos++] = (unsigned short)((c << 2) | k);
               }
             }
-            __syncthreads();
-            const int ng = s_ng;
-            for (int i = tid; i < ng; i += blockDim.x) pair_solve<SOLVER>(sItem[nitems + i], sTc, sM, sH, sC, sT, sR, nvp, sp);
-            __syncthreads();
           }
-        }
-        // refresh this thread's copies: owned vertices from the per-vertex
-        // minimum, ghost vertices from this sweep's own result where solved
-        // (not after the last sweep: only the owned values are read then)
-        if (it == niter_p - 1) break;
-  #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int c = tid + j * blockDim.x;
-          if (c < nep) {
-            const float4 tv = sTc[c];
-            const float4 rv = sR[c];
-            const ushort4 cv = cvv[j];
-            const unsigned nd = need[j];
-            float4 nv;
-            nv.x = cv.x < nvp ? sT[cv.x] : ((nd & 1u) ? rv.x : tv.x);
-            nv.y = cv.y < nvp ? sT[cv.y] : ((nd & 2u) ? rv.y : tv.y);
-            nv.z = cv.z < nvp ? sT[cv.z] : ((nd & 4u) ? rv.z : tv.z);
-            nv.w = cv.w < nvp ? sT[cv.w] : ((nd & 8u) ? rv.w : tv.w);
-            const unsigned chg = (nv.x != tv.x ? 1u : 0u) | (nv.y != tv.y ? 2u : 0u) | (nv.z != tv.z ? 4u : 0u) |
-                                 (nv.w != tv.w ? 8u : 0u);
-            sTc[c] = nv;
-            flags = (flags & ~(0xFu << (8 * j))) | (chg << (8 * j));
-          }
-        }
-        // no barrier here: every thread refreshes only its own copies, and the
-        // next sweep's solves read them after the barrier that follows its
-        // listing
-      }
-      __syncthreads();
-      // the next list entry is drawn here (draw_patch in two parts), its
-      // atomic in flight during the copy-out below; s_li was read by every
-      // thread before the barrier above, and is read again after the one
-      // below
-      int drawn = 0;
-      if (tid == 0) {
-        s_n[0] = s_n[1] = 0;  // read by every thread before the barrier above
-        drawn = atomicAdd(next, 1);
-      }
-      // a check that stayed a check keeps its verdict: it writes no values
-      int con = visit ? 1 : check_con;
-      if (visit)
-        for (int i = tid; i < nvp; i += blockDim.x) {
-          const int v = vs + i;
-          const float nt = sT[i];
-          float outv;
-          if (!is_seed(i)) {
-            s.DT_out[v] = nt;
-            con &= (sOld[i] - nt < sp.tol) ? 1 : 0;
-            outv = nt;
-          } else {
-            outv = s.DT[v];
-          }
-          atomicMin(&s_min, __float_as_uint(outv));
-        }
-      if (tid == 0) {
-        if (drawn == count - 1) atomicExch(next, 0);
-        s_li = (int)gridDim.x + drawn;
-      }
-      con = __syncthreads_and(con);
-      li = s_li;
-      if (tid == 0) {
-        if (visit) {
-          atomicAdd(&s.stats[7], (unsigned long long)__ldg(m.patch_bytes + p));
-          s.bcon[p] = con;
-          s.bmin[p] = __uint_as_float(s_min);
-          s.blabel[p] = con ? LS_FAR : LS_ACTIVE;
-        }
-        if (CHECK) {
-          // a check that stayed a check read the visit's slab but wrote no DT_out
-          if (!visit) atomicAdd(&s.stats[7], (unsigned long long)(__ldg(m.patch_bytes + p) - 4 * nvp));
-          if (visit) atomicAdd(&s.stats[8], 1ull);
-          if (visit || !con) {
-            // activated: joins the next iteration's list (marked when visited
-            // here already)
-            const int pos = atomicAdd(&s.counts[nxt], 1);
-            nlist[pos] = visit ? (p | kPrevisited) : p;
-          } else {
-            s.blabel[p] = LS_FAR;
-          }
+          __syncthreads();
+          const int ng = s_ng;
+          for (int i = tid; i < ng; i += blockDim.x) pair_solve<SOLVER>(sItem[nitems + i], sTc, sM, sH, sC, sT, sR, nvp, sp);
+          __syncthreads();
         }
       }
-    } else {
-      __syncthreads();
-      if (tid == 0) s_li = draw_patch(next, count);
-      __syncthreads();
-      li = s_li;
+      // refresh this thread's copies: owned vertices from the per-vertex
+      // minimum, ghost vertices from this sweep's own result where solved
+      // (not after the last sweep: only the owned values are read then)
+      if (it == niter_p - 1) break;
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int c = tid + j * blockDim.x;
+        if (c < nep) {
+          const float4 tv = sTc[c];
+          const float4 rv = sR[c];
+          const ushort4 cv = cvv[j];
+          const unsigned nd = need[j];
+          float4 nv;
+          nv.x = cv.x < nvp ? sT[cv.x] : ((nd & 1u) ? rv.x : tv.x);
+          nv.y = cv.y < nvp ? sT[cv.y] : ((nd & 2u) ? rv.y : tv.y);
+          nv.z = cv.z < nvp ? sT[cv.z] : ((nd & 4u) ? rv.z : tv.z);
+          nv.w = cv.w < nvp ? sT[cv.w] : ((nd & 8u) ? rv.w : tv.w);
+          const unsigned chg = (nv.x != tv.x ? 1u : 0u) | (nv.y != tv.y ? 2u : 0u) | (nv.z != tv.z ? 4u : 0u) |
+                               (nv.w != tv.w ? 8u : 0u);
+          sTc[c] = nv;
+          flags = (flags & ~(0xFu << (8 * j))) | (chg << (8 * j));
+        }
+      }
+      // no barrier here: every thread refreshes only its own copies, and the
+      // next sweep's solves read them after the barrier that follows its
+      // listing
     }
+    __syncthreads();
+    // the next list entry is drawn here (draw_patch in two parts), its
+    // atomic in flight during the copy-out below; s_li was read by every
+    // thread before the barrier above, and is read again after the one
+    // below
+    int drawn = 0;
+    if (tid == 0) {
+      s_n[0] = s_n[1] = 0;  // read by every thread before the barrier above
+      drawn = atomicAdd(next, 1);
+    }
+    // a check that found nothing writes nothing
+    int con = 1;
+    if (visit) {
+      const int slot = s.slot[p] ^ 1;
+      for (int i = tid; i < nvp; i += blockDim.x) {
+        const int v = vs + i;
+        const float nt = sT[i];
+        float outv;
+        if (!is_seed(i)) {
+          reinterpret_cast<int2*>(s.cell + v)[slot] = make_int2(__float_as_int(nt), t);
+          con &= (sOld[i] - nt < sp.tol) ? 1 : 0;
+          outv = nt;
+        } else {
+          outv = __int_as_float(s.cell[v].x);
+        }
+        atomicMin(&s_min[par], __float_as_uint(outv));
+      }
+    }
+    if (tid == 0) {
+      if (drawn == f.count - 1) atomicExch(next, 0);
+      s_li = (int)gridDim.x + drawn;
+    }
+    con = __syncthreads_and(con);
+    li = s_li;
+    if (tid == 0) {
+      if (visit) s.slot[p] ^= 1;
+      s_cnt.visits += visit ? 1 : 0;
+      s_cnt.checks += check ? 1 : 0;
+      s_cnt.early += check && visit ? 1 : 0;
+      // a check that stayed a check read the visit's slab but wrote no values
+      s_cnt.bytes += (unsigned long long)(__ldg(m.patch_bytes + p) - (visit ? 0 : 4 * nvp));
+    }
+    if ((tid >> 5) == ((int)blockDim.x >> 5) - 1)
+      fim_publish(m, s, f, p, con != 0, visit && __uint_as_float(s_min[par]) < patch_par(m, sp, p).bw);
   }
+  if (tid == 0) fim_count_flush(s, f, s_cnt);
   // every phase was waited for (unless a copy stayed in flight after a
   // timeout): the mbarrier can go
   if (tid == 0 && !in_flight) slab_bar_inval(bar);
@@ -1208,64 +1285,15 @@ __host__ __device__ constexpr int pair_minb(int setting) { return setting == 7 ?
 
 template <int SETTING, int SOLVER>
 __global__ void __launch_bounds__(pair_maxt(SETTING), pair_minb(SETTING))
-    k_fim_pair(DevMesh m, DevState s, StepParams sp, int cur, int check) {
-  fim_pair_pass<SOLVER>(m, s, sp, cur, check, blockIdx.x);
-}
-
-// Schedule of one FIM iteration: one warp per patch of the current list.
-__device__ __forceinline__ void schedule_pass(const DevMesh& m, const DevState& s, const StepParams& sp, int cur,
-                                              int vb) {
-  const int count = s.counts[cur];
-  const int* list = cur ? s.list1 : s.list0;
-  int* nlist = cur ? s.list0 : s.list1;
-  const int nxt = cur ^ 1;
-  const int lane = threadIdx.x & 31;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (int w = (vb * blockDim.x + threadIdx.x) >> 5; w < count; w += nwarps) {
-    const int p = list[w] & ~kPrevisited;
-    // the patch's records, loaded together (none depends on the copy-back)
-    const int vs = m.vert_off[p], ve = m.vert_off[p + 1];
-    const int con = s.bcon[p];
-    const float bmin = s.bmin[p];
-    const int a = m.padj_off[p], b = m.padj_off[p + 1];
-    for (int v = vs + lane; v < ve; v += 32)
-      if (!s.seed[v]) s.DT[v] = s.DT_out[v];
-    if (!con) {
-      if (lane == 0) {
-        const int pos = atomicAdd(&s.counts[nxt], 1);
-        nlist[pos] = p;
-      }
-    } else if (bmin < patch_par(m, sp, p).bw) {
-      for (int j0 = a; j0 < b; j0 += 32) {
-        const int j = j0 + lane;
-        int q = -1;
-        bool take = false;
-        if (j < b) {
-          q = m.padj[j];
-          take = atomicCAS(&s.blabel[q], LS_FAR, LS_ACTIVE) == LS_FAR;
-        }
-        const unsigned mask = __ballot_sync(0xffffffffu, take);
-        if (mask) {
-          const int leader = __ffs(mask) - 1;
-          int base = 0;
-          if (lane == leader) base = atomicAdd(&s.counts[2], __popc(mask));
-          base = __shfl_sync(0xffffffffu, base, leader);
-          if (take) s.newlist[base + __popc(mask & ((1u << lane) - 1u))] = q;
-        }
-      }
-    }
-  }
-}
-
-__global__ void k_schedule(DevMesh m, DevState s, StepParams sp, int cur) {
-  schedule_pass(m, s, sp, cur, blockIdx.x);
+    k_fim_pair(DevMesh m, DevState s, StepParams sp, int off) {
+  fim_pair_pass<SOLVER>(m, s, sp, s.ctl[CTL_ITER] + off, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
 // Persistent FIM loop: every iteration of a step's redistance in one
-// cooperative launch (all CTAs resident), the sweep, schedule and check
-// passes separated by grid-wide barriers instead of kernel boundaries.  The
-// passes are the launch-per-pass kernels' bodies, so a step gives the same
+// cooperative launch (all CTAs resident), the iterations separated by
+// grid-wide barriers instead of kernel boundaries.  An iteration is the
+// launch-per-iteration kernels' body, so a step gives the same
 // bits either way (the reference's host loop this replaces:
 // redistance3d.cu:85-224).
 //
@@ -1276,18 +1304,17 @@ __global__ void k_schedule(DevMesh m, DevState s, StepParams sp, int cur) {
 // arrival releases every CTA without a reset or a second word on the
 // critical path.  Every wait is bounded: after sp.spin_limit polls (one if
 // it is negative) the CTA
-// raises the abort word (ctl[3]) and leaves; a CTA that finds the word
+// raises the abort word (CTL_ERR) and leaves; a CTA that finds the word
 // raised, while waiting or after a barrier, leaves too, so an abort ends the
 // whole launch, and the host reports LS_DEVICE_TIMEOUT.  The acq_rel fences
 // on both sides make the passes' global writes (plain stores of every
 // thread, ordered before thread 0 by the CTA barrier) visible to the next
-// pass, which reads them with plain loads: DT, DT_out, lists, counters,
-// labels.
+// iteration, which reads them with plain loads: distances, lists, counters.
 __device__ __forceinline__ bool grid_sync(const DevState& s, const StepParams& sp, unsigned& epoch) {
   __shared__ int s_go;
   __syncthreads();
   if (threadIdx.x == 0) {
-    volatile int* abort_word = s.ctl + 3;
+    volatile int* abort_word = s.ctl + CTL_ERR;
     int go = 1;
     epoch += 1;
     const unsigned target = epoch * gridDim.x;
@@ -1303,7 +1330,7 @@ __device__ __forceinline__ bool grid_sync(const DevState& s, const StepParams& s
         break;
       }
       if (++polls > (sp.spin_limit < 0 ? 0u : (unsigned)sp.spin_limit)) {
-        atomicExch(s.ctl + 3, 1);
+        atomicExch(s.ctl + CTL_ERR, 1);
         go = 0;
         break;
       }
@@ -1317,9 +1344,6 @@ __device__ __forceinline__ bool grid_sync(const DevState& s, const StepParams& s
   return s_go != 0;
 }
 
-// The loop: iteration i sweeps list (i & 1) while it is not empty, at most
-// sp.max_fim_iters iterations (the cap sets ctl[1]).
-//
 // A cooperative launch places consecutive CTAs on the same SM (CTAs 0-19 of
 // a 760-CTA grid on four SMs, measured), while an ordinary launch spreads
 // them over the SMs; the passes give list entry b to CTA b first, so a short
@@ -1368,42 +1392,41 @@ __device__ __forceinline__ int spread_index(const DevState& s, const StepParams&
   return s_vb;
 }
 
+// The loop: iterations until the list is empty.  The cap is hit when an
+// iteration beyond the first sp.max_fim_iters visits a patch (its list may
+// hold candidates only, all found converged): seen when a list follows it.
 template <class Pass>
 __device__ __forceinline__ void fim_loop_persistent(const DevMesh& m, const DevState& s, const StepParams& sp,
                                                     Pass&& pass) {
-  int cur = 0;
   unsigned epoch = 0;  // barriers passed (thread 0)
   bool ok = true;
+  const int t0 = s.ctl[CTL_ITER];  // read by every CTA before the first barrier
   const int vb = spread_index(s, sp, epoch, &ok);
   if (!ok) return;
   for (int it = 0;; ++it) {
-    const int count = *reinterpret_cast<volatile int*>(s.counts + cur);
-    if (count == 0) break;
-    if (it >= sp.max_fim_iters) {
-      if (blockIdx.x == 0 && threadIdx.x == 0) s.ctl[1] = 1;
-      break;
+    const int t = t0 + it;
+    const volatile int* n = s.ctl + CTL_VISITS + t % 3;
+    const bool done = n[0] + n[CTL_CANDS - CTL_VISITS] == 0;
+    if (done || it > sp.max_fim_iters) {
+      if (!done && blockIdx.x == 0 && threadIdx.x == 0) s.ctl[CTL_CAP] = 1;
+      return;
     }
-    pass(cur, 0, vb);
+    // above every stamp this iteration uses, also if the launch is abandoned
+    if (blockIdx.x == 0 && threadIdx.x == 0) s.ctl[CTL_ITER] = t + 1;
+    pass(t, vb);
     if (!grid_sync(s, sp, epoch)) return;
-    schedule_pass(m, s, sp, cur, vb);
-    if (!grid_sync(s, sp, epoch)) return;
-    pass(cur, 1, vb);
-    if (!grid_sync(s, sp, epoch)) return;
-    cur ^= 1;
   }
 }
 
 template <int SETTING, int SOLVER>
 __global__ void __launch_bounds__(pair_maxt(SETTING), pair_minb(SETTING))
     k_fim_pair_persist(DevMesh m, DevState s, StepParams sp) {
-  fim_loop_persistent(m, s, sp,
-                      [&](int cur, int check, int vb) { fim_pair_pass<SOLVER>(m, s, sp, cur, check, vb); });
+  fim_loop_persistent(m, s, sp, [&](int t, int vb) { fim_pair_pass<SOLVER>(m, s, sp, t, vb); });
 }
 
 template <int D1, int MAXT, bool XDIV, int MINB, bool PREC>
 __global__ void __launch_bounds__(MAXT, MINB) k_fim_persist(DevMesh m, DevState s, StepParams sp) {
-  fim_loop_persistent(m, s, sp,
-                      [&](int cur, int check, int vb) { fim_copy_pass<D1, XDIV, PREC>(m, s, sp, cur, check, vb); });
+  fim_loop_persistent(m, s, sp, [&](int t, int vb) { fim_copy_pass<D1, XDIV, PREC>(m, s, sp, t, vb); });
 }
 
 // Narrowband (K14) fused with the sign recovery (K10b) and the vertex-update
@@ -1414,21 +1437,22 @@ __global__ void k_narrowband(DevMesh m, DevState s, StepParams sp) {
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  const int base = s.ctl[CTL_BASE];
   unsigned cnt = 0, pv = 0, npc = 0;
   for (int p = warp_id_global(); p < m.nparts; p += nwarps) {
     const int vs = m.vert_off[p], ve = m.vert_off[p + 1];
     const PatchPar pp = patch_par(m, sp, p);
     unsigned mn = 0x7f800000u;
     for (int v = vs + lane; v < ve; v += 32) {
-      const float d = s.DT[v];
+      const float d = dt_before(s.cell[v], kStampMax, base, sp.largenum);
       mn = min(mn, __float_as_uint(d));
       cnt += (d <= pp.bw);
       const float mag = (d >= sp.largenum || pp.scale == 1.f) ? d : d * pp.scale;
-      s.phi[v] = s.sign[v] ? mag : -mag;
+      s.phi[v] = s.phi[v] < 0.f ? -mag : mag;  // the sign phi had before the redistance
     }
     mn = __reduce_min_sync(0xffffffffu, mn);
     if (lane == 0 && __uint_as_float(mn) <= pp.bw) {
-      const int pos = atomicAdd(&s.counts[3], 1);
+      const int pos = atomicAdd(s.ctl + CTL_NB, 1);
       s.nblist[pos] = p;
       pv += ve - vs;
       npc += 1;
@@ -1671,7 +1695,7 @@ __device__ __forceinline__ void update_patches(const DevMesh& m, const DevState&
   float* sC = sX + (D1 == 4 ? 3 * slab : 0);  // per copy: aH[4] aV[4] curv[4] vol g0 g1 g2
   const bool curvature = sp.update_kind == 1;
   const int stride = 15;
-  const int count = s.counts[3];
+  const int count = s.ctl[CTL_NB];
   for (int li = blockIdx.x; li < count; li += gridDim.x) {
     const int p = s.nblist[li];
     const PatchPar pp = patch_par(m, sp, p);
@@ -1763,7 +1787,7 @@ __global__ void __launch_bounds__(384, 3) k_update_384(DevMesh m, DevState s, St
 __global__ void k_copy_phi(DevMesh m, DevState s) {
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  const int count = s.counts[3];
+  const int count = s.ctl[CTL_NB];
   for (int w = warp_id_global(); w < count; w += nwarps) {
     const int p = s.nblist[w];
     for (int v = m.vert_off[p] + lane; v < m.vert_off[p + 1]; v += 32) s.phi[v] = s.phi_out[v];
@@ -1774,6 +1798,13 @@ __global__ void k_copy_phi(DevMesh m, DevState s) {
 __global__ void k_unpermute(DevMesh m, const float* phi, float* out) {
   for (int o = blockIdx.x * blockDim.x + threadIdx.x; o < m.nv; o += gridDim.x * blockDim.x)
     out[o] = phi[__ldg(m.ipermute + o)];
+}
+
+// FIM distances in the layout's order (diagnostics)
+__global__ void k_distances(DevMesh m, DevState s, float LN, float* out) {
+  const int base = s.ctl[CTL_BASE];
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < m.nv; v += gridDim.x * blockDim.x)
+    out[v] = dt_before(s.cell[v], kStampMax, base, LN);
 }
 
 // out[new] = in[old]
@@ -1821,6 +1852,7 @@ __global__ void k_nb_vertices(DevMesh m, DevState s, DevLearn lr, int nb) {
     int base = 0;
     if (lane == 0) base = atomicAdd(&lr.cnt[0], nvp);
     base = __shfl_sync(0xffffffffu, base, 0);
+    if (lane == 0) s.slot[p] = 0;  // k_warm_apply writes the first half: the first visit writes the other
     for (int i = lane; i < nvp; i += 32) lr.vlist[base + i] = vs + i;
   }
 }
@@ -1829,10 +1861,11 @@ __global__ void k_nb_vertices(DevMesh m, DevState s, DevLearn lr, int nb) {
 // search that follows overwrites the seeds.
 __global__ void k_warm_apply(DevState s, DevLearn lr, float LN, float margin) {
   const int n = lr.cnt[0];
+  const int stamp = s.ctl[CTL_BASE] + 1;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int v = lr.vlist[i];
     const float w = fminf(fabsf(lr.pred[i]) + margin, LN);
-    s.DT[v] = w;
+    *reinterpret_cast<int2*>(s.cell + v) = make_int2(__float_as_int(w), stamp);
     lr.warm[v] = w;
   }
 }
@@ -1840,7 +1873,7 @@ __global__ void k_warm_apply(DevState s, DevLearn lr, float LN, float margin) {
 // Support check after the FIM from a warm start: an owned non-seed vertex
 // whose value lies more than tol below every local solve of its elements
 // (its support) was set by the warm start, not by the wavefront; it is
-// reset to LARGENUM and its patch joins list0 for another FIM loop.  One
+// reset to LARGENUM and its patch joins the list of another FIM loop.  One
 // CTA per patch over all patches; patches without a reached vertex skip.
 template <int D1, bool XDIV>
 __global__ void __launch_bounds__(384) k_support(DevMesh m, DevState s, StepParams sp, DevLearn lr, float tol,
@@ -1849,13 +1882,20 @@ __global__ void __launch_bounds__(384) k_support(DevMesh m, DevState s, StepPara
   float* sT = smem;
   float* sC = smem + sp.lvp + sp.lgp;  // owned candidates
   const int tid = threadIdx.x;
+  const int base = s.ctl[CTL_BASE], t0 = s.ctl[CTL_ITER];
+  // LARGENUM over the newest value of vertex v
+  auto drop = [&](int v) {
+    const DtCell c = s.cell[v];
+    reinterpret_cast<int2*>(s.cell + v)[c.w > c.y ? 1 : 0].x = __float_as_int(sp.largenum);
+  };
   for (int p = blockIdx.x; p < m.nparts; p += gridDim.x) {
     const int vs = m.vert_off[p], nvp = m.vert_off[p + 1] - vs;
     const int gs = m.ghost_off[p], ngp = m.ghost_off[p + 1] - gs;
     const int es = m.ele_off[p], nep = m.ele_off[p + 1] - es;
     int reached = 0;
     for (int i = tid; i < nvp + ngp; i += blockDim.x) {
-      const float d = s.DT[i < nvp ? vs + i : __ldg(m.ghost_ids + gs + i - nvp)];
+      const float d =
+          dt_before(s.cell[i < nvp ? vs + i : __ldg(m.ghost_ids + gs + i - nvp)], kStampMax, base, sp.largenum);
       sT[i] = d;
       if (i < nvp) {
         sC[i] = __int_as_float(0x7f800000);
@@ -1880,8 +1920,8 @@ __global__ void __launch_bounds__(384) k_support(DevMesh m, DevState s, StepPara
     int bad = 0;
     for (int i = tid; i < nvp; i += blockDim.x) {
       const int v = vs + i;
-      if (!s.seed[v] && sT[i] < sp.largenum && sT[i] < sC[i] - tol) {
-        s.DT[v] = sp.largenum;
+      if (!dt_is_seed(s.cell[v], base) && sT[i] < sp.largenum && sT[i] < sC[i] - tol) {
+        drop(v);
         bad++;
       }
     }
@@ -1890,15 +1930,13 @@ __global__ void __launch_bounds__(384) k_support(DevMesh m, DevState s, StepPara
       // reset every non-seed vertex of the patch: values that leaned on the
       // unsupported ones are recomputed in the same FIM loop
       for (int i = tid; i < nvp; i += blockDim.x)
-        if (!s.seed[vs + i]) s.DT[vs + i] = sp.largenum;
+        if (!dt_is_seed(s.cell[vs + i], base)) drop(vs + i);
     }
     if (tid == 0 && bad) {
       atomicAdd(&lr.cnt[1], bad);
-      if (atomicCAS(&s.blabel[p], LS_FAR, LS_ACTIVE) == LS_FAR) {
-        const int pos = atomicAdd(&s.counts[0], 1);
-        s.list0[pos] = p;
-        atomicAdd(&lr.cnt[3], 1);
-      }
+      s.pend[p] = 2 * t0;  // the lists are empty: only this CTA appends p
+      s.lists[(size_t)(t0 % 3) * m.nparts + atomicAdd(s.ctl + CTL_VISITS + t0 % 3, 1)] = p;
+      atomicAdd(&lr.cnt[3], 1);
     }
     __syncthreads();
   }
@@ -1906,12 +1944,13 @@ __global__ void __launch_bounds__(384) k_support(DevMesh m, DevState s, StepPara
 
 // Warm-set vertices whose final value differs from the warm start by more
 // than tol (FIM frame).
-__global__ void k_moved(DevState s, DevLearn lr, float tol) {
+__global__ void k_moved(DevState s, DevLearn lr, float LN, float tol) {
   const int n = lr.cnt[0];
+  const int base = s.ctl[CTL_BASE];
   int moved = 0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int v = lr.vlist[i];
-    moved += (fabsf(s.DT[v] - lr.warm[v]) > tol) ? 1 : 0;
+    moved += (fabsf(dt_before(s.cell[v], kStampMax, base, LN) - lr.warm[v]) > tol) ? 1 : 0;
   }
   moved = __reduce_add_sync(0xffffffffu, moved);
   if ((threadIdx.x & 31) == 0 && moved) atomicAdd(&lr.cnt[2], moved);
@@ -1938,8 +1977,8 @@ cudaError_t launch_learn(int op, const DevMesh& m, const DevState& s, const Step
       k_warm_apply<<<L.flat_grid, 256, 0, st>>>(s, lr, sp.largenum, fa);
       break;
     case LEARN_SEED_WARM:
-      if (m.dim == 3) k_seed<4><<<L.seed_grid, L.fim_block, 0, st>>>(m, s, 0, sp.scale, 1);
-      else k_seed<3><<<L.seed_grid, L.fim_block, 0, st>>>(m, s, 0, sp.scale, 1);
+      if (m.dim == 3) k_seed<4><<<L.seed_grid, L.fim_block, 0, st>>>(m, s, sp.scale, 1);
+      else k_seed<3><<<L.seed_grid, L.fim_block, 0, st>>>(m, s, sp.scale, 1);
       break;
     case LEARN_SUPPORT: {
       const int smem = (int)sizeof(float) * (2 * sp.lvp + sp.lgp);
@@ -1953,7 +1992,7 @@ cudaError_t launch_learn(int op, const DevMesh& m, const DevState& s, const Step
       break;
     }
     case LEARN_MOVED:
-      k_moved<<<L.flat_grid, 256, 0, st>>>(s, lr, fa);
+      k_moved<<<L.flat_grid, 256, 0, st>>>(s, lr, sp.largenum, fa);
       break;
     case LEARN_TARGETS:
       k_targets<<<L.flat_grid, 256, 0, st>>>(s, lr, fa, sp.largenum);
@@ -1964,14 +2003,14 @@ cudaError_t launch_learn(int op, const DevMesh& m, const DevState& s, const Step
   return cudaGetLastError();
 }
 
-cudaError_t launch_reset(const DevMesh& m, const DevState& s, const StepParams& sp, const Launch& L, cudaStream_t st) {
-  k_reset<<<L.flat_grid, 256, 0, st>>>(s, m.nv, sp.largenum);
+cudaError_t launch_begin(const DevState& s, int restart, cudaStream_t st) {
+  k_begin<<<1, 256, 0, st>>>(s, restart);
   return cudaGetLastError();
 }
 
-cudaError_t launch_seed(const DevMesh& m, const DevState& s, int use_all, float scale, const Launch& L, cudaStream_t st) {
-  if (m.dim == 3) k_seed<4><<<L.seed_grid, L.fim_block, 0, st>>>(m, s, use_all, scale, 0);
-  else k_seed<3><<<L.seed_grid, L.fim_block, 0, st>>>(m, s, use_all, scale, 0);
+cudaError_t launch_seed(const DevMesh& m, const DevState& s, const StepParams& sp, const Launch& L, cudaStream_t st) {
+  if (m.dim == 3) k_seed<4><<<L.seed_grid, L.fim_block, 0, st>>>(m, s, sp.scale, 0);
+  else k_seed<3><<<L.seed_grid, L.fim_block, 0, st>>>(m, s, sp.scale, 0);
   return cudaGetLastError();
 }
 
@@ -2014,23 +2053,23 @@ __host__ __device__ inline bool use_pair(const DevMesh& m, const StepParams& sp,
   return m.dim == 3 && !m.capped && !(sp.tau > 0.f) && L.pair_block > 0;
 }
 
-cudaError_t launch_pair(const DevMesh& m, const DevState& s, const StepParams& sp, int cur, int c, const Launch& L,
+cudaError_t launch_pair(const DevMesh& m, const DevState& s, const StepParams& sp, int off, const Launch& L,
                         cudaStream_t st) {
-  void* args[] = {(void*)&m, (void*)&s, (void*)&sp, (void*)&cur, (void*)&c};
+  void* args[] = {(void*)&m, (void*)&s, (void*)&sp, (void*)&off};
   return cudaLaunchKernel(LS_PAIR_KERNEL(sp), dim3((unsigned)L.fim_grid), dim3((unsigned)L.pair_block), args,
                           (size_t)pair_smem(sp, sp.lep), st);
 }
 
-cudaError_t launch_sweep(const DevMesh& m, const DevState& s, const StepParams& sp, int cur, bool check,
-                         const Launch& L, cudaStream_t st) {
+// One FIM iteration: the off-th of a loop body (stamp CTL_ITER + off).
+cudaError_t launch_fim(const DevMesh& m, const DevState& s, const StepParams& sp, int off, const Launch& L,
+                       cudaStream_t st) {
   const bool xd = sp.xdiv != 0;
   const bool pr = sp.tau > 0.f;
-  const int c = check ? 1 : 0;
   // precision-form kernels: one 384-class register budget (2 CTAs/SM) and
   // the deferred-solve queue in shared memory
   const int psmem = L.fim_smem + (int)sizeof(DeferredSolve) * kDeferCap;
 #define LS_FIM(D, T, X, B, P) \
-  k_fim<D, T, X, B, P><<<L.fim_grid, L.fim_block, P ? psmem : L.fim_smem, st>>>(m, s, sp, cur, c)
+  k_fim<D, T, X, B, P><<<L.fim_grid, L.fim_block, P ? psmem : L.fim_smem, st>>>(m, s, sp, off)
 #define LS_FIM3(T, B) \
   do { \
     if (xd) { if (pr) LS_FIM(4, T, true, (T == 384 ? 2 : 1), true); else LS_FIM(4, T, true, B, false); } \
@@ -2042,25 +2081,25 @@ cudaError_t launch_sweep(const DevMesh& m, const DevState& s, const StepParams& 
   const bool compact = kLbSkip && m.dim == 3 && !m.capped;
   if (use_pair(m, sp, L)) {
     // tetrahedra: compacted solves, two copies per thread
-    return launch_pair(m, s, sp, cur, c, L, st);
+    return launch_pair(m, s, sp, off, L, st);
   } else if (compact && pr) {
     // fast build, tetrahedra, precision form: compacted solves, FP64 repeats
     // run densely after each sweep's FP32 pass
     const int cs = compact_smem(sp, L.fim_block <= 384 ? 384 : L.fim_block <= 512 ? 512 : 1024);
-    if (L.fim_block <= 384) k_fim_compact<384, 2, true><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, cur, c);
-    else if (L.fim_block <= 512) k_fim_compact<512, 1, true><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, cur, c);
-    else k_fim_compact<1024, 1, true><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, cur, c);
+    if (L.fim_block <= 384) k_fim_compact<384, 2, true><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, off);
+    else if (L.fim_block <= 512) k_fim_compact<512, 1, true><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, off);
+    else k_fim_compact<1024, 1, true><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, off);
   } else if (compact) {
     // fast build, tetrahedra: compacted solves
     const int cs = compact_smem(sp, L.fim_block <= 384 ? 384 : L.fim_block <= 512 ? 512 : 1024);
     if (L.fim_block <= 384) {
-      if (sp.ctas == 2) k_fim_compact<384, 2, false><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, cur, c);
-      else if (sp.ctas == 4) k_fim_compact<384, 4, false><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, cur, c);
-      else k_fim_compact<384, 3, false><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, cur, c);
+      if (sp.ctas == 2) k_fim_compact<384, 2, false><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, off);
+      else if (sp.ctas == 4) k_fim_compact<384, 4, false><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, off);
+      else k_fim_compact<384, 3, false><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, off);
     } else if (L.fim_block <= 512) {
-      k_fim_compact<512, 1, false><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, cur, c);
+      k_fim_compact<512, 1, false><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, off);
     } else {
-      k_fim_compact<1024, 1, false><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, cur, c);
+      k_fim_compact<1024, 1, false><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, off);
     }
   } else if (m.dim == 3) {
     if (L.fim_block <= 384) {
@@ -2082,7 +2121,7 @@ cudaError_t launch_sweep(const DevMesh& m, const DevState& s, const StepParams& 
   return cudaGetLastError();
 }
 
-// The persistent form of the sweep kernel launch_sweep would pick, where it
+// The persistent form of the kernel launch_fim would pick, where it
 // has one: the two-copies-per-thread kernel, or the one-copy kernel with
 // 384-thread blocks (bit-exact build, triangles, meshes with capped slots).
 // Cooperative launch: the runtime refuses a grid that cannot be resident.
@@ -2153,12 +2192,6 @@ cudaError_t configure_persistent(const DevMesh& m, const StepParams& sp, Launch&
   return cudaSuccess;
 }
 
-cudaError_t launch_schedule(const DevMesh& m, const DevState& s, const StepParams& sp, int cur, const Launch& L,
-                            cudaStream_t st) {
-  k_schedule<<<L.warp_grid, 256, 0, st>>>(m, s, sp, cur);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_narrowband(const DevMesh& m, const DevState& s, const StepParams& sp, const Launch& L,
                               cudaStream_t st) {
   k_narrowband<<<L.warp_grid, 256, 0, st>>>(m, s, sp);
@@ -2178,6 +2211,12 @@ cudaError_t launch_update(const DevMesh& m, const DevState& s, const StepParams&
 
 cudaError_t launch_unpermute(const DevMesh& m, const float* phi, float* out, const Launch& L, cudaStream_t st) {
   k_unpermute<<<L.flat_grid, 256, 0, st>>>(m, phi, out);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_distances(const DevMesh& m, const DevState& s, const StepParams& sp, float* out, const Launch& L,
+                             cudaStream_t st) {
+  k_distances<<<L.flat_grid, 256, 0, st>>>(m, s, sp.largenum, out);
   return cudaGetLastError();
 }
 
@@ -2273,7 +2312,8 @@ cudaError_t configure_launch(const DevMesh& m, const StepParams& sp, Launch& L) 
   }
   if (e != cudaSuccess) return e;
   if (occ < 1) occ = 1;
-  L.fim_grid = L.sms * occ;
+  // no more CTAs than patches: a small mesh's launches are short
+  L.fim_grid = std::min(L.sms * occ, m.nparts);
   L.seed_grid = L.sms * 8;
   L.upd_block = L.fim_block > 512 ? 512 : L.fim_block;
   const int slab = sp.lvp + sp.lgp;
@@ -2298,8 +2338,8 @@ cudaError_t configure_launch(const DevMesh& m, const StepParams& sp, Launch& L) 
 
 
 const KernelSet& kernel_table() {
-  static const KernelSet t = {configure_launch,  launch_reset,  launch_seed,      launch_sweep,
-                              launch_schedule,   launch_fim_persistent, launch_narrowband, launch_update,
-                              launch_unpermute,  launch_permute, launch_learn,     launch_geometry};
+  static const KernelSet t = {configure_launch, launch_begin, launch_seed,      launch_fim,
+                              launch_fim_persistent, launch_narrowband, launch_update, launch_distances,
+                              launch_unpermute, launch_permute, launch_learn,  launch_geometry};
   return t;
 }

@@ -5,7 +5,7 @@
 // (src/core3d/cuda/redistance3d.cu:85-224).  Here the lists, labels and
 // convergence flags stay on the device; the host only launches a fixed
 // chunk of FIM iterations (captured once as a CUDA graph) and reads one
-// counter per chunk to learn whether the active list has drained.
+// counter per chunk to learn whether the list has drained.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -42,7 +42,7 @@ Solver::~Solver() {
   if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
   if (graph_) cudaGraphDestroy(graph_);
   for (void* p : allocs_) cudaFree(p);
-  if (h_counts_) cudaFreeHost(h_counts_);
+  if (h_ctl_) cudaFreeHost(h_ctl_);
   if (h_stats_) cudaFreeHost(h_stats_);
   if (h_stage_) cudaFreeHost(h_stage_);
   if (h_snap_) cudaFreeHost(h_snap_);
@@ -157,8 +157,8 @@ std::string Solver::init(const Layout& L, const SolverConfig& cfg, const float* 
   cfg_ = cfg;
   K_ = cfg.bit_exact ? &kernels_exact() : &kernels_fast();
   if (L.lep > 1024) { status_ = 2; return "a patch has more than 1024 element copies"; }
-  // active-list entries carry the visited-ahead mark above the patch id
-  if (L.nparts >= kPrevisited) return "too many patches";
+  // the limit the patch lists always had (30-bit patch ids)
+  if (L.nparts >= (1 << 30)) return "too many patches";
   LS_TRY(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "stream");
   {
     int dev = 0;
@@ -270,30 +270,27 @@ std::string Solver::init(const Layout& L, const SolverConfig& cfg, const float* 
   // step state
   LS_TRY(dalloc(A, &s_.phi, nv), "alloc");
   LS_TRY(dalloc(A, &s_.phi_out, nv), "alloc");
-  LS_TRY(dalloc(A, &s_.DT, nv), "alloc");
-  LS_TRY(dalloc(A, &s_.DT_out, nv), "alloc");
-  LS_TRY(dalloc(A, &s_.seed, nv), "alloc");
-  LS_TRY(dalloc(A, &s_.sign, nv), "alloc");
-  LS_TRY(dalloc(A, &s_.blabel, np), "alloc");
-  LS_TRY(dalloc(A, &s_.bcon, np), "alloc");
-  LS_TRY(dalloc(A, &s_.bmin, np), "alloc");
-  LS_TRY(dalloc(A, &s_.list0, np), "alloc");
-  LS_TRY(dalloc(A, &s_.list1, np), "alloc");
-  LS_TRY(dalloc(A, &s_.newlist, np), "alloc");
+  LS_TRY(dalloc(A, &s_.cell, nv), "alloc");
+  LS_TRY(dalloc(A, &s_.slot, np), "alloc");
+  LS_TRY(dalloc(A, &s_.pend, np), "alloc");
+  LS_TRY(dalloc(A, &s_.reach, np), "alloc");
+  LS_TRY(dalloc(A, &s_.lists, (size_t)3 * np), "alloc");
   LS_TRY(dalloc(A, &s_.nblist, np), "alloc");
-  LS_TRY(dalloc(A, &s_.counts, 8), "alloc");
+  LS_TRY(dalloc(A, &s_.ctl, CTL_WORDS), "alloc");
   LS_TRY(dalloc(A, &s_.stats, 9), "alloc");
-  LS_TRY(dalloc(A, &s_.ctl, 4), "alloc");
   LS_TRY(dalloc(A, &s_.sched, 4), "alloc");
   LS_TRY(dalloc(A, &s_.gbar, kGridBarrierWords), "alloc");
   LS_TRY(cudaMemsetAsync(s_.gbar, 0, sizeof(unsigned) * kGridBarrierWords, stream_), "memset");
   LS_TRY(dalloc(A, &d_tmp_, nv), "alloc");
-  LS_TRY(cudaMemsetAsync(s_.counts, 0, sizeof(int) * 8, stream_), "memset");
+  LS_TRY(cudaMemsetAsync(s_.slot, 0, sizeof(int) * np, stream_), "memset");
+  LS_TRY(cudaMemsetAsync(s_.ctl, 0, sizeof(int) * CTL_WORDS, stream_), "memset");
   LS_TRY(cudaMemsetAsync(s_.stats, 0, sizeof(unsigned long long) * 9, stream_), "memset");
-  LS_TRY(cudaMemsetAsync(s_.ctl, 0, sizeof(int) * 4, stream_), "memset");
   LS_TRY(cudaMemsetAsync(s_.sched, 0, sizeof(int) * 4, stream_), "memset");
   LS_TRY(cudaMemsetAsync(s_.phi, 0, sizeof(float) * nv, stream_), "memset");
-  LS_TRY(cudaMallocHost((void**)&h_counts_, sizeof(int) * 12), "pinned");
+  LS_TRY(cudaMallocHost((void**)&h_ctl_, sizeof(int) * CTL_WORDS), "pinned");
+  std::memset(h_ctl_, 0, sizeof(int) * CTL_WORDS);
+  // a few steps below the limit, so that every handle's stamps restart early in its life
+  LS_TRY(restart_stamps(kStampLimit - 32), "stamps");
   LS_TRY(cudaMallocHost((void**)&h_stats_, sizeof(unsigned long long) * 9), "pinned");
   LS_TRY(cudaMallocHost((void**)&h_stage_, sizeof(float) * nv), "pinned");
 
@@ -346,25 +343,66 @@ std::string Solver::init(const Layout& L, const SolverConfig& cfg, const float* 
   return "";
 }
 
-// Step control kernels (host orchestration, same for both kernel builds).
+// Step control kernel (host orchestration, same for both kernel builds): end
+// of one FIM loop body of `chunk` iterations.  Continue while the next list
+// is not empty.  The cap: iterations beyond the first `cap` that visited a
+// patch (a list can hold candidates only, all found converged, so whether
+// the cap is exceeded shows one body later); it sets CTL_CAP, so that the
+// host reports a timeout.
 namespace {
-// End of one FIM loop body (graph_chunk iterations): continue while the
-// active list is not empty, at most max_bodies bodies per step; the cap
-// sets ctl[1] so that the host reports a timeout.
-__global__ void k_loop_cond(const int* counts, int* ctl, cudaGraphConditionalHandle h, int max_bodies) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    const int b = ++ctl[0];
-    const bool more = counts[0] > 0 && ctl[3] == 0;  // a FIM kernel wait that ran out ends the loop
-    if (more && b >= max_bodies) ctl[1] = 1;
-    cudaGraphSetConditional(h, (more && b < max_bodies) ? 1u : 0u);
-  }
+__device__ __forceinline__ bool body_end(int* ctl, int chunk, int cap) {
+  ctl[CTL_BODIES] += 1;
+  const int t = ctl[CTL_ITER] + chunk;
+  ctl[CTL_ITER] = t;
+  const bool more = ctl[CTL_VISITS + t % 3] + ctl[CTL_CANDS + t % 3] > 0;
+  const bool over = ctl[CTL_ITERS] > cap;
+  if (over) ctl[CTL_CAP] = 1;
+  return more && !over && ctl[CTL_ERR] == 0;  // a FIM kernel wait that ran out ends the loop
 }
-// After the narrowband: the next step's seed search is restricted to it
-// when it is not empty.
-__global__ void k_step_tail(const int* counts, int* ctl) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) ctl[2] = counts[3] > 0 ? 1 : 0;
+__global__ void k_body_end(int* ctl, int chunk, int cap) {
+  if (threadIdx.x == 0) body_end(ctl, chunk, cap);
+}
+__global__ void k_loop_cond(int* ctl, cudaGraphConditionalHandle h, int chunk, int cap) {
+  if (threadIdx.x == 0) cudaGraphSetConditional(h, body_end(ctl, chunk, cap) ? 1u : 0u);
 }
 }  // namespace
+
+// Clears every stamped array and starts the stamps again from `from`.
+cudaError_t Solver::restart_stamps(int from) {
+  cudaError_t e = cudaMemsetAsync(s_.cell, 0xff, sizeof(DtCell) * (size_t)m_.nv, stream_);
+  if (e == cudaSuccess) e = cudaMemsetAsync(s_.pend, 0xff, sizeof(int) * m_.nparts, stream_);
+  if (e == cudaSuccess) e = cudaMemsetAsync(s_.reach, 0xff, sizeof(int) * m_.nparts, stream_);
+  h_ctl_[CTL_ITER] = from;
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(s_.ctl + CTL_ITER, h_ctl_ + CTL_ITER, sizeof(int), cudaMemcpyHostToDevice, stream_);
+  return e;
+}
+
+// The step control words on the host, and the stream idle.
+cudaError_t Solver::read_ctl() {
+  cudaError_t e = cudaMemcpyAsync(h_ctl_, s_.ctl, sizeof(int) * CTL_WORDS, cudaMemcpyDeviceToHost, stream_);
+  return e == cudaSuccess ? cudaStreamSynchronize(stream_) : e;
+}
+
+// Whether the step's FIM loop ended as it should.
+std::string Solver::fim_status() {
+  if (h_ctl_[CTL_ERR]) {
+    status_ = 3;
+    return h_ctl_[CTL_ERR] == 1 ? "a grid barrier wait of the persistent FIM kernel timed out"
+                                : "a geometry slab copy wait of the FIM kernel timed out";
+  }
+  if (h_ctl_[CTL_CAP]) {
+    status_ = 3;
+    return "FIM did not converge within max_fim_iters iterations";
+  }
+  return "";
+}
+
+// Iterations after which the loop gives up: the cap rounded up to whole bodies.
+int Solver::iter_cap() const {
+  const long long c = cfg_.graph_chunk, cap = ((long long)cfg_.max_fim_iters + c - 1) / c * c;
+  return (int)std::min<long long>(cap, 0x7fffffff);
+}
 
 // One time step as one graph: seed part, a while node running FIM loop
 // bodies of graph_chunk iterations until the active list drains (or the
@@ -377,7 +415,7 @@ __global__ void k_step_tail(const int* counts, int* ctl) {
 bool Solver::build_persistent_graph(std::string* err) {
   cudaGraph_t g = nullptr;
   if (cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return false;
-  cudaError_t e = step_persistent_launches(-1);
+  cudaError_t e = step_persistent_launches();
   cudaError_t e2 = cudaStreamEndCapture(stream_, &g);
   if (e != cudaSuccess || e2 != cudaSuccess || !g) {
     if (g) cudaGraphDestroy(g);
@@ -394,30 +432,23 @@ bool Solver::build_persistent_graph(std::string* err) {
   return true;
 }
 
-// One step of the persistent form, launch by launch (use_all < 0: the seed
-// kernel decides from the step-control flag, as in a graph).
-cudaError_t Solver::step_persistent_launches(int use_all) {
-  cudaError_t err = cudaMemsetAsync(s_.counts, 0, sizeof(int) * 3, stream_);
-  if (err == cudaSuccess) err = cudaMemsetAsync(s_.counts + 4, 0, sizeof(int), stream_);
-  if (err == cudaSuccess) err = cudaMemsetAsync(s_.ctl, 0, sizeof(int) * 2, stream_);
-  if (err == cudaSuccess) err = cudaMemsetAsync(s_.ctl + 3, 0, sizeof(int), stream_);
-  if (err == cudaSuccess) err = cudaMemsetAsync(s_.gbar, 0, sizeof(unsigned) * kGridBarrierWords, stream_);
-  // the patch-draw counters are zero after every complete launch; a launch
-  // abandoned on a barrier timeout can leave them set
-  if (err == cudaSuccess) err = cudaMemsetAsync(s_.sched, 0, sizeof(int) * 2, stream_);
-  if (err == cudaSuccess) err = K_->reset(m_, s_, sp_, L_, stream_);
-  if (err == cudaSuccess) err = cudaMemsetAsync(s_.blabel, 0, sizeof(int) * m_.nparts, stream_);
-  if (err == cudaSuccess) err = K_->seed(m_, s_, use_all, sp_.scale, L_, stream_);
-  if (err == cudaSuccess) err = cudaMemsetAsync(s_.counts + 3, 0, sizeof(int), stream_);
-  if (err == cudaSuccess) err = K_->fim_persistent(m_, s_, sp_, L_, stream_);
-  if (err == cudaSuccess) err = K_->narrowband(m_, s_, sp_, L_, stream_);
-  if (err == cudaSuccess) {
-    k_step_tail<<<1, 32, 0, stream_>>>(s_.counts, s_.ctl);
-    err = cudaGetLastError();
-  }
+// The parts of a step before and after its FIM loop.
+cudaError_t Solver::step_head() {
+  cudaError_t e = K_->begin(s_, 0, stream_);
+  return e == cudaSuccess ? K_->seed(m_, s_, sp_, L_, stream_) : e;
+}
+cudaError_t Solver::step_tail() {
+  cudaError_t e = K_->narrowband(m_, s_, sp_, L_, stream_);
   if (cfg_.update_kind != 2)
-    for (int it = 0; it < cfg_.inside_niter && err == cudaSuccess; ++it) err = K_->update(m_, s_, sp_, L_, stream_);
-  return err;
+    for (int it = 0; it < cfg_.inside_niter && e == cudaSuccess; ++it) e = K_->update(m_, s_, sp_, L_, stream_);
+  return e;
+}
+
+// One step of the persistent form, launch by launch.
+cudaError_t Solver::step_persistent_launches() {
+  cudaError_t err = step_head();
+  if (err == cudaSuccess) err = K_->fim_persistent(m_, s_, sp_, L_, stream_);
+  return err == cudaSuccess ? step_tail() : err;
 }
 
 std::string Solver::build_graph() {
@@ -428,31 +459,15 @@ std::string Solver::build_graph() {
     return "";  // no graph: the persistent step launches kernel by kernel
   }
   const int chunk = cfg_.graph_chunk;
-  const int max_bodies = (cfg_.max_fim_iters + chunk - 1) / chunk;
   cudaGraph_t pre = nullptr, post = nullptr;
   cudaError_t err = cudaSuccess;
-  // seed part
   LS_TRY(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "capture begin");
-  err = cudaMemsetAsync(s_.counts, 0, sizeof(int) * 3, stream_);
-  if (err == cudaSuccess) err = cudaMemsetAsync(s_.counts + 4, 0, sizeof(int), stream_);
-  if (err == cudaSuccess) err = cudaMemsetAsync(s_.ctl, 0, sizeof(int) * 2, stream_);
-  if (err == cudaSuccess) err = cudaMemsetAsync(s_.ctl + 3, 0, sizeof(int), stream_);
-  if (err == cudaSuccess) err = K_->reset(m_, s_, sp_, L_, stream_);
-  if (err == cudaSuccess) err = cudaMemsetAsync(s_.blabel, 0, sizeof(int) * m_.nparts, stream_);
-  if (err == cudaSuccess) err = K_->seed(m_, s_, -1, sp_.scale, L_, stream_);
-  if (err == cudaSuccess) err = cudaMemsetAsync(s_.counts + 3, 0, sizeof(int), stream_);
+  err = step_head();
   cudaError_t e2 = cudaStreamEndCapture(stream_, &pre);
   LS_TRY(err, "capture seed part");
   LS_TRY(e2, "capture end");
-  // narrowband + update part
   LS_TRY(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "capture begin");
-  err = K_->narrowband(m_, s_, sp_, L_, stream_);
-  if (err == cudaSuccess) {
-    k_step_tail<<<1, 32, 0, stream_>>>(s_.counts, s_.ctl);
-    err = cudaGetLastError();
-  }
-  if (cfg_.update_kind != 2)
-    for (int it = 0; it < cfg_.inside_niter && err == cudaSuccess; ++it) err = K_->update(m_, s_, sp_, L_, stream_);
+  err = step_tail();
   e2 = cudaStreamEndCapture(stream_, &post);
   LS_TRY(err, "capture update part");
   LS_TRY(e2, "capture end");
@@ -472,14 +487,9 @@ std::string Solver::build_graph() {
   LS_TRY(cudaStreamBeginCaptureToGraph(stream_, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal),
          "capture body");
   err = cudaSuccess;
-  for (int i = 0; i < chunk && err == cudaSuccess; ++i) {
-    const int cur = i & 1;
-    err = K_->sweep(m_, s_, sp_, cur, false, L_, stream_);
-    if (err == cudaSuccess) err = K_->schedule(m_, s_, sp_, cur, L_, stream_);
-    if (err == cudaSuccess) err = K_->sweep(m_, s_, sp_, cur, true, L_, stream_);
-  }
+  for (int i = 0; i < chunk && err == cudaSuccess; ++i) err = K_->fim(m_, s_, sp_, i, L_, stream_);
   if (err == cudaSuccess) {
-    k_loop_cond<<<1, 32, 0, stream_>>>(s_.counts, s_.ctl, hc, max_bodies);
+    k_loop_cond<<<1, 32, 0, stream_>>>(s_.ctl, hc, chunk, iter_cap());
     err = cudaGetLastError();
   }
   e2 = cudaStreamEndCapture(stream_, &body);
@@ -493,41 +503,27 @@ std::string Solver::build_graph() {
 }
 
 std::string Solver::fim_loop(const StepParams& sp) {
-  long long launched = 0;
-  auto prof = [&](int kind, auto&& fn) -> cudaError_t {
+  auto prof = [&](auto&& fn) -> cudaError_t {
     if (!cfg_.profile) return fn();
     ProfEvent pe;
-    cudaError_t e = prof_fim_begin(pe, kind);
+    cudaError_t e = prof_fim_begin(pe, 0);
     if (e != cudaSuccess) return e;
     e = fn();
     cudaError_t e2 = prof_fim_end(pe);
     return e != cudaSuccess ? e : e2;
   };
-  // a wait of the FIM kernels that runs out sets ctl[3] (read at every sync)
-  LS_TRY(cudaMemsetAsync(s_.ctl + 3, 0, sizeof(int), stream_), "memset");
   while (true) {
-    for (int i = 0; i < cfg_.graph_chunk; ++i) {
-      const int cur = i & 1;
-      LS_TRY(prof(0, [&] { return K_->sweep(m_, s_, sp, cur, false, L_, stream_); }), "sweep");
-      LS_TRY(prof(2, [&] { return K_->schedule(m_, s_, sp, cur, L_, stream_); }), "schedule");
-      LS_TRY(prof(1, [&] { return K_->sweep(m_, s_, sp, cur, true, L_, stream_); }), "check");
-    }
-    launched += cfg_.graph_chunk;
-    st_.kernel_launches += 3LL * cfg_.graph_chunk;
-    LS_TRY(cudaMemcpyAsync(h_counts_, s_.counts, sizeof(int) * 8, cudaMemcpyDeviceToHost, stream_), "d2h");
-    LS_TRY(cudaMemcpyAsync(h_counts_ + 8, s_.ctl, sizeof(int) * 4, cudaMemcpyDeviceToHost, stream_), "d2h");
-    LS_TRY(cudaStreamSynchronize(stream_), "fim sync");
-    if (h_counts_[11]) {
-      status_ = 3;
-      return "a geometry slab copy wait of the FIM kernel timed out";
-    }
-    if (h_counts_[0] == 0) break;
-    if (launched >= cfg_.max_fim_iters) {
-      status_ = 3;
-      return "FIM did not converge within max_fim_iters iterations";
-    }
+    for (int i = 0; i < cfg_.graph_chunk; ++i)
+      LS_TRY(prof([&] { return K_->fim(m_, s_, sp, i, L_, stream_); }), "FIM iteration");
+    k_body_end<<<1, 32, 0, stream_>>>(s_.ctl, cfg_.graph_chunk, iter_cap());
+    LS_TRY(cudaGetLastError(), "body end");
+    st_.kernel_launches += cfg_.graph_chunk + 1;
+    LS_TRY(read_ctl(), "fim sync");
+    std::string r = fim_status();
+    if (!r.empty()) return r;
+    const int cur = h_ctl_[CTL_ITER] % 3;
+    if (h_ctl_[CTL_VISITS + cur] + h_ctl_[CTL_CANDS + cur] == 0) return "";
   }
-  return "";
 }
 
 std::string Solver::one_step(bool* empty_nb) {
@@ -543,79 +539,45 @@ std::string Solver::one_step(bool* empty_nb) {
     prof_.push_back(pe);
     return e;
   };
+  if (h_ctl_[CTL_ITER] > kStampLimit) LS_TRY(restart_stamps(0), "stamps");
   if (net_ || collect_) return learned_step(empty_nb);
-  if (graph_exec_ && !cfg_.profile) {
-    LS_TRY(cudaGraphLaunch(graph_exec_, stream_), "graph launch");
-    LS_TRY(cudaMemcpyAsync(h_counts_, s_.counts, sizeof(int) * 8, cudaMemcpyDeviceToHost, stream_), "d2h");
-    LS_TRY(cudaMemcpyAsync(h_counts_ + 8, s_.ctl, sizeof(int) * 4, cudaMemcpyDeviceToHost, stream_), "d2h");
-    LS_TRY(cudaStreamSynchronize(stream_), "step sync");
-    const int bodies = h_counts_[8];
-    st_.kernel_launches += persistent_ ? 5LL + (cfg_.update_kind != 2 ? 2LL * cfg_.inside_niter : 0)
-                                       : 5LL + (3LL * cfg_.graph_chunk + 1) * bodies +
-                                             (cfg_.update_kind != 2 ? 2LL * cfg_.inside_niter : 0);
-    if (h_counts_[11]) {
-      status_ = 3;
-      return h_counts_[11] == 1 ? "a grid barrier wait of the persistent FIM kernel timed out"
-                                : "a geometry slab copy wait of the FIM kernel timed out";
+  const long long upd = cfg_.update_kind != 2 ? 2LL * cfg_.inside_niter : 0;  // update, copy-back
+  if (persistent_ || (graph_exec_ && !cfg_.profile)) {
+    // the whole step in one go: its graph, or the persistent form launch by
+    // launch (profiled: the FIM loop kernel's time is recorded as the sweep time)
+    if (graph_exec_ && !cfg_.profile) {
+      LS_TRY(cudaGraphLaunch(graph_exec_, stream_), "graph launch");
+    } else {
+      ProfEvent pe{};
+      if (cfg_.profile) LS_TRY(prof_fim_begin(pe, 0), "event");
+      LS_TRY(step_persistent_launches(), "persistent step");
+      if (cfg_.profile) LS_TRY(prof_fim_end(pe), "event");
     }
-    if (h_counts_[9]) {
-      status_ = 3;
-      return "FIM did not converge within max_fim_iters iterations";
-    }
-    have_nb_ = h_counts_[3] != 0;
+    LS_TRY(read_ctl(), "step sync");
+    // begin, seed, the FIM loop, narrowband and the updates
+    st_.kernel_launches += 3 + upd + (persistent_ ? 1LL : (cfg_.graph_chunk + 1LL) * h_ctl_[CTL_BODIES]);
+    std::string r = fim_status();
+    if (!r.empty()) return r;
+    have_nb_ = h_ctl_[CTL_NB] != 0;
     *empty_nb = !have_nb_;
     return "";
   }
-  const int use_all = have_nb_ ? 0 : 1;
-  if (persistent_) {
-    // the persistent step launch by launch (profiled: the FIM loop kernel's
-    // time is recorded as the sweep time)
-    ProfEvent pe{};
-    if (cfg_.profile) LS_TRY(prof_fim_begin(pe, 0), "event");
-    LS_TRY(step_persistent_launches(use_all), "persistent step");
-    if (cfg_.profile) LS_TRY(prof_fim_end(pe), "event");
-    LS_TRY(cudaMemcpyAsync(h_counts_, s_.counts, sizeof(int) * 8, cudaMemcpyDeviceToHost, stream_), "d2h");
-    LS_TRY(cudaMemcpyAsync(h_counts_ + 8, s_.ctl, sizeof(int) * 4, cudaMemcpyDeviceToHost, stream_), "d2h");
-    LS_TRY(cudaStreamSynchronize(stream_), "step sync");
-    st_.kernel_launches += 5LL + (cfg_.update_kind != 2 ? 2LL * cfg_.inside_niter : 0);
-    if (h_counts_[11]) {
-      status_ = 3;
-      return h_counts_[11] == 1 ? "a grid barrier wait of the persistent FIM kernel timed out"
-                                : "a geometry slab copy wait of the FIM kernel timed out";
-    }
-    if (h_counts_[9]) {
-      status_ = 3;
-      return "FIM did not converge within max_fim_iters iterations";
-    }
-    have_nb_ = h_counts_[3] != 0;
-    *empty_nb = !have_nb_;
-    return "";
-  }
-  LS_TRY(cudaMemsetAsync(s_.counts, 0, sizeof(int) * 3, stream_), "memset");
-  LS_TRY(cudaMemsetAsync(s_.counts + 4, 0, sizeof(int), stream_), "memset");
-  LS_TRY(K_->reset(m_, s_, sp_, L_, stream_), "reset");
-  LS_TRY(cudaMemsetAsync(s_.blabel, 0, sizeof(int) * m_.nparts, stream_), "memset");
-  LS_TRY(prof(3, [&] { return K_->seed(m_, s_, use_all, sp_.scale, L_, stream_); }), "seed");
-  LS_TRY(cudaMemsetAsync(s_.counts + 3, 0, sizeof(int), stream_), "memset");
-  st_.kernel_launches += 4;  // reset, seed, narrowband, step tail
+  LS_TRY(K_->begin(s_, 0, stream_), "begin");
+  LS_TRY(prof(3, [&] { return K_->seed(m_, s_, sp_, L_, stream_); }), "seed");
+  st_.kernel_launches += 3;  // begin, seed, narrowband
   std::string r = fim_loop(sp_);
   if (!r.empty()) return r;
   LS_TRY(prof(4, [&] { return K_->narrowband(m_, s_, sp_, L_, stream_); }), "narrowband");
-  k_step_tail<<<1, 32, 0, stream_>>>(s_.counts, s_.ctl);
-  LS_TRY(cudaGetLastError(), "step tail");
-  LS_TRY(cudaMemcpyAsync(h_counts_, s_.counts, sizeof(int) * 8, cudaMemcpyDeviceToHost, stream_), "d2h");
-  LS_TRY(cudaStreamSynchronize(stream_), "nb sync");
-  if (h_counts_[3] == 0) {
+  LS_TRY(read_ctl(), "nb sync");
+  have_nb_ = h_ctl_[CTL_NB] != 0;
+  if (!have_nb_) {
     *empty_nb = true;
-    have_nb_ = false;
     return "";
   }
-  have_nb_ = true;
   if (cfg_.update_kind != 2) {
-    for (int it = 0; it < cfg_.inside_niter; ++it) {
+    for (int it = 0; it < cfg_.inside_niter; ++it)
       LS_TRY(prof(5, [&] { return K_->update(m_, s_, sp_, L_, stream_); }), "update");
-      st_.kernel_launches += 2;  // update, copy-back
-    }
+    st_.kernel_launches += upd;
   }
   return "";
 }
@@ -702,14 +664,10 @@ std::string Solver::learned_step(bool* empty_nb) {
   *empty_nb = false;
   const bool prev = have_nb_;
   const bool warm = net_ && prev;
-  int nb_prev = 0;
-  LS_TRY(cudaMemsetAsync(s_.counts, 0, sizeof(int) * 3, stream_), "memset");
-  LS_TRY(cudaMemsetAsync(s_.counts + 4, 0, sizeof(int), stream_), "memset");
-  LS_TRY(K_->reset(m_, s_, sp_, L_, stream_), "reset");
+  LS_TRY(K_->begin(s_, 0, stream_), "begin");
   if (prev) {
-    LS_TRY(cudaMemcpyAsync(h_counts_, s_.counts, sizeof(int) * 8, cudaMemcpyDeviceToHost, stream_), "d2h");
-    LS_TRY(cudaStreamSynchronize(stream_), "sync");
-    nb_prev = h_counts_[3];
+    LS_TRY(read_ctl(), "sync");
+    const int nb_prev = h_ctl_[CTL_NB_PREV];
     LS_TRY(cudaMemsetAsync(lr_.cnt, 0, sizeof(int) * 4, stream_), "memset");
     LS_TRY(K_->learn(LEARN_NB_VERTICES, m_, s_, sp_, lr_, nb_prev, 0.f, L_, stream_), "warm set");
     mlp::k_features<<<L_.flat_grid, 256, 0, stream_>>>(0, lr_.vlist, lr_.cnt, adj_off_, adj_, m_.xyz, m_.nv, s_.phi,
@@ -723,10 +681,8 @@ std::string Solver::learned_step(bool* empty_nb) {
       st_.kernel_launches += 2;
     }
   }
-  LS_TRY(cudaMemsetAsync(s_.blabel, 0, sizeof(int) * m_.nparts, stream_), "memset");
   if (warm) LS_TRY(K_->learn(LEARN_SEED_WARM, m_, s_, sp_, lr_, 0, 0.f, L_, stream_), "seed");
-  else LS_TRY(K_->seed(m_, s_, prev ? 0 : 1, sp_.scale, L_, stream_), "seed");
-  LS_TRY(cudaMemsetAsync(s_.counts + 3, 0, sizeof(int), stream_), "memset");
+  else LS_TRY(K_->seed(m_, s_, sp_, L_, stream_), "seed");
   st_.kernel_launches += 2;
   std::string r = fim_loop(sp_);
   if (!r.empty()) return r;
@@ -735,14 +691,12 @@ std::string Solver::learned_step(bool* empty_nb) {
     const int max_rounds = 16;
     bool clean = false;
     for (int round = 0; round < max_rounds; ++round) {
-      LS_TRY(cudaMemsetAsync(s_.counts, 0, sizeof(int) * 3, stream_), "memset");
       LS_TRY(K_->learn(LEARN_SUPPORT, m_, s_, sp_, lr_, support_patch_ ? 1 : 0, support_tol_, L_, stream_),
              "support");
-      LS_TRY(cudaMemcpyAsync(h_counts_, s_.counts, sizeof(int) * 8, cudaMemcpyDeviceToHost, stream_), "d2h");
-      LS_TRY(cudaStreamSynchronize(stream_), "sync");
+      LS_TRY(read_ctl(), "sync");
       st_.kernel_launches += 1;
       st_.support_rounds++;
-      if (h_counts_[0] == 0) {
+      if (h_ctl_[CTL_VISITS + h_ctl_[CTL_ITER] % 3] == 0) {
         clean = true;
         break;
       }
@@ -752,12 +706,8 @@ std::string Solver::learned_step(bool* empty_nb) {
     if (!clean) {
       // plain FIM from the seeds: the fallback
       st_.learned_fallbacks++;
-      LS_TRY(cudaMemsetAsync(s_.counts, 0, sizeof(int) * 3, stream_), "memset");
-      LS_TRY(cudaMemcpyAsync(s_.counts + 3, &nb_prev, sizeof(int), cudaMemcpyHostToDevice, stream_), "h2d");
-      LS_TRY(K_->reset(m_, s_, sp_, L_, stream_), "reset");
-      LS_TRY(cudaMemsetAsync(s_.blabel, 0, sizeof(int) * m_.nparts, stream_), "memset");
-      LS_TRY(K_->seed(m_, s_, 0, sp_.scale, L_, stream_), "seed");
-      LS_TRY(cudaMemsetAsync(s_.counts + 3, 0, sizeof(int), stream_), "memset");
+      LS_TRY(K_->begin(s_, 1, stream_), "begin");
+      LS_TRY(K_->seed(m_, s_, sp_, L_, stream_), "seed");
       r = fim_loop(sp_);
       if (!r.empty()) return r;
     }
@@ -765,9 +715,7 @@ std::string Solver::learned_step(bool* empty_nb) {
     st_.kernel_launches += 1;
   }
   LS_TRY(K_->narrowband(m_, s_, sp_, L_, stream_), "narrowband");
-  k_step_tail<<<1, 32, 0, stream_>>>(s_.counts, s_.ctl);
-  LS_TRY(cudaGetLastError(), "step tail");
-  st_.kernel_launches += 2;
+  st_.kernel_launches += 1;
   if (collect_ && prev) {
     LS_TRY(K_->learn(LEARN_TARGETS, m_, s_, sp_, lr_, 0, 1.f / sp_.scale, L_, stream_), "targets");
     st_.kernel_launches += 1;
@@ -776,20 +724,19 @@ std::string Solver::learned_step(bool* empty_nb) {
     if (!r.empty()) return r;
     st_.pairs_collected += added;
   }
-  LS_TRY(cudaMemcpyAsync(h_counts_, s_.counts, sizeof(int) * 8, cudaMemcpyDeviceToHost, stream_), "d2h");
-  LS_TRY(cudaMemcpyAsync(h_counts_ + 8, lr_.cnt, sizeof(int) * 4, cudaMemcpyDeviceToHost, stream_), "d2h");
-  LS_TRY(cudaStreamSynchronize(stream_), "sync");
+  int cnt[4] = {};
+  LS_TRY(cudaMemcpyAsync(cnt, lr_.cnt, sizeof(cnt), cudaMemcpyDeviceToHost, stream_), "d2h");
+  LS_TRY(read_ctl(), "sync");
   if (warm) {
-    st_.warm_vertices += h_counts_[8];
-    st_.unsupported_resets += h_counts_[9];
-    st_.moved_vertices += h_counts_[10];
+    st_.warm_vertices += cnt[0];
+    st_.unsupported_resets += cnt[1];
+    st_.moved_vertices += cnt[2];
   }
-  if (h_counts_[3] == 0) {
+  have_nb_ = h_ctl_[CTL_NB] != 0;
+  if (!have_nb_) {
     *empty_nb = true;
-    have_nb_ = false;
     return "";
   }
-  have_nb_ = true;
   if (cfg_.update_kind != 2) {
     for (int it = 0; it < cfg_.inside_niter; ++it) {
       LS_TRY(K_->update(m_, s_, sp_, L_, stream_), "update");
@@ -894,13 +841,17 @@ std::string Solver::eikonal(const int* seeds, const float* values, int nseeds, f
   const Layout& L = *lay_;
   const int nv = m_.nv, np = m_.nparts;
   const float LN = sp_.largenum;
-  std::vector<float> dt(nv, LN);
+  // a step of its own, with the stamps started again: base 0, first iteration 2
+  LS_TRY(restart_stamps(0), "stamps");
+  LS_TRY(K_->begin(s_, 0, stream_), "begin");
+  std::vector<DtCell> cell(nv, make_int4(0, -1, 0, -1));
   std::vector<uint8_t> sd(nv, 0);
-  std::vector<int> act;
+  std::vector<int> act, pend(np, -1);
   for (int i = 0; i < nseeds; ++i) {
     const int v = L.vert_ipermute[seeds[i]];
-    const float a = values[i];
-    dt[v] = (a >= LN) ? LN : a / sp_.scale;
+    const float a = (values[i] >= LN) ? LN : values[i] / sp_.scale;
+    std::memcpy(&cell[v].x, &a, sizeof(float));
+    cell[v].y = 0;
     sd[v] = 1;
   }
   // first active list: the patches one of whose element copies holds a seed
@@ -910,16 +861,19 @@ std::string Solver::eikonal(const int* seeds, const float* values, int nseeds, f
     bool hit = false;
     for (int c = L.ele_offsets[p]; c < L.ele_offsets[p + 1] && !hit; ++c)
       for (int k = 0; k < d1; ++k) hit |= sd[L.conn[(size_t)c * d1 + k]] != 0;
-    if (hit) act.push_back(p);
+    if (hit) {
+      act.push_back(p);
+      pend[p] = 2 * 2;
+    }
   }
-  int counts[8] = {(int)act.size(), 0, 0, 0, 0, 0, 0, 0};
-  LS_TRY(cudaMemcpyAsync(s_.DT, dt.data(), sizeof(float) * nv, cudaMemcpyHostToDevice, stream_), "h2d");
-  LS_TRY(cudaMemcpyAsync(s_.seed, sd.data(), nv, cudaMemcpyHostToDevice, stream_), "h2d");
-  if (!act.empty())
-    LS_TRY(cudaMemcpyAsync(s_.list0, act.data(), sizeof(int) * act.size(), cudaMemcpyHostToDevice, stream_), "h2d");
-  LS_TRY(cudaMemcpyAsync(s_.counts, counts, sizeof(counts), cudaMemcpyHostToDevice, stream_), "h2d");
-  LS_TRY(cudaMemsetAsync(s_.blabel, 0, sizeof(int) * np, stream_), "memset");
-  LS_TRY(cudaMemsetAsync(s_.ctl + 2, 0, sizeof(int), stream_), "memset");
+  const int n = (int)act.size();
+  LS_TRY(cudaMemcpyAsync(s_.cell, cell.data(), sizeof(DtCell) * nv, cudaMemcpyHostToDevice, stream_), "h2d");
+  LS_TRY(cudaMemcpyAsync(s_.pend, pend.data(), sizeof(int) * np, cudaMemcpyHostToDevice, stream_), "h2d");
+  if (n)
+    LS_TRY(cudaMemcpyAsync(s_.lists + (size_t)2 * np, act.data(), sizeof(int) * n, cudaMemcpyHostToDevice, stream_),
+           "h2d");
+  LS_TRY(cudaMemcpyAsync(s_.ctl + CTL_VISITS + 2, &n, sizeof(int), cudaMemcpyHostToDevice, stream_), "h2d");
+  LS_TRY(cudaMemsetAsync(s_.ctl + CTL_NB_VALID, 0, sizeof(int), stream_), "memset");
   StepParams sp = sp_;
   // no narrowband limit: every converged patch that the front has reached
   // (minimum below LARGENUM) activates its neighbours
@@ -927,8 +881,9 @@ std::string Solver::eikonal(const int* seeds, const float* values, int nseeds, f
   std::string r = fim_loop(sp);
   if (!r.empty()) return r;
   if (cfg_.profile) fold_prof(true);
-  LS_TRY(cudaMemcpyAsync(dt.data(), s_.DT, sizeof(float) * nv, cudaMemcpyDeviceToHost, stream_), "d2h");
-  LS_TRY(cudaStreamSynchronize(stream_), "sync");
+  std::vector<float> dt(nv);
+  r = dt_values(dt.data());
+  if (!r.empty()) return r;
   for (int v = 0; v < nv; ++v) out[L.vert_permute[v]] = (dt[v] >= LN) ? LN : dt[v] * sp_.scale;
   have_nb_ = false;  // the step state was overwritten
   stats_stale_ = true;
@@ -939,7 +894,7 @@ std::string Solver::set_phi(const float* phi_orig) {
   std::memcpy(h_stage_, phi_orig, sizeof(float) * m_.nv);
   LS_TRY(cudaMemcpyAsync(d_tmp_, h_stage_, sizeof(float) * m_.nv, cudaMemcpyHostToDevice, stream_), "h2d");
   LS_TRY(K_->permute(m_, d_tmp_, s_.phi, L_, stream_), "permute");
-  LS_TRY(cudaMemsetAsync(s_.ctl + 2, 0, sizeof(int), stream_), "memset");
+  LS_TRY(cudaMemsetAsync(s_.ctl + CTL_NB_VALID, 0, sizeof(int), stream_), "memset");
   LS_TRY(cudaStreamSynchronize(stream_), "sync");
   have_nb_ = false;
   return "";
@@ -954,9 +909,8 @@ std::string Solver::get_phi(float* phi_orig) {
 }
 
 std::string Solver::narrowband(unsigned char* flags) {
-  LS_TRY(cudaMemcpyAsync(h_counts_, s_.counts, sizeof(int) * 8, cudaMemcpyDeviceToHost, stream_), "d2h");
-  LS_TRY(cudaStreamSynchronize(stream_), "sync");
-  const int n = h_counts_[3];
+  LS_TRY(read_ctl(), "d2h");
+  const int n = h_ctl_[CTL_NB];
   std::vector<int> nb(n > 0 ? n : 1);
   if (n > 0) LS_TRY(cudaMemcpy(nb.data(), s_.nblist, sizeof(int) * n, cudaMemcpyDeviceToHost), "d2h");
   std::memset(flags, 0, m_.nparts);
@@ -965,17 +919,18 @@ std::string Solver::narrowband(unsigned char* flags) {
 }
 
 std::string Solver::active_patches(std::vector<int>& out) {
-  LS_TRY(cudaMemcpyAsync(h_counts_, s_.counts, sizeof(int) * 8, cudaMemcpyDeviceToHost, stream_), "d2h");
-  LS_TRY(cudaStreamSynchronize(stream_), "sync");
-  out.assign(h_counts_[0], 0);
-  if (h_counts_[0] > 0) LS_TRY(cudaMemcpy(out.data(), s_.list0, sizeof(int) * h_counts_[0], cudaMemcpyDeviceToHost), "d2h");
-  for (int& p : out) p &= ~kPrevisited;
+  LS_TRY(read_ctl(), "d2h");
+  const int cur = h_ctl_[CTL_ITER] % 3, n = h_ctl_[CTL_VISITS + cur];
+  out.assign(n, 0);
+  if (n > 0)
+    LS_TRY(cudaMemcpy(out.data(), s_.lists + (size_t)cur * m_.nparts, sizeof(int) * n, cudaMemcpyDeviceToHost), "d2h");
   return "";
 }
 
 std::string Solver::dt_values(float* dt) {
+  LS_TRY(K_->distances(m_, s_, sp_, d_tmp_, L_, stream_), "distances");
+  LS_TRY(cudaMemcpyAsync(dt, d_tmp_, sizeof(float) * m_.nv, cudaMemcpyDeviceToHost, stream_), "d2h");
   LS_TRY(cudaStreamSynchronize(stream_), "sync");
-  LS_TRY(cudaMemcpy(dt, s_.DT, sizeof(float) * m_.nv, cudaMemcpyDeviceToHost), "d2h");
   return "";
 }
 

@@ -28,18 +28,21 @@ enum { LEARN_NB_VERTICES = 0, LEARN_WARM, LEARN_SEED_WARM, LEARN_SUPPORT, LEARN_
 // One build of the step kernels (fast or bit-exact).
 struct KernelSet {
   cudaError_t (*configure)(const DevMesh& m, const StepParams& sp, Launch& L);
-  cudaError_t (*reset)(const DevMesh& m, const DevState& s, const StepParams& sp, const Launch& L, cudaStream_t st);
-  cudaError_t (*seed)(const DevMesh& m, const DevState& s, int use_all, float scale, const Launch& L, cudaStream_t st);
-  cudaError_t (*sweep)(const DevMesh& m, const DevState& s, const StepParams& sp, int cur, bool check,
-                       const Launch& L, cudaStream_t st);
-  cudaError_t (*schedule)(const DevMesh& m, const DevState& s, const StepParams& sp, int cur, const Launch& L,
-                          cudaStream_t st);
+  // step control words; restart: again within a step (the previous narrowband's size is kept)
+  cudaError_t (*begin)(const DevState& s, int restart, cudaStream_t st);
+  cudaError_t (*seed)(const DevMesh& m, const DevState& s, const StepParams& sp, const Launch& L, cudaStream_t st);
+  // one FIM iteration, the off-th of a loop body
+  cudaError_t (*fim)(const DevMesh& m, const DevState& s, const StepParams& sp, int off, const Launch& L,
+                     cudaStream_t st);
   // every FIM iteration of a step in one cooperative launch (L.persist_grid > 0)
   cudaError_t (*fim_persistent)(const DevMesh& m, const DevState& s, const StepParams& sp, const Launch& L,
                                 cudaStream_t st);
   cudaError_t (*narrowband)(const DevMesh& m, const DevState& s, const StepParams& sp, const Launch& L,
                             cudaStream_t st);
   cudaError_t (*update)(const DevMesh& m, const DevState& s, const StepParams& sp, const Launch& L, cudaStream_t st);
+  // FIM distances in the layout's vertex order
+  cudaError_t (*distances)(const DevMesh& m, const DevState& s, const StepParams& sp, float* out, const Launch& L,
+                           cudaStream_t st);
   cudaError_t (*unpermute)(const DevMesh& m, const float* phi, float* out, const Launch& L, cudaStream_t st);
   cudaError_t (*permute)(const DevMesh& m, const float* in, float* out, const Launch& L, cudaStream_t st);
   // learned warm start / collection kernels (op: LEARN_*)
@@ -147,7 +150,13 @@ class Solver {
   std::string fim_loop(const StepParams& sp);
   std::string build_graph();
   bool build_persistent_graph(std::string* err);
-  cudaError_t step_persistent_launches(int use_all);
+  cudaError_t step_head();
+  cudaError_t step_tail();
+  cudaError_t step_persistent_launches();
+  cudaError_t restart_stamps(int from);
+  cudaError_t read_ctl();
+  std::string fim_status();
+  int iter_cap() const;
   bool persistent_ = false;        // the step's FIM loop is one cooperative launch
   std::vector<double> mesh_scale_;  // FIM length unit of each mesh (one entry for a single mesh)
   void pull_stats();
@@ -187,7 +196,7 @@ class Solver {
   cudaGraphExec_t graph_exec_ = nullptr;
   cudaGraph_t graph_ = nullptr;
   std::vector<void*> allocs_;
-  int* h_counts_ = nullptr;           // pinned mirror of s_.counts [0..7] and s_.ctl [8..11]
+  int* h_ctl_ = nullptr;              // pinned mirror of the step control words (read_ctl)
   unsigned long long* h_stats_ = nullptr;
   float* h_stage_ = nullptr;          // pinned nv floats
   float* d_tmp_ = nullptr;            // nv floats (caller-order staging)
