@@ -457,6 +457,11 @@ __device__ __forceinline__ float tet_solve_pred(float TA, float TB, float TC, fl
 // point, where the edge candidate gives the same value.
 __device__ __forceinline__ bool in_unit(float l) { return __float_as_uint(l) <= 0x3f800000u; }
 
+// The same test of three numbers.
+__device__ __forceinline__ bool in_unit(float a, float b, float c) {
+  return __vimax3_u32(__float_as_uint(a), __float_as_uint(b), __float_as_uint(c)) <= 0x3f800000u;
+}
+
 // Tet update of D from the face ABC in FP32 without the quadratics (fast
 // build).  It returns the same quantity as tet_solve -- the least T_lin(x) +
 // |x - D| over the face, T_lin interpolating TA, TB, TC, with the reference's
@@ -490,16 +495,37 @@ __device__ __forceinline__ bool in_unit(float l) { return __float_as_uint(l) <= 
 // the independent halves run as pairs -- edges AD and BD, sides BC and AC
 // (both from C), the two interior roots -- with the square roots, side AB
 // and the interior's set-up per lane.
-// Arguments as tet_solve, plus hD.
+// Arguments as tet_solve, plus hD; not all of TA, TB, TC are LARGENUM (the
+// listings leave those solves out).
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
+// The approximate square root, its reciprocal and the reciprocal as the bare
+// hardware operations: with denormals kept, each of the solver's 17 carries
+// a test and a rescaling of its argument.  The arguments here are squared
+// lengths and products of two of them; one below 1.2e-38 stands for a
+// length under 1e-19 (or a face area under 1e-19 of a square unit, whose
+// reciprocal overflows FP32 either way).
+__device__ __forceinline__ float fast_sqrt(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float fast_rsqrt(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float fast_rcp(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
 
 __device__ __forceinline__ float tet_solve_wave(float TA, float TB, float TC, float ACAC, float ACBC, float ACCD,
-                                                float BCBC, float BCCD, float CDCD, float hD, float eps_h, float LN) {
-  if (TA >= LN && TB >= LN && TC >= LN) return LN;
+                                                float BCBC, float BCCD, float CDCD, float hD, float eps_h) {
   // edges AD, BD (lanes x, y) and CD
   const float2 d2 = __fadd2_rn(__fadd2_rn(f2(ACAC, BCBC), f2(ACCD, BCCD)), __fadd2_rn(f2(ACCD, BCCD), f2(CDCD, CDCD)));
-  const float2 ed = __fadd2_rn(f2(TA, TB), f2(sqrtf(d2.x), sqrtf(d2.y)));
-  float best = fminf(fminf(ed.x, ed.y), TC + sqrtf(CDCD));
+  const float2 ed = __fadd2_rn(f2(TA, TB), f2(fast_sqrt(d2.x), fast_sqrt(d2.y)));
+  float best = fminf(fminf(ed.x, ed.y), TC + fast_sqrt(CDCD));
   // sides: x = lam Q + (1 - lam) P with |Q - P|^2 = ff, (Q - P).(D - P) = fw,
   // |D - P|^2 = ww and u = T_Q - T_P.  At the stationary point of
   // T_P + lam u + |x - D| the distance is r = sqrt(ff ww - fw^2) /
@@ -510,8 +536,8 @@ __device__ __forceinline__ float tet_solve_wave(float TA, float TB, float TC, fl
     const float2 u = __fadd2_rn(f2(TB, TA), f2(-TC, -TC));
     const float2 G = __ffma2_rn(ff, f2(CDCD, CDCD), __fmul2_rn(fw, f2(BCCD, ACCD)));  // ff ww - fw^2
     const float2 q = __ffma2_rn(u, f2(-u.x, -u.y), ff);                              // ff - u^2
-    const float2 r = __fmul2_rn(f2(sqrtf(G.x), sqrtf(G.y)), f2(rsqrtf(q.x), rsqrtf(q.y)));
-    const float2 lam = __fmul2_rn(__ffma2_rn(f2(-u.x, -u.y), r, fw), f2(1.f / ff.x, 1.f / ff.y));
+    const float2 r = __fmul2_rn(f2(fast_sqrt(G.x), fast_sqrt(G.y)), f2(fast_rsqrt(q.x), fast_rsqrt(q.y)));
+    const float2 lam = __fmul2_rn(__ffma2_rn(f2(-u.x, -u.y), r, fw), f2(fast_rcp(ff.x), fast_rcp(ff.y)));
     const float2 c = __fadd2_rn(__ffma2_rn(lam, u, f2(TC, TC)), r);
     if (in_unit(lam.x)) best = fminf(best, c.x);
     if (in_unit(lam.y)) best = fminf(best, c.y);
@@ -520,24 +546,24 @@ __device__ __forceinline__ float tet_solve_wave(float TA, float TB, float TC, fl
     const float u = TA - TB;
     const float ff = (BCBC - ACBC) + (ACAC - ACBC), fw = (BCBC + BCCD) - (ACBC + ACCD);
     const float ww = (BCBC + BCCD) + (BCCD + CDCD);
-    const float r = sqrtf(ff * ww - fw * fw) * rsqrtf(ff - u * u);
-    const float lam = (fw - u * r) / ff;
+    const float r = fast_sqrt(ff * ww - fw * fw) * fast_rsqrt(ff - u * u);
+    const float lam = (fw - u * r) * fast_rcp(ff);
     if (in_unit(lam)) best = fminf(best, TB + lam * u + r);
   }
   {  // interior of ABC: x = l1 A + l2 B + l3 C
     const float u1 = TA - TC, u2 = TB - TC;
-    const float idet = 1.f / (ACAC * BCBC - ACBC * ACBC);
-    const float g1 = (BCBC * u1 - ACBC * u2) * idet;  // in-plane gradient, coefficient of -AC
-    const float g2 = (ACAC * u2 - ACBC * u1) * idet;  // and of -BC
+    const float idet = fast_rcp(ACAC * BCBC - ACBC * ACBC);
+    // the reference's h and s, which are also the numerators of the gradient
+    const float h = BCBC * u1 - ACBC * u2, s = ACAC * u2 - ACBC * u1, t = u2 * ACCD - u1 * BCCD;
+    const float g1 = h * idet;  // in-plane gradient, coefficient of -AC
+    const float g2 = s * idet;  // and of -BC
     const float foot1 = (ACBC * BCCD - BCBC * ACCD) * idet;  // D's foot point, weight of A
     // the point downhill of the foot point (lane x) and its mirror uphill
     // (lane y): the reference's SMALLNUM offset in l2 = (s l1 + t) / (h +
     // eps_h) can move the first point out of the face where h is small, and
     // the mirror's point is then the better one, as in the reference
-    const float dl = hD * rsqrtf(1.f - (g1 * u1 + g2 * u2)) * g1;
-    const float TAC = TC - TA, TBC = TC - TB;
-    const float s = TAC * ACBC - TBC * ACAC, t = TAC * BCCD - TBC * ACCD, h = -(TAC * BCBC - TBC * ACBC);
-    const float ih = 1.f / (h + eps_h);
+    const float dl = hD * fast_rsqrt(1.f - (g1 * u1 + g2 * u2)) * g1;
+    const float ih = fast_rcp(h + eps_h);
     const float2 l1 = __fadd2_rn(f2(foot1, foot1), f2(-dl, dl));
     const float2 l2 = __fmul2_rn(__ffma2_rn(f2(s, s), l1, f2(t, t)), f2(ih, ih));
     const float2 l3 = __fadd2_rn(__fadd2_rn(f2(1.f, 1.f), f2(-l1.x, -l1.y)), f2(-l2.x, -l2.y));
@@ -547,9 +573,9 @@ __device__ __forceinline__ float tet_solve_wave(float TA, float TB, float TC, fl
     const float2 a3 = __ffma2_rn(l1, f2(ACCD, ACCD), __ffma2_rn(l2, f2(BCCD, BCCD), f2(CDCD, CDCD)));
     const float2 Q = __ffma2_rn(a1, l1, __ffma2_rn(a2, l2, a3));
     const float2 lin = __ffma2_rn(f2(TA, TA), l1, __ffma2_rn(f2(TB, TB), l2, __fmul2_rn(f2(TC, TC), l3)));
-    const float2 c = __fadd2_rn(lin, f2(sqrtf(Q.x), sqrtf(Q.y)));
-    if (in_unit(l1.x) && in_unit(l2.x) && in_unit(l3.x)) best = fminf(best, c.x);
-    if (in_unit(l1.y) && in_unit(l2.y) && in_unit(l3.y)) best = fminf(best, c.y);
+    const float2 c = __fadd2_rn(lin, f2(fast_sqrt(Q.x), fast_sqrt(Q.y)));
+    if (in_unit(l1.x, l2.x, l3.x)) best = fminf(best, c.x);
+    if (in_unit(l1.y, l2.y, l3.y)) best = fminf(best, c.y);
   }
   return best;
 }

@@ -707,7 +707,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_fim_compact(DevMesh m, DevState 
         if constexpr (PREC)
           r = tet_solve_pred<true>(a0, a1, a2, g0, g1, g2, g3, g4, g5, sp.eps_h, sp.largenum, sp.tau, &ill);
         else
-          r = tet_solve_wave(a0, a1, a2, g0, g1, g2, g3, g4, g5, sH[k * MAXT + cc], sp.eps_h, sp.largenum);
+          r = tet_solve_wave(a0, a1, a2, g0, g1, g2, g3, g4, g5, sH[k * MAXT + cc], sp.eps_h);
         if (PREC && ill) {
           // discriminant cancelled: repeat in FP64 after this pass, densely
           sRep[atomicAdd(&s_rep, 1)] = code;
@@ -841,7 +841,7 @@ __device__ __forceinline__ void pair_solve(int code, const float4* sTc, const fl
   if constexpr (SOLVER == kPairWave) {
     // the target's height: component k of the copy's record, loaded alone
     const float hD = reinterpret_cast<const float*>(sH)[4 * cc + k];
-    r = tet_solve_wave(a0, a1, a2, g0, g1, g2, g3, g4, g5, hD, sp.eps_h, sp.largenum);
+    r = tet_solve_wave(a0, a1, a2, g0, g1, g2, g3, g4, g5, hD, sp.eps_h);
   } else {
     bool d = false;
     r = tet_solve<float, SOLVER == kPairRefXdiv, false, false>(a0, a1, a2, g0, g1, g2, g3, g4, g5, sp.eps_h,
