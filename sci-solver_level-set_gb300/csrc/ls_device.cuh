@@ -492,10 +492,16 @@ __device__ __forceinline__ bool in_unit(float a, float b, float c) {
 // range tests.
 // Evaluation: sm_100 issues one FP32x2 instruction (add, multiply, fused
 // multiply-add, each lane rounded as the scalar operation) for two lanes, so
-// the independent halves run as pairs -- edges AD and BD, sides BC and AC
-// (both from C), the two interior roots -- with the square roots, side AB
-// and the interior's set-up per lane.
-// Arguments as tet_solve, plus hD; not all of TA, TB, TC are LARGENUM (the
+// some independent halves run as pairs -- edges PX and QX, sides RQ and RP
+// (both from R), the two interior roots -- with the square roots, side QP
+// and the interior's set-up per lane.  Every multiply-add is written out:
+// left to the compiler's contraction, the kernels that inline this solver
+// would round differently.
+// Arguments: the face's vertices are P, Q, R and the target X; the dot
+// products of p = P - R, q = Q - R and x = X - R (PP = p.p, PQ = p.q, ...),
+// and hX, X's height over the face.  (tet_solve's ACCD and BCCD are -PX and
+// -QX: with all three vectors from R the four solves of a tet only permute
+// the products, without signs.)  Not all of TP, TQ, TR are LARGENUM (the
 // listings leave those solves out).
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
 // The approximate square root, its reciprocal and the reciprocal as the bare
@@ -520,59 +526,57 @@ __device__ __forceinline__ float fast_rcp(float x) {
   return r;
 }
 
-__device__ __forceinline__ float tet_solve_wave(float TA, float TB, float TC, float ACAC, float ACBC, float ACCD,
-                                                float BCBC, float BCCD, float CDCD, float hD, float eps_h) {
-  // edges AD, BD (lanes x, y) and CD
-  const float2 d2 = __fadd2_rn(__fadd2_rn(f2(ACAC, BCBC), f2(ACCD, BCCD)), __fadd2_rn(f2(ACCD, BCCD), f2(CDCD, CDCD)));
-  const float2 ed = __fadd2_rn(f2(TA, TB), f2(fast_sqrt(d2.x), fast_sqrt(d2.y)));
-  float best = fminf(fminf(ed.x, ed.y), TC + fast_sqrt(CDCD));
-  // sides: x = lam Q + (1 - lam) P with |Q - P|^2 = ff, (Q - P).(D - P) = fw,
-  // |D - P|^2 = ww and u = T_Q - T_P.  At the stationary point of
-  // T_P + lam u + |x - D| the distance is r = sqrt(ff ww - fw^2) /
+__device__ __forceinline__ float tet_solve_wave(float TP, float TQ, float TR, float PP, float PQ, float PX, float QQ,
+                                                float QX, float XX, float hX, float eps_h) {
+  // edges PX, QX (lanes x, y) and RX
+  const float2 d2 = f2((PP - PX) + (XX - PX), (QQ - QX) + (XX - QX));
+  const float2 ed = __fadd2_rn(f2(TP, TQ), f2(fast_sqrt(d2.x), fast_sqrt(d2.y)));
+  float best = fminf(fminf(ed.x, ed.y), TR + fast_sqrt(XX));
+  const float up = TP - TR, uq = TQ - TR;
+  // sides: y = lam F + (1 - lam) B with |F - B|^2 = ff, (F - B).(X - B) = fw,
+  // |X - B|^2 = ww and u = T_F - T_B.  At the stationary point of
+  // T_B + lam u + |y - X| the distance is r = sqrt(ff ww - fw^2) /
   // sqrt(ff - u^2) (no root when ff <= u^2: the rsqrt is then NaN or inf and
   // the candidate is rejected) and lam = (fw - u r) / ff.
-  {  // sides BC (lane x: P = C, Q = B) and AC (lane y: P = C, Q = A)
-    const float2 fw = f2(-BCCD, -ACCD), ff = f2(BCBC, ACAC);
-    const float2 u = __fadd2_rn(f2(TB, TA), f2(-TC, -TC));
-    const float2 G = __ffma2_rn(ff, f2(CDCD, CDCD), __fmul2_rn(fw, f2(BCCD, ACCD)));  // ff ww - fw^2
-    const float2 q = __ffma2_rn(u, f2(-u.x, -u.y), ff);                              // ff - u^2
+  {  // sides RQ (lane x) and RP (lane y), both from R
+    const float2 G = f2(fmaf(QQ, XX, -__fmul_rn(QX, QX)), fmaf(PP, XX, -__fmul_rn(PX, PX)));  // ff ww - fw^2
+    const float2 q = f2(fmaf(-uq, uq, QQ), fmaf(-up, up, PP));                                // ff - u^2
     const float2 r = __fmul2_rn(f2(fast_sqrt(G.x), fast_sqrt(G.y)), f2(fast_rsqrt(q.x), fast_rsqrt(q.y)));
-    const float2 lam = __fmul2_rn(__ffma2_rn(f2(-u.x, -u.y), r, fw), f2(fast_rcp(ff.x), fast_rcp(ff.y)));
-    const float2 c = __fadd2_rn(__ffma2_rn(lam, u, f2(TC, TC)), r);
-    if (in_unit(lam.x)) best = fminf(best, c.x);
-    if (in_unit(lam.y)) best = fminf(best, c.y);
+    const float lx = __fmul_rn(fmaf(-uq, r.x, QX), fast_rcp(QQ)), ly = __fmul_rn(fmaf(-up, r.y, PX), fast_rcp(PP));
+    const float2 c = __fadd2_rn(__ffma2_rn(f2(lx, ly), f2(uq, up), f2(TR, TR)), r);
+    if (in_unit(lx)) best = fminf(best, c.x);
+    if (in_unit(ly)) best = fminf(best, c.y);
   }
-  {  // side AB (P = B, Q = A)
-    const float u = TA - TB;
-    const float ff = (BCBC - ACBC) + (ACAC - ACBC), fw = (BCBC + BCCD) - (ACBC + ACCD);
-    const float ww = (BCBC + BCCD) + (BCCD + CDCD);
-    const float r = fast_sqrt(ff * ww - fw * fw) * fast_rsqrt(ff - u * u);
-    const float lam = (fw - u * r) * fast_rcp(ff);
-    if (in_unit(lam)) best = fminf(best, TB + lam * u + r);
+  {  // side QP, from Q
+    const float u = TP - TQ;
+    const float ff = (QQ - PQ) + (PP - PQ), fw = (QQ - QX) - (PQ - PX);
+    const float r = __fmul_rn(fast_sqrt(fmaf(ff, d2.y, -__fmul_rn(fw, fw))), fast_rsqrt(fmaf(-u, u, ff)));
+    const float lam = __fmul_rn(fmaf(-u, r, fw), fast_rcp(ff));
+    if (in_unit(lam)) best = fminf(best, __fadd_rn(fmaf(lam, u, TQ), r));
   }
-  {  // interior of ABC: x = l1 A + l2 B + l3 C
-    const float u1 = TA - TC, u2 = TB - TC;
-    const float idet = fast_rcp(ACAC * BCBC - ACBC * ACBC);
+  {  // interior: y = l1 P + l2 Q + l3 R
+    const float idet = fast_rcp(fmaf(PP, QQ, -__fmul_rn(PQ, PQ)));
     // the reference's h and s, which are also the numerators of the gradient
-    const float h = BCBC * u1 - ACBC * u2, s = ACAC * u2 - ACBC * u1, t = u2 * ACCD - u1 * BCCD;
-    const float g1 = h * idet;  // in-plane gradient, coefficient of -AC
-    const float g2 = s * idet;  // and of -BC
-    const float foot1 = (ACBC * BCCD - BCBC * ACCD) * idet;  // D's foot point, weight of A
+    const float h = fmaf(QQ, up, -__fmul_rn(PQ, uq)), s = fmaf(PP, uq, -__fmul_rn(PQ, up));
+    const float t = fmaf(up, QX, -__fmul_rn(uq, PX));
+    const float g1 = __fmul_rn(h, idet);  // in-plane gradient, coefficient of P - R
+    const float g2 = __fmul_rn(s, idet);  // and of Q - R
+    const float foot1 = __fmul_rn(fmaf(QQ, PX, -__fmul_rn(PQ, QX)), idet);  // X's foot point, weight of P
     // the point downhill of the foot point (lane x) and its mirror uphill
     // (lane y): the reference's SMALLNUM offset in l2 = (s l1 + t) / (h +
     // eps_h) can move the first point out of the face where h is small, and
     // the mirror's point is then the better one, as in the reference
-    const float dl = hD * fast_rsqrt(1.f - (g1 * u1 + g2 * u2)) * g1;
+    const float dl = __fmul_rn(__fmul_rn(hX, fast_rsqrt(fmaf(-g1, up, fmaf(-g2, uq, 1.f)))), g1);
     const float ih = fast_rcp(h + eps_h);
-    const float2 l1 = __fadd2_rn(f2(foot1, foot1), f2(-dl, dl));
+    const float2 l1 = f2(foot1 - dl, foot1 + dl);
     const float2 l2 = __fmul2_rn(__ffma2_rn(f2(s, s), l1, f2(t, t)), f2(ih, ih));
-    const float2 l3 = __fadd2_rn(__fadd2_rn(f2(1.f, 1.f), f2(-l1.x, -l1.y)), f2(-l2.x, -l2.y));
-    // |x - D|^2 as the quadratic form of (l1, l2), and T_lin(x)
-    const float2 a1 = __ffma2_rn(l1, f2(ACAC, ACAC), __ffma2_rn(l2, f2(ACBC, ACBC), f2(ACCD, ACCD)));
-    const float2 a2 = __ffma2_rn(l1, f2(ACBC, ACBC), __ffma2_rn(l2, f2(BCBC, BCBC), f2(BCCD, BCCD)));
-    const float2 a3 = __ffma2_rn(l1, f2(ACCD, ACCD), __ffma2_rn(l2, f2(BCCD, BCCD), f2(CDCD, CDCD)));
+    const float2 l3 = f2((1.f - l1.x) - l2.x, (1.f - l1.y) - l2.y);
+    // |y - X|^2 as the quadratic form of (l1, l2), and T_lin(y)
+    const float2 a1 = __ffma2_rn(l1, f2(PP, PP), __ffma2_rn(l2, f2(PQ, PQ), f2(-PX, -PX)));
+    const float2 a2 = __ffma2_rn(l1, f2(PQ, PQ), __ffma2_rn(l2, f2(QQ, QQ), f2(-QX, -QX)));
+    const float2 a3 = __ffma2_rn(l1, f2(-PX, -PX), __ffma2_rn(l2, f2(-QX, -QX), f2(XX, XX)));
     const float2 Q = __ffma2_rn(a1, l1, __ffma2_rn(a2, l2, a3));
-    const float2 lin = __ffma2_rn(f2(TA, TA), l1, __ffma2_rn(f2(TB, TB), l2, __fmul2_rn(f2(TC, TC), l3)));
+    const float2 lin = __ffma2_rn(l1, f2(up, up), __ffma2_rn(l2, f2(uq, uq), f2(TR, TR)));
     const float2 c = __fadd2_rn(lin, f2(fast_sqrt(Q.x), fast_sqrt(Q.y)));
     if (in_unit(l1.x, l2.x, l3.x)) best = fminf(best, c.x);
     if (in_unit(l1.y, l2.y, l3.y)) best = fminf(best, c.y);

@@ -707,7 +707,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_fim_compact(DevMesh m, DevState 
         if constexpr (PREC)
           r = tet_solve_pred<true>(a0, a1, a2, g0, g1, g2, g3, g4, g5, sp.eps_h, sp.largenum, sp.tau, &ill);
         else
-          r = tet_solve_wave(a0, a1, a2, g0, g1, g2, g3, g4, g5, sH[k * MAXT + cc], sp.eps_h);
+          r = tet_solve_wave(a0, a1, a2, g0, g1, -g2, g3, -g4, g5, sH[k * MAXT + cc], sp.eps_h);
         if (PREC && ill) {
           // discriminant cancelled: repeat in FP64 after this pass, densely
           sRep[atomicAdd(&s_rep, 1)] = code;
@@ -802,18 +802,22 @@ __global__ void __launch_bounds__(MAXT, MINB) k_fim_compact(DevMesh m, DevState 
 // the reference semantics there).
 constexpr int kPairWave = 0, kPairRef = 1, kPairRefXdiv = 2;
 
-// Can solve k (listed as a candidate: its inputs changed) lower its target
-// T_k?  Not when the three other values are all LARGENUM (the solver returns
-// LARGENUM); with the planar-wave solver also not when min of them plus
-// 0.999 x the target's height over their face is at least T_k (the lower
-// bound of every candidate in exact arithmetic).  The reference solver's
-// FP32 candidates can fall below that bound, so the bit-exact build keeps
-// those solves.
+// The solves (bit k: target k) of a copy with values tv and heights hv that
+// can lower their target T_k.  One cannot when the three other values are
+// all LARGENUM (the solver returns LARGENUM); with the planar-wave solver
+// also not when min of them plus 0.999 x the target's height over their face
+// is at least T_k (the lower bound of every candidate in exact arithmetic,
+// which with three LARGENUMs is no less than T_k either).  The reference
+// solver's FP32 candidates can fall below that bound, so the bit-exact build
+// keeps those solves.
 template <int SOLVER>
-__device__ __forceinline__ bool pair_may_lower(unsigned cand, float mn, float hk, float tk, float LN) {
-  if (!cand || !(mn < LN)) return false;
-  if constexpr (SOLVER == kPairWave) return mn + 0.999f * hk < tk;
-  return true;
+__device__ __forceinline__ unsigned pair_may_lower(const float4& tv, const float4& hv, float LN) {
+  const float m01 = fminf(tv.x, tv.y), m23 = fminf(tv.z, tv.w);
+  const float n0 = fminf(tv.y, m23), n1 = fminf(tv.x, m23), n2 = fminf(m01, tv.w), n3 = fminf(m01, tv.z);
+  if constexpr (SOLVER == kPairWave)
+    return (n0 + 0.999f * hv.x < tv.x ? 1u : 0u) | (n1 + 0.999f * hv.y < tv.y ? 2u : 0u) |
+           (n2 + 0.999f * hv.z < tv.z ? 4u : 0u) | (n3 + 0.999f * hv.w < tv.w ? 8u : 0u);
+  return (n0 < LN ? 1u : 0u) | (n1 < LN ? 2u : 0u) | (n2 < LN ? 4u : 0u) | (n3 < LN ? 8u : 0u);
 }
 
 // One listed solve of k_fim_pair: solve k of copy cc from the copy values
@@ -825,48 +829,46 @@ __device__ __forceinline__ void pair_solve(int code, const float4* sTc, const fl
   const int cc = code >> 2, k = code & 3;
   const float4 tv = sTc[cc];
   const float TA = tv.x, TB = tv.y, TC = tv.z, TD = tv.w;
-  // the six metric terms of solve k (k_geometry's record: floats 0-5 for
-  // solves 0, 1, 3, floats 6-11 for solve 2), v0 .. v5 = ACAC ACBC ACCD BCBC
-  // BCCD CDCD, or ADAD ADBD ADCD BDBD CDBD CDCD
+  // the six dot products of solve k's base vertex (k_geometry's record:
+  // floats 0-5 from C for the targets A, B, D, floats 6-11 from D for C) and
+  // their order for solve k
   const float2* mp = reinterpret_cast<const float2*>(sM) + 6 * cc + (k == 2 ? 3 : 0);
   const float2 p0 = mp[0], p1 = mp[1], p2 = mp[2];
-  const float v0 = p0.x, v1 = p0.y, v2 = p1.x, v3 = p1.y, v4 = p2.x, v5 = p2.y;
-  // the permuted arguments of solve k (solve_copy's four calls)
-  float a0, a1, a2, g0, g1, g2, g3, g4, g5, own;
-  if (k == 3) { a0 = TA; a1 = TB; a2 = TC; g0 = v0; g1 = v1; g2 = v2; g3 = v3; g4 = v4; g5 = v5; own = TD; }
-  else if (k == 0) { a0 = TB; a1 = TD; a2 = TC; g0 = v3; g1 = -v4; g2 = -v1; g3 = v5; g4 = v2; g5 = v0; own = TA; }
-  else if (k == 1) { a0 = TA; a1 = TD; a2 = TC; g0 = v0; g1 = -v2; g2 = -v1; g3 = v5; g4 = v4; g5 = v3; own = TB; }
-  else { a0 = TA; a1 = TB; a2 = TD; g0 = v0; g1 = v1; g2 = -v2; g3 = v3; g4 = -v4; g5 = v5; own = TC; }
+  const float aa = p0.x, ab = p0.y, ad = p1.x, bb = p1.y, bd = p2.x, dd = p2.y;
+  const bool k0 = k == 0, k1 = k == 1, lo = k < 2;
+  const float tp = k0 ? TB : TA, tq = lo ? TD : TB, tr = k == 2 ? TD : TC;
+  const float PP = k0 ? bb : aa, PQ = k0 ? bd : k1 ? ad : ab, PX = lo ? ab : ad;
+  const float QQ = lo ? dd : bb, QX = k0 ? ad : bd, XX = k0 ? aa : k1 ? bb : dd;
   float r;
   if constexpr (SOLVER == kPairWave) {
     // the target's height: component k of the copy's record, loaded alone
-    const float hD = reinterpret_cast<const float*>(sH)[4 * cc + k];
-    r = tet_solve_wave(a0, a1, a2, g0, g1, g2, g3, g4, g5, hD, sp.eps_h);
+    const float hX = reinterpret_cast<const float*>(sH)[4 * cc + k];
+    r = tet_solve_wave(tp, tq, tr, PP, PQ, PX, QQ, QX, XX, hX, sp.eps_h);
   } else {
     bool d = false;
-    r = tet_solve<float, SOLVER == kPairRefXdiv, false, false>(a0, a1, a2, g0, g1, g2, g3, g4, g5, sp.eps_h,
-                                                                sp.eps_h64, sp.largenum, 0.f, d, own);
+    r = tet_solve<float, SOLVER == kPairRefXdiv, false, false>(tp, tq, tr, PP, PQ, -PX, QQ, -QX, XX, sp.eps_h,
+                                                                sp.eps_h64, sp.largenum, 0.f, d);
   }
-  const float nw = fminf(own, r);
-  // the target's slab index: component k of the copy's connectivity
+  // the target's slab index: component k of the copy's connectivity.  An
+  // owned target's shared value is already at most the copy's
   const int tk = reinterpret_cast<const unsigned short*>(sC)[4 * cc + k];
-  if (tk < nvp) atomicMin(reinterpret_cast<int*>(&sT[tk]), __float_as_int(nw));
-  else reinterpret_cast<float*>(sR)[4 * cc + k] = nw;
+  if (tk < nvp) atomicMin(reinterpret_cast<int*>(&sT[tk]), __float_as_int(r));
+  else reinterpret_cast<float*>(sR)[4 * cc + k] = fminf(reinterpret_cast<const float*>(sTc)[4 * cc + k], r);
 }
 
 // Per-copy geometry of the two-copies-per-thread sweep, computed once per
-// mesh: the copy's metric terms (copy_metric) as three float4 -- ACAC ACBC
-// ACCD BCBC | BCCD CDCD ADAD ADBD | ADCD BDBD CDBD CDCD, so that floats 0-5
-// hold the six terms solves 0, 1 and 3 permute and floats 6-11 the six of
-// solve 2 -- and the heights of its four vertices over their opposite faces,
+// mesh: the dot products of the edge vectors from C to A, B, D (floats 0-5:
+// AA AB AD BB BD DD) and from D to A, B, C (floats 6-11) as three float4 --
+// copy_metric's terms, whose CD is -(D from C), with signs so that the four
+// solves only permute them -- and the heights of its four vertices over their opposite faces,
 // the same expressions the one-copy kernels evaluate per visit.
 __global__ void k_geometry(DevMesh m, float4* gm, float4* gh) {
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < m.full; c += stride) {
     float Mt[11];
     copy_metric<4>(m, c, Mt);
-    gm[3 * c] = make_float4(Mt[0], Mt[1], Mt[2], Mt[3]);
-    gm[3 * c + 1] = make_float4(Mt[4], Mt[5], Mt[6], Mt[7]);
+    gm[3 * c] = make_float4(Mt[0], Mt[1], -Mt[2], Mt[3]);
+    gm[3 * c + 1] = make_float4(-Mt[4], Mt[5], Mt[6], Mt[7]);
     gm[3 * c + 2] = make_float4(Mt[8], Mt[9], Mt[10], Mt[5]);
     const float ACAC = Mt[0], ACBC = Mt[1], ACCD = Mt[2], BCBC = Mt[3], BCCD = Mt[4], CDCD = Mt[5];
     const float ADAD = Mt[6], ADBD = Mt[7], BDBD = Mt[9];
@@ -1045,9 +1047,9 @@ __device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& 
       }
     // the copies' connectivity (the previous patch's last reads of sC came
     // before its final barrier) and flags, which only this thread reads:
-    // bits 8j .. 8j+3 the vertices of copy j that changed in the previous
-    // sweep (all on the first), bits 8j+4 .. 8j+7 its ghost vertices
-    unsigned flags = 0u;
+    // bits 0 .. 3 the vertices of copy j that changed in the previous
+    // sweep (all on the first), bits 4 .. 7 its ghost vertices
+    unsigned flags[2] = {0u, 0u};
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       const int c = tid + j * blockDim.x;
@@ -1056,7 +1058,7 @@ __device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& 
         sC[c] = cv;
         const unsigned ghost = (cv.x >= nvp ? 1u : 0u) | (cv.y >= nvp ? 2u : 0u) | (cv.z >= nvp ? 4u : 0u) |
                                (cv.w >= nvp ? 8u : 0u);
-        flags |= (0xFu | (ghost << 4)) << (8 * j);
+        flags[j] = 0xFu | (ghost << 4);
       }
     }
     if (tid == 0) {
@@ -1105,26 +1107,12 @@ __device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& 
         need[j] = 0u;
         // a copy none of whose values changed in the previous sweep lists
         // nothing: its flags are read first
-        const unsigned fl = (flags >> (8 * j)) & 0xFFu;  // zero past nep
-        if (fl & 0xFu) {
-          const float4 tv = sTc[c];
-          const float4 hv = sH[c];
-          const unsigned chg = fl & 0xFu, ghost = fl >> 4;
-          const float LN = sp.largenum;
-          const float m012 = fminf(fminf(tv.x, tv.y), tv.z), m013 = fminf(fminf(tv.x, tv.y), tv.w);
-          const float m023 = fminf(fminf(tv.x, tv.z), tv.w), m123 = fminf(fminf(tv.y, tv.z), tv.w);
-          unsigned cand = 0u;
-          if (chg & 0xEu) cand |= 1u;
-          if (chg & 0xDu) cand |= 2u;
-          if (chg & 0xBu) cand |= 4u;
-          if (chg & 0x7u) cand |= 8u;
-          cand &= (~ghost | allow_ghost) & 0xFu;
-          unsigned nd = 0u;
-          if (pair_may_lower<SOLVER>(cand & 1u, m123, hv.x, tv.x, LN)) nd |= 1u;
-          if (pair_may_lower<SOLVER>(cand & 2u, m023, hv.y, tv.y, LN)) nd |= 2u;
-          if (pair_may_lower<SOLVER>(cand & 4u, m013, hv.z, tv.z, LN)) nd |= 4u;
-          if (pair_may_lower<SOLVER>(cand & 8u, m012, hv.w, tv.w, LN)) nd |= 8u;
-          need[j] = nd;
+        const unsigned chg = flags[j] & 0xFu;  // zero past nep
+        if (chg) {
+          // a solve whose three inputs are unchanged repeats its result: with
+          // one changed vertex every solve but that vertex's own has one
+          const unsigned cand = (chg & (chg - 1u)) ? 0xFu : ~chg;
+          need[j] = pair_may_lower<SOLVER>(sTc[c], sH[c], sp.largenum) & cand & (~(flags[j] >> 4) | allow_ghost) & 0xFu;
         }
       }
       {
@@ -1170,17 +1158,8 @@ __device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& 
           for (int j = 0; j < 2; ++j) {
             const int c = tid + j * blockDim.x;
             if (c < nep) {
-              const float4 tv = sTc[c];
-              const float4 hv = sH[c];
-              const unsigned ghost = (flags >> (8 * j + 4)) & 0xFu;  // all four inputs count as changed
-              const float LN = sp.largenum;
-              const float m012 = fminf(fminf(tv.x, tv.y), tv.z), m013 = fminf(fminf(tv.x, tv.y), tv.w);
-              const float m023 = fminf(fminf(tv.x, tv.z), tv.w), m123 = fminf(fminf(tv.y, tv.z), tv.w);
-              unsigned nd = 0u;
-              if (pair_may_lower<SOLVER>(ghost & 1u, m123, hv.x, tv.x, LN)) nd |= 1u;
-              if (pair_may_lower<SOLVER>(ghost & 2u, m023, hv.y, tv.y, LN)) nd |= 2u;
-              if (pair_may_lower<SOLVER>(ghost & 4u, m013, hv.z, tv.z, LN)) nd |= 4u;
-              if (pair_may_lower<SOLVER>(ghost & 8u, m012, hv.w, tv.w, LN)) nd |= 8u;
+              // (all four inputs count as changed)
+              const unsigned nd = pair_may_lower<SOLVER>(sTc[c], sH[c], sp.largenum) & (flags[j] >> 4);
               need[j] |= nd;
               const int n = __popc(nd);
               if (n) {
@@ -1217,7 +1196,7 @@ __device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& 
           const unsigned chg = (nv.x != tv.x ? 1u : 0u) | (nv.y != tv.y ? 2u : 0u) | (nv.z != tv.z ? 4u : 0u) |
                                (nv.w != tv.w ? 8u : 0u);
           sTc[c] = nv;
-          flags = (flags & ~(0xFu << (8 * j))) | (chg << (8 * j));
+          flags[j] = (flags[j] & ~0xFu) | chg;
         }
       }
       // no barrier here: every thread refreshes only its own copies, and the
