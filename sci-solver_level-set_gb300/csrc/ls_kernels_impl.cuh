@@ -77,13 +77,21 @@ struct FimIter {
   int* next_n;      // and its sizes: [0] visits, [CTL_CANDS - CTL_VISITS] candidates
 };
 
-__device__ __forceinline__ FimIter fim_iter(const DevMesh& m, const DevState& s, int t) {
+// The view of stamp t, or, with rel, of stamp CTL_ITER + t.  The words come
+// through shared memory (all threads call it; a barrier): a word that every
+// thread of the grid loads is a queue of thousands of requests at one L2
+// sector (with 760 CTAs of 192 threads 3 us passed before the first list
+// entry was known, with 216 CTAs 1.1 us).
+__device__ __forceinline__ FimIter fim_iter(const DevMesh& m, const DevState& s, int t, bool rel) {
+  __shared__ int s_ctl[CTL_WORDS];
+  if (threadIdx.x < CTL_WORDS) s_ctl[threadIdx.x] = ld_relaxed(s.ctl + threadIdx.x);
+  __syncthreads();
   FimIter f;
-  const int cur = t % 3, nxt = cur == 2 ? 0 : cur + 1;
-  f.t = t;
-  f.base = ld_relaxed(s.ctl + CTL_BASE);
-  f.nvis = ld_relaxed(s.ctl + CTL_VISITS + cur);
-  f.count = f.nvis + ld_relaxed(s.ctl + CTL_CANDS + cur);
+  f.t = rel ? s_ctl[CTL_ITER] + t : t;
+  const int cur = f.t % 3, nxt = cur == 2 ? 0 : cur + 1;
+  f.base = s_ctl[CTL_BASE];
+  f.nvis = s_ctl[CTL_VISITS + cur];
+  f.count = f.nvis + s_ctl[CTL_CANDS + cur];
   f.list = s.lists + (size_t)cur * m.nparts;
   f.next = s.lists + (size_t)nxt * m.nparts;
   f.next_n = s.ctl + CTL_VISITS + nxt;
@@ -363,11 +371,12 @@ __device__ __forceinline__ void copy_metric(const DevMesh& m, long long c, float
 // instructions: with differently contracted FMAs the check could report a
 // drop of more than the tolerance that the visit never applies, and two
 // patches could re-activate each other without end.
-// t: the iteration's stamp; vb: the CTA's index in the patch assignment
-// (blockIdx.x, or the spread index of the persistent kernel)
+// vb: the CTA's index in the patch assignment (blockIdx.x, or the spread
+// index of the persistent kernel)
 template <int D1, bool XDIV, bool PREC>
-__device__ __forceinline__ void fim_copy_pass(const DevMesh& m, const DevState& s, const StepParams& sp, int t,
-                                              int vb) {
+__device__ __forceinline__ void fim_copy_pass(const DevMesh& m, const DevState& s, const StepParams& sp,
+                                              const FimIter& f, int vb) {
+  if (vb >= f.count) return;  // no entry for this CTA
   extern __shared__ float smem[];
   float* sT = smem;                       // owned + ghost values
   float* sOld = smem + sp.lvp + sp.lgp;   // owned values at the start of the last sweep
@@ -375,7 +384,7 @@ __device__ __forceinline__ void fim_copy_pass(const DevMesh& m, const DevState& 
   __shared__ int s_qn;  // deferred FP64 solves queued in this sweep (precision form)
   DeferredSolve* sQ = reinterpret_cast<DeferredSolve*>(smem + 2 * sp.lvp + sp.lgp);
   if (PREC && threadIdx.x == 0) s_qn = 0;
-  const FimIter f = fim_iter(m, s, t);
+  const int t = f.t;
   const int tid = threadIdx.x;
   FimCount cnt = {};
   int par = 0;
@@ -534,7 +543,7 @@ __device__ __forceinline__ void fim_copy_pass(const DevMesh& m, const DevState& 
 
 template <int D1, int MAXT, bool XDIV, int MINB, bool PREC>
 __global__ void __launch_bounds__(MAXT, MINB) k_fim(DevMesh m, DevState s, StepParams sp, int off) {
-  fim_copy_pass<D1, XDIV, PREC>(m, s, sp, s.ctl[CTL_ITER] + off, blockIdx.x);
+  fim_copy_pass<D1, XDIV, PREC>(m, s, sp, fim_iter(m, s, off, true), blockIdx.x);
 }
 
 // Patch assignment of the sweep kernels: CTA b takes list entry b first
@@ -578,8 +587,9 @@ __global__ void __launch_bounds__(MAXT, MINB) k_fim_compact(DevMesh m, DevState 
   __shared__ unsigned s_min[2];  // patch minimum, by parity of the CTA's patches
   __shared__ int s_n[2];  // listed solves, by sweep parity (reset one sweep ahead)
   __shared__ int s_li;    // list entry of the next patch
-  const int t = s.ctl[CTL_ITER] + off;
-  const FimIter f = fim_iter(m, s, t);
+  const FimIter f = fim_iter(m, s, off, true);
+  if ((int)blockIdx.x >= f.count) return;  // no entry for this CTA
+  const int t = f.t;
   FimCount cnt = {};
   int par = 0;
   const int tid = threadIdx.x;
@@ -970,8 +980,10 @@ __device__ __forceinline__ bool slab_wait(unsigned bar, unsigned parity, bool gi
 // the ghost targets; if it finds the patch unconverged, those are run from
 // the same sweep-start values and the visit goes on.
 template <int SOLVER>
-__device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& s, const StepParams& sp, int t,
-                                              int vb) {
+__device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& s, const StepParams& sp,
+                                              const FimIter& f, int vb) {
+  if (vb >= f.count) return;  // no entry for this CTA
+  const int t = f.t;
   extern __shared__ float4 smem4[];
   float* sT = reinterpret_cast<float*>(smem4);  // owned + ghost values
   float* sOld = sT + sp.lvp + sp.lgp;          // owned values at the start of the last sweep
@@ -990,7 +1002,6 @@ __device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& 
   __shared__ __align__(8) unsigned long long s_bar;  // geometry slab copies of the current patch
   __shared__ int s_err;  // a slab wait ran out: the pass ends
   __shared__ FimCount s_cnt;  // thread 0's work counters (in shared memory for their registers)
-  const FimIter f = fim_iter(m, s, t);
   const int tid = threadIdx.x;
   const unsigned bar = smem_u32addr(&s_bar);
   unsigned phase = 0;      // thread 0: parity of the slab copies' current phase
@@ -1265,7 +1276,7 @@ __host__ __device__ constexpr int pair_minb(int setting) { return setting == 7 ?
 template <int SETTING, int SOLVER>
 __global__ void __launch_bounds__(pair_maxt(SETTING), pair_minb(SETTING))
     k_fim_pair(DevMesh m, DevState s, StepParams sp, int off) {
-  fim_pair_pass<SOLVER>(m, s, sp, s.ctl[CTL_ITER] + off, blockIdx.x);
+  fim_pair_pass<SOLVER>(m, s, sp, fim_iter(m, s, off, true), blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -1392,7 +1403,7 @@ __device__ __forceinline__ void fim_loop_persistent(const DevMesh& m, const DevS
     }
     // above every stamp this iteration uses, also if the launch is abandoned
     if (blockIdx.x == 0 && threadIdx.x == 0) s.ctl[CTL_ITER] = t + 1;
-    pass(t, vb);
+    pass(fim_iter(m, s, t, false), vb);
     if (!grid_sync(s, sp, epoch)) return;
   }
 }
@@ -1400,12 +1411,12 @@ __device__ __forceinline__ void fim_loop_persistent(const DevMesh& m, const DevS
 template <int SETTING, int SOLVER>
 __global__ void __launch_bounds__(pair_maxt(SETTING), pair_minb(SETTING))
     k_fim_pair_persist(DevMesh m, DevState s, StepParams sp) {
-  fim_loop_persistent(m, s, sp, [&](int t, int vb) { fim_pair_pass<SOLVER>(m, s, sp, t, vb); });
+  fim_loop_persistent(m, s, sp, [&](const FimIter& f, int vb) { fim_pair_pass<SOLVER>(m, s, sp, f, vb); });
 }
 
 template <int D1, int MAXT, bool XDIV, int MINB, bool PREC>
 __global__ void __launch_bounds__(MAXT, MINB) k_fim_persist(DevMesh m, DevState s, StepParams sp) {
-  fim_loop_persistent(m, s, sp, [&](int t, int vb) { fim_copy_pass<D1, XDIV, PREC>(m, s, sp, t, vb); });
+  fim_loop_persistent(m, s, sp, [&](const FimIter& f, int vb) { fim_copy_pass<D1, XDIV, PREC>(m, s, sp, f, vb); });
 }
 
 // Narrowband (K14) fused with the sign recovery (K10b) and the vertex-update
@@ -1437,11 +1448,14 @@ __global__ void k_narrowband(DevMesh m, DevState s, StepParams sp) {
       npc += 1;
     }
   }
-  atomicAdd(&s_cnt, (unsigned long long)cnt);
-  if (lane == 0) { atomicAdd(&s_pv, (unsigned long long)pv); atomicAdd(&s_np, (unsigned long long)npc); }
+  cnt = __reduce_add_sync(0xffffffffu, cnt);
+  if (lane == 0 && cnt) atomicAdd(&s_cnt, (unsigned long long)cnt);
+  if (lane == 0 && npc) { atomicAdd(&s_pv, (unsigned long long)pv); atomicAdd(&s_np, (unsigned long long)npc); }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    atomicAdd(&s.stats[2], s_cnt);
+  // most CTAs hold no narrowband patch: same-address atomics are served one
+  // after another
+  if (threadIdx.x == 0 && s_cnt) atomicAdd(&s.stats[2], s_cnt);
+  if (threadIdx.x == 0 && s_np) {
     atomicAdd(&s.stats[3], s_pv);
     atomicAdd(&s.stats[4], s_np);
   }
@@ -2293,7 +2307,7 @@ cudaError_t configure_launch(const DevMesh& m, const StepParams& sp, Launch& L) 
   if (occ < 1) occ = 1;
   // no more CTAs than patches: a small mesh's launches are short
   L.fim_grid = std::min(L.sms * occ, m.nparts);
-  L.seed_grid = L.sms * 8;
+  L.seed_grid = std::min(L.sms * 8, m.nparts);
   L.upd_block = L.fim_block > 512 ? 512 : L.fim_block;
   const int slab = sp.lvp + sp.lgp;
   L.upd_smem = (int)sizeof(float) * (slab * (m.dim == 3 ? 4 : 1) + sp.lep * 16);
@@ -2309,9 +2323,9 @@ cudaError_t configure_launch(const DevMesh& m, const StepParams& sp, Launch& L) 
   }
   if (e != cudaSuccess) return e;
   if (occ < 1) occ = 1;
-  L.upd_grid = L.sms * occ;
-  L.warp_grid = L.sms * 8;
-  L.flat_grid = L.sms * 8;
+  L.upd_grid = std::min(L.sms * occ, m.nparts);
+  L.warp_grid = std::min(L.sms * 8, (m.nparts + 7) / 8);   // 8 warps, one patch each
+  L.flat_grid = std::min(L.sms * 8, (m.nv + 255) / 256);
   return configure_persistent(m, sp, L);
 }
 
