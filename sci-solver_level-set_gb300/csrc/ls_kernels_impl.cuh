@@ -367,6 +367,14 @@ __device__ __forceinline__ void copy_metric(const DevMesh& m, long long c, float
   }
 }
 
+// The sweep of k_fim: one element copy per thread.  The owned values live in
+// two buffers: a sweep reads its copies' registers and takes the minima into
+// one buffer, the next sweep into the other, so that one barrier separates
+// them, and a visit's last sweep leaves the values it started from in the
+// other buffer for the convergence test.  Every copy adds its present values
+// to the minima too, so a buffer needs no refresh from the other.  A sweep in
+// which no copy lowered anything ends the visit: the remaining ones would
+// change nothing, and the convergence test sees no drop, as after them.
 // A candidate's check is the first sweep of its visit, run by the same
 // instructions: with differently contracted FMAs the check could report a
 // drop of more than the tolerance that the visit never applies, and two
@@ -378,8 +386,8 @@ __device__ __forceinline__ void fim_copy_pass(const DevMesh& m, const DevState& 
                                               const FimIter& f, int vb) {
   if (vb >= f.count) return;  // no entry for this CTA
   extern __shared__ float smem[];
-  float* sT = smem;                       // owned + ghost values
-  float* sOld = smem + sp.lvp + sp.lgp;   // owned values at the start of the last sweep
+  float* const buf0 = smem;                      // owned + ghost values at the start, then odd sweeps' minima
+  float* const buf1 = smem + sp.lvp + sp.lgp;    // even sweeps' minima
   __shared__ unsigned s_min[2];           // patch minimum, by parity of the CTA's patches
   __shared__ int s_qn;  // deferred FP64 solves queued in this sweep (precision form)
   DeferredSolve* sQ = reinterpret_cast<DeferredSolve*>(smem + 2 * sp.lvp + sp.lgp);
@@ -397,14 +405,20 @@ __device__ __forceinline__ void fim_copy_pass(const DevMesh& m, const DevState& 
     const int slot = s.slot[p] ^ 1;
     int niter = visit ? sp.niter : 1;
     if (tid == 0) (visit ? cnt.visits : cnt.checks)++;
-    for (int i = tid; i < nvp + ngp; i += blockDim.x)
-      sT[i] = dt_before(s.cell[i < nvp ? vs + i : __ldg(m.ghost_ids + gs + i - nvp)], t, f.base, sp.largenum);
+    for (int i = tid; i < nvp + ngp; i += blockDim.x) {
+      const float d = dt_before(s.cell[i < nvp ? vs + i : __ldg(m.ghost_ids + gs + i - nvp)], t, f.base, sp.largenum);
+      buf0[i] = d;
+      if (i < nvp) buf1[i] = d;
+    }
     if (tid == 0) s_min[par] = 0x7f800000u;
     __syncthreads();
     const bool act = tid < nep;
     int idx[4] = {0, 0, 0, 0};
     float T[4] = {0.f, 0.f, 0.f, 0.f};
+    // the fast build's triangles use the planar-wave form
+    constexpr bool WAVE = kLbSkip && D1 == 3;
     float Mt[11];
+    TriGeo tg;
     int nflag = 0;
     // corners whose value is the vertex's: owned, and within the reference's
     // per-vertex slot limit where that applies (others stay private)
@@ -417,15 +431,22 @@ __device__ __forceinline__ void fim_copy_pass(const DevMesh& m, const DevState& 
       for (int k = 0; k < D1; ++k)
         if (idx[k] < nvp && !((capm >> k) & 1u)) shared_k |= 1u << k;
 #pragma unroll
-      for (int k = 0; k < D1; ++k) T[k] = sT[idx[k]];
-      copy_metric<D1>(m, (long long)es + tid, Mt);
+      for (int k = 0; k < D1; ++k) T[k] = buf0[idx[k]];
+      if constexpr (WAVE) {
+        const long long c = (long long)es + tid;
+        tg = tri_geo(__ldg(m.lc + c), __ldg(m.lc + m.full + c), __ldg(m.lc + 2 * m.full + c));
+      } else {
+        copy_metric<D1>(m, (long long)es + tid, Mt);
+      }
     }
+    float* sT = buf0;    // minima of the last sweep
+    float* sOld = buf1;  // owned values at its start
 #pragma unroll 1
     for (int it = 0; it < niter; ++it) {
-      if (it == niter - 1) {
-        for (int i = tid; i < nvp; i += blockDim.x) sOld[i] = sT[i];
-        __syncthreads();
-      }
+      float* const w = sOld;
+      sOld = sT;
+      sT = w;
+      bool low = false;  // this copy lowers a value
       int qpos[4] = {-1, -1, -1, -1};
       if (act) {
         float nw[4];
@@ -452,16 +473,21 @@ __device__ __forceinline__ void fim_copy_pass(const DevMesh& m, const DevState& 
             }
             nw[k] = fminf(T[k], rr[k]);
           }
+        } else if constexpr (WAVE) {
+          nw[0] = fminf(T[0], tri_solve_wave<0>(tg, T));
+          nw[1] = fminf(T[1], tri_solve_wave<1>(tg, T));
+          nw[2] = fminf(T[2], tri_solve_wave<2>(tg, T));
         } else {
           solve_copy<D1, XDIV>(Mt, T, nw, sp.eps_h, sp.eps_h64, sp.largenum);
         }
 #pragma unroll
         for (int k = 0; k < D1; ++k) {
+          low |= nw[k] < T[k];
           if ((shared_k >> k) & 1u) atomicMin(reinterpret_cast<int*>(&sT[idx[k]]), __float_as_int(nw[k]));
           else T[k] = nw[k];
         }
       }
-      __syncthreads();
+      const bool any = __syncthreads_or(low);
       if constexpr (PREC && D1 == 4) {
         const int nq = min(s_qn, kDeferCap);
         for (int i = tid; i < nq; i += blockDim.x) {
@@ -504,8 +530,13 @@ __device__ __forceinline__ void fim_copy_pass(const DevMesh& m, const DevState& 
           cnt.visits++;
           cnt.bytes += (unsigned long long)(__ldg(m.patch_bytes + p) - 4 * nvp);
         }
+      } else if (PREC) {
+        __syncthreads();  // the queue's reset and results, before the next sweep fills it
+      } else if (!any) {
+        // (the precision form counts its repeats in every sweep, so it runs them all)
+        sOld = sT;
+        break;
       }
-      __syncthreads();
     }
     // a check that found nothing writes nothing
     int con = 1;
