@@ -108,7 +108,7 @@ constexpr int kStampLimit = 1 << 29;
 // Device step state.
 struct DevState {
   float* phi;
-  float* phi_out;
+  float* phi_rd;    // phi after the redistance, before the update
   DtCell* cell;     // per vertex: FIM distance
   int* slot;        // per patch: the half of its vertices' cells that its last visit wrote
   // per patch, stamps: 2t = in the list of iteration t and not done with it,

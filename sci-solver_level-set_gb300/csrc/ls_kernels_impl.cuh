@@ -26,9 +26,7 @@
 //     per thread, the default for patches of up to 384 copies).
 //   k_narrowband   patch narrowband, phi := sign * DT, vertex-update count (K14 + K10b)
 //   k_update       advection (K16) or mean-curvature update on narrowband patches
-//                  (k_update_384: the same for patches of up to 384 copies,
-//                  three CTAs per SM)
-//   k_copy_phi     phi := phi_out on narrowband patches (K15)
+//   k_copy_phi     phi_rd := phi there, between inside iterations (K15)
 //   k_unpermute    phi in the caller's vertex order (K18)
 //
 // Patch visits read a contiguous slab: owned vertex values [vs, ve) plus a
@@ -188,9 +186,15 @@ __device__ __forceinline__ void fim_count_flush(const DevState& s, const FimIter
 
 // Seed search (redistance_kernels3d.h:623-770): an element copy whose
 // vertex values include an exact zero or differ in sign marks those
-// vertices as seeds with DT = |phi|; the patch joins list0.
+// vertices as seeds with DT = |phi|; the patch joins the first list.
+// The patch's phi is staged in shared memory once (a copy's four gathers
+// through ghost ids were the kernel), and a patch whose values have one sign
+// and no zero has no such copy: its connectivity is not read.  128^3 step:
+// 21.7 us before.
+constexpr int kSeedBlock = 128;
 template <int D1>
-__global__ void k_seed(DevMesh m, DevState s, float scale, int warm) {
+__global__ void __launch_bounds__(kSeedBlock) k_seed(DevMesh m, DevState s, StepParams sp, int warm) {
+  extern __shared__ float smem[];
   const int nprev = s.ctl[CTL_NB_PREV];
   const int base = s.ctl[CTL_BASE], t0 = s.ctl[CTL_ITER];
   int* list = s.lists + (size_t)(t0 % 3) * m.nparts;
@@ -198,30 +202,39 @@ __global__ void k_seed(DevMesh m, DevState s, float scale, int warm) {
   const int count = nprev ? nprev : m.nparts;
   for (int li = blockIdx.x; li < count; li += gridDim.x) {
     const int p = nprev ? s.nblist[li] : li;
-    const float sc = m.patch_mesh ? __ldg(&m.mesh_par[m.patch_mesh[p]]).y : scale;
     const int vs = m.vert_off[p], nvp = m.vert_off[p + 1] - vs;
-    const int gs = m.ghost_off[p];
+    const int gs = m.ghost_off[p], ngp = m.ghost_off[p + 1] - gs;
     const int es = m.ele_off[p], nep = m.ele_off[p + 1] - es;
+    // bit 0: a value not <= 0, bit 1: one not >= 0, bit 2: a zero
+    int seen = 0;
+    for (int i = threadIdx.x; i < nvp + ngp; i += blockDim.x) {
+      const float v = s.phi[i < nvp ? vs + i : m.ghost_ids[gs + i - nvp]];
+      smem[i] = v;
+      seen |= (v <= 0.f ? 0 : 1) | (v >= 0.f ? 0 : 2) | (v == 0.f ? 4 : 0);
+    }
+    const bool pos = __syncthreads_or(seen & 1), neg = __syncthreads_or(seen & 2), zero = __syncthreads_or(seen & 4);
     int found = 0;
-    for (int c = threadIdx.x; c < nep; c += blockDim.x) {
-      const ushort4 cv = m.conn[es + c];
-      const int idx[4] = {cv.x, cv.y, cv.z, cv.w};
-      int gv[D1];
-      float val[D1];
-      bool allpos = true, allneg = true;
+    if ((pos && neg) || zero) {
+      const float sc = m.patch_mesh ? __ldg(&m.mesh_par[m.patch_mesh[p]]).y : sp.scale;
+      for (int c = threadIdx.x; c < nep; c += blockDim.x) {
+        const ushort4 cv = m.conn[es + c];
+        const int idx[4] = {cv.x, cv.y, cv.z, cv.w};
+        float val[D1];
+        bool allpos = true, allneg = true;
 #pragma unroll
-      for (int k = 0; k < D1; ++k) {
-        gv[k] = idx[k] < nvp ? vs + idx[k] : m.ghost_ids[gs + idx[k] - nvp];
-        val[k] = s.phi[gv[k]];
-        allpos &= (val[k] >= 0.f);
-        allneg &= (val[k] <= 0.f);
-      }
-      const bool cross = !(allpos || allneg);
+        for (int k = 0; k < D1; ++k) {
+          val[k] = smem[idx[k]];
+          allpos &= (val[k] >= 0.f);
+          allneg &= (val[k] <= 0.f);
+        }
+        const bool cross = !(allpos || allneg);
 #pragma unroll
-      for (int k = 0; k < D1; ++k) {
-        if (cross || val[k] == 0.f) {
-          *reinterpret_cast<int2*>(s.cell + gv[k]) = make_int2(__float_as_int(fabsf(val[k]) / sc), base);
-          found = 1;
+        for (int k = 0; k < D1; ++k) {
+          if (cross || val[k] == 0.f) {
+            const int gv = idx[k] < nvp ? vs + idx[k] : m.ghost_ids[gs + idx[k] - nvp];
+            *reinterpret_cast<int2*>(s.cell + gv) = make_int2(__float_as_int(fabsf(val[k]) / sc), base);
+            found = 1;
+          }
         }
       }
     }
@@ -1451,8 +1464,11 @@ __global__ void __launch_bounds__(MAXT, MINB) k_fim_persist(DevMesh m, DevState 
 }
 
 // Narrowband (K14) fused with the sign recovery (K10b) and the vertex-update
-// count: one warp per patch over every patch.
-__global__ void k_narrowband(DevMesh m, DevState s, StepParams sp) {
+// count: one warp per patch over every patch.  The redistanced phi goes to
+// phi_rd; outside the narrowband (or with no update, last != 0) it is the
+// step's result and goes to phi too.  The update then reads phi_rd and
+// writes phi, so that no copy pass follows it.
+__global__ void k_narrowband(DevMesh m, DevState s, StepParams sp, int last) {
   __shared__ unsigned long long s_cnt, s_pv, s_np;
   if (threadIdx.x == 0) { s_cnt = 0; s_pv = 0; s_np = 0; }
   __syncthreads();
@@ -1469,10 +1485,13 @@ __global__ void k_narrowband(DevMesh m, DevState s, StepParams sp) {
       mn = min(mn, __float_as_uint(d));
       cnt += (d <= pp.bw);
       const float mag = (d >= sp.largenum || pp.scale == 1.f) ? d : d * pp.scale;
-      s.phi[v] = s.phi[v] < 0.f ? -mag : mag;  // the sign phi had before the redistance
+      s.phi_rd[v] = s.phi[v] < 0.f ? -mag : mag;  // the sign phi had before the redistance
     }
     mn = __reduce_min_sync(0xffffffffu, mn);
-    if (lane == 0 && __uint_as_float(mn) <= pp.bw) {
+    const bool nb = __uint_as_float(mn) <= pp.bw;
+    if (!nb || last)
+      for (int v = vs + lane; v < ve; v += 32) s.phi[v] = s.phi_rd[v];
+    if (lane == 0 && nb) {
       const int pos = atomicAdd(s.ctl + CTL_NB, 1);
       s.nblist[pos] = p;
       pv += ve - vs;
@@ -1497,19 +1516,39 @@ __global__ void k_narrowband(DevMesh m, DevState s, StepParams sp) {
 // meshFIM2d_kernels.h:37-362) or mean curvature (meshFIM3d.cu:103-267 in the
 // reference form, or the lumped-mass form).  One CTA per patch; per-copy
 // contributions go to shared memory, each owned vertex sums its slots in the
-// reference order.
+// reference order.  KIND is a template parameter, so that a copy computes and
+// stores only what its update sums: a record of two float4 (advection: aH,
+// aV; curvature: curv, then volume and volume-weighted gradient), and aV too
+// where the reference's curvature gate needs it.  Blocks of 128 threads, many
+// per SM: while one patch's few owned vertices sum their slots (a serial
+// chain of about 24), other patches' copies compute.  128^3 curvature: 42 us
+// (79 us with 352 threads, every quantity computed and a copy pass after it;
+// this kernel with 384 threads: 71 us, and no faster on 163 patches).
+enum { UPD_ADVECT = 0, UPD_CURVATURE = 1, UPD_CURVATURE_REF = 2 };
+constexpr int kUpdBlock = 128;
+// float4 of a copy's record
+__host__ __device__ constexpr int upd_record(int kind) { return kind == UPD_CURVATURE_REF ? 3 : 2; }
 struct Contrib {
   float aH[4], aV[4], curv[4], vol, g0, g1, g2;
 };
 
-template <int D1>
+// 1 / x for the quotients by one divisor (fast build: one reciprocal and
+// products; the bit-exact build divides each as the reference does)
+template <typename T>
+struct Divisor {
+  T x;
+  __device__ __forceinline__ explicit Divisor(T d) : x(kLbSkip ? T(1) / d : d) {}
+  __device__ __forceinline__ T operator()(T a) const { return kLbSkip ? a * x : a / x; }
+};
+
+template <int D1, int KIND>
 __device__ __forceinline__ void update_copy(const DevMesh& m, const StepParams& sp, long long c,
                                             long long c_first, const float* sPhi, const float* sX,
                                             int nslab, const int idx[4], Contrib& o) {
 #pragma unroll
   for (int k = 0; k < 4; ++k) { o.aH[k] = 0.f; o.aV[k] = 0.f; o.curv[k] = 0.f; }
   o.vol = 0.f; o.g0 = 0.f; o.g1 = 0.f; o.g2 = 0.f;
-  const bool curvature = sp.update_kind == 1;
+  constexpr bool curvature = KIND != UPD_ADVECT;
   float e[4];
 #pragma unroll
   for (int k = 0; k < D1; ++k) e[k] = sPhi[idx[k]];
@@ -1582,10 +1621,11 @@ __device__ __forceinline__ void update_copy(const DevMesh& m, const StepParams& 
     const float b14 = a12 * a33 + a13 * a22 + a23 * a32 - a12 * a23 - a13 * a32 - a22 * a33;
     const float b24 = a11 * a23 + a13 * a31 + a21 * a33 - a11 * a33 - a13 * a21 - a23 * a31;
     const float b34 = a11 * a32 + a12 * a21 + a22 * a31 - a11 * a22 - a12 * a31 - a21 * a32;
-    float nN[4][3] = {{b11 / det, b21 / det, b31 / det},
-                      {b12 / det, b22 / det, b32 / det},
-                      {b13 / det, b23 / det, b33 / det},
-                      {b14 / det, b24 / det, b34 / det}};
+    const Divisor<float> over_det(det);
+    float nN[4][3] = {{over_det(b11), over_det(b21), over_det(b31)},
+                      {over_det(b12), over_det(b22), over_det(b32)},
+                      {over_det(b13), over_det(b23), over_det(b33)},
+                      {over_det(b14), over_det(b24), over_det(b34)}};
     float gp0 = 0.f, gp1 = 0.f, gp2 = 0.f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -1594,51 +1634,59 @@ __device__ __forceinline__ void update_copy(const DevMesh& m, const StepParams& 
       gp2 += nN[i][2] * e[i];
     }
     const float absg = sqrtf(gp0 * gp0 + gp1 * gp1 + gp2 * gp2);
-    float sg0, sg1, sg2;
-    if (curvature) {
-      sg0 = 1.f; sg1 = 0.f; sg2 = 1.f;
-    } else {
-      const long long cs = sp.ref_compat ? c_first : c;
-      sg0 = __ldg(m.sig + cs); sg1 = __ldg(m.sig + m.full + cs); sg2 = __ldg(m.sig + 2 * m.full + cs);
-    }
-    float K[4], Kp[4], Km[4], H = 0.f, beta = 0.f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      K[i] = volume * (sg0 * nN[i][0] + sg1 * nN[i][1] + sg2 * nN[i][2]);
-      H += K[i] * e[i];
-      Kp[i] = fmaxf(K[i], 0.f);
-      Km[i] = fminf(K[i], 0.f);
-      beta += Km[i];
-    }
-    beta = 1.0f / beta;
-    const bool hpass = (double)fabsf(H) > (curvature ? 1e-16 : 1e-8);
-    float at[4] = {0.f, 0.f, 0.f, 0.f};
-    if (hpass) {
-      float alpha[4], theta = 0.f;
+    bool hpass = true;
+    if constexpr (KIND != UPD_CURVATURE) {
+      float sg0, sg1, sg2;
+      if constexpr (curvature) {
+        sg0 = 1.f; sg1 = 0.f; sg2 = 1.f;
+      } else {
+        const long long cs = sp.ref_compat ? c_first : c;
+        sg0 = __ldg(m.sig + cs); sg1 = __ldg(m.sig + m.full + cs); sg2 = __ldg(m.sig + 2 * m.full + cs);
+      }
+      float K[4], Kp[4], Km[4], H = 0.f, beta = 0.f;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float d = Kp[i] * beta *
-                        (Km[0] * (e[i] - e[0]) + Km[1] * (e[i] - e[1]) + Km[2] * (e[i] - e[2]) + Km[3] * (e[i] - e[3]));
-        alpha[i] = d / H;
-        theta += fmaxf(0.f, alpha[i]);
+        K[i] = volume * (sg0 * nN[i][0] + sg1 * nN[i][1] + sg2 * nN[i][2]);
+        H += K[i] * e[i];
+        Kp[i] = fmaxf(K[i], 0.f);
+        Km[i] = fminf(K[i], 0.f);
+        beta += Km[i];
+      }
+      beta = 1.0f / beta;
+      // |H| > 1e-16, |H| > 1e-8 as the reference compares them, in double:
+      // the nearest floats lie above and below those numbers
+      hpass = curvature ? fabsf(H) >= 1e-16f : fabsf(H) > 1e-8f;
+      float at[4] = {0.f, 0.f, 0.f, 0.f};
+      if (hpass) {
+        float alpha[4], theta = 0.f;
+        const Divisor<float> over_h(H);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float d = Kp[i] * beta *
+                          (Km[0] * (e[i] - e[0]) + Km[1] * (e[i] - e[1]) + Km[2] * (e[i] - e[2]) + Km[3] * (e[i] - e[3]));
+          alpha[i] = over_h(d);
+          theta += fmaxf(0.f, alpha[i]);
+        }
+        const Divisor<float> over_theta(theta);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) at[i] = over_theta(fmaxf(alpha[i], 0.f));
       }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) at[i] = fmaxf(alpha[i], 0.f) / theta;
+      for (int i = 0; i < 4; ++i) { o.aH[i] = at[i] * H; o.aV[i] = at[i] * volume; }
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { o.aH[i] = at[i] * H; o.aV[i] = at[i] * volume; }
-    if (curvature) {
-      const bool gate = sp.ref_compat ? hpass : (absg > 0.f);
+    if constexpr (curvature) {
+      const bool gate = KIND == UPD_CURVATURE_REF ? hpass : (absg > 0.f);
       if (gate) {
         o.vol = volume;
         o.g0 = volume * gp0; o.g1 = volume * gp1; o.g2 = volume * gp2;
+        const Divisor<float> over_absg(absg);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           float acc = 0.f;
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const int jj = (i + j) & 3;
-            acc += (nN[i][0] * nN[jj][0] + nN[i][1] * nN[jj][1] + nN[i][2] * nN[jj][2]) / absg * e[jj];
+            acc += over_absg(nN[i][0] * nN[jj][0] + nN[i][1] * nN[jj][1] + nN[i][2] * nN[jj][2]) * e[jj];
           }
           o.curv[i] = volume * acc;
         }
@@ -1677,7 +1725,7 @@ __device__ __forceinline__ void update_copy(const DevMesh& m, const StepParams& 
       // below are formed in every case, as in the reference
       // (meshFIM2d_kernels.h:198-236): a non-finite H then reaches the sums
       float at[3] = {0.f, 0.f, 0.f};
-      if ((double)fabsf(H) > 1e-8) {
+      if (fabsf(H) > 1e-8f) {  // the double comparison with 1e-8, see above
         float alpha[3], theta = 0.f;
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
@@ -1710,15 +1758,14 @@ __device__ __forceinline__ void update_copy(const DevMesh& m, const StepParams& 
   }
 }
 
-template <int D1>
-__device__ __forceinline__ void update_patches(const DevMesh& m, const DevState& s, const StepParams& sp) {
-  extern __shared__ float smem[];
-  const int slab = sp.lvp + sp.lgp;
-  float* sPhi = smem;                // slab
-  float* sX = smem + slab;           // 3 * slab (3D only)
-  float* sC = sX + (D1 == 4 ? 3 * slab : 0);  // per copy: aH[4] aV[4] curv[4] vol g0 g1 g2
-  const bool curvature = sp.update_kind == 1;
-  const int stride = 15;
+template <int D1, int KIND>
+__global__ void __launch_bounds__(kUpdBlock, 8) k_update(DevMesh m, DevState s, StepParams sp) {
+  extern __shared__ float4 smem4[];
+  constexpr int REC = upd_record(KIND);
+  constexpr bool curvature = KIND != UPD_ADVECT;
+  float4* sC = smem4;                                          // [lep][REC]
+  float* sPhi = reinterpret_cast<float*>(smem4 + REC * sp.lep);  // slab
+  float* sX = sPhi + sp.lvp + sp.lgp;                          // 3 * slab (3D only)
   const int count = s.ctl[CTL_NB];
   for (int li = blockIdx.x; li < count; li += gridDim.x) {
     const int p = s.nblist[li];
@@ -1729,7 +1776,7 @@ __device__ __forceinline__ void update_patches(const DevMesh& m, const DevState&
     const int nslab = nvp + ngp;
     for (int i = threadIdx.x; i < nslab; i += blockDim.x) {
       const int v = i < nvp ? vs + i : __ldg(m.ghost_ids + gs + i - nvp);
-      sPhi[i] = s.phi[v];
+      sPhi[i] = s.phi_rd[v];
       if (D1 == 4) {
         sX[i] = __ldg(m.xyz + v);
         sX[nslab + i] = __ldg(m.xyz + m.nv + v);
@@ -1741,13 +1788,16 @@ __device__ __forceinline__ void update_patches(const DevMesh& m, const DevState&
       const ushort4 cv = m.conn[es + c];
       const int idx[4] = {cv.x, cv.y, cv.z, D1 == 4 ? cv.w : 0};
       Contrib o;
-      update_copy<D1>(m, sp, (long long)es + c, es, sPhi, sX, nslab, idx, o);
-      float* dst = sC + (size_t)c * stride;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) { dst[k] = o.aH[k]; dst[4 + k] = o.aV[k]; dst[8 + k] = o.curv[k]; }
-      dst[12] = o.vol; dst[13] = o.g0; dst[14] = o.g1;
-      // g2 packed separately below the copies
-      sC[(size_t)nep * stride + c] = o.g2;
+      update_copy<D1, KIND>(m, sp, (long long)es + c, es, sPhi, sX, nslab, idx, o);
+      float4* dst = sC + (size_t)c * REC;
+      if constexpr (curvature) {
+        dst[0] = make_float4(o.curv[0], o.curv[1], o.curv[2], o.curv[3]);
+        dst[1] = make_float4(o.vol, o.g0, o.g1, o.g2);
+        if constexpr (REC > 2) dst[2] = make_float4(o.aV[0], o.aV[1], o.aV[2], o.aV[3]);
+      } else {
+        dst[0] = make_float4(o.aH[0], o.aH[1], o.aH[2], o.aH[3]);
+        dst[1] = make_float4(o.aV[0], o.aV[1], o.aV[2], o.aV[3]);
+      }
     }
     __syncthreads();
     for (int i = threadIdx.x; i < nvp; i += blockDim.x) {
@@ -1758,63 +1808,65 @@ __device__ __forceinline__ void update_patches(const DevMesh& m, const DevState&
       const int b = (m.capped && !curvature) ? min(m.vslot_off[v + 1], a + m.slot_cap) : m.vslot_off[v + 1];
       const float oldT = sPhi[i];
       float res = oldT;
-      if (!curvature) {
+      if constexpr (!curvature) {
         float up = 0.f, down = 0.f;
+#pragma unroll 4
         for (int q = a; q < b; ++q) {
           const int sl = m.vslot[q];
-          up += sC[(sl >> 2) * stride + (sl & 3)];
+          const float* src = reinterpret_cast<const float*>(sC + (size_t)(sl >> 2) * REC) + (sl & 3);
+          up += src[0];
+          down += src[4];
         }
-        for (int q = a; q < b; ++q) {
-          const int sl = m.vslot[q];
-          down += sC[(sl >> 2) * stride + 4 + (sl & 3)];
-        }
-        if ((double)fabsf(down) > 1e-8) res = oldT - pp.dt * (up / down);
+        if (fabsf(down) > 1e-8f) res = oldT - pp.dt * (up / down);
       } else {
         float down = 0.f, gd = 0.f, g0 = 0.f, g1 = 0.f, g2 = 0.f, cu = 0.f;
+#pragma unroll 4
         for (int q = a; q < b; ++q) {
           const int sl = m.vslot[q];
-          const float* src = sC + (sl >> 2) * stride;
-          down += src[4 + (sl & 3)];
-          g0 += src[13];
-          g1 += src[14];
-          g2 += sC[(size_t)nep * stride + (sl >> 2)];
-          gd += src[12];
-          cu += src[8 + (sl & 3)];
+          const float4* rec = sC + (size_t)(sl >> 2) * REC;
+          const float4 gv = rec[1];
+          g0 += gv.y;
+          g1 += gv.z;
+          g2 += gv.w;
+          gd += gv.x;
+          cu += reinterpret_cast<const float*>(rec)[sl & 3];
+          if constexpr (REC > 2) down += reinterpret_cast<const float*>(rec + 2)[sl & 3];
         }
         const float node_eik = sqrtf(g0 * g0 + g1 * g1 + g2 * g2) / gd;
-        if (sp.ref_compat && D1 == 4) {
-          if ((double)fabsf(down) > 1e-16) res = oldT - pp.cc * node_eik * (cu / gd) * pp.dt;
+        if constexpr (KIND == UPD_CURVATURE_REF) {
+          if (fabsf(down) >= 1e-16f) res = oldT - pp.cc * node_eik * (cu / gd) * pp.dt;
         } else if (gd > 0.f) {
           // the reference's normalisation (curv_up / sum of element volumes)
           res = oldT - pp.cc * node_eik * (cu / gd) * pp.dt;
         }
       }
-      s.phi_out[v] = res;
+      s.phi[v] = res;
     }
     __syncthreads();
   }
 }
 
-template <int D1>
-__global__ void __launch_bounds__(512) k_update(DevMesh m, DevState s, StepParams sp) {
-  update_patches<D1>(m, s, sp);
+// The update of the mesh's dimension and the step's kind (the reference's
+// curvature form exists for tetrahedra only).
+inline const void* update_kernel(const DevMesh& m, const StepParams& sp) {
+  if (m.dim == 2)
+    return sp.update_kind == 1 ? (const void*)k_update<3, UPD_CURVATURE> : (const void*)k_update<3, UPD_ADVECT>;
+  if (sp.update_kind != 1) return (const void*)k_update<4, UPD_ADVECT>;
+  return sp.ref_compat ? (const void*)k_update<4, UPD_CURVATURE_REF> : (const void*)k_update<4, UPD_CURVATURE>;
+}
+inline int update_record(const DevMesh& m, const StepParams& sp) {
+  return upd_record(m.dim == 3 && sp.update_kind == 1 && sp.ref_compat ? UPD_CURVATURE_REF : UPD_ADVECT);
 }
 
-// tetrahedra with patches of up to 384 element copies: three CTAs per SM
-// (which caps the registers at 56 without spills; the 512-thread form keeps
-// two)
-__global__ void __launch_bounds__(384, 3) k_update_384(DevMesh m, DevState s, StepParams sp) {
-  update_patches<4>(m, s, sp);
-}
-
-// phi := phi_out on narrowband patches (CopyOutBack_levelset3d)
+// phi_rd := phi on narrowband patches, between the inside iterations of a
+// step (CopyOutBack_levelset3d)
 __global__ void k_copy_phi(DevMesh m, DevState s) {
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int count = s.ctl[CTL_NB];
   for (int w = warp_id_global(); w < count; w += nwarps) {
     const int p = s.nblist[w];
-    for (int v = m.vert_off[p] + lane; v < m.vert_off[p + 1]; v += 32) s.phi[v] = s.phi_out[v];
+    for (int v = m.vert_off[p] + lane; v < m.vert_off[p + 1]; v += 32) s.phi_rd[v] = s.phi[v];
   }
 }
 
@@ -1986,7 +2038,7 @@ __global__ void k_targets(DevState s, DevLearn lr, float inv_h, float LN) {
   const int n = lr.cnt[0];
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int v = lr.vlist[i];
-    const float ph = s.phi[v];
+    const float ph = s.phi_rd[v];
     lr.target[i] = fabsf(ph) >= LN ? __int_as_float(0x7fc00000) : ph * (lr.vinv_h ? lr.vinv_h[v] : inv_h);
   }
 }
@@ -2001,8 +2053,8 @@ cudaError_t launch_learn(int op, const DevMesh& m, const DevState& s, const Step
       k_warm_apply<<<L.flat_grid, 256, 0, st>>>(s, lr, sp.largenum, fa);
       break;
     case LEARN_SEED_WARM:
-      if (m.dim == 3) k_seed<4><<<L.seed_grid, L.fim_block, 0, st>>>(m, s, sp.scale, 1);
-      else k_seed<3><<<L.seed_grid, L.fim_block, 0, st>>>(m, s, sp.scale, 1);
+      if (m.dim == 3) k_seed<4><<<L.seed_grid, kSeedBlock, L.seed_smem, st>>>(m, s, sp, 1);
+      else k_seed<3><<<L.seed_grid, kSeedBlock, L.seed_smem, st>>>(m, s, sp, 1);
       break;
     case LEARN_SUPPORT: {
       const int smem = (int)sizeof(float) * (2 * sp.lvp + sp.lgp);
@@ -2033,8 +2085,8 @@ cudaError_t launch_begin(const DevState& s, int restart, cudaStream_t st) {
 }
 
 cudaError_t launch_seed(const DevMesh& m, const DevState& s, const StepParams& sp, const Launch& L, cudaStream_t st) {
-  if (m.dim == 3) k_seed<4><<<L.seed_grid, L.fim_block, 0, st>>>(m, s, sp.scale, 0);
-  else k_seed<3><<<L.seed_grid, L.fim_block, 0, st>>>(m, s, sp.scale, 0);
+  if (m.dim == 3) k_seed<4><<<L.seed_grid, kSeedBlock, L.seed_smem, st>>>(m, s, sp, 0);
+  else k_seed<3><<<L.seed_grid, kSeedBlock, L.seed_smem, st>>>(m, s, sp, 0);
   return cudaGetLastError();
 }
 
@@ -2218,19 +2270,18 @@ cudaError_t configure_persistent(const DevMesh& m, const StepParams& sp, Launch&
 
 cudaError_t launch_narrowband(const DevMesh& m, const DevState& s, const StepParams& sp, const Launch& L,
                               cudaStream_t st) {
-  k_narrowband<<<L.warp_grid, 256, 0, st>>>(m, s, sp);
+  k_narrowband<<<L.warp_grid, 256, 0, st>>>(m, s, sp, sp.update_kind == 2 ? 1 : 0);
   return cudaGetLastError();
 }
 
-cudaError_t launch_update(const DevMesh& m, const DevState& s, const StepParams& sp, const Launch& L,
+// One inside iteration of the step's update (first: the narrowband kernel
+// has just written phi_rd).
+cudaError_t launch_update(const DevMesh& m, const DevState& s, const StepParams& sp, int first, const Launch& L,
                           cudaStream_t st) {
-  if (m.dim == 3 && L.upd_block <= 384) k_update_384<<<L.upd_grid, L.upd_block, L.upd_smem, st>>>(m, s, sp);
-  else if (m.dim == 3) k_update<4><<<L.upd_grid, L.upd_block, L.upd_smem, st>>>(m, s, sp);
-  else k_update<3><<<L.upd_grid, L.upd_block, L.upd_smem, st>>>(m, s, sp);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  k_copy_phi<<<L.warp_grid, 256, 0, st>>>(m, s);
-  return cudaGetLastError();
+  if (!first) k_copy_phi<<<L.warp_grid, 256, 0, st>>>(m, s);
+  void* args[] = {(void*)&m, (void*)&s, (void*)&sp};
+  return cudaLaunchKernel(update_kernel(m, sp), dim3((unsigned)L.upd_grid), dim3((unsigned)L.upd_block), args,
+                          (size_t)L.upd_smem, st);
 }
 
 cudaError_t launch_unpermute(const DevMesh& m, const float* phi, float* out, const Launch& L, cudaStream_t st) {
@@ -2338,13 +2389,18 @@ cudaError_t configure_launch(const DevMesh& m, const StepParams& sp, Launch& L) 
   if (occ < 1) occ = 1;
   // no more CTAs than patches: a small mesh's launches are short
   L.fim_grid = std::min(L.sms * occ, m.nparts);
-  L.seed_grid = std::min(L.sms * 8, m.nparts);
-  L.upd_block = L.fim_block > 512 ? 512 : L.fim_block;
+  L.seed_grid = std::min(L.sms * 16, m.nparts);
+  L.seed_smem = (int)sizeof(float) * (sp.lvp + sp.lgp);
+  if (L.seed_smem > 48 * 1024) {
+    e = cudaFuncSetAttribute(m.dim == 3 ? (const void*)k_seed<4> : (const void*)k_seed<3>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, L.seed_smem);
+    if (e != cudaSuccess) return e;
+  }
+  L.upd_block = kUpdBlock;
   const int slab = sp.lvp + sp.lgp;
-  L.upd_smem = (int)sizeof(float) * (slab * (m.dim == 3 ? 4 : 1) + sp.lep * 16);
+  L.upd_smem = (int)sizeof(float) * slab * (m.dim == 3 ? 4 : 1) + (int)sizeof(float4) * sp.lep * update_record(m, sp);
   {
-    const void* fn = m.dim == 3 ? (L.upd_block <= 384 ? (const void*)k_update_384 : (const void*)k_update<4>)
-                                : (const void*)k_update<3>;
+    const void* fn = update_kernel(m, sp);
     if (L.upd_smem > 48 * 1024) {
       e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, L.upd_smem);
       if (e != cudaSuccess) return e;

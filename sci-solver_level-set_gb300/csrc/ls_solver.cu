@@ -269,7 +269,7 @@ std::string Solver::init(const Layout& L, const SolverConfig& cfg, const float* 
   }
   // step state
   LS_TRY(dalloc(A, &s_.phi, nv), "alloc");
-  LS_TRY(dalloc(A, &s_.phi_out, nv), "alloc");
+  LS_TRY(dalloc(A, &s_.phi_rd, nv), "alloc");
   LS_TRY(dalloc(A, &s_.cell, nv), "alloc");
   LS_TRY(dalloc(A, &s_.slot, np), "alloc");
   LS_TRY(dalloc(A, &s_.pend, np), "alloc");
@@ -440,7 +440,7 @@ cudaError_t Solver::step_head() {
 cudaError_t Solver::step_tail() {
   cudaError_t e = K_->narrowband(m_, s_, sp_, L_, stream_);
   if (cfg_.update_kind != 2)
-    for (int it = 0; it < cfg_.inside_niter && e == cudaSuccess; ++it) e = K_->update(m_, s_, sp_, L_, stream_);
+    for (int it = 0; it < cfg_.inside_niter && e == cudaSuccess; ++it) e = K_->update(m_, s_, sp_, it == 0, L_, stream_);
   return e;
 }
 
@@ -541,7 +541,8 @@ std::string Solver::one_step(bool* empty_nb) {
   };
   if (h_ctl_[CTL_ITER] > kStampLimit) LS_TRY(restart_stamps(0), "stamps");
   if (net_ || collect_) return learned_step(empty_nb);
-  const long long upd = cfg_.update_kind != 2 ? 2LL * cfg_.inside_niter : 0;  // update, copy-back
+  // updates, and the copies between them
+  const long long upd = cfg_.update_kind != 2 ? 2LL * cfg_.inside_niter - 1 : 0;
   if (persistent_ || (graph_exec_ && !cfg_.profile)) {
     // the whole step in one go: its graph, or the persistent form launch by
     // launch (profiled: the FIM loop kernel's time is recorded as the sweep time)
@@ -576,7 +577,7 @@ std::string Solver::one_step(bool* empty_nb) {
   }
   if (cfg_.update_kind != 2) {
     for (int it = 0; it < cfg_.inside_niter; ++it)
-      LS_TRY(prof(5, [&] { return K_->update(m_, s_, sp_, L_, stream_); }), "update");
+      LS_TRY(prof(5, [&] { return K_->update(m_, s_, sp_, it == 0, L_, stream_); }), "update");
     st_.kernel_launches += upd;
   }
   return "";
@@ -739,8 +740,8 @@ std::string Solver::learned_step(bool* empty_nb) {
   }
   if (cfg_.update_kind != 2) {
     for (int it = 0; it < cfg_.inside_niter; ++it) {
-      LS_TRY(K_->update(m_, s_, sp_, L_, stream_), "update");
-      st_.kernel_launches += 2;
+      LS_TRY(K_->update(m_, s_, sp_, it == 0, L_, stream_), "update");
+      st_.kernel_launches += it == 0 ? 1 : 2;
     }
   }
   return "";

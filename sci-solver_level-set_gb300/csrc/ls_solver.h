@@ -18,7 +18,7 @@ struct Launch {
   int pair_block;  // threads of the two-copies-per-thread sweep kernel (0: not used)
   int persist_grid;  // CTAs of the persistent FIM kernel (all resident; 0: no persistent form here)
   int upd_grid, upd_block, upd_smem;
-  int seed_grid;
+  int seed_grid, seed_smem;
   int warp_grid;
   int flat_grid;
 };
@@ -39,7 +39,8 @@ struct KernelSet {
                                 cudaStream_t st);
   cudaError_t (*narrowband)(const DevMesh& m, const DevState& s, const StepParams& sp, const Launch& L,
                             cudaStream_t st);
-  cudaError_t (*update)(const DevMesh& m, const DevState& s, const StepParams& sp, const Launch& L, cudaStream_t st);
+  cudaError_t (*update)(const DevMesh& m, const DevState& s, const StepParams& sp, int first, const Launch& L,
+                        cudaStream_t st);
   // FIM distances in the layout's vertex order
   cudaError_t (*distances)(const DevMesh& m, const DevState& s, const StepParams& sp, float* out, const Launch& L,
                            cudaStream_t st);
