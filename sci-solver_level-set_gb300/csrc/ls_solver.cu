@@ -43,6 +43,7 @@ Solver::~Solver() {
   if (graph_) cudaGraphDestroy(graph_);
   for (void* p : allocs_) cudaFree(p);
   if (h_ctl_) cudaFreeHost(h_ctl_);
+  if (d_seeds_) cudaFree(d_seeds_);
   if (h_stats_) cudaFreeHost(h_stats_);
   if (h_stage_) cudaFreeHost(h_stage_);
   if (h_snap_) cudaFreeHost(h_snap_);
@@ -53,6 +54,8 @@ Solver::~Solver() {
     cudaEventDestroy(pe.b);
   }
   for (cudaEvent_t e : ev_pool_) cudaEventDestroy(e);
+  for (cudaEvent_t e : ev_chunk_)
+    if (e) cudaEventDestroy(e);
   if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -287,8 +290,10 @@ std::string Solver::init(const Layout& L, const SolverConfig& cfg, const float* 
   LS_TRY(cudaMemsetAsync(s_.stats, 0, sizeof(unsigned long long) * 9, stream_), "memset");
   LS_TRY(cudaMemsetAsync(s_.sched, 0, sizeof(int) * 4, stream_), "memset");
   LS_TRY(cudaMemsetAsync(s_.phi, 0, sizeof(float) * nv, stream_), "memset");
-  LS_TRY(cudaMallocHost((void**)&h_ctl_, sizeof(int) * CTL_WORDS), "pinned");
-  std::memset(h_ctl_, 0, sizeof(int) * CTL_WORDS);
+  LS_TRY(cudaMallocHost((void**)&h_ctl_, sizeof(int) * 3 * CTL_WORDS), "pinned");
+  std::memset(h_ctl_, 0, sizeof(int) * 3 * CTL_WORDS);
+  h_chunk_ = h_ctl_ + CTL_WORDS;
+  for (cudaEvent_t& e : ev_chunk_) LS_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
   // a few steps below the limit, so that every handle's stamps restart early in its life
   LS_TRY(restart_stamps(kStampLimit - 32), "stamps");
   LS_TRY(cudaMallocHost((void**)&h_stats_, sizeof(unsigned long long) * 9), "pinned");
@@ -502,6 +507,11 @@ std::string Solver::build_graph() {
   return "";
 }
 
+// Iterations launched one by one, in chunks of graph_chunk.  The next chunk
+// is enqueued before the host waits for the last one's control words, so the
+// GPU does not idle for the round trip (about 15 us a chunk); the chunk
+// behind the one that drains the list finds it empty.  Profiled steps wait
+// for each chunk (their launches are counted).
 std::string Solver::fim_loop(const StepParams& sp) {
   auto prof = [&](auto&& fn) -> cudaError_t {
     if (!cfg_.profile) return fn();
@@ -512,18 +522,25 @@ std::string Solver::fim_loop(const StepParams& sp) {
     cudaError_t e2 = prof_fim_end(pe);
     return e != cudaSuccess ? e : e2;
   };
-  while (true) {
+  const int ahead = cfg_.profile ? 0 : 1;
+  for (int k = 0;; ++k) {
     for (int i = 0; i < cfg_.graph_chunk; ++i)
       LS_TRY(prof([&] { return K_->fim(m_, s_, sp, i, L_, stream_); }), "FIM iteration");
     k_body_end<<<1, 32, 0, stream_>>>(s_.ctl, cfg_.graph_chunk, iter_cap());
     LS_TRY(cudaGetLastError(), "body end");
     st_.kernel_launches += cfg_.graph_chunk + 1;
-    LS_TRY(read_ctl(), "fim sync");
-    std::string r = fim_status();
-    if (!r.empty()) return r;
-    const int cur = h_ctl_[CTL_ITER] % 3;
-    if (h_ctl_[CTL_VISITS + cur] + h_ctl_[CTL_CANDS + cur] == 0) return "";
+    int* const mine = h_chunk_ + (k & 1) * CTL_WORDS;
+    LS_TRY(cudaMemcpyAsync(mine, s_.ctl, sizeof(int) * CTL_WORDS, cudaMemcpyDeviceToHost, stream_), "d2h");
+    LS_TRY(cudaEventRecord(ev_chunk_[k & 1], stream_), "event");
+    if (k < ahead) continue;
+    const int done = (k - ahead) & 1;
+    LS_TRY(cudaEventSynchronize(ev_chunk_[done]), "fim sync");
+    const int* c = h_chunk_ + done * CTL_WORDS;
+    const int cur = c[CTL_ITER] % 3;
+    if (c[CTL_ERR] || c[CTL_CAP] || c[CTL_VISITS + cur] + c[CTL_CANDS + cur] == 0) break;
   }
+  LS_TRY(read_ctl(), "fim end");
+  return fim_status();
 }
 
 std::string Solver::one_step(bool* empty_nb) {
@@ -834,46 +851,81 @@ std::string Solver::step_host(const float* phi_in, float* phi_out) {
   return "";
 }
 
+// Standalone eikonal solve: the seeds, the first list and the result on the
+// device (host loops over the copies, the cells and the permutation took 7 of
+// 10.5 ms at 64^3).
+namespace {
+// The last of several values given for one vertex counts.
+__global__ void k_eik_order(DevMesh m, const int* seeds, int n, int* order) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) atomicMax(order + __ldg(m.ipermute + seeds[i]), i);
+}
+__global__ void k_eik_seed(DevMesh m, DevState s, const int* seeds, const float* values, int n, const int* order,
+                           float scale, float LN) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int v = __ldg(m.ipermute + seeds[i]);
+  if (order[v] != i) return;
+  const float a = values[i] >= LN ? LN : values[i] / scale;
+  *reinterpret_cast<int2*>(s.cell + v) = make_int2(__float_as_int(a), s.ctl[CTL_BASE]);
+}
+// The patches one of whose element copies holds a seed (the list the seed
+// kernel makes at the start of a time step): a patch's copies' vertices are
+// its own and its ghosts.  One warp per patch.
+__global__ void k_eik_list(DevMesh m, DevState s) {
+  const int lane = threadIdx.x & 31, nwarps = (gridDim.x * blockDim.x) >> 5;
+  const int base = s.ctl[CTL_BASE], t0 = s.ctl[CTL_ITER];
+  for (int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < m.nparts; p += nwarps) {
+    const int vs = m.vert_off[p], nvp = m.vert_off[p + 1] - vs;
+    const int gs = m.ghost_off[p], ngp = m.ghost_off[p + 1] - gs;
+    bool hit = false;
+    for (int i = lane; i < nvp + ngp; i += 32)
+      hit |= dt_is_seed(s.cell[i < nvp ? vs + i : __ldg(m.ghost_ids + gs + i - nvp)], base);
+    if (__any_sync(0xffffffffu, hit) && lane == 0) {
+      s.lists[(size_t)(t0 % 3) * m.nparts + atomicAdd(s.ctl + CTL_VISITS + t0 % 3, 1)] = p;
+      s.pend[p] = 2 * t0;
+    }
+  }
+}
+// out[old]: the distance in the caller's units
+__global__ void k_eik_out(DevMesh m, DevState s, float scale, float LN, float* out) {
+  const int base = s.ctl[CTL_BASE];
+  for (int o = blockIdx.x * blockDim.x + threadIdx.x; o < m.nv; o += gridDim.x * blockDim.x) {
+    const float d = dt_before(s.cell[__ldg(m.ipermute + o)], kStampMax, base, LN);
+    out[o] = d >= LN ? LN : d * scale;
+  }
+}
+}  // namespace
+
 std::string Solver::eikonal(const int* seeds, const float* values, int nseeds, float* out) {
   if (m_.patch_mesh) {
     status_ = 1;
     return "the standalone eikonal solve takes one mesh, not a batch";
   }
-  const Layout& L = *lay_;
-  const int nv = m_.nv, np = m_.nparts;
+  const int nv = m_.nv, n = nseeds;
   const float LN = sp_.largenum;
-  // a step of its own, with the stamps started again: base 0, first iteration 2
-  LS_TRY(restart_stamps(0), "stamps");
+  if (h_ctl_[CTL_ITER] > kStampLimit) LS_TRY(restart_stamps(0), "stamps");
   LS_TRY(K_->begin(s_, 0, stream_), "begin");
-  std::vector<DtCell> cell(nv, make_int4(0, -1, 0, -1));
-  std::vector<uint8_t> sd(nv, 0);
-  std::vector<int> act, pend(np, -1);
-  for (int i = 0; i < nseeds; ++i) {
-    const int v = L.vert_ipermute[seeds[i]];
-    const float a = (values[i] >= LN) ? LN : values[i] / sp_.scale;
-    std::memcpy(&cell[v].x, &a, sizeof(float));
-    cell[v].y = 0;
-    sd[v] = 1;
-  }
-  // first active list: the patches one of whose element copies holds a seed
-  // (the list the seed kernel makes at the start of a time step)
-  const int d1 = m_.dim + 1;
-  for (int p = 0; p < np; ++p) {
-    bool hit = false;
-    for (int c = L.ele_offsets[p]; c < L.ele_offsets[p + 1] && !hit; ++c)
-      for (int k = 0; k < d1; ++k) hit |= sd[L.conn[(size_t)c * d1 + k]] != 0;
-    if (hit) {
-      act.push_back(p);
-      pend[p] = 2 * 2;
+  if (n > 0) {
+    if (n > seed_cap_) {
+      // seeds and values of the largest call so far
+      if (d_seeds_) LS_TRY(cudaFree(d_seeds_), "free");
+      d_seeds_ = nullptr;
+      seed_cap_ = 0;
+      LS_TRY(cudaMalloc((void**)&d_seeds_, (sizeof(int) + sizeof(float)) * (size_t)n), "alloc");
+      seed_cap_ = n;
     }
+    float* d_values = reinterpret_cast<float*>(d_seeds_ + seed_cap_);
+    int* order = reinterpret_cast<int*>(d_tmp_);
+    LS_TRY(cudaMemcpyAsync(d_seeds_, seeds, sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, stream_), "h2d");
+    LS_TRY(cudaMemcpyAsync(d_values, values, sizeof(float) * (size_t)n, cudaMemcpyHostToDevice, stream_), "h2d");
+    LS_TRY(cudaMemsetAsync(order, 0xff, sizeof(int) * (size_t)nv, stream_), "memset");
+    const int grid = (n + 255) / 256;
+    k_eik_order<<<grid, 256, 0, stream_>>>(m_, d_seeds_, n, order);
+    k_eik_seed<<<grid, 256, 0, stream_>>>(m_, s_, d_seeds_, d_values, n, order, sp_.scale, LN);
+    k_eik_list<<<L_.warp_grid, 256, 0, stream_>>>(m_, s_);
+    LS_TRY(cudaGetLastError(), "eikonal seeds");
   }
-  const int n = (int)act.size();
-  LS_TRY(cudaMemcpyAsync(s_.cell, cell.data(), sizeof(DtCell) * nv, cudaMemcpyHostToDevice, stream_), "h2d");
-  LS_TRY(cudaMemcpyAsync(s_.pend, pend.data(), sizeof(int) * np, cudaMemcpyHostToDevice, stream_), "h2d");
-  if (n)
-    LS_TRY(cudaMemcpyAsync(s_.lists + (size_t)2 * np, act.data(), sizeof(int) * n, cudaMemcpyHostToDevice, stream_),
-           "h2d");
-  LS_TRY(cudaMemcpyAsync(s_.ctl + CTL_VISITS + 2, &n, sizeof(int), cudaMemcpyHostToDevice, stream_), "h2d");
   LS_TRY(cudaMemsetAsync(s_.ctl + CTL_NB_VALID, 0, sizeof(int), stream_), "memset");
   StepParams sp = sp_;
   // no narrowband limit: every converged patch that the front has reached
@@ -882,10 +934,14 @@ std::string Solver::eikonal(const int* seeds, const float* values, int nseeds, f
   std::string r = fim_loop(sp);
   if (!r.empty()) return r;
   if (cfg_.profile) fold_prof(true);
-  std::vector<float> dt(nv);
-  r = dt_values(dt.data());
-  if (!r.empty()) return r;
-  for (int v = 0; v < nv; ++v) out[L.vert_permute[v]] = (dt[v] >= LN) ? LN : dt[v] * sp_.scale;
+  // to the caller's pageable array where the GPU can write it (step_host)
+  float* const dst = pageable_ ? out : d_tmp_;
+  k_eik_out<<<L_.flat_grid, 256, 0, stream_>>>(m_, s_, sp_.scale, LN, dst);
+  LS_TRY(cudaGetLastError(), "eikonal result");
+  if (!pageable_)
+    LS_TRY(cudaMemcpyAsync(h_stage_, d_tmp_, sizeof(float) * nv, cudaMemcpyDeviceToHost, stream_), "d2h");
+  LS_TRY(cudaStreamSynchronize(stream_), "sync");
+  if (!pageable_) std::memcpy(out, h_stage_, sizeof(float) * nv);
   have_nb_ = false;  // the step state was overwritten
   stats_stale_ = true;
   return "";

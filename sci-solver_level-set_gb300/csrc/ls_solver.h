@@ -198,6 +198,10 @@ class Solver {
   cudaGraph_t graph_ = nullptr;
   std::vector<void*> allocs_;
   int* h_ctl_ = nullptr;              // pinned mirror of the step control words (read_ctl)
+  int* h_chunk_ = nullptr;            // two more, of the last chunks of fim_loop
+  cudaEvent_t ev_chunk_[2] = {};
+  int* d_seeds_ = nullptr;            // eikonal seeds and values, room for seed_cap_ of each
+  int seed_cap_ = 0;
   unsigned long long* h_stats_ = nullptr;
   float* h_stage_ = nullptr;          // pinned nv floats
   float* d_tmp_ = nullptr;            // nv floats (caller-order staging)
