@@ -16,7 +16,7 @@
 //   g_W_l = d_l^T a_{l-1} (fp32 accumulate);  g_b_l = sum_samples d_l
 //   d_{l-1} = bf16((d_l W_l) * [a_{l-1} > 0])
 //
-// One CTA of 128 threads handles a tile of 128 samples.  Operand tiles use
+// One CTA of 256 threads handles a tile of 128 samples.  Operand tiles use
 // the no-swizzle K-major core-matrix layout of the tensor core: element
 // (row r, k) of a 128 x 128 BF16 tile sits at byte
 //   (r / 8) * 2048 + (k / 8) * 128 + (r % 8) * 16 + (k % 8) * 2,
@@ -25,7 +25,15 @@
 // (M = N = 128, K = 16) covers two core matrices along K; the K loop
 // advances both descriptors by 256 bytes.  The accumulator (M = 128) keeps
 // row r in tensor-memory lane r, column n in column n; warp w of the CTA
-// reads lanes 32w..32w+31 with tcgen05.ld.
+// reads lanes 32 (w % 4) .. +31 with tcgen05.ld, warps 0-3 the columns below
+// 64, warps 4-7 the others.
+// The same bytes are the MN-major operand of the transposed product: its
+// core matrices hold 8 K rows of 8 contiguous M/N elements, 128 bytes apart
+// along M/N and 2048 along K, so the leading and stride offsets swap, the K
+// loop advances by 4096 bytes and the instruction descriptor's transpose bit
+// is set.  The weight gradients d^T a and the back-propagation d W therefore
+// read the tiles of d, a and W that the forward pass uses; nothing is
+// transposed.
 //
 // Every wait on an mbarrier is bounded (about one second of clock cycles);
 // on expiry the kernel records the error, waits (bounded) for its MMAs,
@@ -49,7 +57,8 @@ namespace mlp {
 namespace {
 
 constexpr int F = 128;        // features = hidden width
-constexpr int TILE = 128;     // samples per CTA
+constexpr int TILE = 128;     // samples per tile
+constexpr int THREADS = 256;  // of the network kernels' CTAs
 constexpr int TILE_BYTES = TILE * F * 2;   // one BF16 operand tile (32 KB)
 constexpr uint32_t LBO = 128, SBO = 2048;  // core-matrix strides (bytes)
 // kind::f16 instruction descriptor: D fp32 (bits 4-5 = 1), A bf16 (bits
@@ -57,6 +66,7 @@ constexpr uint32_t LBO = 128, SBO = 2048;  // core-matrix strides (bytes)
 // M >> 4 at bits 24-28
 constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(F >> 3) << 17) |
                            ((uint32_t)(TILE >> 4) << 24);
+constexpr uint32_t IDESC_TA = 1u << 15, IDESC_TB = 1u << 16;  // A, B MN-major
 constexpr long long WAIT_CYCLES = 2000000000LL;  // ~1 s at 2 GHz
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -65,12 +75,13 @@ __device__ __forceinline__ uint32_t tile_off(int r, int k) {
   return (uint32_t)((r >> 3) * SBO + (k >> 3) * LBO + (r & 7) * 16 + (k & 7) * 2);
 }
 
-// shared-memory matrix descriptor, no swizzle (layout type 0), version 1
-__device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
+// shared-memory matrix descriptor, no swizzle (layout type 0), version 1;
+// mn: the tile read as an MN-major operand
+__device__ __forceinline__ uint64_t make_desc(uint32_t saddr, bool mn) {
   uint64_t d = 0;
   d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
-  d |= (uint64_t)((LBO >> 4) & 0x3FFFu) << 16;
-  d |= (uint64_t)((SBO >> 4) & 0x3FFFu) << 32;
+  d |= (uint64_t)(((mn ? SBO : LBO) >> 4) & 0x3FFFu) << 16;
+  d |= (uint64_t)(((mn ? LBO : SBO) >> 4) & 0x3FFFu) << 32;
   d |= (uint64_t)1 << 46;
   return d;
 }
@@ -89,11 +100,11 @@ __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::be
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-__device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, int accumulate) {
+__device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, int accumulate) {
   asm volatile(
       "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
-      "l"(a), "l"(b), "r"(IDESC), "r"(accumulate)
+      "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 
@@ -139,16 +150,19 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// row r of a [rows][128] BF16 global matrix -> tile row r (16-byte chunks)
-__device__ __forceinline__ void load_row(uint8_t* tile, int r, const __nv_bfloat16* src) {
-  const uint4* s = reinterpret_cast<const uint4*>(src);
-#pragma unroll 4
-  for (int j = 0; j < F / 8; ++j) *reinterpret_cast<uint4*>(tile + tile_off(r, j * 8)) = __ldg(s + j);
-}
-
-__device__ __forceinline__ void zero_row(uint8_t* tile, int r) {
-#pragma unroll 4
-  for (int j = 0; j < F / 8; ++j) *reinterpret_cast<uint4*>(tile + tile_off(r, j * 8)) = make_uint4(0, 0, 0, 0);
+// rows [s0, s0 + 128) of a [n][128] BF16 global matrix -> a tile (zeros past
+// n), by all threads: a warp takes 8 rows x 4 chunks of 16 bytes at a time,
+// whole 64-byte pieces of the rows, and its stores fall on all banks
+__device__ __forceinline__ void load_rows(uint8_t* tile, const __nv_bfloat16* X, int s0, int n) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rl = lane & 7, cl = lane >> 3;
+#pragma unroll
+  for (int k = 0; k < 64 / (THREADS / 32); ++k) {
+    const int i = warp + k * (THREADS / 32);  // 16 row groups x 4 chunk groups
+    const int r = (i >> 2) * 8 + rl, c = ((i & 3) * 4 + cl) * 8;
+    const uint4 v = s0 + r < n ? __ldg(reinterpret_cast<const uint4*>(X + (size_t)(s0 + r) * F + c)) : make_uint4(0, 0, 0, 0);
+    *reinterpret_cast<uint4*>(tile + tile_off(r, c)) = v;
+  }
 }
 
 // 8 floats -> 8 BF16 (round to nearest even) in one 16-byte chunk
@@ -171,16 +185,12 @@ __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__floa
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// Weight copies for the tensor cores: BF16 tiles in the operand layout above
-// (tile_off), so that one bulk asynchronous copy of 32 KB stages a layer's
-// weights.  Wt[l]: rows = output feature, K = input feature (B operand of
-// the forward); WTt[l]: rows = input feature, K = output feature (B operand
-// of the backward's dH = d W).
-__device__ __forceinline__ void store_weight(__nv_bfloat16* Wt, __nv_bfloat16* WTt, int i, float p) {
+// Weight copy for the tensor cores: BF16 tiles in the operand layout above
+// (tile_off; rows = output feature, K = input feature), so that one bulk
+// asynchronous copy of 32 KB stages a layer's weights.
+__device__ __forceinline__ void store_weight(__nv_bfloat16* Wt, int i, float p) {
   const int l = i / (F * F), o = (i / F) % F, in = i % F;
-  const __nv_bfloat16 v = __float2bfloat16_rn(p);
-  Wt[(size_t)l * F * F + tile_off(o, in) / 2] = v;
-  WTt[(size_t)l * F * F + tile_off(in, o) / 2] = v;
+  Wt[(size_t)l * F * F + tile_off(o, in) / 2] = __float2bfloat16_rn(p);
 }
 
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
@@ -199,12 +209,14 @@ __device__ __forceinline__ void bulk_tile(uint8_t* dst, const __nv_bfloat16* src
 }
 
 // MMAs of one 128 x 128 x 128 product that add to the accumulator when acc
-// is set (thread 0 only)
-__device__ __forceinline__ void mma_tile_acc(uint32_t tmem_d, const uint8_t* a, const uint8_t* b, bool acc) {
+// is set (thread 0 only); ta, tb: the tile is read as an MN-major operand
+__device__ __forceinline__ void mma_tile(uint32_t tmem_d, const uint8_t* a, bool ta, const uint8_t* b, bool tb, bool acc) {
   const uint32_t sa = smem_u32(a), sb = smem_u32(b);
+  const uint32_t ka = ta ? 2 * SBO : 2 * LBO, kb = tb ? 2 * SBO : 2 * LBO;
+  const uint32_t idesc = IDESC | (ta ? IDESC_TA : 0u) | (tb ? IDESC_TB : 0u);
 #pragma unroll
   for (int ks = 0; ks < F / 16; ++ks)
-    mma(tmem_d, make_desc(sa + ks * 2 * LBO), make_desc(sb + ks * 2 * LBO), (acc || ks > 0) ? 1 : 0);
+    mma(tmem_d, make_desc(sa + ks * ka, ta), make_desc(sb + ks * kb, tb), idesc, (acc || ks > 0) ? 1 : 0);
 }
 
 struct SmemW {
@@ -214,23 +226,59 @@ struct SmemW {
   int fail;
 };
 
+// The half of a layer's epilogue that belongs to this thread: its sample
+// row's 64 columns (from column 64 * (warp / 4)) of bf16(relu(z + b)) to tile
+// `out` (when given), their values added up with the weights w4 in column
+// order (last layer).  The two halves of a row's sum are one chain: the lower
+// columns' partial sum goes through s_out to the upper ones' thread.
+__device__ __forceinline__ float layer_epilogue(uint32_t tz, const float* s_b, uint8_t* out, const float* s_w4,
+                                                float* s_out) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int r = (warp & 3) * 32 + lane, c0 = (warp >> 2) * 64;
+  float v[64];
+  tmem_ld32(tz + ((uint32_t)((warp & 3) * 32) << 16) + c0, v);
+  tmem_ld32(tz + ((uint32_t)((warp & 3) * 32) << 16) + c0 + 32, v + 32);
+#pragma unroll
+  for (int j = 0; j < 64; ++j) v[j] = bf16r(fmaxf(v[j] + s_b[c0 + j], 0.f));
+  if (out) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) *reinterpret_cast<uint4*>(out + tile_off(r, c0 + q * 8)) = pack8(v + q * 8);
+  }
+  float sum = 0.f;
+  if (s_w4) {
+    if (warp < 4) {
+#pragma unroll
+      for (int j = 0; j < 64; ++j) sum += v[j] * s_w4[j];
+      s_out[r] = sum;
+    }
+    __syncthreads();
+    if (warp >= 4) {
+      sum = s_out[r];
+#pragma unroll
+      for (int j = 0; j < 64; ++j) sum += v[j] * s_w4[64 + j];
+    }
+  }
+  return sum;  // complete in warps 4-7
+}
+
 // ---------------------------------------------------------------------------
-// Forward.  X [n][128] BF16 rows; Wt the three weight tiles; b [3][128],
-// w4 [128], b4 [1] fp32; y [n]; A (optional) [3][n][128] BF16 activations
-// a_1..a_3 for the backward pass.  n_dev (optional) overrides n from device
-// memory (graph replays with a device-side sample count).  Each CTA stages
-// the weights once (three bulk copies) and then runs the sample tiles
-// blockIdx.x, blockIdx.x + gridDim.x, ... through the three layers.
-__global__ void __launch_bounds__(128, 1)
+// Forward.  X [n][128] BF16 rows; Wt the three weight tiles; P4 = [b (3 x
+// 128) | w4 (128) | b4] fp32; y [n].  n_dev (optional) overrides n from
+// device memory (a device-side sample count).  Each CTA stages the weights
+// once (three bulk copies) and then runs the sample tiles blockIdx.x,
+// blockIdx.x + gridDim.x, ... through the three layers.
+__global__ void __launch_bounds__(THREADS, 1)
     k_mlp_fwd(const __nv_bfloat16* __restrict__ X, int n, const int* n_dev, const __nv_bfloat16* __restrict__ Wt,
-              const float* __restrict__ b, const float* __restrict__ w4, const float* __restrict__ b4,
-              float* __restrict__ y, __nv_bfloat16* __restrict__ A, int* err) {
+              const float* __restrict__ P4, float* __restrict__ y, int* err) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* act = base;                       // activation tile (A operand)
   uint8_t* wt = base + TILE_BYTES;           // 3 weight tiles (B operands)
-  SmemW* sm = reinterpret_cast<SmemW*>(base + 4 * TILE_BYTES);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  float* s_b = reinterpret_cast<float*>(base + 4 * TILE_BYTES);  // [3][128] biases
+  float* s_w4 = s_b + 3 * F;                                      // [128]
+  float* s_out = s_w4 + F;                                        // [128]
+  SmemW* sm = reinterpret_cast<SmemW*>(s_out + F);
+  const int tid = threadIdx.x, warp = tid >> 5;
   if (n_dev) n = *n_dev;
   const int ntiles = (n + TILE - 1) / TILE;
   if ((int)blockIdx.x >= ntiles) return;  // whole CTA exits before any tensor-core work
@@ -241,6 +289,7 @@ __global__ void __launch_bounds__(128, 1)
     mbar_expect_tx(&sm->bar_w, 3 * TILE_BYTES);
     for (int l = 0; l < 3; ++l) bulk_tile(wt + l * TILE_BYTES, Wt + (size_t)l * F * F, &sm->bar_w);
   }
+  for (int i = tid; i < 4 * F; i += THREADS) s_b[i] = __ldg(P4 + i);  // b and w4
   __syncwarp();
   if (warp == 0) tmem_alloc(&sm->tmem, 128);
   fence_before();
@@ -251,9 +300,7 @@ __global__ void __launch_bounds__(128, 1)
   bool ok = true, weights = false, mma_pending = false;
   for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
     const int s0 = tile * TILE;
-    const int s = s0 + tid;  // sample row tid of the operand tile
-    if (s < n) load_row(act, tid, X + (size_t)s * F);
-    else zero_row(act, tid);
+    load_rows(act, X, s0, n);
     fence_async_smem();
     fence_before();
     __syncthreads();
@@ -266,7 +313,7 @@ __global__ void __launch_bounds__(128, 1)
     float out = 0.f;
     for (int l = 0; l < 3 && ok; ++l) {
       if (tid == 0) {
-        mma_tile_acc(tmem, act, wt + l * TILE_BYTES, false);
+        mma_tile(tmem, act, false, wt + l * TILE_BYTES, false, false);
         mma_commit(&sm->bar);
       }
       mma_pending = true;
@@ -275,35 +322,13 @@ __global__ void __launch_bounds__(128, 1)
       mma_pending = false;
       phase ^= 1;
       fence_after();
-      const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
-      const int r = warp * 32 + lane;  // sample row of this thread
-      for (int c = 0; c < F / 32; ++c) {
-        float v[32];
-        tmem_ld32(trow + c * 32, v);
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = bf16r(fmaxf(v[j] + __ldg(b + l * F + c * 32 + j), 0.f));
-        if (l < 2) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(act + tile_off(r, c * 32 + q * 8)) = pack8(v + q * 8);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) out += v[j] * __ldg(w4 + c * 32 + j);
-        }
-        if (A && s0 + r < n) {
-          uint4* dst = reinterpret_cast<uint4*>(A + ((size_t)l * n + s0 + r) * F + c * 32);
-#pragma unroll
-          for (int q = 0; q < 4; ++q) dst[q] = pack8(v + q * 8);
-        }
-      }
+      out = layer_epilogue(tmem, s_b + l * F, l < 2 ? act : nullptr, l == 2 ? s_w4 : nullptr, s_out);
       fence_before();
       fence_async_smem();
       __syncthreads();
       fence_after();
     }
-    if (ok) {
-      const int r = warp * 32 + lane;
-      if (s0 + r < n) y[s0 + r] = out + __ldg(b4);
-    }
+    if (ok && tid >= TILE && s0 + tid - TILE < n) y[s0 + tid - TILE] = out + __ldg(P4 + 4 * F);
   }
   if (!ok) {
     sm->fail = 1;
@@ -318,40 +343,95 @@ __global__ void __launch_bounds__(128, 1)
   if (warp == 0) tmem_dealloc(tmem, 128);
 }
 
+// Column sums of a tile in sample order (the order is part of the result:
+// Adam turns the last bit of a small gradient into a step).  Thread c < 128
+// sums column c.  Eight columns share 16 bytes, and the four such groups of
+// a warp lie on the same banks for one sample, so group g runs g samples
+// behind: the four read different rows of the core matrices, without
+// conflicts.
+__device__ __forceinline__ float column_sum(const uint8_t* tile) {
+  const int c = threadIdx.x & (TILE - 1), lag = (threadIdx.x & 31) >> 3;
+  float sum = 0.f;
+#pragma unroll 8
+  for (int k = 0; k < TILE + 3; ++k) {
+    const int r = k - lag;
+    if (r >= 0 && r < TILE) sum += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(tile + tile_off(r, c)));
+  }
+  return sum;
+}
+
+// Weighted column sums sum_s w_s tile[s][c] of a tile's halves h of 64
+// samples (w in shared memory) to s_part[h][c]: the samples of each 32 add up
+// as a butterfly does (16 apart, then 8, 4, 2, 1), and the two 32s of a half.
+// Thread (h, j, q) has the samples 64 h + 8 i + q of the columns 8 j .. 8 j + 7.
+__device__ __forceinline__ void weighted_column_sums(const uint8_t* tile, const float* w, float* s_part) {
+  const int q = threadIdx.x & 7, j = (threadIdx.x >> 3) & 15, h = threadIdx.x >> 7;
+  float a[2][8];
+#pragma unroll
+  for (int g = 0; g < 2; ++g) {
+    float v[4][8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = 64 * h + 32 * g + 8 * i + q;
+      const uint4 raw = *reinterpret_cast<const uint4*>(tile + tile_off(r, 8 * j));
+      const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(&raw);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[i][k] = __fmul_rn(w[r], __bfloat162float(hb[k]));
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) a[g][k] = (v[0][k] + v[2][k]) + (v[1][k] + v[3][k]);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+      for (int k = 0; k < 8; ++k) a[g][k] += __shfl_xor_sync(0xffffffffu, a[g][k], o);
+  }
+  if (q == 0)
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s_part[h * F + 8 * j + k] = a[0][k] + a[1][k];
+}
+
 // ---------------------------------------------------------------------------
-// Backward.  Each CTA runs the sample tiles blockIdx.x, blockIdx.x +
-// gridDim.x, ...; the three weight gradients accumulate in tensor memory
-// across its tiles (gW_l in columns [128 l, 128 l + 128), the back-propagated
-// dH of the current layer in [384, 512)); the bias, w4 and b4 gradients and
-// the loss accumulate in shared memory and registers.  At the end the CTA
-// writes its sums as row blockIdx.x of Gp [gridDim.x][NG_STRIDE], laid out as G =
-// [gW (3x128x128) | gb (3x128) | gw4 (128) | gb4 (1) | loss (1)]; k_mlp_reduce
-// adds the rows in a fixed order (no atomics in global memory, the same
-// gradient bits on every run).  WTt: the transposed weight tiles (layers 1
-// and 2 are staged once per CTA by bulk copies); A the forward activations;
-// t the targets.
+// Gradients: forward and backward of a batch in one kernel.  Each CTA runs
+// the sample tiles blockIdx.x, blockIdx.x + gridDim.x, ...  A tile's
+// activations stay in shared memory (X, a_1, a_2; a_3 takes W_1's place,
+// which is staged again for the next tile, and the deltas d_3, d_2, d_1 take
+// a_3's), and the transposed products read the same tiles as MN-major
+// operands.  The three weight gradients accumulate in tensor memory across
+// the CTA's tiles (gW_l in columns [128 l, 128 l + 128); z and dH of the
+// current layer in [384, 512)); the bias, w4 and b4 gradients and the loss
+// accumulate in shared memory and registers.  At the end the CTA writes its
+// sums as row blockIdx.x of Gp [gridDim.x][NG_STRIDE], laid out as G =
+// [gW (3x128x128) | gb (3x128) | gw4 (128) | gb4 (1) | loss (1)]; the rows
+// are added in a fixed order (no atomics in global memory, the same gradient
+// bits on every run).
+// Bound by the chain of a tile (six products with their epilogues, about
+// 2 us each): at 8,192 samples 64 CTAs have one tile each.  The separate
+// forward (19.5 us) and backward (70.7 us: explicit 2-byte transposes of d
+// and a, 640 shuffles for gw4, 2-byte loads of the activations) took 90 us
+// for such a batch.
 constexpr int NG_ROW = 3 * F * F + 3 * F + F + 1 + 1;
 // rows of Gp start on 16-byte boundaries (the weight gradients are stored as
 // float4)
 constexpr int NG_STRIDE = (NG_ROW + 3) & ~3;
 
-__global__ void __launch_bounds__(128, 1)
-    k_mlp_bwd(const __nv_bfloat16* __restrict__ X, int n, const __nv_bfloat16* __restrict__ WTt,
-              const float* __restrict__ w4, const __nv_bfloat16* __restrict__ A, const float* __restrict__ y,
-              const float* __restrict__ t, float inv_n, float* __restrict__ Gp, int* err) {
+__global__ void __launch_bounds__(THREADS, 1)
+    k_mlp_grad(const __nv_bfloat16* __restrict__ X, int n, const __nv_bfloat16* __restrict__ Wt,
+               const float* __restrict__ P4, const float* __restrict__ t, float inv_n, float* __restrict__ Gp, int* err) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* dT = base;                   // A operand of gW: d^T  (rows = out, K = samples)
-  uint8_t* aT = base + TILE_BYTES;      // B operand of gW: a^T  (rows = in,  K = samples)
-  uint8_t* dN = base + 2 * TILE_BYTES;  // A operand of dH: d    (rows = samples, K = out)
-  uint8_t* wN1 = base + 3 * TILE_BYTES;  // B operand of dH for layer 1: W_1^T (rows = in, K = out)
-  uint8_t* wN2 = base + 4 * TILE_BYTES;  // the same for layer 2
-  // bias and w4 gradients, each entry owned by one thread (fixed summation
-  // order: the gradients come out the same on every run)
-  float* s_gb = reinterpret_cast<float*>(base + 5 * TILE_BYTES);  // [3][128] bias gradients
-  float* s_gw4 = s_gb + 3 * F;                                     // [128]
-  float* s_gw4w = s_gw4 + F;                                       // [4][128] the tile's per-warp w4 sums
-  float* s_red = s_gw4w + 4 * F;                                   // [2][4] per-warp gb4 and loss
+  uint8_t* tD = base;                       // W_1, then a_3, then the deltas
+  uint8_t* tW2 = base + TILE_BYTES;
+  uint8_t* tW3 = base + 2 * TILE_BYTES;
+  uint8_t* tX = base + 3 * TILE_BYTES;
+  uint8_t* tA1 = base + 4 * TILE_BYTES;
+  uint8_t* tA2 = base + 5 * TILE_BYTES;
+  float* s_b = reinterpret_cast<float*>(base + 6 * TILE_BYTES);  // [3][128] biases
+  float* s_w4 = s_b + 3 * F;                                      // [128]
+  float* s_out = s_w4 + F;                                        // [128]
+  float* s_dy = s_out + F;                                        // [128]
+  float* s_g = s_dy + F;         // [4][128] gradient sums gb_1, gb_2, gb_3, gw4, each entry one thread's
+  float* s_part = s_g + 4 * F;   // [2][128] the tile's gw4 by halves
+  float* s_red = s_part + 2 * F;  // [2][4] per-warp gb4 and loss
   SmemW* sm = reinterpret_cast<SmemW*>(s_red + 8);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ntiles = (n + TILE - 1) / TILE;
@@ -360,140 +440,139 @@ __global__ void __launch_bounds__(128, 1)
     mbar_init(&sm->bar, 1);
     mbar_init(&sm->bar_w, 1);
     sm->fail = 0;
-    mbar_expect_tx(&sm->bar_w, 2 * TILE_BYTES);
-    bulk_tile(wN1, WTt + (size_t)1 * F * F, &sm->bar_w);
-    bulk_tile(wN2, WTt + (size_t)2 * F * F, &sm->bar_w);
+    mbar_expect_tx(&sm->bar_w, 3 * TILE_BYTES);
+    bulk_tile(tD, Wt, &sm->bar_w);
+    bulk_tile(tW2, Wt + (size_t)F * F, &sm->bar_w);
+    bulk_tile(tW3, Wt + (size_t)2 * F * F, &sm->bar_w);
   }
-  for (int i = tid; i < 4 * F; i += blockDim.x) s_gb[i] = 0.f;  // s_gb and s_gw4
+  for (int i = tid; i < 4 * F; i += THREADS) s_b[i] = __ldg(P4 + i);  // b and w4
+  for (int i = tid; i < 4 * F; i += THREADS) s_g[i] = 0.f;
   __syncwarp();
   if (warp == 0) tmem_alloc(&sm->tmem, 512);
   fence_before();
   __syncthreads();
   fence_after();
-  const uint32_t tm = sm->tmem;
-  const int r = tid;                // sample row of this thread in the operand phase
-  const int rr = warp * 32 + lane;  // accumulator row of this thread (the same index)
-  const uint32_t trow = tm + ((uint32_t)(warp * 32) << 16);
-  float gb4_acc = 0.f, loss_acc = 0.f;
-  uint32_t phase = 0;
-  bool ok = true, weights = false, mma_pending = false, first = true;
-  for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-    const int s0 = tile * TILE;
-    const int s = s0 + r;
-    const bool valid = s < n;
-    // output layer
-    float dy = 0.f;
-    if (valid) {
-      const float e = y[s] - t[s];
-      dy = e * inv_n;
-      loss_acc += 0.5f * e * e * inv_n;
-    }
-    gb4_acc += dy;
-    // d_3 = bf16(dy w4 [a_3 > 0]); its column sums are gb_3
-    const __nv_bfloat16* a3 = A + ((size_t)2 * n + (valid ? s : s0)) * F;
-    for (int c = 0; c < F; c += 8) {
-      float av[8], dv[8];
-      if (valid) {
-        const uint4 raw = __ldg(reinterpret_cast<const uint4*>(a3 + c));
-        const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(&raw);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) av[j] = __bfloat162float(hb[j]);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) av[j] = 0.f;
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) dv[j] = bf16r(av[j] > 0.f ? dy * __ldg(w4 + c + j) : 0.f);
-      *reinterpret_cast<uint4*>(dN + tile_off(r, c)) = pack8(dv);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) *reinterpret_cast<__nv_bfloat16*>(dT + tile_off(c + j, r)) = __float2bfloat16_rn(dv[j]);
-    }
-    // gw4[j] += sum_r dy_r a3[r][j]: warp sums through shuffles, added up
-    // per column after the next barrier
-    for (int c = 0; c < F; ++c) {
-      float v = valid ? dy * __bfloat162float(a3[c]) : 0.f;
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == 0) s_gw4w[warp * F + c] = v;
-    }
-    for (int l = 2; l >= 0 && ok; --l) {
-      // B operand of gW_l: a_{l-1}^T (a_0 = X)
-      {
-        const __nv_bfloat16* src = l == 0 ? (X + (size_t)(valid ? s : s0) * F)
-                                          : (A + ((size_t)(l - 1) * n + (valid ? s : s0)) * F);
-        for (int c = 0; c < F; c += 8) {
-          uint4 raw = valid ? __ldg(reinterpret_cast<const uint4*>(src + c)) : make_uint4(0, 0, 0, 0);
-          const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(&raw);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) *reinterpret_cast<__nv_bfloat16*>(aT + tile_off(c + j, r)) = hb[j];
-        }
-      }
-      fence_async_smem();
-      fence_before();
-      __syncthreads();
-      fence_after();
-      if (!weights) {
-        ok = __syncthreads_and(mbar_wait(&sm->bar_w, 0)) != 0;
-        weights = ok;
-        if (!ok) break;
-      }
-      // gb_l: thread tid sums row tid of d^T (the tile's samples in order;
-      // padding samples are zero); the tensor cores only read dT meanwhile
-      {
-        float sum = 0.f;
-        for (int k = 0; k < TILE; k += 8) {
-          const uint4 raw = *reinterpret_cast<const uint4*>(dT + tile_off(tid, k));
-          const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(&raw);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) sum += __bfloat162float(hb[j]);
-        }
-        s_gb[l * F + tid] += sum;
-        if (l == 2) s_gw4[tid] += (s_gw4w[tid] + s_gw4w[F + tid]) + (s_gw4w[2 * F + tid] + s_gw4w[3 * F + tid]);
-      }
-      if (tid == 0) {
-        mma_tile_acc(tm + l * 128, dT, aT, !first);                   // gW_l (+)= d_l^T a_{l-1}
-        if (l > 0) mma_tile_acc(tm + 384, dN, l == 2 ? wN2 : wN1, false);  // dH = d_l W_l
-        mma_commit(&sm->bar);
-      }
-      mma_pending = true;
-      ok = __syncthreads_and(mbar_wait(&sm->bar, phase)) != 0;
-      if (!ok) break;
+  const uint32_t tm = sm->tmem, tz = tm + 384;
+  const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+  const int r = (warp & 3) * 32 + lane;  // sample row of this thread
+  const int c0 = (warp >> 2) * 64;       // and its first column
+  const float b4 = __ldg(P4 + 4 * F);
+  float gb4_acc = 0.f, loss_acc = 0.f;  // warps 4-7
+  uint32_t phase = 0, phase_w = 0;
+  bool ok = true, w_pending = true, mma_pending = false, first = true;
+  // one group of MMAs issued by thread 0, waited for by all
+  auto finish = [&]() {
+    mma_pending = true;
+    ok = __syncthreads_and(mbar_wait(&sm->bar, phase)) != 0;
+    if (ok) {
       mma_pending = false;
       phase ^= 1;
       fence_after();
-      if (l > 0) {
-        // d_{l-1} for sample rr = bf16(dH * [a_{l-1} > 0]); its column sums are gb_{l-1}
-        const int sr = s0 + rr;
-        const bool vr = sr < n;
-        const __nv_bfloat16* ap = A + ((size_t)(l - 1) * n + (vr ? sr : s0)) * F;
-        for (int c = 0; c < F / 32; ++c) {
-          float v[32];
-          tmem_ld32(trow + 384 + c * 32, v);
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float a = vr ? __bfloat162float(ap[c * 32 + j]) : 0.f;
-            v[j] = bf16r(a > 0.f ? v[j] : 0.f);
-          }
-#pragma unroll
-          for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(dN + tile_off(rr, c * 32 + q * 8)) = pack8(v + q * 8);
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            *reinterpret_cast<__nv_bfloat16*>(dT + tile_off(c * 32 + j, rr)) = __float2bfloat16_rn(v[j]);
-        }
-      }
-      fence_before();
-      __syncthreads();
-      fence_after();
     }
+    return ok;
+  };
+  // generic writes to the tiles, before the tensor cores (or a bulk copy) use them
+  auto publish = [&]() {
+    fence_async_smem();
+    fence_before();
+    __syncthreads();
+    fence_after();
+  };
+  for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+    const int s0 = tile * TILE;
+    if (!first && tid == 0) {
+      // (the deltas' last product is done and the barrier after it passed)
+      mbar_expect_tx(&sm->bar_w, TILE_BYTES);
+      bulk_tile(tD, Wt, &sm->bar_w);
+    }
+    w_pending = true;
+    const bool valid = s0 + r < n;
+    const float tv = warp >= 4 && valid ? __ldg(t + s0 + r) : 0.f;
+    load_rows(tX, X, s0, n);
+    publish();
+    ok = __syncthreads_and(mbar_wait(&sm->bar_w, phase_w)) != 0;
+    if (!ok) break;
+    w_pending = false;
+    phase_w ^= 1;
+    // forward
+    float out = 0.f;
+    for (int l = 0; l < 3; ++l) {
+      if (tid == 0) {
+        mma_tile(tz, l == 0 ? tX : l == 1 ? tA1 : tA2, false, l == 0 ? tD : l == 1 ? tW2 : tW3, false, false);
+        mma_commit(&sm->bar);
+      }
+      if (!finish()) break;
+      out = layer_epilogue(tz, s_b + l * F, l == 0 ? tA1 : l == 1 ? tA2 : tD, l == 2 ? s_w4 : nullptr, s_out);
+      if (l < 2) publish();
+    }
+    if (!ok) break;
+    // output layer
+    if (warp >= 4) {
+      float dy = 0.f;
+      if (valid) {
+        const float e = (out + b4) - tv;
+        dy = e * inv_n;
+        loss_acc += 0.5f * e * e * inv_n;
+      }
+      gb4_acc += dy;
+      s_dy[r] = dy;
+    }
+    __syncthreads();
+    weighted_column_sums(tD, s_dy, s_part);
+    __syncthreads();
+    if (tid < F) s_g[3 * F + tid] += s_part[tid] + s_part[F + tid];  // gw4
+    // d_3 = bf16(dy w4 [a_3 > 0]) over a_3
+    {
+      const float dy = s_dy[r];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        uint4* p = reinterpret_cast<uint4*>(tD + tile_off(r, c0 + q * 8));
+        const uint4 raw = *p;
+        const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(&raw);
+        float dv[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) dv[k] = __bfloat162float(hb[k]) > 0.f ? dy * s_w4[c0 + q * 8 + k] : 0.f;
+        *p = pack8(dv);
+      }
+    }
+    publish();
+    for (int l = 2; l >= 0; --l) {
+      const uint8_t* below = l == 2 ? tA2 : l == 1 ? tA1 : tX;  // a_l, the layer's input
+      if (tid == 0) {
+        mma_tile(tm + l * 128, tD, true, below, true, !first);                            // gW_l (+)= d^T a_l
+        if (l > 0) mma_tile(tz, tD, false, l == 2 ? tW3 : tW2, true, false);  // dH = d W
+        mma_commit(&sm->bar);
+      }
+      if (tid < F) s_g[l * F + tid] += column_sum(tD);  // gb_l, while the tensor cores read the same tile
+      if (!finish()) break;
+      if (l > 0) {
+        // the next delta, bf16(dH [a_l > 0])
+        float v[64];
+        tmem_ld32(tz + lanes + c0, v);
+        tmem_ld32(tz + lanes + c0 + 32, v + 32);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const uint4 raw = *reinterpret_cast<const uint4*>(below + tile_off(r, c0 + q * 8));
+          const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(&raw);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) v[q * 8 + k] = __bfloat162float(hb[k]) > 0.f ? v[q * 8 + k] : 0.f;
+          *reinterpret_cast<uint4*>(tD + tile_off(r, c0 + q * 8)) = pack8(v + q * 8);
+        }
+        publish();
+      }
+    }
+    if (!ok) break;
+    publish();  // before the next tile's copies land over this one's
     first = false;
   }
   if (ok) {
     float* row = Gp + (size_t)blockIdx.x * NG_STRIDE;
-    // weight gradients: row rr of each gW_l from tensor memory
+    // weight gradients: row r's 64 columns of each gW_l from tensor memory
     for (int l = 0; l < 3; ++l)
-      for (int c = 0; c < F / 32; ++c) {
+      for (int c = 0; c < 64; c += 32) {
         float v[32];
-        tmem_ld32(trow + l * 128 + c * 32, v);
-        float4* dst = reinterpret_cast<float4*>(row + ((size_t)l * F + rr) * F + c * 32);
+        tmem_ld32(tm + lanes + l * 128 + c0 + c, v);
+        float4* dst = reinterpret_cast<float4*>(row + ((size_t)l * F + r) * F + c0 + c);
 #pragma unroll
         for (int q = 0; q < 8; ++q) dst[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
       }
@@ -501,12 +580,13 @@ __global__ void __launch_bounds__(128, 1)
       gb4_acc += __shfl_xor_sync(0xffffffffu, gb4_acc, o);
       loss_acc += __shfl_xor_sync(0xffffffffu, loss_acc, o);
     }
-    if (lane == 0) {
-      s_red[warp] = gb4_acc;
-      s_red[4 + warp] = loss_acc;
+    if (lane == 0 && warp >= 4) {
+      s_red[warp - 4] = gb4_acc;
+      s_red[warp] = loss_acc;
     }
     __syncthreads();
-    for (int i = tid; i < 4 * F; i += blockDim.x) row[3 * F * F + i] = s_gb[i];  // gb and gw4
+    // gb and gw4
+    for (int i = tid; i < 4 * F; i += THREADS) row[3 * F * F + i] = s_g[i];
     if (tid == 0) {
       row[3 * F * F + 4 * F] = (s_red[0] + s_red[1]) + (s_red[2] + s_red[3]);
       row[3 * F * F + 4 * F + 1] = (s_red[4] + s_red[5]) + (s_red[6] + s_red[7]);
@@ -514,48 +594,83 @@ __global__ void __launch_bounds__(128, 1)
   } else {
     sm->fail = 1;
     if (err) atomicExch(err, 1);
-    if (!weights) mbar_wait(&sm->bar_w, 0);
+    // drain (bounded) before the tensor memory goes
+    if (w_pending) mbar_wait(&sm->bar_w, phase_w);
     if (mma_pending) mbar_wait(&sm->bar, phase);
   }
   fence_before();
   __syncthreads();
   fence_after();
-  if (warp == 0) tmem_dealloc(sm->tmem, 512);
+  if (warp == 0) tmem_dealloc(tm, 512);
 }
 
-// G[i] = sum over the rows of Gp (fixed order); the loss of the batch is
-// also added to *loss_acc when it is given (the epoch's sum on the device).
-__global__ void k_mlp_reduce(const float* __restrict__ Gp, int rows, float* __restrict__ G, float* loss_acc) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NG_ROW; i += gridDim.x * blockDim.x) {
-    float sum = 0.f;
-    for (int r = 0; r < rows; ++r) sum += Gp[(size_t)r * NG_STRIDE + i];
-    G[i] = sum;
-    if (loss_acc && i == NG_ROW - 1) *loss_acc += sum;
+// Sum of column i over the rows of Gp, in row order.
+__device__ __forceinline__ float row_sum(const float* __restrict__ Gp, int rows, int i) {
+  float sum = 0.f;
+  int r = 0;
+  for (; r + 8 <= rows; r += 8) {
+    float v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = __ldg(Gp + (size_t)(r + k) * NG_STRIDE + i);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) sum += v[k];
   }
+  for (; r < rows; ++r) sum += __ldg(Gp + (size_t)r * NG_STRIDE + i);
+  return sum;
+}
+
+// G[i] = sum over the rows of Gp (fixed order).
+__global__ void k_mlp_reduce(const float* __restrict__ Gp, int rows, float* __restrict__ G) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NG_ROW; i += gridDim.x * blockDim.x)
+    G[i] = row_sum(Gp, rows, i);
 }
 
 // ---------------------------------------------------------------------------
-// Adam on the fp32 master parameters P = [W (3x128x128) | b (3x128) | w4 |
-// b4]; refreshes the BF16 weight tiles.
-__global__ void k_adam(float* __restrict__ P, const float* __restrict__ G, float* __restrict__ M1,
+// Gradient reduction and Adam in one pass: each thread adds up its
+// parameter's rows of Gp (fixed order) and steps the fp32 master parameter P
+// = [W (3x128x128) | b (3x128) | w4 | b4], refreshing the BF16 weight tiles;
+// the batch's loss is added to *loss_acc (the epoch's sum on the device).
+__global__ void k_adam(float* __restrict__ P, const float* __restrict__ Gp, int rows, float* __restrict__ M1,
                        float* __restrict__ M2, int np, float lr, float b1, float b2, float eps, float c1, float c2,
-                       __nv_bfloat16* __restrict__ Wt, __nv_bfloat16* __restrict__ WTt) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
-    const float g = G[i];
-    const float m = b1 * M1[i] + (1.f - b1) * g;
-    const float v = b2 * M2[i] + (1.f - b2) * g * g;
-    M1[i] = m;
-    M2[i] = v;
-    const float p = P[i] - lr * (m * c1) / (sqrtf(v * c2) + eps);
-    P[i] = p;
-    if (i < 3 * F * F) store_weight(Wt, WTt, i, p);
+                       __nv_bfloat16* __restrict__ Wt, float* __restrict__ loss_acc) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= NG_ROW) return;
+  const float g = row_sum(Gp, rows, i);
+  if (i >= np) {
+    *loss_acc += g;
+    return;
   }
+  const float m = b1 * M1[i] + (1.f - b1) * g;
+  const float v = b2 * M2[i] + (1.f - b2) * g * g;
+  M1[i] = m;
+  M2[i] = v;
+  const float p = P[i] - lr * (m * c1) / (sqrtf(v * c2) + eps);
+  P[i] = p;
+  if (i < 3 * F * F) store_weight(Wt, i, p);
 }
 
-__global__ void k_pack_weights(const float* __restrict__ P, __nv_bfloat16* __restrict__ Wt,
-                               __nv_bfloat16* __restrict__ WTt) {
+__global__ void k_pack_weights(const float* __restrict__ P, __nv_bfloat16* __restrict__ Wt) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * F * F; i += gridDim.x * blockDim.x)
-    store_weight(Wt, WTt, i, P[i]);
+    store_weight(Wt, i, P[i]);
+}
+
+// BF16 copies of fp32 values, four per thread at a time; vec: both arrays
+// start on a boundary of four values.  `in` may be the caller's host array
+// where the GPU can read it: the conversion then costs the transfer alone.
+__global__ void k_to_bf16(const float* __restrict__ in, size_t n, int vec, __nv_bfloat16* __restrict__ out) {
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; 4 * i < n; i += stride) {
+    if (vec && 4 * i + 4 <= n) {
+      const float4 v = *reinterpret_cast<const float4*>(in + 4 * i);
+      __nv_bfloat162 p[2] = {__floats2bfloat162_rn(v.x, v.y), __floats2bfloat162_rn(v.z, v.w)};
+      *reinterpret_cast<uint2*>(out + 4 * i) = *reinterpret_cast<uint2*>(p);
+    } else {
+      float v[4];
+      for (int k = 0; k < 4; ++k) v[k] = 4 * i + k < n ? in[4 * i + k] : 0.f;
+      for (int k = 0; k < 4; ++k)
+        if (4 * i + k < n) out[4 * i + k] = __float2bfloat16_rn(v[k]);
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -636,8 +751,9 @@ namespace {
 constexpr int NP = 3 * F * F + 3 * F + F + 1;  // master parameters
 constexpr int NG = NP + 1;                      // gradients + loss
 static_assert(NG == NG_ROW, "gradient row layout");
-size_t fwd_smem() { return 4 * (size_t)TILE_BYTES + 1024 + 64; }
-size_t bwd_smem() { return 5 * (size_t)TILE_BYTES + (8 * F + 8) * sizeof(float) + 1024 + 64; }
+size_t fwd_smem() { return 4 * (size_t)TILE_BYTES + 5 * F * sizeof(float) + 1024 + 64; }
+size_t grad_smem() { return 6 * (size_t)TILE_BYTES + (12 * F + 8) * sizeof(float) + 1024 + 64; }
+size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 }  // namespace
 
 #define MLP_TRY(expr, what)                                                     \
@@ -647,6 +763,8 @@ size_t bwd_smem() { return 5 * (size_t)TILE_BYTES + (8 * F + 8) * sizeof(float) 
   } while (0)
 
 Net::~Net() {
+  if (ws_) cudaFree(ws_);
+  if (h_end_) cudaFreeHost(h_end_);
   for (void* p : allocs_) cudaFree(p);
   if (PX_) cudaFree(PX_);
   if (PT_) cudaFree(PT_);
@@ -666,14 +784,16 @@ std::string Net::init(unsigned long long seed) {
   MLP_TRY(alloc((void**)&M1_, sizeof(float) * NP), "alloc");
   MLP_TRY(alloc((void**)&M2_, sizeof(float) * NP), "alloc");
   MLP_TRY(alloc((void**)&Wb_, sizeof(__nv_bfloat16) * 3 * F * F), "alloc");
-  MLP_TRY(alloc((void**)&WTb_, sizeof(__nv_bfloat16) * 3 * F * F), "alloc");
-  MLP_TRY(alloc((void**)&err_, sizeof(int)), "alloc");
-  MLP_TRY(alloc((void**)&loss_acc_, sizeof(float)), "alloc");
+  // the error word, then the epoch's loss: read together
+  MLP_TRY(alloc((void**)&err_, 2 * sizeof(int)), "alloc");
+  loss_acc_ = reinterpret_cast<float*>(err_ + 1);
+  MLP_TRY(cudaMallocHost((void**)&h_end_, 2 * sizeof(int)), "pinned");
   {
     int dev = 0;
     MLP_TRY(cudaGetDevice(&dev), "device");
     MLP_TRY(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev), "device");
     if (sms_ < 1) sms_ = 1;
+    if (cudaDeviceGetAttribute(&pageable_, cudaDevAttrPageableMemoryAccess, dev) != cudaSuccess) pageable_ = 0;
   }
   // one partial-gradient row per backward CTA (at most one CTA per SM)
   MLP_TRY(alloc((void**)&Gp_, sizeof(float) * (size_t)NG_STRIDE * sms_), "alloc");
@@ -681,7 +801,7 @@ std::string Net::init(unsigned long long seed) {
   MLP_TRY(cudaMemsetAsync(M2_, 0, sizeof(float) * NP, stream_), "memset");
   MLP_TRY(cudaMemsetAsync(err_, 0, sizeof(int), stream_), "memset");
   MLP_TRY(cudaFuncSetAttribute(k_mlp_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem()), "attr");
-  MLP_TRY(cudaFuncSetAttribute(k_mlp_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bwd_smem()), "attr");
+  MLP_TRY(cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grad_smem()), "attr");
   // He-uniform initialisation of the weights, zero biases
   std::mt19937_64 rng(seed);
   std::vector<float> p(NP, 0.f);
@@ -695,7 +815,7 @@ std::string Net::init(unsigned long long seed) {
 
 std::string Net::set_params(const float* host) {
   MLP_TRY(cudaMemcpyAsync(P_, host, sizeof(float) * NP, cudaMemcpyHostToDevice, stream_), "h2d");
-  k_pack_weights<<<96, 256, 0, stream_>>>(P_, Wb_, WTb_);
+  k_pack_weights<<<96, 256, 0, stream_>>>(P_, Wb_);
   MLP_TRY(cudaGetLastError(), "pack");
   MLP_TRY(cudaMemsetAsync(M1_, 0, sizeof(float) * NP, stream_), "memset");
   MLP_TRY(cudaMemsetAsync(M2_, 0, sizeof(float) * NP, stream_), "memset");
@@ -712,135 +832,142 @@ std::string Net::get_params(float* host) {
 
 int Net::num_params() { return NP; }
 
-std::string Net::check_err() {
-  int e = 0;
-  MLP_TRY(cudaMemcpyAsync(&e, err_, sizeof(int), cudaMemcpyDeviceToHost, stream_), "d2h");
+// Waits for the stream; the error word and, when given, the epoch's loss.
+std::string Net::finish(float* loss) {
+  MLP_TRY(cudaMemcpyAsync(h_end_, err_, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream_), "d2h");
   MLP_TRY(cudaStreamSynchronize(stream_), "sync");
-  if (e) {
+  if (loss) std::memcpy(loss, h_end_ + 1, sizeof(float));
+  if (h_end_[0]) {
     cudaMemsetAsync(err_, 0, sizeof(int), stream_);
     return "tensor-core wait timed out";
   }
   return "";
 }
 
-std::string Net::forward_dev(const __nv_bfloat16* X, int n, const int* n_dev, int max_n, float* y,
-                             __nv_bfloat16* acts, cudaStream_t st) {
+// Workspace of the host-buffer entry points: grown to the largest call, kept
+// up to kWorkspaceKeep bytes (trim, with the stream idle).
+char* Net::workspace(size_t bytes) {
+  if (bytes > ws_bytes_) {
+    if (ws_) cudaFree(ws_);
+    ws_ = nullptr;
+    ws_bytes_ = 0;
+    if (cudaMalloc((void**)&ws_, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      ws_ = nullptr;
+      return nullptr;
+    }
+    ws_bytes_ = bytes;
+  }
+  return ws_;
+}
+std::string Net::trim(std::string r) {
+  if (ws_bytes_ > kWorkspaceKeep) {
+    cudaStreamSynchronize(stream_);
+    cudaFree(ws_);
+    ws_ = nullptr;
+    ws_bytes_ = 0;
+  }
+  return r;
+}
+size_t Net::staging_bytes(size_t n) const { return pageable_ ? 0 : align256(n * F * sizeof(float)); }
+
+// Host rows -> BF16 on the device, through the GPU's own access to the
+// caller's array where it has it, otherwise through `staging`.
+std::string Net::upload_rows(const float* Xh, size_t n, __nv_bfloat16* X, char* staging) {
+  const float* src = Xh;
+  if (!pageable_) {
+    MLP_TRY(cudaMemcpyAsync(staging, Xh, sizeof(float) * n * F, cudaMemcpyHostToDevice, stream_), "h2d");
+    src = reinterpret_cast<const float*>(staging);
+  }
+  const size_t quads = (n * F + 3) / 4;
+  const int grid = (int)std::min<size_t>((quads + 255) / 256, (size_t)sms_ * 8);
+  k_to_bf16<<<grid, 256, 0, stream_>>>(src, n * F, (reinterpret_cast<uintptr_t>(src) & 15) == 0, X);
+  MLP_TRY(cudaGetLastError(), "conversion");
+  return "";
+}
+
+std::string Net::forward_dev(const __nv_bfloat16* X, int n, const int* n_dev, int max_n, float* y, cudaStream_t st) {
   // one CTA per SM at most, each over several sample tiles (the weights are
   // staged once per CTA)
   const int tiles = (max_n + TILE - 1) / TILE;
   const int grid = tiles < sms_ ? tiles : sms_;
   if (grid <= 0) return "";
-  k_mlp_fwd<<<grid, 128, fwd_smem(), st>>>(X, n, n_dev, Wb_, P_ + 3 * F * F, P_ + 3 * F * F + 3 * F,
-                                            P_ + 3 * F * F + 4 * F, y, acts, err_);
+  k_mlp_fwd<<<grid, THREADS, fwd_smem(), st>>>(X, n, n_dev, Wb_, P_ + 3 * F * F, y, err_);
   MLP_TRY(cudaGetLastError(), "mlp forward");
   return "";
 }
 
-std::string Net::backward_dev(const __nv_bfloat16* X, int n, const __nv_bfloat16* acts, const float* y,
-                              const float* t, cudaStream_t st, float* loss_sink) {
+std::string Net::gradient_rows(const __nv_bfloat16* X, int n, const float* t, int* rows) {
   const int tiles = (n + TILE - 1) / TILE;
-  const int grid = tiles < sms_ ? tiles : sms_;
-  if (grid <= 0) return "";
-  k_mlp_bwd<<<grid, 128, bwd_smem(), st>>>(X, n, WTb_, P_ + 3 * F * F + 4 * F - F, acts, y, t, 1.f / n, Gp_, err_);
-  MLP_TRY(cudaGetLastError(), "mlp backward");
-  k_mlp_reduce<<<(NG + 255) / 256, 256, 0, st>>>(Gp_, grid, G_, loss_sink);
-  MLP_TRY(cudaGetLastError(), "mlp gradient reduction");
+  *rows = tiles < sms_ ? tiles : sms_;
+  if (*rows <= 0) return "";
+  k_mlp_grad<<<*rows, THREADS, grad_smem(), stream_>>>(X, n, Wb_, P_ + 3 * F * F, t, 1.f / n, Gp_, err_);
+  MLP_TRY(cudaGetLastError(), "mlp gradients");
   return "";
 }
 
 std::string Net::predict(const float* Xh, int n, float* yh) {
   if (n <= 0) return "";
-  std::vector<__nv_bfloat16> xb((size_t)n * F);
-  for (size_t i = 0; i < xb.size(); ++i) xb[i] = __float2bfloat16_rn(Xh[i]);
-  __nv_bfloat16* X = nullptr;
-  float* y = nullptr;
-  MLP_TRY(cudaMalloc(&X, sizeof(__nv_bfloat16) * xb.size()), "alloc");
-  cudaError_t e = cudaMalloc(&y, sizeof(float) * n);
-  if (e != cudaSuccess) { cudaFree(X); return std::string("alloc: ") + cudaGetErrorString(e); }
-  std::string r;
-  e = cudaMemcpyAsync(X, xb.data(), sizeof(__nv_bfloat16) * xb.size(), cudaMemcpyHostToDevice, stream_);
-  if (e == cudaSuccess) r = forward_dev(X, n, nullptr, n, y, nullptr, stream_);
-  else r = std::string("h2d: ") + cudaGetErrorString(e);
+  const size_t bx = align256(sizeof(__nv_bfloat16) * (size_t)n * F), by = align256(sizeof(float) * (size_t)n);
+  char* w = workspace(bx + by + staging_bytes(n));
+  if (!w) return "alloc";
+  __nv_bfloat16* X = reinterpret_cast<__nv_bfloat16*>(w);
+  float* y = reinterpret_cast<float*>(w + bx);
+  std::string r = upload_rows(Xh, n, X, w + bx + by);
+  if (r.empty()) r = forward_dev(X, n, nullptr, n, y, stream_);
   if (r.empty()) {
-    e = cudaMemcpyAsync(yh, y, sizeof(float) * n, cudaMemcpyDeviceToHost, stream_);
+    cudaError_t e = cudaMemcpyAsync(yh, y, sizeof(float) * n, cudaMemcpyDeviceToHost, stream_);
     if (e != cudaSuccess) r = std::string("d2h: ") + cudaGetErrorString(e);
   }
-  cudaStreamSynchronize(stream_);
-  cudaFree(X);
-  cudaFree(y);
-  if (r.empty()) r = check_err();
-  return r;
+  const std::string f = finish(nullptr);
+  return trim(r.empty() ? f : r);
 }
 
 std::string Net::gradients(const float* Xh, const float* th, int n, float* gh, float* loss) {
   if (n <= 0) return "empty batch";
-  std::vector<__nv_bfloat16> xb((size_t)n * F);
-  for (size_t i = 0; i < xb.size(); ++i) xb[i] = __float2bfloat16_rn(Xh[i]);
-  std::vector<void*> tmp;
-  auto fin = [&](const std::string& r) {
-    cudaStreamSynchronize(stream_);
-    for (void* p : tmp) cudaFree(p);
-    return r;
+  const size_t bx = align256(sizeof(__nv_bfloat16) * (size_t)n * F), bt = align256(sizeof(float) * (size_t)n);
+  char* w = workspace(bx + bt + staging_bytes(n));
+  if (!w) return "alloc";
+  __nv_bfloat16* X = reinterpret_cast<__nv_bfloat16*>(w);
+  float* t = reinterpret_cast<float*>(w + bx);
+  auto body = [&]() -> std::string {
+    std::string r = upload_rows(Xh, n, X, w + bx + bt);
+    if (!r.empty()) return r;
+    MLP_TRY(cudaMemcpyAsync(t, th, sizeof(float) * n, cudaMemcpyHostToDevice, stream_), "h2d");
+    int rows = 0;
+    r = gradient_rows(X, n, t, &rows);
+    if (!r.empty()) return r;
+    k_mlp_reduce<<<(NG + 255) / 256, 256, 0, stream_>>>(Gp_, rows, G_);
+    MLP_TRY(cudaGetLastError(), "mlp gradient reduction");
+    MLP_TRY(cudaMemcpyAsync(gh, G_, sizeof(float) * NP, cudaMemcpyDeviceToHost, stream_), "d2h");
+    MLP_TRY(cudaMemcpyAsync(loss_acc_, G_ + NP, sizeof(float), cudaMemcpyDeviceToDevice, stream_), "loss");
+    return "";
   };
-  __nv_bfloat16 *X = nullptr, *Aa = nullptr;
-  float *y = nullptr, *t = nullptr;
-  if (cudaMalloc(&X, sizeof(__nv_bfloat16) * xb.size()) != cudaSuccess) return fin("alloc");
-  tmp.push_back(X);
-  if (cudaMalloc(&Aa, sizeof(__nv_bfloat16) * 3 * (size_t)n * F) != cudaSuccess) return fin("alloc");
-  tmp.push_back(Aa);
-  if (cudaMalloc(&y, sizeof(float) * n) != cudaSuccess) return fin("alloc");
-  tmp.push_back(y);
-  if (cudaMalloc(&t, sizeof(float) * n) != cudaSuccess) return fin("alloc");
-  tmp.push_back(t);
-  cudaMemcpyAsync(X, xb.data(), sizeof(__nv_bfloat16) * xb.size(), cudaMemcpyHostToDevice, stream_);
-  cudaMemcpyAsync(t, th, sizeof(float) * n, cudaMemcpyHostToDevice, stream_);
-  cudaMemsetAsync(G_, 0, sizeof(float) * NG, stream_);
-  std::string r = forward_dev(X, n, nullptr, n, y, Aa, stream_);
-  if (r.empty()) r = backward_dev(X, n, Aa, y, t, stream_);
-  if (!r.empty()) return fin(r);
-  cudaMemcpyAsync(gh, G_, sizeof(float) * NP, cudaMemcpyDeviceToHost, stream_);
+  std::string r = body();
   float l = 0.f;
-  cudaMemcpyAsync(&l, G_ + NP, sizeof(float), cudaMemcpyDeviceToHost, stream_);
-  r = fin("");
+  const std::string f = finish(&l);
   if (loss) *loss = l;
-  if (r.empty()) r = check_err();
-  return r;
+  return trim(r.empty() ? f : r);
 }
 
 std::string Net::train(const float* Xh, const float* th, int n, int epochs, int batch, float lr, float* last_loss) {
   if (n <= 0 || batch <= 0 || epochs <= 0) return "empty training set";
-  std::vector<__nv_bfloat16> xb((size_t)n * F);
-  for (size_t i = 0; i < xb.size(); ++i) xb[i] = __float2bfloat16_rn(Xh[i]);
-  return train_dev_upload(xb.data(), th, n, epochs, batch, lr, last_loss);
-}
-
-std::string Net::train_dev_upload(const __nv_bfloat16* xb, const float* th, int n, int epochs, int batch, float lr,
-                                  float* last_loss) {
-  std::vector<void*> tmp;
-  auto fin = [&](const std::string& r) {
-    cudaStreamSynchronize(stream_);
-    for (void* p : tmp) cudaFree(p);
-    return r;
-  };
-  __nv_bfloat16 *X = nullptr, *Aa = nullptr;
-  float *y = nullptr, *t = nullptr;
-  const int bmax = batch < n ? batch : n;
-  if (cudaMalloc(&X, sizeof(__nv_bfloat16) * (size_t)n * F) != cudaSuccess) return fin("alloc");
-  tmp.push_back(X);
-  if (cudaMalloc(&t, sizeof(float) * n) != cudaSuccess) return fin("alloc");
-  tmp.push_back(t);
-  if (cudaMalloc(&Aa, sizeof(__nv_bfloat16) * 3 * (size_t)bmax * F) != cudaSuccess) return fin("alloc");
-  tmp.push_back(Aa);
-  if (cudaMalloc(&y, sizeof(float) * bmax) != cudaSuccess) return fin("alloc");
-  tmp.push_back(y);
-  cudaMemcpyAsync(X, xb, sizeof(__nv_bfloat16) * (size_t)n * F, cudaMemcpyHostToDevice, stream_);
-  cudaMemcpyAsync(t, th, sizeof(float) * n, cudaMemcpyHostToDevice, stream_);
-  std::string r = train_device(X, t, n, epochs, batch, lr, Aa, y, last_loss);
-  return fin(r);
+  const size_t bx = align256(sizeof(__nv_bfloat16) * (size_t)n * F), bt = align256(sizeof(float) * (size_t)n);
+  char* w = workspace(bx + bt + staging_bytes(n));
+  if (!w) return "alloc";
+  __nv_bfloat16* X = reinterpret_cast<__nv_bfloat16*>(w);
+  float* t = reinterpret_cast<float*>(w + bx);
+  std::string r = upload_rows(Xh, n, X, w + bx + bt);
+  if (r.empty() &&
+      cudaMemcpyAsync(t, th, sizeof(float) * (size_t)n, cudaMemcpyHostToDevice, stream_) != cudaSuccess)
+    r = "h2d";
+  if (r.empty()) r = train_device(X, t, n, epochs, batch, lr, last_loss);
+  cudaStreamSynchronize(stream_);
+  return trim(r);
 }
 
 std::string Net::train_device(const __nv_bfloat16* X, const float* t, int n, int epochs, int batch, float lr,
-                              __nv_bfloat16* Aa, float* y, float* last_loss) {
+                              float* last_loss) {
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   float loss_sum = 0.f;
   int loss_cnt = 0;
@@ -850,24 +977,22 @@ std::string Net::train_device(const __nv_bfloat16* X, const float* t, int n, int
     loss_cnt = 0;
     for (int s0 = 0; s0 < n; s0 += batch) {
       const int m = (n - s0) < batch ? (n - s0) : batch;
-      const __nv_bfloat16* Xb = X + (size_t)s0 * F;
-      std::string r = forward_dev(Xb, m, nullptr, m, y, Aa, stream_);
-      if (r.empty()) r = backward_dev(Xb, m, Aa, y, t + s0, stream_, loss_acc_);
+      int rows = 0;
+      std::string r = gradient_rows(X + (size_t)s0 * F, m, t + s0, &rows);
       if (!r.empty()) return r;
       ++step_;
       const float c1 = 1.f / (1.f - std::pow(b1, (float)step_));
       const float c2 = 1.f / (1.f - std::pow(b2, (float)step_));
-      k_adam<<<(NP + 255) / 256, 256, 0, stream_>>>(P_, G_, M1_, M2_, NP, lr, b1, b2, eps, c1, c2, Wb_, WTb_);
+      k_adam<<<(NG + 127) / 128, 128, 0, stream_>>>(P_, Gp_, rows, M1_, M2_, NP, lr, b1, b2, eps, c1, c2, Wb_,
+                                                    loss_acc_);
       MLP_TRY(cudaGetLastError(), "adam");
       ++loss_cnt;
     }
-    MLP_TRY(cudaMemcpyAsync(&loss_sum, loss_acc_, sizeof(float), cudaMemcpyDeviceToHost, stream_), "d2h");
-    MLP_TRY(cudaStreamSynchronize(stream_), "sync");
-    std::string r = check_err();
+    std::string r = finish(&loss_sum);
     if (!r.empty()) return r;
   }
   if (last_loss) *last_loss = loss_cnt ? loss_sum / loss_cnt : 0.f;
-  return check_err();
+  return "";
 }
 
 std::string Net::reserve_pairs(long long cap) {
@@ -944,7 +1069,7 @@ std::string Net::eval_pairs(long long first, long long count, float* abs_err) {
   if (count > 0x7fffffffLL) return "too many pairs";
   float* y = nullptr;
   MLP_TRY(cudaMalloc(&y, sizeof(float) * (size_t)count), "alloc");
-  std::string r = forward_dev(PX_ + (size_t)first * F, (int)count, nullptr, (int)count, y, nullptr, stream_);
+  std::string r = forward_dev(PX_ + (size_t)first * F, (int)count, nullptr, (int)count, y, stream_);
   std::vector<float> yh((size_t)count), th((size_t)count);
   if (r.empty() &&
       (cudaMemcpyAsync(yh.data(), y, sizeof(float) * (size_t)count, cudaMemcpyDeviceToHost, stream_) != cudaSuccess ||
@@ -955,7 +1080,7 @@ std::string Net::eval_pairs(long long first, long long count, float* abs_err) {
   cudaFree(y);
   if (!r.empty()) return r;
   for (long long i = 0; i < count; ++i) abs_err[i] = std::fabs(yh[(size_t)i] - th[(size_t)i]);
-  return check_err();
+  return finish(nullptr);
 }
 
 std::string Net::train_pairs(int epochs, int batch, float lr, unsigned long long seed, float* last_loss) {
@@ -974,23 +1099,18 @@ std::string Net::train_pairs(int epochs, int batch, float lr, unsigned long long
     return r;
   };
   int* dperm = nullptr;
-  __nv_bfloat16 *Xs = nullptr, *Aa = nullptr;
-  float *ts = nullptr, *y = nullptr;
-  const int bmax = (long long)batch < n ? batch : (int)n;
+  __nv_bfloat16* Xs = nullptr;
+  float* ts = nullptr;
   if (cudaMalloc(&dperm, sizeof(int) * (size_t)n) != cudaSuccess) return fin("alloc");
   tmp.push_back(dperm);
   if (cudaMalloc(&Xs, sizeof(__nv_bfloat16) * (size_t)n * F) != cudaSuccess) return fin("alloc");
   tmp.push_back(Xs);
   if (cudaMalloc(&ts, sizeof(float) * (size_t)n) != cudaSuccess) return fin("alloc");
   tmp.push_back(ts);
-  if (cudaMalloc(&Aa, sizeof(__nv_bfloat16) * 3 * (size_t)bmax * F) != cudaSuccess) return fin("alloc");
-  tmp.push_back(Aa);
-  if (cudaMalloc(&y, sizeof(float) * bmax) != cudaSuccess) return fin("alloc");
-  tmp.push_back(y);
   cudaMemcpyAsync(dperm, perm.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, stream_);
   k_gather_pairs<<<4096, 256, 0, stream_>>>(PX_, PT_, dperm, n, Xs, ts);
   if (cudaGetLastError() != cudaSuccess) return fin("gather pairs");
-  return fin(train_device(Xs, ts, (int)n, epochs, batch, lr, Aa, y, last_loss));
+  return fin(train_device(Xs, ts, (int)n, epochs, batch, lr, last_loss));
 }
 
 }  // namespace mlp

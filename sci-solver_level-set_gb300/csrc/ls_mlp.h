@@ -27,18 +27,8 @@ class Net {
   std::string predict(const float* X, int n, float* y);
   std::string gradients(const float* X, const float* t, int n, float* g, float* loss);
   std::string train(const float* X, const float* t, int n, int epochs, int batch, float lr, float* last_loss);
-  std::string train_dev_upload(const __nv_bfloat16* X, const float* t, int n, int epochs, int batch, float lr,
-                               float* last_loss);
-  // device entry points on stream st
-  std::string forward_dev(const __nv_bfloat16* X, int n, const int* n_dev, int max_n, float* y,
-                          __nv_bfloat16* acts, cudaStream_t st);
-  // gradients of the batch into G (its loss also added to *loss_sink when
-  // given, on the device)
-  std::string backward_dev(const __nv_bfloat16* X, int n, const __nv_bfloat16* acts, const float* y, const float* t,
-                           cudaStream_t st, float* loss_sink = nullptr);
-  std::string train_device(const __nv_bfloat16* X, const float* t, int n, int epochs, int batch, float lr,
-                           __nv_bfloat16* acts, float* y, float* last_loss);
-  std::string check_err();
+  // device entry point on stream st
+  std::string forward_dev(const __nv_bfloat16* X, int n, const int* n_dev, int max_n, float* y, cudaStream_t st);
   // training pairs (device buffer owned by the network)
   std::string reserve_pairs(long long cap);
   std::string clear_pairs();
@@ -50,12 +40,25 @@ class Net {
   std::string eval_pairs(long long first, long long count, float* abs_err);
 
  private:
+  static constexpr size_t kWorkspaceKeep = (size_t)256 << 20;
+  std::string finish(float* loss);
+  char* workspace(size_t bytes);
+  std::string trim(std::string r);
+  size_t staging_bytes(size_t n) const;
+  std::string upload_rows(const float* Xh, size_t n, __nv_bfloat16* X, char* staging);
+  // gradients of the batch as *rows rows of Gp_, one per CTA
+  std::string gradient_rows(const __nv_bfloat16* X, int n, const float* t, int* rows);
+  std::string train_device(const __nv_bfloat16* X, const float* t, int n, int epochs, int batch, float lr,
+                           float* last_loss);
+  char* ws_ = nullptr;  // workspace of the host-buffer entry points
+  size_t ws_bytes_ = 0;
+  int* h_end_ = nullptr;  // pinned mirror of the error word and the loss
+  int pageable_ = 0;      // the GPU can access pageable host memory directly
   cudaStream_t stream_ = nullptr;
   std::vector<void*> allocs_;
   float *P_ = nullptr, *G_ = nullptr, *M1_ = nullptr, *M2_ = nullptr;
-  // BF16 weight tiles in the tensor-core operand layout (forward, transposed)
-  __nv_bfloat16 *Wb_ = nullptr, *WTb_ = nullptr;
-  float* Gp_ = nullptr;        // per-CTA partial gradients of the backward pass [sms_][NG]
+  __nv_bfloat16* Wb_ = nullptr;  // BF16 weight tiles in the tensor-core operand layout
+  float* Gp_ = nullptr;        // per-CTA partial gradients [sms_][NG]
   float* loss_acc_ = nullptr;  // the epoch's summed batch losses (device)
   int sms_ = 1;
   int* err_ = nullptr;

@@ -693,7 +693,7 @@ std::string Solver::learned_step(bool* empty_nb) {
     LS_TRY(cudaGetLastError(), "features");
     st_.kernel_launches += 2;
     if (warm) {
-      std::string r = net_->forward_dev(X_, 0, lr_.cnt, m_.nv, lr_.pred, nullptr, stream_);
+      std::string r = net_->forward_dev(X_, 0, lr_.cnt, m_.nv, lr_.pred, stream_);
       if (!r.empty()) return r;
       LS_TRY(K_->learn(LEARN_WARM, m_, s_, sp_, lr_, 0, margin_, L_, stream_), "warm apply");
       st_.kernel_launches += 2;
