@@ -56,7 +56,6 @@ struct ls_batch {
   std::vector<int> vbase;  // first vertex of each member in the merged numbering
   std::unique_ptr<lsgb::Layout> layout;
   std::unique_ptr<lsgb::Solver> solver;
-  std::vector<float> stage;
   std::string err;
 };
 
@@ -702,7 +701,6 @@ ls_status ls_batch_setup(ls_batch* b) {
     b->solver.reset();
     return s;
   }
-  b->stage.assign(vb, 0.f);
   return bsolver_status(b, b->solver->set_phi(phi.data()));
 }
 
@@ -835,10 +833,7 @@ ls_status ls_batch_get_phi(ls_batch* b, int index, float* phi) {
   if (!b || !phi) return LS_BAD_INPUT;
   if (!b->solver) return bfail(b, LS_NOT_READY, "call ls_batch_setup first");
   if (index < 0 || index >= (int)b->members.size()) return bfail(b, LS_BAD_INPUT, "bad member index");
-  std::string r = b->solver->get_phi(b->stage.data());
-  if (!r.empty()) return bsolver_status(b, r);
-  std::memcpy(phi, b->stage.data() + b->vbase[index], sizeof(float) * (size_t)b->members[index].nv);
-  return LS_OK;
+  return bsolver_status(b, b->solver->get_phi(phi, b->vbase[index], b->members[index].nv));
 }
 
 ls_status ls_batch_get_stats(ls_batch* b, ls_stats* s) {

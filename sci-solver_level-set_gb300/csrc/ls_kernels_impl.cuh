@@ -1870,10 +1870,11 @@ __global__ void k_copy_phi(DevMesh m, DevState s) {
   }
 }
 
-// out[old] = phi[new] (kernel_compute_vertT_before_permute3d), as a gather
-__global__ void k_unpermute(DevMesh m, const float* phi, float* out) {
-  for (int o = blockIdx.x * blockDim.x + threadIdx.x; o < m.nv; o += gridDim.x * blockDim.x)
-    out[o] = phi[__ldg(m.ipermute + o)];
+// out[old - first] = phi[new] for n vertices from `first` on in the caller's
+// order (kernel_compute_vertT_before_permute3d), as a gather
+__global__ void k_unpermute(DevMesh m, const float* phi, int first, int n, float* out) {
+  for (int o = blockIdx.x * blockDim.x + threadIdx.x; o < n; o += gridDim.x * blockDim.x)
+    out[o] = phi[__ldg(m.ipermute + first + o)];
 }
 
 // FIM distances in the layout's order (diagnostics)
@@ -2284,8 +2285,9 @@ cudaError_t launch_update(const DevMesh& m, const DevState& s, const StepParams&
                           (size_t)L.upd_smem, st);
 }
 
-cudaError_t launch_unpermute(const DevMesh& m, const float* phi, float* out, const Launch& L, cudaStream_t st) {
-  k_unpermute<<<L.flat_grid, 256, 0, st>>>(m, phi, out);
+cudaError_t launch_unpermute(const DevMesh& m, const float* phi, int first, int n, float* out, const Launch& L,
+                             cudaStream_t st) {
+  k_unpermute<<<std::min(L.flat_grid, (n + 255) / 256), 256, 0, st>>>(m, phi, first, n, out);
   return cudaGetLastError();
 }
 

@@ -785,14 +785,19 @@ void Solver::pull_stats() {
   fold_prof(true);
 }
 
+// One row of a run's history: where the GPU can write the caller's array, the
+// row is on its way when this returns and complete when the stream is (run
+// ends with a wait); the next step is enqueued behind it.
+std::string Solver::emit_phi(float* row) {
+  if (!pageable_) return get_phi(row);
+  LS_TRY(K_->unpermute(m_, s_.phi, 0, m_.nv, row, L_, stream_), "unpermute");
+  return "";
+}
+
 std::string Solver::run(int nsteps, float* history, int* steps_done) {
   int done = 0;
-  if (history) {
-    LS_TRY(K_->unpermute(m_, s_.phi, d_tmp_, L_, stream_), "unpermute");
-    LS_TRY(cudaMemcpyAsync(h_stage_, d_tmp_, sizeof(float) * m_.nv, cudaMemcpyDeviceToHost, stream_), "d2h");
-    LS_TRY(cudaStreamSynchronize(stream_), "sync");
-    std::memcpy(history, h_stage_, sizeof(float) * m_.nv);
-  }
+  std::string h;
+  if (history && !(h = emit_phi(history)).empty()) return h;
   LS_TRY(cudaEventRecord(ev0_, stream_), "event");
   for (int s = 0; s < nsteps; ++s) {
     bool empty = false;
@@ -801,12 +806,7 @@ std::string Solver::run(int nsteps, float* history, int* steps_done) {
     if (cfg_.profile) fold_prof(true);
     if (empty) break;
     done++;
-    if (history) {
-      LS_TRY(K_->unpermute(m_, s_.phi, d_tmp_, L_, stream_), "unpermute");
-      LS_TRY(cudaMemcpyAsync(h_stage_, d_tmp_, sizeof(float) * m_.nv, cudaMemcpyDeviceToHost, stream_), "d2h");
-      LS_TRY(cudaStreamSynchronize(stream_), "sync");
-      std::memcpy(history + (size_t)(s + 1) * m_.nv, h_stage_, sizeof(float) * m_.nv);
-    }
+    if (history && !(h = emit_phi(history + (size_t)(s + 1) * m_.nv)).empty()) return h;
   }
   LS_TRY(cudaEventRecord(ev1_, stream_), "event");
   LS_TRY(cudaEventSynchronize(ev1_), "event sync");
@@ -838,13 +838,11 @@ std::string Solver::step_host(const float* phi_in, float* phi_out) {
   if (!r.empty()) return r;
   if (cfg_.profile) fold_prof(true);
   if (pageable_) {
-    LS_TRY(K_->unpermute(m_, s_.phi, phi_out, L_, stream_), "unpermute out");
+    LS_TRY(K_->unpermute(m_, s_.phi, 0, nv, phi_out, L_, stream_), "unpermute out");
     LS_TRY(cudaStreamSynchronize(stream_), "sync");
   } else {
-    LS_TRY(K_->unpermute(m_, s_.phi, d_tmp_, L_, stream_), "unpermute");
-    LS_TRY(cudaMemcpyAsync(h_stage_, d_tmp_, sizeof(float) * nv, cudaMemcpyDeviceToHost, stream_), "d2h");
-    LS_TRY(cudaStreamSynchronize(stream_), "sync");
-    std::memcpy(phi_out, h_stage_, sizeof(float) * nv);
+    r = get_phi(phi_out);
+    if (!r.empty()) return r;
   }
   if (!empty) st_.steps_run++;
   stats_stale_ = true;
@@ -948,20 +946,26 @@ std::string Solver::eikonal(const int* seeds, const float* values, int nseeds, f
 }
 
 std::string Solver::set_phi(const float* phi_orig) {
-  std::memcpy(h_stage_, phi_orig, sizeof(float) * m_.nv);
-  LS_TRY(cudaMemcpyAsync(d_tmp_, h_stage_, sizeof(float) * m_.nv, cudaMemcpyHostToDevice, stream_), "h2d");
-  LS_TRY(K_->permute(m_, d_tmp_, s_.phi, L_, stream_), "permute");
+  const float* src = phi_orig;
+  if (!pageable_) {
+    std::memcpy(h_stage_, phi_orig, sizeof(float) * m_.nv);
+    LS_TRY(cudaMemcpyAsync(d_tmp_, h_stage_, sizeof(float) * m_.nv, cudaMemcpyHostToDevice, stream_), "h2d");
+    src = d_tmp_;
+  }
+  LS_TRY(K_->permute(m_, src, s_.phi, L_, stream_), "permute");
   LS_TRY(cudaMemsetAsync(s_.ctl + CTL_NB_VALID, 0, sizeof(int), stream_), "memset");
   LS_TRY(cudaStreamSynchronize(stream_), "sync");
   have_nb_ = false;
   return "";
 }
 
-std::string Solver::get_phi(float* phi_orig) {
-  LS_TRY(K_->unpermute(m_, s_.phi, d_tmp_, L_, stream_), "unpermute");
-  LS_TRY(cudaMemcpyAsync(h_stage_, d_tmp_, sizeof(float) * m_.nv, cudaMemcpyDeviceToHost, stream_), "d2h");
+std::string Solver::get_phi(float* phi_orig, int first, int n) {
+  float* const dst = pageable_ ? phi_orig : d_tmp_;
+  LS_TRY(K_->unpermute(m_, s_.phi, first, n, dst, L_, stream_), "unpermute");
+  if (!pageable_)
+    LS_TRY(cudaMemcpyAsync(h_stage_, d_tmp_, sizeof(float) * n, cudaMemcpyDeviceToHost, stream_), "d2h");
   LS_TRY(cudaStreamSynchronize(stream_), "sync");
-  std::memcpy(phi_orig, h_stage_, sizeof(float) * m_.nv);
+  if (!pageable_) std::memcpy(phi_orig, h_stage_, sizeof(float) * n);
   return "";
 }
 

@@ -44,7 +44,9 @@ struct KernelSet {
   // FIM distances in the layout's vertex order
   cudaError_t (*distances)(const DevMesh& m, const DevState& s, const StepParams& sp, float* out, const Launch& L,
                            cudaStream_t st);
-  cudaError_t (*unpermute)(const DevMesh& m, const float* phi, float* out, const Launch& L, cudaStream_t st);
+  // n vertices from `first` on in the caller's order
+  cudaError_t (*unpermute)(const DevMesh& m, const float* phi, int first, int n, float* out, const Launch& L,
+                           cudaStream_t st);
   cudaError_t (*permute)(const DevMesh& m, const float* in, float* out, const Launch& L, cudaStream_t st);
   // learned warm start / collection kernels (op: LEARN_*)
   cudaError_t (*learn)(int op, const DevMesh& m, const DevState& s, const StepParams& sp, const DevLearn& lr, int arg,
@@ -114,7 +116,8 @@ class Solver {
   // Upload the layout and the per-copy data; phi0 / vel in the caller's order.
   std::string init(const Layout& L, const SolverConfig& cfg, const float* vel);
   std::string set_phi(const float* phi_orig);          // host, caller order
-  std::string get_phi(float* phi_orig);                // host, caller order
+  std::string get_phi(float* phi_orig) { return get_phi(phi_orig, 0, m_.nv); }  // host, caller order
+  std::string get_phi(float* phi_orig, int first, int n);  // n vertices from `first` on
   // Run nsteps; history (optional) gets phi after each step (host, caller order).
   std::string run(int nsteps, float* history, int* steps_done);
   std::string step_host(const float* phi_in, float* phi_out);
@@ -151,6 +154,7 @@ class Solver {
   std::string fim_loop(const StepParams& sp);
   std::string build_graph();
   bool build_persistent_graph(std::string* err);
+  std::string emit_phi(float* row);
   cudaError_t step_head();
   cudaError_t step_tail();
   cudaError_t step_persistent_launches();
