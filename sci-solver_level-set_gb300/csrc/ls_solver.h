@@ -153,6 +153,7 @@ class Solver {
   std::string learn_buffers();
   std::string fim_loop(const StepParams& sp);
   std::string build_graph();
+  int first_bodies() const { return m_.dim == 3 ? 3 : 2; }  // loop bodies' worth of iterations before the loop
   bool build_persistent_graph(std::string* err);
   std::string emit_phi(float* row);
   cudaError_t step_head();
