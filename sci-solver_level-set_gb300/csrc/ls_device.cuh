@@ -496,7 +496,12 @@ __device__ __forceinline__ bool in_unit(float a, float b, float c) {
 // (both from R), the two interior roots -- with the square roots, side QP
 // and the interior's set-up per lane.  Every multiply-add is written out:
 // left to the compiler's contraction, the kernels that inline this solver
-// would round differently.
+// would round differently.  Of a difference of products the first is fused;
+// s has its products in the other order than g2's numerator, and the weights
+// of T_lin are those of all three vertices: a value's last bit decides range
+// tests and the front's last patches, so cheaper forms of these (shared
+// numerators, differences to TR: 1 % of the FIM time) were not worth another
+// set of bits.
 // Arguments: the face's vertices are P, Q, R and the target X; the dot
 // products of p = P - R, q = Q - R and x = X - R (PP = p.p, PQ = p.q, ...),
 // and hX, X's height over the face.  (tet_solve's ACCD and BCCD are -PX and
@@ -556,17 +561,17 @@ __device__ __forceinline__ float tet_solve_wave(float TP, float TQ, float TR, fl
   }
   {  // interior: y = l1 P + l2 Q + l3 R
     const float idet = fast_rcp(fmaf(PP, QQ, -__fmul_rn(PQ, PQ)));
-    // the reference's h and s, which are also the numerators of the gradient
-    const float h = fmaf(QQ, up, -__fmul_rn(PQ, uq)), s = fmaf(PP, uq, -__fmul_rn(PQ, up));
-    const float t = fmaf(up, QX, -__fmul_rn(uq, PX));
-    const float g1 = __fmul_rn(h, idet);  // in-plane gradient, coefficient of P - R
-    const float g2 = __fmul_rn(s, idet);  // and of Q - R
-    const float foot1 = __fmul_rn(fmaf(QQ, PX, -__fmul_rn(PQ, QX)), idet);  // X's foot point, weight of P
+    // the reference's h (also the numerator of g1), s and t
+    const float h = fmaf(QQ, up, -__fmul_rn(PQ, uq));
+    const float s = fmaf(-up, PQ, __fmul_rn(uq, PP)), t = fmaf(up, QX, -__fmul_rn(uq, PX));
+    const float g1 = __fmul_rn(h, idet);                                   // in-plane gradient, coefficient of P - R
+    const float g2 = __fmul_rn(fmaf(PP, uq, -__fmul_rn(PQ, up)), idet);  // and of Q - R
+    const float foot1 = __fmul_rn(fmaf(PQ, -QX, __fmul_rn(QQ, PX)), idet);  // X's foot point, weight of P
     // the point downhill of the foot point (lane x) and its mirror uphill
     // (lane y): the reference's SMALLNUM offset in l2 = (s l1 + t) / (h +
     // eps_h) can move the first point out of the face where h is small, and
     // the mirror's point is then the better one, as in the reference
-    const float dl = __fmul_rn(__fmul_rn(hX, fast_rsqrt(fmaf(-g1, up, fmaf(-g2, uq, 1.f)))), g1);
+    const float dl = __fmul_rn(__fmul_rn(hX, fast_rsqrt(__fsub_rn(1.f, fmaf(g1, up, __fmul_rn(g2, uq))))), g1);
     const float ih = fast_rcp(h + eps_h);
     const float2 l1 = f2(foot1 - dl, foot1 + dl);
     const float2 l2 = __fmul2_rn(__ffma2_rn(f2(s, s), l1, f2(t, t)), f2(ih, ih));
@@ -576,7 +581,7 @@ __device__ __forceinline__ float tet_solve_wave(float TP, float TQ, float TR, fl
     const float2 a2 = __ffma2_rn(l1, f2(PQ, PQ), __ffma2_rn(l2, f2(QQ, QQ), f2(-QX, -QX)));
     const float2 a3 = __ffma2_rn(l1, f2(-PX, -PX), __ffma2_rn(l2, f2(-QX, -QX), f2(XX, XX)));
     const float2 Q = __ffma2_rn(a1, l1, __ffma2_rn(a2, l2, a3));
-    const float2 lin = __ffma2_rn(l1, f2(up, up), __ffma2_rn(l2, f2(uq, uq), f2(TR, TR)));
+    const float2 lin = __ffma2_rn(f2(TP, TP), l1, __ffma2_rn(f2(TQ, TQ), l2, __fmul2_rn(f2(TR, TR), l3)));
     const float2 c = __fadd2_rn(lin, f2(fast_sqrt(Q.x), fast_sqrt(Q.y)));
     if (in_unit(l1.x, l2.x, l3.x)) best = fminf(best, c.x);
     if (in_unit(l1.y, l2.y, l3.y)) best = fminf(best, c.y);
