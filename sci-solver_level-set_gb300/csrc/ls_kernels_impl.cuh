@@ -851,19 +851,27 @@ __global__ void __launch_bounds__(MAXT, MINB) k_fim_compact(DevMesh m, DevState 
 
 // Local solver of the two-copies-per-thread sweep: the fast build's
 // planar-wave solver with the lower-bound skip (kPairWave), or the
-// reference's solver in its operand order, every listed solve run (the
+// reference's solver in its operand order (the
 // bit-exact build; kPairRefXdiv with the interior division in double, as
 // the reference semantics there).
 constexpr int kPairWave = 0, kPairRef = 1, kPairRefXdiv = 2;
 
 // The solves (bit k: target k) of a copy with values tv and heights hv that
 // can lower their target T_k.  One cannot when the three other values are
-// all LARGENUM (the solver returns LARGENUM); with the planar-wave solver
-// also not when min of them plus 0.999 x the target's height over their face
-// is at least T_k (the lower bound of every candidate in exact arithmetic,
-// which with three LARGENUMs is no less than T_k either).  The reference
-// solver's FP32 candidates can fall below that bound, so the bit-exact build
-// keeps those solves.
+// all LARGENUM (the solver returns LARGENUM), nor when min of them plus the
+// target's height over their face is at least T_k: every candidate is a value
+// T_lin(y) + |y - X| at a point y of the face.
+// Planar-wave solver: 0.999 x the height (with three LARGENUMs the sum is no
+// less than T_k either).
+// Reference solver (bit-exact build): what its FP32 candidates satisfy
+// whatever their rounding.  With weights in [0, 1], T_lin rounds to at least
+// min (1 - 4e-7).  The squared distance is the quadratic form of the solve's
+// six FP32 products, at least det3 / det2 = h^2, evaluated to 5e-7 of the sum
+// S of their magnitudes: where h^2 >= 1e-4 S its root is at least 0.997 h.
+// So min (1 - 1e-6) + 0.99 h (hv, 0 for flat tets: ref_height) bounds them,
+// with room for the rounding of the test itself, and the solves left out
+// change no bit.  48^3 step: 525 M -> 288 M warp instructions, its FIM launches
+// 1077 -> 683 us.
 template <int SOLVER>
 __device__ __forceinline__ unsigned pair_may_lower(const float4& tv, const float4& hv, float LN) {
   const float m01 = fminf(tv.x, tv.y), m23 = fminf(tv.z, tv.w);
@@ -871,7 +879,9 @@ __device__ __forceinline__ unsigned pair_may_lower(const float4& tv, const float
   if constexpr (SOLVER == kPairWave)
     return (n0 + 0.999f * hv.x < tv.x ? 1u : 0u) | (n1 + 0.999f * hv.y < tv.y ? 2u : 0u) |
            (n2 + 0.999f * hv.z < tv.z ? 4u : 0u) | (n3 + 0.999f * hv.w < tv.w ? 8u : 0u);
-  return (n0 < LN ? 1u : 0u) | (n1 < LN ? 2u : 0u) | (n2 < LN ? 4u : 0u) | (n3 < LN ? 8u : 0u);
+  constexpr float lo = 1.f - 1e-6f;
+  return (n0 < LN && n0 * lo + hv.x < tv.x ? 1u : 0u) | (n1 < LN && n1 * lo + hv.y < tv.y ? 2u : 0u) |
+         (n2 < LN && n2 * lo + hv.z < tv.z ? 4u : 0u) | (n3 < LN && n3 * lo + hv.w < tv.w ? 8u : 0u);
 }
 
 // One listed solve of k_fim_pair: solve k of copy cc from the copy values
@@ -916,6 +926,19 @@ __device__ __forceinline__ void pair_solve(int code, const float4* sTc, const fl
 // copy_metric's terms, whose CD is -(D from C), with signs so that the four
 // solves only permute them -- and the heights of its four vertices over their opposite faces,
 // the same expressions the one-copy kernels evaluate per visit.
+// (The bit-exact build's heights are ref_height's.)
+// 0.99 x the height of x over the plane of p, q from their products, where
+// the tet is far enough from flat for pair_may_lower's bound (0 elsewhere).
+__device__ __forceinline__ float ref_height(float PP_, float PQ_, float PX_, float QQ_, float QX_, float XX_) {
+  const double PP = PP_, PQ = PQ_, PX = PX_, QQ = QQ_, QX = QX_, XX = XX_;
+  const double S = PP + QQ + XX + 2.0 * (fabs(PQ) + fabs(PX) + fabs(QX));
+  const double det2 = PP * QQ - PQ * PQ;
+  const double det3 = PP * (QQ * XX - QX * QX) - PQ * (PQ * XX - QX * PX) + PX * (PQ * QX - QQ * PX);
+  if (!(det2 >= 1e-6 * S * S)) return 0.f;
+  const double h2 = det3 / det2;
+  return h2 >= 1e-4 * S ? (float)(0.99 * sqrt(h2)) : 0.f;
+}
+
 __global__ void k_geometry(DevMesh m, float4* gm, float4* gh) {
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < m.full; c += stride) {
@@ -928,10 +951,18 @@ __global__ void k_geometry(DevMesh m, float4* gm, float4* gh) {
     const float ADAD = Mt[6], ADBD = Mt[7], BDBD = Mt[9];
     const float det3 = ACAC * (BCBC * CDCD - BCCD * BCCD) - ACBC * (ACBC * CDCD - BCCD * ACCD) +
                        ACCD * (ACBC * BCCD - BCBC * ACCD);
+#ifdef LS_KERNELS_EXACT
+    (void)det3;
+    const float aa = ACAC, ab = ACBC, ad = -ACCD, bb = BCBC, bd = -BCCD, dd = CDCD;
+    // the products in each solve's order (pair_solve)
+    gh[c] = make_float4(ref_height(bb, bd, ab, dd, ad, aa), ref_height(aa, ad, ab, dd, bd, bb),
+                        ref_height(ADAD, ADBD, Mt[8], BDBD, Mt[10], CDCD), ref_height(aa, ab, ad, bb, bd, dd));
+#else
     gh[c] = make_float4(sqrtf(fmaxf(det3 / (BCBC * CDCD - BCCD * BCCD), 0.f)),   // A over BCD
                         sqrtf(fmaxf(det3 / (ACAC * CDCD - ACCD * ACCD), 0.f)),   // B over ACD
                         sqrtf(fmaxf(det3 / (ADAD * BDBD - ADBD * ADBD), 0.f)),   // C over ABD
                         sqrtf(fmaxf(det3 / (ACAC * BCBC - ACBC * ACBC), 0.f)));  // D over ABC
+#endif
   }
 }
 
