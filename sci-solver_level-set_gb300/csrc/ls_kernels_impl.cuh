@@ -314,21 +314,28 @@ __device__ __forceinline__ void solve_copy_flags(const float* Mt, const float T[
   r[2] = tet_solve<float, XDIV, true>(TA, TB, TD, ADAD, ADBD, -ADCD, BDBD, -CDBD, CDCD, eps_h, eps_h64, LN, tau, ill[2], TC);
 }
 
-// The FP64 repeat of solve k of a tet copy (same argument order as above).
-__device__ __noinline__ float solve_k_fp64(const float* Mt, const float T[4], int k, double eps_h64, float LN) {
+// The FP64 repeat of solve k of a tet copy (the argument order of the calls
+// above), or part `part` of it (tet_part_f64).  The arguments are selected
+// first, so that the lanes of a warp run one solve together whatever their k.
+struct RepeatArgs {
+  float t0, t1, t2, g0, g1, g2, g3, g4, g5;
+};
+__device__ __forceinline__ RepeatArgs repeat_args(const float* Mt, const float T[4], int k) {
   const float ACAC = Mt[0], ACBC = Mt[1], ACCD = Mt[2], BCBC = Mt[3], BCCD = Mt[4];
   const float CDCD = Mt[5], ADAD = Mt[6], ADBD = Mt[7], ADCD = Mt[8], BDBD = Mt[9], CDBD = Mt[10];
-  const float TA = T[0], TB = T[1], TC = T[2], TD = T[3];
-  const double L64 = LN;
+  const bool k0 = k == 0, k1 = k == 1, k2 = k == 2, lo = k < 2;
+  RepeatArgs a;
+  a.t0 = k0 ? T[1] : T[0]; a.t1 = lo ? T[3] : T[1]; a.t2 = k2 ? T[3] : T[2];
+  a.g0 = k0 ? BCBC : k2 ? ADAD : ACAC; a.g1 = k0 ? -BCCD : k1 ? -ACCD : k2 ? ADBD : ACBC;
+  a.g2 = lo ? -ACBC : k2 ? -ADCD : ACCD; a.g3 = lo ? CDCD : k2 ? BDBD : BCBC;
+  a.g4 = k0 ? ACCD : k2 ? -CDBD : BCCD; a.g5 = k0 ? ACAC : k1 ? BCBC : CDCD;
+  return a;
+}
+__device__ __noinline__ float solve_k_fp64(const float* Mt, const float T[4], int k, double eps_h64, float LN) {
+  const RepeatArgs a = repeat_args(Mt, T, k);
   bool d = false;
-  double r;
-  switch (k) {
-    case 3: r = tet_solve<double, false, false>(TA, TB, TC, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD, eps_h64, eps_h64, L64, 0.0, d); break;
-    case 0: r = tet_solve<double, false, false>(TB, TD, TC, BCBC, -BCCD, -ACBC, CDCD, ACCD, ACAC, eps_h64, eps_h64, L64, 0.0, d); break;
-    case 1: r = tet_solve<double, false, false>(TA, TD, TC, ACAC, -ACCD, -ACBC, CDCD, BCCD, BCBC, eps_h64, eps_h64, L64, 0.0, d); break;
-    default: r = tet_solve<double, false, false>(TA, TB, TD, ADAD, ADBD, -ADCD, BDBD, -CDBD, CDCD, eps_h64, eps_h64, L64, 0.0, d); break;
-  }
-  return (float)r;
+  return (float)tet_solve<double, false, false>(a.t0, a.t1, a.t2, a.g0, a.g1, a.g2, a.g3, a.g4, a.g5, eps_h64, eps_h64,
+                                                (double)LN, 0.0, d);
 }
 
 // One deferred FP64 solve: the copy (CTA-local index << 2 | solve) and its
@@ -764,7 +771,9 @@ __global__ void __launch_bounds__(MAXT, MINB) k_fim_compact(DevMesh m, DevState 
           r = tet_solve_wave(a0, a1, a2, g0, g1, -g2, g3, -g4, g5, sH[k * MAXT + cc], sp.eps_h);
         if (PREC && ill) {
           // discriminant cancelled: repeat in FP64 after this pass, densely
+          // (a ghost target's result starts from its value)
           sRep[atomicAdd(&s_rep, 1)] = code;
+          sR[k * MAXT + cc] = own;
           continue;
         }
         const float nw = fminf(own, r);
@@ -775,22 +784,29 @@ __global__ void __launch_bounds__(MAXT, MINB) k_fim_compact(DevMesh m, DevState 
       }
       __syncthreads();
       if constexpr (PREC) {
-        const int nrep = s_rep;
-        for (int i = tid; i < nrep; i += blockDim.x) {
-          const int code = sRep[i];
-          const int cc = code >> 2, k = code & 3;
-          float Mq[11], Tq[4];
+        // each repeat's four parts on warps of different SM quarters (warp w
+        // runs on quarter w % 4); blocks of fewer than four warps take several
+        // parts per warp
+        const int nrep = s_rep, nw = blockDim.x >> 5, warp = tid >> 5;
+        const int groups = nw >> 2, pstep = groups ? 4 : nw;
+        const int first = groups ? (warp >> 2) * 32 + (tid & 31) : (tid & 31), step = groups ? groups * 32 : 32;
+        if (!groups || warp < 4 * groups)
+          for (int part = groups ? (warp & 3) : warp; part < 4; part += pstep)
+            for (int i = first; i < nrep; i += step) {
+              const int code = sRep[i];
+              const int cc = code >> 2, k = code & 3;
+              float Mq[11], Tq[4];
 #pragma unroll
-          for (int j = 0; j < 11; ++j) Mq[j] = sM[j * MAXT + cc];
+              for (int j = 0; j < 11; ++j) Mq[j] = sM[j * MAXT + cc];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) Tq[j] = sTc[j * MAXT + cc];
-          const float nw = fminf(Tq[k], solve_k_fp64(Mq, Tq, k, sp.eps_h64, sp.largenum));
-          const ushort4 cv = sC[cc];
-          const int tk = k == 0 ? cv.x : k == 1 ? cv.y : k == 2 ? cv.z : cv.w;
-          if (tk < nvp) atomicMin(reinterpret_cast<int*>(&sT[tk]), __float_as_int(nw));
-          else sR[k * MAXT + cc] = nw;
-          nflag++;
-        }
+              for (int j = 0; j < 4; ++j) Tq[j] = sTc[j * MAXT + cc];
+              const RepeatArgs a = repeat_args(Mq, Tq, k);
+              const float r = (float)tet_part_f64(part, a.t0, a.t1, a.t2, a.g0, a.g1, a.g2, a.g3, a.g4, a.g5, sp.eps_h64);
+              const ushort4 cv = sC[cc];
+              const int tk = k == 0 ? cv.x : k == 1 ? cv.y : k == 2 ? cv.z : cv.w;
+              atomicMin(reinterpret_cast<int*>(tk < nvp ? &sT[tk] : &sR[k * MAXT + cc]), __float_as_int(r));
+              if (part == 0) nflag++;
+            }
         __syncthreads();
         if (tid == 0) s_rep = 0;
       }
