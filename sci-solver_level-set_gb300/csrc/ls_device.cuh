@@ -98,7 +98,7 @@ enum {
   CTL_ITER = 12,    // stamp of the first iteration of the next loop body
   CTL_BASE = 13,    // base stamp of the step
   CTL_ITERS = 14,   // iterations of this step that visited a patch
-  CTL_LAST = 15,    // stamp of the last of them
+  CTL_LAST = 15,    // stamp of the last iteration that visited a patch
   CTL_WORDS = 16
 };
 // Stamps restart (every stamped array cleared) between steps once they pass
@@ -125,6 +125,14 @@ struct DevState {
                     // arrivals since the launch started, [2 + smid] CTAs on SM smid
 };
 constexpr int kGridBarrierWords = 2 + 1024;
+
+// Counts iteration t of this step if it visited a patch (one thread, once for
+// each iteration: when the next one starts, or at the end of a loop body).
+__device__ __forceinline__ void count_iteration(int* ctl, unsigned long long* stats, int t) {
+  if (*reinterpret_cast<volatile int*>(ctl + CTL_LAST) != t) return;
+  ctl[CTL_ITERS] += 1;
+  atomicAdd(&stats[5], 1ull);
+}
 
 // Learned warm start / training-pair collection buffers (null when off).
 struct DevLearn {

@@ -98,6 +98,7 @@ __device__ __forceinline__ FimIter fim_iter(const DevMesh& m, const DevState& s,
     const int aft = nxt == 2 ? 0 : nxt + 1;
     s.ctl[CTL_VISITS + aft] = 0;
     s.ctl[CTL_CANDS + aft] = 0;
+    if (t > 0 || !rel) count_iteration(s.ctl, s.stats, f.t - 1);  // (a body's last one: at its end)
   }
   return f;
 }
@@ -174,10 +175,7 @@ struct FimCount {
 __device__ __forceinline__ void fim_count_flush(const DevState& s, const FimIter& f, const FimCount& n) {
   if (n.visits) {
     atomicAdd(&s.stats[0], (unsigned long long)n.visits);
-    if (atomicMax(s.ctl + CTL_LAST, f.t) < f.t) {
-      atomicAdd(s.ctl + CTL_ITERS, 1);
-      atomicAdd(&s.stats[5], 1ull);
-    }
+    s.ctl[CTL_LAST] = f.t;  // counted as an iteration by count_iteration
   }
   if (n.checks) atomicAdd(&s.stats[1], (unsigned long long)n.checks);
   if (n.early) atomicAdd(&s.stats[8], (unsigned long long)n.early);
@@ -425,14 +423,33 @@ __device__ __forceinline__ void fim_copy_pass(const DevMesh& m, const DevState& 
     const int slot = s.slot[p] ^ 1;
     int niter = visit ? sp.niter : 1;
     if (tid == 0) (visit ? cnt.visits : cnt.checks)++;
+    // the copy's own loads are in flight while the slab is gathered
+    const bool act = tid < nep;
+    ushort4 cv = make_ushort4(0, 0, 0, 0);
+    unsigned capm = 0u;
+    float lc0 = 0.f, lc1 = 0.f, lc2 = 0.f;
+    if (act) {
+      cv = m.conn[es + tid];
+      if (m.capped) capm = m.capped[es + tid];
+      if constexpr (D1 == 3) {
+        const long long c = (long long)es + tid;
+        lc0 = __ldg(m.lc + c); lc1 = __ldg(m.lc + m.full + c); lc2 = __ldg(m.lc + 2 * m.full + c);
+      }
+    }
+    bool sd0 = false;  // the owned vertex tid is a seed (its value in v0)
+    float v0 = 0.f;
     for (int i = tid; i < nvp + ngp; i += blockDim.x) {
-      const float d = dt_before(s.cell[i < nvp ? vs + i : __ldg(m.ghost_ids + gs + i - nvp)], t, f.base, sp.largenum);
+      const DtCell cell = s.cell[i < nvp ? vs + i : __ldg(m.ghost_ids + gs + i - nvp)];
+      const float d = dt_before(cell, t, f.base, sp.largenum);
+      if (i == tid) {
+        sd0 = dt_is_seed(cell, f.base);
+        v0 = d;
+      }
       buf0[i] = d;
       if (i < nvp) buf1[i] = d;
     }
     if (tid == 0) s_min[par] = 0x7f800000u;
     __syncthreads();
-    const bool act = tid < nep;
     int idx[4] = {0, 0, 0, 0};
     float T[4] = {0.f, 0.f, 0.f, 0.f};
     // the fast build's triangles use the planar-wave form
@@ -444,17 +461,14 @@ __device__ __forceinline__ void fim_copy_pass(const DevMesh& m, const DevState& 
     // per-vertex slot limit where that applies (others stay private)
     unsigned shared_k = 0u;
     if (act) {
-      const ushort4 cv = m.conn[es + tid];
       idx[0] = cv.x; idx[1] = cv.y; idx[2] = cv.z; idx[3] = cv.w;
-      const unsigned capm = m.capped ? (unsigned)m.capped[es + tid] : 0u;
 #pragma unroll
       for (int k = 0; k < D1; ++k)
         if (idx[k] < nvp && !((capm >> k) & 1u)) shared_k |= 1u << k;
 #pragma unroll
       for (int k = 0; k < D1; ++k) T[k] = buf0[idx[k]];
       if constexpr (WAVE) {
-        const long long c = (long long)es + tid;
-        tg = tri_geo(__ldg(m.lc + c), __ldg(m.lc + m.full + c), __ldg(m.lc + 2 * m.full + c));
+        tg = tri_geo(lc0, lc1, lc2);
       } else {
         copy_metric<D1>(m, (long long)es + tid, Mt);
       }
@@ -541,7 +555,7 @@ __device__ __forceinline__ void fim_copy_pass(const DevMesh& m, const DevState& 
         // first sweep this was
         int c0 = 1;
         for (int i = tid; i < nvp; i += blockDim.x)
-          if (!dt_is_seed(s.cell[vs + i], f.base)) c0 &= (sOld[i] - sT[i] < sp.tol) ? 1 : 0;
+          if (!(i == tid ? sd0 : dt_is_seed(s.cell[vs + i], f.base))) c0 &= (sOld[i] - sT[i] < sp.tol) ? 1 : 0;
         if (__syncthreads_and(c0)) break;
         visit = true;
         niter = sp.niter;
@@ -564,14 +578,17 @@ __device__ __forceinline__ void fim_copy_pass(const DevMesh& m, const DevState& 
       for (int i = tid; i < nvp; i += blockDim.x) {
         const int v = vs + i;
         const float nt = sT[i];
-        float outv;
-        const DtCell c = s.cell[v];
-        if (!dt_is_seed(c, f.base)) {
+        float outv = v0;
+        bool sd = sd0;
+        if (i != tid) {
+          const DtCell c = s.cell[v];
+          sd = dt_is_seed(c, f.base);
+          outv = __int_as_float(c.x);
+        }
+        if (!sd) {
           reinterpret_cast<int2*>(s.cell + v)[slot] = make_int2(__float_as_int(nt), t);
           con &= (sOld[i] - nt < sp.tol) ? 1 : 0;
           outv = nt;
-        } else {
-          outv = __int_as_float(c.x);
         }
         atomicMin(&s_min[par], __float_as_uint(outv));
       }
@@ -1093,6 +1110,11 @@ __device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& 
   __shared__ __align__(8) unsigned long long s_bar;  // geometry slab copies of the current patch
   __shared__ int s_err;  // a slab wait ran out: the pass ends
   __shared__ FimCount s_cnt;  // thread 0's work counters (in shared memory for their registers)
+  // the patch's half for this visit's results, and its visit's bytes: loaded
+  // with the slab, so that the end of the visit does not wait for them
+  __shared__ int s_slot, s_bytes;
+  // a list of no more entries than CTAs has none left to draw
+  const bool draws = f.count > (int)gridDim.x;
   const int tid = threadIdx.x;
   const unsigned bar = smem_u32addr(&s_bar);
   unsigned phase = 0;      // thread 0: parity of the slab copies' current phase
@@ -1122,6 +1144,7 @@ __device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& 
     // and connectivity load (the previous patch's last reads of sM and sH
     // came before its final barrier)
     if (tid == 0) geo_issue(m, es, nep, sM, sH, bar);
+    const int slot0 = tid == 0 ? s.slot[p] : 0, bytes0 = tid == 0 ? __ldg(m.patch_bytes + p) : 0;
     // every load of the patch's own slab is issued before any of them is
     // stored (values, seed flags, connectivity: independent round trips
     // that overlap; a ghost value waits only for its id), then stored.
@@ -1166,6 +1189,8 @@ __device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& 
     if (tid == 0) {
       s_min[par] = 0x7f800000u;
       s_ng = 0;
+      s_slot = slot0 ^ 1;
+      s_bytes = bytes0;
       if (!slab_wait(bar, phase, sp.spin_limit < 0)) {
         // abandoned: the host reports a timeout; the copies are waited for
         // once more so that none is in flight when the CTA leaves
@@ -1313,12 +1338,12 @@ __device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& 
     int drawn = 0;
     if (tid == 0) {
       s_n[0] = s_n[1] = 0;  // read by every thread before the barrier above
-      drawn = atomicAdd(next, 1);
+      if (draws) drawn = atomicAdd(next, 1);
     }
     // a check that found nothing writes nothing
     int con = 1;
     if (visit) {
-      const int slot = s.slot[p] ^ 1;
+      const int slot = s_slot;
       for (int i = tid; i < nvp; i += blockDim.x) {
         const int v = vs + i;
         const float nt = sT[i];
@@ -1334,18 +1359,18 @@ __device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& 
       }
     }
     if (tid == 0) {
-      if (drawn == f.count - 1) atomicExch(next, 0);
-      s_li = (int)gridDim.x + drawn;
+      if (draws && drawn == f.count - 1) atomicExch(next, 0);
+      s_li = (int)gridDim.x + drawn;  // without draws: past the list
     }
     con = __syncthreads_and(con);
     li = s_li;
     if (tid == 0) {
-      if (visit) s.slot[p] ^= 1;
+      if (visit) s.slot[p] = s_slot;
       s_cnt.visits += visit ? 1 : 0;
       s_cnt.checks += check ? 1 : 0;
       s_cnt.early += check && visit ? 1 : 0;
       // a check that stayed a check read the visit's slab but wrote no values
-      s_cnt.bytes += (unsigned long long)(__ldg(m.patch_bytes + p) - (visit ? 0 : 4 * nvp));
+      s_cnt.bytes += (unsigned long long)(s_bytes - (visit ? 0 : 4 * nvp));
     }
     if ((tid >> 5) == ((int)blockDim.x >> 5) - 1)
       fim_publish(m, s, f, p, con != 0, visit && __uint_as_float(s_min[par]) < patch_par(m, sp, p).bw);
@@ -1489,7 +1514,10 @@ __device__ __forceinline__ void fim_loop_persistent(const DevMesh& m, const DevS
     const volatile int* n = s.ctl + CTL_VISITS + t % 3;
     const bool done = n[0] + n[CTL_CANDS - CTL_VISITS] == 0;
     if (done || it > sp.max_fim_iters) {
-      if (!done && blockIdx.x == 0 && threadIdx.x == 0) s.ctl[CTL_CAP] = 1;
+      if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (!done) s.ctl[CTL_CAP] = 1;
+        if (it > 0) count_iteration(s.ctl, s.stats, t - 1);
+      }
       return;
     }
     // above every stamp this iteration uses, also if the launch is abandoned

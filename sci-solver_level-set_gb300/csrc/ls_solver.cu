@@ -355,20 +355,21 @@ std::string Solver::init(const Layout& L, const SolverConfig& cfg, const float* 
 // the cap is exceeded shows one body later); it sets CTL_CAP, so that the
 // host reports a timeout.
 namespace {
-__device__ __forceinline__ bool body_end(int* ctl, int chunk, int cap) {
+__device__ __forceinline__ bool body_end(int* ctl, unsigned long long* stats, int chunk, int cap) {
   ctl[CTL_BODIES] += 1;
   const int t = ctl[CTL_ITER] + chunk;
+  count_iteration(ctl, stats, t - 1);
   ctl[CTL_ITER] = t;
   const bool more = ctl[CTL_VISITS + t % 3] + ctl[CTL_CANDS + t % 3] > 0;
   const bool over = ctl[CTL_ITERS] > cap;
   if (over) ctl[CTL_CAP] = 1;
   return more && !over && ctl[CTL_ERR] == 0;  // a FIM kernel wait that ran out ends the loop
 }
-__global__ void k_body_end(int* ctl, int chunk, int cap) {
-  if (threadIdx.x == 0) body_end(ctl, chunk, cap);
+__global__ void k_body_end(int* ctl, unsigned long long* stats, int chunk, int cap) {
+  if (threadIdx.x == 0) body_end(ctl, stats, chunk, cap);
 }
-__global__ void k_loop_cond(int* ctl, cudaGraphConditionalHandle h, int chunk, int cap) {
-  if (threadIdx.x == 0) cudaGraphSetConditional(h, body_end(ctl, chunk, cap) ? 1u : 0u);
+__global__ void k_loop_cond(int* ctl, unsigned long long* stats, cudaGraphConditionalHandle h, int chunk, int cap) {
+  if (threadIdx.x == 0) cudaGraphSetConditional(h, body_end(ctl, stats, chunk, cap) ? 1u : 0u);
 }
 }  // namespace
 
@@ -489,7 +490,7 @@ std::string Solver::build_graph() {
   err = step_head();
   for (int i = 0; i < first && err == cudaSuccess; ++i) err = K_->fim(m_, s_, sp_, i, L_, stream_);
   if (err == cudaSuccess) {
-    k_loop_cond<<<1, 32, 0, stream_>>>(s_.ctl, hc, first, iter_cap());
+    k_loop_cond<<<1, 32, 0, stream_>>>(s_.ctl, s_.stats, hc, first, iter_cap());
     err = cudaGetLastError();
   }
   const cudaGraphNode_t* deps = nullptr;
@@ -516,7 +517,7 @@ std::string Solver::build_graph() {
   err = cudaSuccess;
   for (int i = 0; i < chunk && err == cudaSuccess; ++i) err = K_->fim(m_, s_, sp_, i, L_, stream_);
   if (err == cudaSuccess) {
-    k_loop_cond<<<1, 32, 0, stream_>>>(s_.ctl, hc, chunk, iter_cap());
+    k_loop_cond<<<1, 32, 0, stream_>>>(s_.ctl, s_.stats, hc, chunk, iter_cap());
     err = cudaGetLastError();
   }
   e2 = cudaStreamEndCapture(stream_, &body);
@@ -547,7 +548,7 @@ std::string Solver::fim_loop(const StepParams& sp) {
   for (int k = 0;; ++k) {
     for (int i = 0; i < cfg_.graph_chunk; ++i)
       LS_TRY(prof([&] { return K_->fim(m_, s_, sp, i, L_, stream_); }), "FIM iteration");
-    k_body_end<<<1, 32, 0, stream_>>>(s_.ctl, cfg_.graph_chunk, iter_cap());
+    k_body_end<<<1, 32, 0, stream_>>>(s_.ctl, s_.stats, cfg_.graph_chunk, iter_cap());
     LS_TRY(cudaGetLastError(), "body end");
     st_.kernel_launches += cfg_.graph_chunk + 1;
     int* const mine = h_chunk_ + (k & 1) * CTL_WORDS;
