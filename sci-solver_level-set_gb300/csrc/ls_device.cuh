@@ -99,7 +99,12 @@ enum {
   CTL_BASE = 13,    // base stamp of the step
   CTL_ITERS = 14,   // iterations of this step that visited a patch
   CTL_LAST = 15,    // stamp of the last iteration that visited a patch
-  CTL_WORDS = 16
+  // a run enqueues a step before it knows how the previous one ended (host-set
+  // CTL_CHAIN, 0 outside a run's later steps): if that one ran out of
+  // narrowband or failed, the step finds CTL_STOP set and does nothing
+  CTL_CHAIN = 16,
+  CTL_STOP = 17,
+  CTL_WORDS = 32
 };
 // Stamps restart (every stamped array cleared) between steps once they pass
 // this limit; a new handle starts a few steps below it.

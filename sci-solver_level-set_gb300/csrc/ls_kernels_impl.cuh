@@ -50,6 +50,8 @@ __global__ void k_begin(DevState s, int restart) {
   int* c = s.ctl;
   for (int i = threadIdx.x; i < kGridBarrierWords; i += blockDim.x) s.gbar[i] = 0u;
   if (threadIdx.x == 0) {
+    c[CTL_STOP] = c[CTL_CHAIN] && (c[CTL_NB] == 0 || c[CTL_CAP] || c[CTL_ERR]) ? 1 : 0;
+    if (c[CTL_STOP]) return;
     for (int i = 0; i < 3; ++i) c[CTL_VISITS + i] = c[CTL_CANDS + i] = 0;
     if (!restart) {
       c[CTL_NB_PREV] = c[CTL_NB_VALID] ? c[CTL_NB] : 0;
@@ -89,12 +91,12 @@ __device__ __forceinline__ FimIter fim_iter(const DevMesh& m, const DevState& s,
   const int cur = f.t % 3, nxt = cur == 2 ? 0 : cur + 1;
   f.base = s_ctl[CTL_BASE];
   f.nvis = s_ctl[CTL_VISITS + cur];
-  f.count = f.nvis + s_ctl[CTL_CANDS + cur];
+  f.count = s_ctl[CTL_STOP] ? 0 : f.nvis + s_ctl[CTL_CANDS + cur];
   f.list = s.lists + (size_t)cur * m.nparts;
   f.next = s.lists + (size_t)nxt * m.nparts;
   f.next_n = s.ctl + CTL_VISITS + nxt;
   // the list after the next one was read by the previous iteration
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  if (blockIdx.x == 0 && threadIdx.x == 0 && !s_ctl[CTL_STOP]) {
     const int aft = nxt == 2 ? 0 : nxt + 1;
     s.ctl[CTL_VISITS + aft] = 0;
     s.ctl[CTL_CANDS + aft] = 0;
@@ -193,6 +195,7 @@ constexpr int kSeedBlock = 128;
 template <int D1>
 __global__ void __launch_bounds__(kSeedBlock) k_seed(DevMesh m, DevState s, StepParams sp, int warm) {
   extern __shared__ float smem[];
+  if (s.ctl[CTL_STOP]) return;
   const int nprev = s.ctl[CTL_NB_PREV];
   const int base = s.ctl[CTL_BASE], t0 = s.ctl[CTL_ITER];
   int* list = s.lists + (size_t)(t0 % 3) * m.nparts;
@@ -1512,7 +1515,7 @@ __device__ __forceinline__ void fim_loop_persistent(const DevMesh& m, const DevS
   for (int it = 0;; ++it) {
     const int t = t0 + it;
     const volatile int* n = s.ctl + CTL_VISITS + t % 3;
-    const bool done = n[0] + n[CTL_CANDS - CTL_VISITS] == 0;
+    const bool done = n[0] + n[CTL_CANDS - CTL_VISITS] == 0 || ld_relaxed(s.ctl + CTL_STOP);
     if (done || it > sp.max_fim_iters) {
       if (blockIdx.x == 0 && threadIdx.x == 0) {
         if (!done) s.ctl[CTL_CAP] = 1;
@@ -1544,6 +1547,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_fim_persist(DevMesh m, DevState 
 // step's result and goes to phi too.  The update then reads phi_rd and
 // writes phi, so that no copy pass follows it.
 __global__ void k_narrowband(DevMesh m, DevState s, StepParams sp, int last) {
+  if (s.ctl[CTL_STOP]) return;
   __shared__ unsigned long long s_cnt, s_pv, s_np;
   if (threadIdx.x == 0) { s_cnt = 0; s_pv = 0; s_np = 0; }
   __syncthreads();
@@ -1841,7 +1845,7 @@ __global__ void __launch_bounds__(kUpdBlock, 8) k_update(DevMesh m, DevState s, 
   float4* sC = smem4;                                          // [lep][REC]
   float* sPhi = reinterpret_cast<float*>(smem4 + REC * sp.lep);  // slab
   float* sX = sPhi + sp.lvp + sp.lgp;                          // 3 * slab (3D only)
-  const int count = s.ctl[CTL_NB];
+  const int count = s.ctl[CTL_STOP] ? 0 : s.ctl[CTL_NB];
   for (int li = blockIdx.x; li < count; li += gridDim.x) {
     const int p = s.nblist[li];
     const PatchPar pp = patch_par(m, sp, p);
@@ -1938,7 +1942,7 @@ inline int update_record(const DevMesh& m, const StepParams& sp) {
 __global__ void k_copy_phi(DevMesh m, DevState s) {
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  const int count = s.ctl[CTL_NB];
+  const int count = s.ctl[CTL_STOP] ? 0 : s.ctl[CTL_NB];
   for (int w = warp_id_global(); w < count; w += nwarps) {
     const int p = s.nblist[w];
     for (int v = m.vert_off[p] + lane; v < m.vert_off[p + 1]; v += 32) s.phi_rd[v] = s.phi[v];
@@ -1946,8 +1950,10 @@ __global__ void k_copy_phi(DevMesh m, DevState s) {
 }
 
 // out[old - first] = phi[new] for n vertices from `first` on in the caller's
-// order (kernel_compute_vertT_before_permute3d), as a gather
-__global__ void k_unpermute(DevMesh m, const float* phi, int first, int n, float* out) {
+// order (kernel_compute_vertT_before_permute3d), as a gather; with ctl only
+// if the step that phi is the result of was done
+__global__ void k_unpermute(DevMesh m, const float* phi, int first, int n, float* out, const int* ctl) {
+  if (ctl && (ctl[CTL_STOP] || ctl[CTL_NB] == 0 || ctl[CTL_CAP] || ctl[CTL_ERR])) return;
   for (int o = blockIdx.x * blockDim.x + threadIdx.x; o < n; o += gridDim.x * blockDim.x)
     out[o] = phi[__ldg(m.ipermute + first + o)];
 }
@@ -2360,9 +2366,9 @@ cudaError_t launch_update(const DevMesh& m, const DevState& s, const StepParams&
                           (size_t)L.upd_smem, st);
 }
 
-cudaError_t launch_unpermute(const DevMesh& m, const float* phi, int first, int n, float* out, const Launch& L,
-                             cudaStream_t st) {
-  k_unpermute<<<std::min(L.flat_grid, (n + 255) / 256), 256, 0, st>>>(m, phi, first, n, out);
+cudaError_t launch_unpermute(const DevMesh& m, const float* phi, int first, int n, float* out, const int* ctl,
+                             const Launch& L, cudaStream_t st) {
+  k_unpermute<<<std::min(L.flat_grid, (n + 255) / 256), 256, 0, st>>>(m, phi, first, n, out, ctl);
   return cudaGetLastError();
 }
 

@@ -356,6 +356,7 @@ std::string Solver::init(const Layout& L, const SolverConfig& cfg, const float* 
 // host reports a timeout.
 namespace {
 __device__ __forceinline__ bool body_end(int* ctl, unsigned long long* stats, int chunk, int cap) {
+  if (ctl[CTL_STOP]) return false;
   ctl[CTL_BODIES] += 1;
   const int t = ctl[CTL_ITER] + chunk;
   count_iteration(ctl, stats, t - 1);
@@ -379,9 +380,10 @@ cudaError_t Solver::restart_stamps(int from) {
   if (e == cudaSuccess) e = cudaMemsetAsync(s_.pend, 0xff, sizeof(int) * m_.nparts, stream_);
   if (e == cudaSuccess) e = cudaMemsetAsync(s_.reach, 0xff, sizeof(int) * m_.nparts, stream_);
   h_ctl_[CTL_ITER] = from;
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(s_.ctl + CTL_ITER, h_ctl_ + CTL_ITER, sizeof(int), cudaMemcpyHostToDevice, stream_);
-  return e;
+  if (e != cudaSuccess) return e;
+  if (from == 0) return cudaMemsetAsync(s_.ctl + CTL_ITER, 0, sizeof(int), stream_);
+  e = cudaMemcpyAsync(s_.ctl + CTL_ITER, h_ctl_ + CTL_ITER, sizeof(int), cudaMemcpyHostToDevice, stream_);
+  return e == cudaSuccess ? cudaStreamSynchronize(stream_) : e;  // h_ctl_ is read until then
 }
 
 // The step control words on the host, and the stream idle.
@@ -565,6 +567,20 @@ std::string Solver::fim_loop(const StepParams& sp) {
   return fim_status();
 }
 
+// A step run in one go has ended with the control words in h_ctl_.
+std::string Solver::step_done(bool* empty_nb) {
+  // begin, seed, the FIM loop, narrowband, the updates and the copies between them
+  const long long upd = cfg_.update_kind != 2 ? 2LL * cfg_.inside_niter - 1 : 0;
+  st_.kernel_launches += 3 + upd + (persistent_ ? 1LL
+                                                : (cfg_.graph_chunk + 1LL) * h_ctl_[CTL_BODIES] +
+                                                      (first_bodies() - 1LL) * cfg_.graph_chunk);
+  std::string r = fim_status();
+  if (!r.empty()) return r;
+  have_nb_ = h_ctl_[CTL_NB] != 0;
+  *empty_nb = !have_nb_;
+  return "";
+}
+
 std::string Solver::one_step(bool* empty_nb) {
   *empty_nb = false;
   auto prof = [&](int kind, auto&& fn) -> cudaError_t {
@@ -580,8 +596,6 @@ std::string Solver::one_step(bool* empty_nb) {
   };
   if (h_ctl_[CTL_ITER] > kStampLimit) LS_TRY(restart_stamps(0), "stamps");
   if (net_ || collect_) return learned_step(empty_nb);
-  // updates, and the copies between them
-  const long long upd = cfg_.update_kind != 2 ? 2LL * cfg_.inside_niter - 1 : 0;
   if (persistent_ || (graph_exec_ && !cfg_.profile)) {
     // the whole step in one go: its graph, or the persistent form launch by
     // launch (profiled: the FIM loop kernel's time is recorded as the sweep time)
@@ -594,15 +608,7 @@ std::string Solver::one_step(bool* empty_nb) {
       if (cfg_.profile) LS_TRY(prof_fim_end(pe), "event");
     }
     LS_TRY(read_ctl(), "step sync");
-    // begin, seed, the FIM loop, narrowband and the updates
-    st_.kernel_launches += 3 + upd + (persistent_ ? 1LL
-                                                  : (cfg_.graph_chunk + 1LL) * h_ctl_[CTL_BODIES] +
-                                                        (first_bodies() - 1LL) * cfg_.graph_chunk);
-    std::string r = fim_status();
-    if (!r.empty()) return r;
-    have_nb_ = h_ctl_[CTL_NB] != 0;
-    *empty_nb = !have_nb_;
-    return "";
+    return step_done(empty_nb);
   }
   LS_TRY(K_->begin(s_, 0, stream_), "begin");
   LS_TRY(prof(3, [&] { return K_->seed(m_, s_, sp_, L_, stream_); }), "seed");
@@ -619,7 +625,7 @@ std::string Solver::one_step(bool* empty_nb) {
   if (cfg_.update_kind != 2) {
     for (int it = 0; it < cfg_.inside_niter; ++it)
       LS_TRY(prof(5, [&] { return K_->update(m_, s_, sp_, it == 0, L_, stream_); }), "update");
-    st_.kernel_launches += upd;
+    st_.kernel_launches += 2LL * cfg_.inside_niter - 1;
   }
   return "";
 }
@@ -814,8 +820,42 @@ void Solver::pull_stats() {
 // ends with a wait); the next step is enqueued behind it.
 std::string Solver::emit_phi(float* row) {
   if (!pageable_) return get_phi(row);
-  LS_TRY(K_->unpermute(m_, s_.phi, 0, m_.nv, row, L_, stream_), "unpermute");
+  LS_TRY(K_->unpermute(m_, s_.phi, 0, m_.nv, row, nullptr, L_, stream_), "unpermute");
   return "";
+}
+
+// Steps of a run as graphs, each enqueued before the host knows how the
+// previous one ended (the round trip, about 15 us, is behind the next step).
+// A step behind one that ran out of narrowband or failed does nothing
+// (CTL_STOP), and neither does its history row.
+std::string Solver::run_chained(int nsteps, float* history, int* done) {
+  std::string r;
+  bool empty = false;
+  auto settle = [&](int s) -> std::string {
+    const int* c = h_chunk_ + (s & 1) * CTL_WORDS;
+    LS_TRY(cudaEventSynchronize(ev_chunk_[s & 1]), "step sync");
+    std::memcpy(h_ctl_, c, sizeof(int) * CTL_WORDS);
+    std::string e = step_done(&empty);
+    if (e.empty() && !empty) ++*done;
+    return e;
+  };
+  int s = 0;
+  for (; s < nsteps && r.empty() && !empty; ++s) {
+    if (h_ctl_[CTL_ITER] > kStampLimit) LS_TRY(restart_stamps(0), "stamps");
+    LS_TRY(cudaGraphLaunch(graph_exec_, stream_), "graph launch");
+    if (history)
+      LS_TRY(K_->unpermute(m_, s_.phi, 0, m_.nv, history + (size_t)(s + 1) * m_.nv, s_.ctl, L_, stream_), "unpermute");
+    LS_TRY(cudaMemcpyAsync(h_chunk_ + (s & 1) * CTL_WORDS, s_.ctl, sizeof(int) * CTL_WORDS, cudaMemcpyDeviceToHost,
+                           stream_), "d2h");
+    LS_TRY(cudaEventRecord(ev_chunk_[s & 1], stream_), "event");
+    if (s == 0) LS_TRY(cudaMemsetAsync(s_.ctl + CTL_CHAIN, 1, sizeof(int), stream_), "memset");
+    if (s > 0) r = settle(s - 1);
+  }
+  // the last enqueued step, unless the one before it ended the run
+  if (r.empty() && !empty && s > 0) r = settle(s - 1);
+  LS_TRY(cudaMemsetAsync(s_.ctl + CTL_CHAIN, 0, sizeof(int), stream_), "memset");
+  LS_TRY(cudaStreamSynchronize(stream_), "run sync");
+  return r;
 }
 
 std::string Solver::run(int nsteps, float* history, int* steps_done) {
@@ -823,7 +863,12 @@ std::string Solver::run(int nsteps, float* history, int* steps_done) {
   std::string h;
   if (history && !(h = emit_phi(history)).empty()) return h;
   LS_TRY(cudaEventRecord(ev0_, stream_), "event");
-  for (int s = 0; s < nsteps; ++s) {
+  const bool chained = nsteps > 1 && graph_exec_ && !cfg_.profile && !net_ && !collect_ && (!history || pageable_);
+  if (chained) {
+    h = run_chained(nsteps, history, &done);
+    if (!h.empty()) return h;
+  }
+  for (int s = 0; s < nsteps && !chained; ++s) {
     bool empty = false;
     std::string r = one_step(&empty);
     if (!r.empty()) return r;
@@ -862,7 +907,7 @@ std::string Solver::step_host(const float* phi_in, float* phi_out) {
   if (!r.empty()) return r;
   if (cfg_.profile) fold_prof(true);
   if (pageable_) {
-    LS_TRY(K_->unpermute(m_, s_.phi, 0, nv, phi_out, L_, stream_), "unpermute out");
+    LS_TRY(K_->unpermute(m_, s_.phi, 0, nv, phi_out, nullptr, L_, stream_), "unpermute out");
     LS_TRY(cudaStreamSynchronize(stream_), "sync");
   } else {
     r = get_phi(phi_out);
@@ -985,7 +1030,7 @@ std::string Solver::set_phi(const float* phi_orig) {
 
 std::string Solver::get_phi(float* phi_orig, int first, int n) {
   float* const dst = pageable_ ? phi_orig : d_tmp_;
-  LS_TRY(K_->unpermute(m_, s_.phi, first, n, dst, L_, stream_), "unpermute");
+  LS_TRY(K_->unpermute(m_, s_.phi, first, n, dst, nullptr, L_, stream_), "unpermute");
   if (!pageable_)
     LS_TRY(cudaMemcpyAsync(h_stage_, d_tmp_, sizeof(float) * n, cudaMemcpyDeviceToHost, stream_), "d2h");
   LS_TRY(cudaStreamSynchronize(stream_), "sync");

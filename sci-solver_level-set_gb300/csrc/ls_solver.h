@@ -44,9 +44,9 @@ struct KernelSet {
   // FIM distances in the layout's vertex order
   cudaError_t (*distances)(const DevMesh& m, const DevState& s, const StepParams& sp, float* out, const Launch& L,
                            cudaStream_t st);
-  // n vertices from `first` on in the caller's order
-  cudaError_t (*unpermute)(const DevMesh& m, const float* phi, int first, int n, float* out, const Launch& L,
-                           cudaStream_t st);
+  // n vertices from `first` on in the caller's order (ctl: only if the step was done)
+  cudaError_t (*unpermute)(const DevMesh& m, const float* phi, int first, int n, float* out, const int* ctl,
+                           const Launch& L, cudaStream_t st);
   cudaError_t (*permute)(const DevMesh& m, const float* in, float* out, const Launch& L, cudaStream_t st);
   // learned warm start / collection kernels (op: LEARN_*)
   cudaError_t (*learn)(int op, const DevMesh& m, const DevState& s, const StepParams& sp, const DevLearn& lr, int arg,
@@ -156,6 +156,8 @@ class Solver {
   int first_bodies() const { return m_.dim == 3 ? 3 : 2; }  // loop bodies' worth of iterations before the loop
   bool build_persistent_graph(std::string* err);
   std::string emit_phi(float* row);
+  std::string run_chained(int nsteps, float* history, int* done);
+  std::string step_done(bool* empty_nb);
   cudaError_t step_head();
   cudaError_t step_tail();
   cudaError_t step_persistent_launches();
