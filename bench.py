@@ -606,8 +606,7 @@ def main():
     ps = ls.stats()
     ls.set_profile(False)
     peak, peak_kind = load_peaks()
-    # the FIM patch kernel: sweep launches and neighbour-check launches (a
-    # check that activates its patch runs the patch's visit in the same launch)
+    # the FIM patch kernel: one launch per iteration (its checks and visits)
     fim_launches = max(ps["n_sweep"] + ps["n_check"], 1)
     sweep_ms = (ps["ms_sweep"] + ps["ms_check"]) / fim_launches
     bytes_per_launch = ps["sweep_slab_bytes"] / fim_launches
@@ -615,12 +614,12 @@ def main():
     step_ms_prof = (ps["ms_sweep"] + ps["ms_check"] + ps["ms_schedule"] + ps["ms_seed"] + ps["ms_narrowband"]
                     + ps["ms_update"])
     kernel_ms = {k: ps["ms_" + k] / prof_steps for k in ("sweep", "check", "schedule", "seed", "narrowband", "update")}
-    # the sweep kernel the run used: two element copies per thread at the
-    # setting 5 (patches of up to 384 copies), one per thread otherwise
-    sweep_kernel = "k_fim_pair" if ls.get_params().fim_ctas_per_sm == 5 else "k_fim_compact"
+    # the FIM kernel the run used: k_fim_pair at the settings 5 to 7 (patches
+    # of up to 384 copies), one copy per thread otherwise
+    sweep_kernel = "k_fim_pair" if ls.get_params().fim_ctas_per_sm in (5, 6, 7) else "k_fim_compact"
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": profile_traffic(bytes_per_launch),
-                "kernel": sweep_kernel + " (FIM patch sweep and check launches)",
+                "kernel": sweep_kernel + " (FIM iterations: checks, visits and the next list)",
                 "traffic_source": "this run's algorithmic bytes per launch x the DRAM/algorithmic ratio of an ncu "
                                   "capture (dram__bytes_read.sum + dram__bytes_write.sum) of this kernel build's "
                                   "first FIM launches at 96^3, profiles/k_fim_sweep_c3.md",
@@ -628,10 +627,10 @@ def main():
                 "peak_source": peak_kind,
                 "share_of_step": ((ps["ms_sweep"] + ps["ms_check"]) / step_ms_prof) if step_ms_prof > 0 else None,
                 "algorithmic_bytes_per_launch": bytes_per_launch, "avg_launch_ms": sweep_ms,
-                # the FIM kernel is bound by instruction issue of the local
-                # solvers, not by HBM: issue slots active from the committed
-                # ncu capture of its sweep and check launches
-                "limiter": "SM instruction issue (FP32/ALU/MUFU of the local solvers); DRAM at 4-13 % of peak",
+                # the FIM kernel is bound by instruction issue and the barriers
+                # between listing and solving, not by HBM: issue slots active
+                # from the committed ncu capture
+                "limiter": "SM instruction issue and CTA barriers (listing and local solvers); DRAM at 10-20 % of peak",
                 "issue_slots_active": profile_value("issue_slots_active")}
 
     cpu = None

@@ -306,6 +306,20 @@ std::string Solver::init(const Layout& L, const SolverConfig& cfg, const float* 
   sp_.tau = (cfg.fp64_flagged && L.dim == 3) ? (float)cfg.fp64_tau : 0.f;
   sp_.xdiv = (cfg.bit_exact && ref) ? 1 : 0;
   sp_.ctas = (cfg.fim_ctas >= 2 && cfg.fim_ctas <= 7) ? cfg.fim_ctas : 5;
+  if (sp_.ctas == 5 && !cfg.bit_exact && L.dim == 3) {
+    // The default's tet sweep on large meshes: its six-CTA form (56 instead of
+    // 64 registers, a few spilled), where the lists are long enough for the
+    // sixth CTA to hide more than the spills cost.  Step times with 64 / 56
+    // registers: 32^3 (1,331 patches) 229 / 232 us, 48^3 (4,913) 323 / 319,
+    // 64^3 (10,648) 436 / 431, 80^3 (19,683) 605 / 590, 112^3 (54,872) 1009 /
+    // 958, 128^3 (79,507) 1108 / 1070; graph patches of 16 vertices, 64^3
+    // (17,165) 791 / 778, 80^3 (33,000) 966 / 987.  The bit-exact build's
+    // solver spills more: 48^3 726 / 783 us.  Same results.
+    int dev = 0, sms = 0;
+    LS_TRY(cudaGetDevice(&dev), "device");
+    LS_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "device");
+    if (np >= 100 * sms) sp_.ctas = 6;
+  }
   sp_.tol = (float)cfg.smallnum;
   sp_.eps_h64 = cfg.smallnum;
   sp_.eps_h = (float)sp_.eps_h64;
