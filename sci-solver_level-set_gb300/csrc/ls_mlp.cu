@@ -404,12 +404,20 @@ __device__ __forceinline__ void weighted_column_sums(const uint8_t* tile, const 
 // [gW (3x128x128) | gb (3x128) | gw4 (128) | gb4 (1) | loss (1)]; the rows
 // are added in a fixed order (no atomics in global memory, the same gradient
 // bits on every run).
-// Bound by the chain of a tile (six products with their epilogues, about
-// 2 us each): at 8,192 samples 64 CTAs have one tile each.  The separate
-// forward (19.5 us) and backward (70.7 us: explicit 2-byte transposes of d
-// and a, 640 shuffles for gw4, 2-byte loads of the activations) took 90 us
-// for such a batch.
+// Bound by the chain of a tile (six products with their epilogues): at 8,192
+// samples 64 CTAs have one tile each, 24.5 us.  The separate forward (19.5
+// us) and backward (70.7 us: explicit 2-byte transposes of d and a, 640
+// shuffles for gw4, 2-byte loads of the activations) took 90 us for such a
+// batch; this kernel with rows of Gp in parameter order 30 us.
+// A row's weight gradients lie as the accumulators are read out, four columns
+// of 128 rows at a time (whole 512-byte stores of a warp).
 constexpr int NG_ROW = 3 * F * F + 3 * F + F + 1 + 1;
+// The element of G's order at place j of a row.
+__device__ __forceinline__ int grad_element(int j) {
+  if (j >= 3 * F * F) return j;
+  const int l = j / (F * F), c = (j / (4 * F)) % (F / 4), r = (j / 4) % F;
+  return (l * F + r) * F + c * 4 + j % 4;
+}
 // rows of Gp start on 16-byte boundaries (the weight gradients are stored as
 // float4)
 constexpr int NG_STRIDE = (NG_ROW + 3) & ~3;
@@ -572,9 +580,9 @@ __global__ void __launch_bounds__(THREADS, 1)
       for (int c = 0; c < 64; c += 32) {
         float v[32];
         tmem_ld32(tm + lanes + l * 128 + c0 + c, v);
-        float4* dst = reinterpret_cast<float4*>(row + ((size_t)l * F + r) * F + c0 + c);
+        float4* dst = reinterpret_cast<float4*>(row) + (size_t)(l * (F / 4) + (c0 + c) / 4) * F + r;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) dst[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        for (int q = 0; q < 8; ++q) dst[q * F] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
       }
     for (int o = 16; o > 0; o >>= 1) {
       gb4_acc += __shfl_xor_sync(0xffffffffu, gb4_acc, o);
@@ -604,7 +612,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   if (warp == 0) tmem_dealloc(tm, 512);
 }
 
-// Sum of column i over the rows of Gp, in row order.
+// Sum of place i of the rows of Gp, in row order.
 __device__ __forceinline__ float row_sum(const float* __restrict__ Gp, int rows, int i) {
   float sum = 0.f;
   int r = 0;
@@ -622,7 +630,7 @@ __device__ __forceinline__ float row_sum(const float* __restrict__ Gp, int rows,
 // G[i] = sum over the rows of Gp (fixed order).
 __global__ void k_mlp_reduce(const float* __restrict__ Gp, int rows, float* __restrict__ G) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NG_ROW; i += gridDim.x * blockDim.x)
-    G[i] = row_sum(Gp, rows, i);
+    G[grad_element(i)] = row_sum(Gp, rows, i);
 }
 
 // ---------------------------------------------------------------------------
@@ -633,9 +641,10 @@ __global__ void k_mlp_reduce(const float* __restrict__ Gp, int rows, float* __re
 __global__ void k_adam(float* __restrict__ P, const float* __restrict__ Gp, int rows, float* __restrict__ M1,
                        float* __restrict__ M2, int np, float lr, float b1, float b2, float eps, float c1, float c2,
                        __nv_bfloat16* __restrict__ Wt, float* __restrict__ loss_acc) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= NG_ROW) return;
-  const float g = row_sum(Gp, rows, i);
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= NG_ROW) return;
+  const float g = row_sum(Gp, rows, j);
+  const int i = grad_element(j);
   if (i >= np) {
     *loss_acc += g;
     return;
@@ -769,11 +778,16 @@ Net::~Net() {
   if (PX_) cudaFree(PX_);
   if (PT_) cudaFree(PT_);
   if (pair_count_) cudaFree(pair_count_);
+  for (cudaEvent_t e : uploaded_)
+    if (e) cudaEventDestroy(e);
+  if (upload_) cudaStreamDestroy(upload_);
   if (stream_) cudaStreamDestroy(stream_);
 }
 
 std::string Net::init(unsigned long long seed) {
   MLP_TRY(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "stream");
+  MLP_TRY(cudaStreamCreateWithFlags(&upload_, cudaStreamNonBlocking), "stream");
+  for (cudaEvent_t& e : uploaded_) MLP_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
   auto alloc = [&](void** p, size_t bytes) -> cudaError_t {
     cudaError_t e = cudaMalloc(p, bytes);
     if (e == cudaSuccess) allocs_.push_back(*p);
@@ -873,15 +887,15 @@ size_t Net::staging_bytes(size_t n) const { return pageable_ ? 0 : align256(n * 
 
 // Host rows -> BF16 on the device, through the GPU's own access to the
 // caller's array where it has it, otherwise through `staging`.
-std::string Net::upload_rows(const float* Xh, size_t n, __nv_bfloat16* X, char* staging) {
+std::string Net::upload_rows(const float* Xh, size_t n, __nv_bfloat16* X, char* staging, cudaStream_t st) {
   const float* src = Xh;
   if (!pageable_) {
-    MLP_TRY(cudaMemcpyAsync(staging, Xh, sizeof(float) * n * F, cudaMemcpyHostToDevice, stream_), "h2d");
+    MLP_TRY(cudaMemcpyAsync(staging, Xh, sizeof(float) * n * F, cudaMemcpyHostToDevice, st), "h2d");
     src = reinterpret_cast<const float*>(staging);
   }
   const size_t quads = (n * F + 3) / 4;
   const int grid = (int)std::min<size_t>((quads + 255) / 256, (size_t)sms_ * 8);
-  k_to_bf16<<<grid, 256, 0, stream_>>>(src, n * F, (reinterpret_cast<uintptr_t>(src) & 15) == 0, X);
+  k_to_bf16<<<grid, 256, 0, st>>>(src, n * F, (reinterpret_cast<uintptr_t>(src) & 15) == 0, X);
   MLP_TRY(cudaGetLastError(), "conversion");
   return "";
 }
@@ -913,7 +927,7 @@ std::string Net::predict(const float* Xh, int n, float* yh) {
   if (!w) return "alloc";
   __nv_bfloat16* X = reinterpret_cast<__nv_bfloat16*>(w);
   float* y = reinterpret_cast<float*>(w + bx);
-  std::string r = upload_rows(Xh, n, X, w + bx + by);
+  std::string r = upload_rows(Xh, n, X, w + bx + by, stream_);
   if (r.empty()) r = forward_dev(X, n, nullptr, n, y, stream_);
   if (r.empty()) {
     cudaError_t e = cudaMemcpyAsync(yh, y, sizeof(float) * n, cudaMemcpyDeviceToHost, stream_);
@@ -931,7 +945,7 @@ std::string Net::gradients(const float* Xh, const float* th, int n, float* gh, f
   __nv_bfloat16* X = reinterpret_cast<__nv_bfloat16*>(w);
   float* t = reinterpret_cast<float*>(w + bx);
   auto body = [&]() -> std::string {
-    std::string r = upload_rows(Xh, n, X, w + bx + bt);
+    std::string r = upload_rows(Xh, n, X, w + bx + bt, stream_);
     if (!r.empty()) return r;
     MLP_TRY(cudaMemcpyAsync(t, th, sizeof(float) * n, cudaMemcpyHostToDevice, stream_), "h2d");
     int rows = 0;
@@ -957,17 +971,31 @@ std::string Net::train(const float* Xh, const float* th, int n, int epochs, int 
   if (!w) return "alloc";
   __nv_bfloat16* X = reinterpret_cast<__nv_bfloat16*>(w);
   float* t = reinterpret_cast<float*>(w + bx);
-  std::string r = upload_rows(Xh, n, X, w + bx + bt);
-  if (r.empty() &&
-      cudaMemcpyAsync(t, th, sizeof(float) * (size_t)n, cudaMemcpyHostToDevice, stream_) != cudaSuccess)
-    r = "h2d";
-  if (r.empty()) r = train_device(X, t, n, epochs, batch, lr, last_loss);
+  // The rows arrive in up to kUploads pieces of whole batches on a stream of
+  // their own, the first epoch's batches wait for theirs: the transfer (150 us
+  // for 25.6 MB) runs behind the training of the pieces before.
+  const size_t batches = ((size_t)n + batch - 1) / batch;
+  const size_t per = (batches + kUploads - 1) / kUploads * (size_t)batch;  // rows of a piece
+  auto body = [&]() -> std::string {
+    MLP_TRY(cudaMemcpyAsync(t, th, sizeof(float) * (size_t)n, cudaMemcpyHostToDevice, stream_), "h2d");
+    int piece = 0;
+    for (size_t r0 = 0; r0 < (size_t)n; r0 += per, ++piece) {
+      const size_t rows = std::min(per, (size_t)n - r0);
+      std::string r = upload_rows(Xh + r0 * F, rows, X + r0 * F, w + bx + bt + (pageable_ ? 0 : r0 * F * sizeof(float)),
+                                  upload_);
+      if (!r.empty()) return r;
+      MLP_TRY(cudaEventRecord(uploaded_[piece], upload_), "event");
+    }
+    return train_device(X, t, n, epochs, batch, lr, last_loss, per);
+  };
+  std::string r = body();
+  cudaStreamSynchronize(upload_);
   cudaStreamSynchronize(stream_);
   return trim(r);
 }
 
 std::string Net::train_device(const __nv_bfloat16* X, const float* t, int n, int epochs, int batch, float lr,
-                              float* last_loss) {
+                              float* last_loss, size_t piece_rows) {
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   float loss_sum = 0.f;
   int loss_cnt = 0;
@@ -977,6 +1005,8 @@ std::string Net::train_device(const __nv_bfloat16* X, const float* t, int n, int
     loss_cnt = 0;
     for (int s0 = 0; s0 < n; s0 += batch) {
       const int m = (n - s0) < batch ? (n - s0) : batch;
+      if (piece_rows && ep == 0 && (size_t)s0 % piece_rows == 0)
+        MLP_TRY(cudaStreamWaitEvent(stream_, uploaded_[(size_t)s0 / piece_rows], 0), "wait");
       int rows = 0;
       std::string r = gradient_rows(X + (size_t)s0 * F, m, t + s0, &rows);
       if (!r.empty()) return r;
@@ -1110,7 +1140,7 @@ std::string Net::train_pairs(int epochs, int batch, float lr, unsigned long long
   cudaMemcpyAsync(dperm, perm.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, stream_);
   k_gather_pairs<<<4096, 256, 0, stream_>>>(PX_, PT_, dperm, n, Xs, ts);
   if (cudaGetLastError() != cudaSuccess) return fin("gather pairs");
-  return fin(train_device(Xs, ts, (int)n, epochs, batch, lr, last_loss));
+  return fin(train_device(Xs, ts, (int)n, epochs, batch, lr, last_loss, 0));
 }
 
 }  // namespace mlp

@@ -45,11 +45,15 @@ class Net {
   char* workspace(size_t bytes);
   std::string trim(std::string r);
   size_t staging_bytes(size_t n) const;
-  std::string upload_rows(const float* Xh, size_t n, __nv_bfloat16* X, char* staging);
+  std::string upload_rows(const float* Xh, size_t n, __nv_bfloat16* X, char* staging, cudaStream_t st);
   // gradients of the batch as *rows rows of Gp_, one per CTA
   std::string gradient_rows(const __nv_bfloat16* X, int n, const float* t, int* rows);
+  // piece_rows > 0: the rows arrive in pieces of that many (uploaded_)
   std::string train_device(const __nv_bfloat16* X, const float* t, int n, int epochs, int batch, float lr,
-                           float* last_loss);
+                           float* last_loss, size_t piece_rows);
+  static constexpr int kUploads = 8;
+  cudaStream_t upload_ = nullptr;
+  cudaEvent_t uploaded_[kUploads] = {};
   char* ws_ = nullptr;  // workspace of the host-buffer entry points
   size_t ws_bytes_ = 0;
   int* h_end_ = nullptr;  // pinned mirror of the error word and the loss
