@@ -465,68 +465,6 @@ __device__ __forceinline__ float tet_solve_pred(float TA, float TB, float TC, fl
   return fminf(TD, fminf(FaceTBC, fminf(FaceTAB, FaceTAC)));
 }
 
-// One of the four quadratics of tet_solve in double, with its candidates, for
-// the precision form's repeats (part 0: side BC and edge CD, 1: side AB and
-// edge BD, 2: side AC and edge AD, 3: the interior); the least of the four
-// parts is tet_solve's result.  The FP64 rate is 1/64 of FP32's, so that a
-// double instruction of one warp, however few of its lanes have a solve,
-// holds its SM quarter's pipe for 64 cycles: a repeat as a whole took one
-// quarter 9 us while the other three idled, its parts run on all four.  A
-// quadratic's two roots share one reciprocal.  `part` is the same in all
-// lanes of a warp.
-__device__ __forceinline__ double tet_part_f64(int part, double TA, double TB, double TC, double ACAC, double ACBC,
-                                               double ACCD, double BCBC, double BCCD, double CDCD, double eps_h) {
-  const double TAC = TC - TA, TBC = TC - TB, TAB = TB - TA;
-  double p, q, r, best;
-  double s = 0.0, t = 0.0, ih = 0.0;
-  if (part == 0) {
-    p = BCBC * TBC * TBC - BCBC * BCBC;
-    q = (BCCD + BCCD) * TBC * TBC - 2.0 * BCBC * BCCD;
-    r = TBC * TBC * CDCD - BCCD * BCCD;
-    best = TC + sqrt(CDCD);
-  } else if (part == 1) {
-    const double gx = ACAC - ACBC, gy = ACBC - BCBC, gz = ACCD - BCCD, TT = TAB * TAB;
-    const double xx = TT * ACAC - gx * gx, yy = TT * BCBC - gy * gy, xy = 2.0 * (TT * ACBC - gx * gy);
-    const double xz = 2.0 * (TT * ACCD - gx * gz), yz = 2.0 * (TT * BCCD - gy * gz);
-    p = xx + yy - xy;
-    q = -2.0 * yy + xy + xz - yz;
-    r = yy + yz + (TT * CDCD - gz * gz);
-    best = TB + sqrt((BCBC + BCCD) + (BCCD + CDCD));
-  } else if (part == 2) {
-    p = ACAC * TAC * TAC - ACAC * ACAC;
-    q = (ACCD + ACCD) * TAC * TAC - 2.0 * ACAC * ACCD;
-    r = TAC * TAC * CDCD - ACCD * ACCD;
-    best = TA + sqrt((ACAC + ACCD) + (ACCD + CDCD));
-  } else {
-    const double h = -(TAC * BCBC - TBC * ACBC);
-    s = TAC * ACBC - TBC * ACAC;
-    t = TAC * BCCD - TBC * ACCD;
-    const double TT = TAC * TAC;
-    const double xx = TT * ACAC - ACAC * ACAC, yy = TT * BCBC - ACBC * ACBC, xy = 2.0 * (TT * ACBC - ACAC * ACBC);
-    const double xz = 2.0 * (TT * ACCD - ACAC * ACCD), yz = 2.0 * (TT * BCCD - ACBC * ACCD);
-    p = xx * h * h + yy * s * s + xy * s * h;
-    q = 2.0 * yy * s * t + xy * t * h + xz * h * h + yz * s * h;
-    r = yy * t * t + yz * t * h + (TT * CDCD - ACCD * ACCD) * h * h;
-    ih = 1.0 / (h + eps_h);
-    best = 1e300;
-  }
-  // a negative discriminant gives NaN roots, which fail every range test
-  const double sq = sqrt(q * q - 4.0 * p * r), inv = 1.0 / (2.0 * p);
-#pragma unroll
-  for (int sgn = 0; sgn < 2; ++sgn) {
-    const double l = (sgn ? -q - sq : -q + sq) * inv;
-    // the weights of A, B, C
-    const double k = 1.0 - l, l2 = (s * l + t) * ih;
-    const double wa = part == 0 ? 0.0 : l, wb = part == 0 ? l : part == 1 ? k : part == 2 ? 0.0 : l2;
-    const double wc = part == 1 ? 0.0 : part == 3 ? k - l2 : k;
-    if (l >= 0.0 && l <= 1.0 && wb >= 0.0 && wb <= 1.0 && wc >= 0.0 && wc <= 1.0)
-      best = fmin(best, TA * wa + TB * wb + TC * wc +
-                            sqrt((wa * ACAC + wb * ACBC + ACCD) * wa + (wa * ACBC + wb * BCBC + BCCD) * wb +
-                                 (wa * ACCD + wb * BCCD + CDCD)));
-  }
-  return best;
-}
-
 // l in [+0, 1] as one unsigned compare of the bits (negative values, -0.0
 // and NaN fail).  A candidate rejected for l = -0.0 sits at the side's end
 // point, where the edge candidate gives the same value.

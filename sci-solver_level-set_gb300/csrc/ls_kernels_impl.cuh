@@ -316,8 +316,8 @@ __device__ __forceinline__ void solve_copy_flags(const float* Mt, const float T[
 }
 
 // The FP64 repeat of solve k of a tet copy (the argument order of the calls
-// above), or part `part` of it (tet_part_f64).  The arguments are selected
-// first, so that the lanes of a warp run one solve together whatever their k.
+// above).  The arguments are selected first, so that the lanes of a warp run
+// one solve together whatever their k.
 struct RepeatArgs {
   float t0, t1, t2, g0, g1, g2, g3, g4, g5;
 };
@@ -791,9 +791,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_fim_compact(DevMesh m, DevState 
           r = tet_solve_wave(a0, a1, a2, g0, g1, -g2, g3, -g4, g5, sH[k * MAXT + cc], sp.eps_h);
         if (PREC && ill) {
           // discriminant cancelled: repeat in FP64 after this pass, densely
-          // (a ghost target's result starts from its value)
           sRep[atomicAdd(&s_rep, 1)] = code;
-          sR[k * MAXT + cc] = own;
           continue;
         }
         const float nw = fminf(own, r);
@@ -804,29 +802,27 @@ __global__ void __launch_bounds__(MAXT, MINB) k_fim_compact(DevMesh m, DevState 
       }
       __syncthreads();
       if constexpr (PREC) {
-        // each repeat's four parts on warps of different SM quarters (warp w
-        // runs on quarter w % 4); blocks of fewer than four warps take several
-        // parts per warp
-        const int nrep = s_rep, nw = blockDim.x >> 5, warp = tid >> 5;
-        const int groups = nw >> 2, pstep = groups ? 4 : nw;
-        const int first = groups ? (warp >> 2) * 32 + (tid & 31) : (tid & 31), step = groups ? groups * 32 : 32;
-        if (!groups || warp < 4 * groups)
-          for (int part = groups ? (warp & 3) : warp; part < 4; part += pstep)
-            for (int i = first; i < nrep; i += step) {
-              const int code = sRep[i];
-              const int cc = code >> 2, k = code & 3;
-              float Mq[11], Tq[4];
+        // one repeat per thread: the FP64 rate is 1/64 of FP32's, so a double
+        // instruction of a warp holds its SM quarter's pipe for 64 cycles however
+        // few of its lanes have a repeat; with the arguments selected first the
+        // four targets' repeats share one pass (33^3 FIM launches of a step 2300
+        // -> 1350 us)
+        const int nrep = s_rep;
+        for (int i = tid; i < nrep; i += blockDim.x) {
+          const int code = sRep[i];
+          const int cc = code >> 2, k = code & 3;
+          float Mq[11], Tq[4];
 #pragma unroll
-              for (int j = 0; j < 11; ++j) Mq[j] = sM[j * MAXT + cc];
+          for (int j = 0; j < 11; ++j) Mq[j] = sM[j * MAXT + cc];
 #pragma unroll
-              for (int j = 0; j < 4; ++j) Tq[j] = sTc[j * MAXT + cc];
-              const RepeatArgs a = repeat_args(Mq, Tq, k);
-              const float r = (float)tet_part_f64(part, a.t0, a.t1, a.t2, a.g0, a.g1, a.g2, a.g3, a.g4, a.g5, sp.eps_h64);
-              const ushort4 cv = sC[cc];
-              const int tk = k == 0 ? cv.x : k == 1 ? cv.y : k == 2 ? cv.z : cv.w;
-              atomicMin(reinterpret_cast<int*>(tk < nvp ? &sT[tk] : &sR[k * MAXT + cc]), __float_as_int(r));
-              if (part == 0) nflag++;
-            }
+          for (int j = 0; j < 4; ++j) Tq[j] = sTc[j * MAXT + cc];
+          const float nw = fminf(Tq[k], solve_k_fp64(Mq, Tq, k, sp.eps_h64, sp.largenum));
+          const ushort4 cv = sC[cc];
+          const int tk = k == 0 ? cv.x : k == 1 ? cv.y : k == 2 ? cv.z : cv.w;
+          if (tk < nvp) atomicMin(reinterpret_cast<int*>(&sT[tk]), __float_as_int(nw));
+          else sR[k * MAXT + cc] = nw;
+          nflag++;
+        }
         __syncthreads();
         if (tid == 0) s_rep = 0;
       }
