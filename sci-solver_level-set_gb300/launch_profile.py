@@ -6,7 +6,8 @@ Builds the curvature-flow workload of the benchmark at n^3 cells (seeded
 jittered cube, three spheres, 3x3x3-vertex patches), turns per-kernel
 profiling on before the first step and runs `steps` time steps kernel by
 kernel.  It prints one line per FIM launch (the first `launches` of them,
-all when 0): kind (sweep / check), device time from CUDA events on the
+all when 0; one launch is one FIM iteration, its checks and visits
+together): kind (always sweep), device time from CUDA events on the
 library's stream, and the algorithmic slab bytes of the patch visits and
 checks that launch ran, then their sums.
 
