@@ -595,8 +595,24 @@ std::string Solver::step_done(bool* empty_nb) {
   return "";
 }
 
+// Nothing may be in flight that reads or writes a caller's array when a call
+// returns an error: the caller may free it then.
+std::string Solver::settled(std::string r) {
+  if (!r.empty()) cudaStreamSynchronize(stream_);
+  return r;
+}
+
+// Ends a chain of steps (run_chained), also one whose end failed before.
+cudaError_t Solver::end_chain() {
+  if (!chained_) return cudaSuccess;
+  const cudaError_t e = cudaMemsetAsync(s_.ctl + CTL_CHAIN, 0, sizeof(int), stream_);
+  if (e == cudaSuccess) chained_ = false;
+  return e;
+}
+
 std::string Solver::one_step(bool* empty_nb) {
   *empty_nb = false;
+  LS_TRY(end_chain(), "memset");
   auto prof = [&](int kind, auto&& fn) -> cudaError_t {
     if (!cfg_.profile) return fn();
     ProfEvent pe;
@@ -833,7 +849,7 @@ void Solver::pull_stats() {
 // row is on its way when this returns and complete when the stream is (run
 // ends with a wait); the next step is enqueued behind it.
 std::string Solver::emit_phi(float* row) {
-  if (!pageable_) return get_phi(row);
+  if (!pageable_) return store_phi(row, 0, m_.nv);
   LS_TRY(K_->unpermute(m_, s_.phi, 0, m_.nv, row, nullptr, L_, stream_), "unpermute");
   return "";
 }
@@ -843,6 +859,15 @@ std::string Solver::emit_phi(float* row) {
 // A step behind one that ran out of narrowband or failed does nothing
 // (CTL_STOP), and neither does its history row.
 std::string Solver::run_chained(int nsteps, float* history, int* done) {
+  LS_TRY(end_chain(), "memset");
+  std::string r = enqueue_chain(nsteps, history, done);
+  const cudaError_t e = end_chain();
+  if (r.empty()) r = check(e, "memset");
+  if (r.empty()) r = check(cudaStreamSynchronize(stream_), "run sync");
+  return r;
+}
+
+std::string Solver::enqueue_chain(int nsteps, float* history, int* done) {
   std::string r;
   bool empty = false;
   auto settle = [&](int s) -> std::string {
@@ -862,17 +887,18 @@ std::string Solver::run_chained(int nsteps, float* history, int* done) {
     LS_TRY(cudaMemcpyAsync(h_chunk_ + (s & 1) * CTL_WORDS, s_.ctl, sizeof(int) * CTL_WORDS, cudaMemcpyDeviceToHost,
                            stream_), "d2h");
     LS_TRY(cudaEventRecord(ev_chunk_[s & 1], stream_), "event");
-    if (s == 0) LS_TRY(cudaMemsetAsync(s_.ctl + CTL_CHAIN, 1, sizeof(int), stream_), "memset");
+    if (s == 0) {
+      chained_ = true;
+      LS_TRY(cudaMemsetAsync(s_.ctl + CTL_CHAIN, 1, sizeof(int), stream_), "memset");
+    }
     if (s > 0) r = settle(s - 1);
   }
   // the last enqueued step, unless the one before it ended the run
   if (r.empty() && !empty && s > 0) r = settle(s - 1);
-  LS_TRY(cudaMemsetAsync(s_.ctl + CTL_CHAIN, 0, sizeof(int), stream_), "memset");
-  LS_TRY(cudaStreamSynchronize(stream_), "run sync");
   return r;
 }
 
-std::string Solver::run(int nsteps, float* history, int* steps_done) {
+std::string Solver::run_steps(int nsteps, float* history, int* steps_done) {
   int done = 0;
   std::string h;
   if (history && !(h = emit_phi(history)).empty()) return h;
@@ -902,7 +928,7 @@ std::string Solver::run(int nsteps, float* history, int* steps_done) {
   return "";
 }
 
-std::string Solver::step_host(const float* phi_in, float* phi_out) {
+std::string Solver::step_buffers(const float* phi_in, float* phi_out) {
   const int nv = m_.nv;
   if (pageable_) {
     // the GPU reads and writes the caller's pageable host arrays directly
@@ -924,7 +950,7 @@ std::string Solver::step_host(const float* phi_in, float* phi_out) {
     LS_TRY(K_->unpermute(m_, s_.phi, 0, nv, phi_out, nullptr, L_, stream_), "unpermute out");
     LS_TRY(cudaStreamSynchronize(stream_), "sync");
   } else {
-    r = get_phi(phi_out);
+    r = store_phi(phi_out, 0, nv);
     if (!r.empty()) return r;
   }
   if (!empty) st_.steps_run++;
@@ -978,7 +1004,7 @@ __global__ void k_eik_out(DevMesh m, DevState s, float scale, float LN, float* o
 }
 }  // namespace
 
-std::string Solver::eikonal(const int* seeds, const float* values, int nseeds, float* out) {
+std::string Solver::solve_eikonal(const int* seeds, const float* values, int nseeds, float* out) {
   if (m_.patch_mesh) {
     status_ = 1;
     return "the standalone eikonal solve takes one mesh, not a batch";
@@ -986,6 +1012,7 @@ std::string Solver::eikonal(const int* seeds, const float* values, int nseeds, f
   const int nv = m_.nv, n = nseeds;
   const float LN = sp_.largenum;
   if (h_ctl_[CTL_ITER] > kStampLimit) LS_TRY(restart_stamps(0), "stamps");
+  LS_TRY(end_chain(), "memset");
   LS_TRY(K_->begin(s_, 0, stream_), "begin");
   if (n > 0) {
     if (n > seed_cap_) {
@@ -1028,7 +1055,7 @@ std::string Solver::eikonal(const int* seeds, const float* values, int nseeds, f
   return "";
 }
 
-std::string Solver::set_phi(const float* phi_orig) {
+std::string Solver::load_phi(const float* phi_orig) {
   const float* src = phi_orig;
   if (!pageable_) {
     std::memcpy(h_stage_, phi_orig, sizeof(float) * m_.nv);
@@ -1042,7 +1069,7 @@ std::string Solver::set_phi(const float* phi_orig) {
   return "";
 }
 
-std::string Solver::get_phi(float* phi_orig, int first, int n) {
+std::string Solver::store_phi(float* phi_orig, int first, int n) {
   float* const dst = pageable_ ? phi_orig : d_tmp_;
   LS_TRY(K_->unpermute(m_, s_.phi, first, n, dst, nullptr, L_, stream_), "unpermute");
   if (!pageable_)

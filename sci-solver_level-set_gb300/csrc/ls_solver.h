@@ -115,15 +115,19 @@ class Solver {
   ~Solver();
   // Upload the layout and the per-copy data; phi0 / vel in the caller's order.
   std::string init(const Layout& L, const SolverConfig& cfg, const float* vel);
-  std::string set_phi(const float* phi_orig);          // host, caller order
-  std::string get_phi(float* phi_orig) { return get_phi(phi_orig, 0, m_.nv); }  // host, caller order
-  std::string get_phi(float* phi_orig, int first, int n);  // n vertices from `first` on
+  std::string set_phi(const float* phi_orig) { return settled(load_phi(phi_orig)); }  // host, caller order
+  std::string get_phi(float* phi_orig) { return get_phi(phi_orig, 0, m_.nv); }        // host, caller order
+  std::string get_phi(float* phi_orig, int first, int n) {  // n vertices from `first` on
+    return settled(store_phi(phi_orig, first, n));
+  }
   // Run nsteps; history (optional) gets phi after each step (host, caller order).
-  std::string run(int nsteps, float* history, int* steps_done);
-  std::string step_host(const float* phi_in, float* phi_out);
+  std::string run(int nsteps, float* history, int* steps_done) { return settled(run_steps(nsteps, history, steps_done)); }
+  std::string step_host(const float* phi_in, float* phi_out) { return settled(step_buffers(phi_in, phi_out)); }
   // Distance from arbitrary seed vertices (caller order), whole mesh, no
   // narrowband limit; out: nv floats in the caller's order.
-  std::string eikonal(const int* seeds, const float* values, int nseeds, float* out);
+  std::string eikonal(const int* seeds, const float* values, int nseeds, float* out) {
+    return settled(solve_eikonal(seeds, values, nseeds, out));
+  }
   std::string narrowband(unsigned char* flags);
   std::string active_patches(std::vector<int>& out);
   std::string dt_values(float* dt_new_order);
@@ -156,7 +160,17 @@ class Solver {
   int first_bodies() const { return m_.dim == 3 ? 3 : 2; }  // loop bodies' worth of iterations before the loop
   bool build_persistent_graph(std::string* err);
   std::string emit_phi(float* row);
+  // the calls above, with work on the caller's arrays still in flight on an error
+  std::string settled(std::string r);
+  std::string run_steps(int nsteps, float* history, int* steps_done);
+  std::string step_buffers(const float* phi_in, float* phi_out);
+  std::string solve_eikonal(const int* seeds, const float* values, int nseeds, float* out);
+  std::string load_phi(const float* phi_orig);
+  std::string store_phi(float* phi_orig, int first, int n);
   std::string run_chained(int nsteps, float* history, int* done);
+  std::string enqueue_chain(int nsteps, float* history, int* done);
+  cudaError_t end_chain();
+  bool chained_ = false;  // CTL_CHAIN is set on the device
   std::string step_done(bool* empty_nb);
   cudaError_t step_head();
   cudaError_t step_tail();

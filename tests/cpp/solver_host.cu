@@ -1,0 +1,185 @@
+// solver_host.cu -- the orchestration of ls_solver.cu on the CPU, over the
+// runtime of fake_cuda.h and a set of kernels that only keep the step control
+// words as the real ones do.  Each argument names a check; the program prints
+// what does not hold and returns the number of failures.
+#include <cstdio>
+#include <memory>
+#include <sstream>
+
+#include "fake_cuda.h"
+
+#define private public
+#include "ls_solver.h"
+#undef private
+
+namespace lsgb {
+namespace {
+int failures = 0;
+#define CHECK(cond, ...)            \
+  do {                              \
+    if (!(cond)) {                  \
+      ++failures;                   \
+      std::printf("FAILED: ");      \
+      std::printf(__VA_ARGS__);     \
+      std::printf(" [%s]\n", #cond); \
+    }                               \
+  } while (0)
+
+// Steps with a narrowband that the fake kernels still have to give.
+int nb_steps = 1 << 30;
+int fim_captured = 0;  // FIM launches captured or enqueued since it was cleared
+
+void begin_words(int* c) {
+  c[CTL_STOP] = c[CTL_CHAIN] && (c[CTL_NB] == 0 || c[CTL_CAP] || c[CTL_ERR]) ? 1 : 0;
+  if (c[CTL_STOP]) return;
+  c[CTL_NB] = c[CTL_BODIES] = c[CTL_CAP] = c[CTL_ERR] = 0;
+  c[CTL_BASE] = c[CTL_ITER];
+  c[CTL_ITER] += 2;
+}
+void step_words(const DevState& s, int nv) {
+  int* c = s.ctl;
+  begin_words(c);
+  if (c[CTL_STOP]) return;
+  c[CTL_ITER] += 12;
+  c[CTL_BODIES] = 1;
+  c[CTL_NB] = nb_steps-- > 0 ? 1 : 0;
+  if (c[CTL_NB])
+    for (int v = 0; v < nv; ++v) s.phi[v] += 1.f;
+}
+
+cudaError_t put(cudaStream_t st, fake::Work w) {
+  FAKE_CALL("kernel");
+  fake::enqueue(fake::of(st), std::move(w));
+  return cudaSuccess;
+}
+
+KernelSet make_kernels() {
+  KernelSet k{};
+  k.configure = [](const DevMesh&, const StepParams&, Launch& L) {
+    L = Launch{};
+    L.sms = 152;
+    L.warp_grid = L.flat_grid = 1;
+    return cudaSuccess;
+  };
+  k.begin = [](const DevState& s, int, cudaStream_t st) { return put(st, [=] { begin_words(s.ctl); }); };
+  k.seed = [](const DevMesh&, const DevState&, const StepParams&, const Launch&, cudaStream_t st) { return put(st, [] {}); };
+  k.fim = [](const DevMesh&, const DevState& s, const StepParams&, int off, const Launch&, cudaStream_t st) {
+    ++fim_captured;
+    return put(st, [=] { if (off == 0 && !s.ctl[CTL_STOP]) s.ctl[CTL_ITER] += 4; });
+  };
+  k.narrowband = [](const DevMesh& m, const DevState& s, const StepParams&, const Launch&, cudaStream_t st) {
+    return put(st, [=] {
+      s.ctl[CTL_NB] = nb_steps-- > 0 ? 1 : 0;
+      if (s.ctl[CTL_NB]) for (int v = 0; v < m.nv; ++v) s.phi[v] += 1.f;
+    });
+  };
+  k.update = [](const DevMesh&, const DevState&, const StepParams&, int, const Launch&, cudaStream_t st) { return put(st, [] {}); };
+  k.unpermute = [](const DevMesh& m, const float* phi, int first, int n, float* out, const int* ctl, const Launch&, cudaStream_t st) {
+    return put(st, [=] {
+      if (ctl && (ctl[CTL_STOP] || ctl[CTL_NB] == 0)) return;
+      for (int o = 0; o < n; ++o) out[o] = phi[m.ipermute[first + o]];
+    });
+  };
+  k.permute = [](const DevMesh& m, const float* in, float* out, const Launch&, cudaStream_t st) {
+    return put(st, [=] { for (int o = 0; o < m.nv; ++o) out[m.ipermute[o]] = in[o]; });
+  };
+  k.geometry = [](const DevMesh&, float4*, float4*, const Launch&, cudaStream_t st) { return put(st, [] {}); };
+  return k;
+}
+
+// A strip of two triangles (dim 2) or one tetrahedron in one patch.
+Layout make_layout(int dim) {
+  Layout L;
+  const float xyz[12] = {0, 0, 0, 1, 0, 0, 0, 1, 0, dim == 2 ? 1.f : 0.f, dim == 2 ? 1.f : 0.f, dim == 2 ? 0.f : 1.f};
+  const int tri[6] = {0, 1, 2, 1, 3, 2}, tet[4] = {0, 1, 2, 3}, npart[4] = {0, 0, 0, 0};
+  const std::string r = build_layout(dim, 4, xyz, dim == 2 ? 2 : 1, dim == 2 ? tri : tet, npart, 1, L);
+  CHECK(r.empty(), "layout: %s", r.c_str());
+  return L;
+}
+
+struct Rig {
+  Layout L;
+  std::unique_ptr<Solver> s{new Solver()};
+  std::vector<float> phi{1.f, 2.f, 3.f, 4.f};
+  explicit Rig(const SolverConfig& cfg, int dim = 3) : L(make_layout(dim)) {
+    fake::st.fail_at = -1;
+    const std::string r = s->init(L, cfg, nullptr);
+    CHECK(r.empty(), "init: %s", r.c_str());
+    Solver* p = s.get();
+    fake::st.step = [p] { step_words(p->s_, p->m_.nv); };
+    CHECK(s->set_phi(phi.data()).empty(), "set_phi");
+  }
+};
+
+// Whichever runtime call of an entry point fails: nothing that it enqueued is
+// left in flight when it returns, and the handle's next step is a step.
+void errors() {
+  struct Entry { const char* name; int graph, pageable; std::function<std::string(Solver&, float*)> f; };
+  const int n = 4;
+  const int seed[1] = {1};
+  const float value[1] = {0.f};
+  std::vector<Entry> entries;
+  for (int graph : {1, 0})
+    for (int pageable : {1, 0}) {
+      entries.push_back({"run with history", graph, pageable, [=](Solver& s, float* b) { int d; return s.run(5, b, &d); }});
+      entries.push_back({"run", graph, pageable, [=](Solver& s, float*) { int d; return s.run(5, nullptr, &d); }});
+      entries.push_back({"step_host", graph, pageable, [=](Solver& s, float* b) { return s.step_host(b, b + n); }});
+      entries.push_back({"set_phi", graph, pageable, [=](Solver& s, float* b) { return s.set_phi(b); }});
+      entries.push_back({"get_phi", graph, pageable, [=](Solver& s, float* b) { return s.get_phi(b); }});
+      entries.push_back({"eikonal", graph, pageable, [=](Solver& s, float* b) { return s.eikonal(seed, value, 1, b); }});
+    }
+  for (const Entry& e : entries) {
+    int failed = 0;
+    for (int k = 0;; ++k) {
+      SolverConfig cfg;
+      cfg.use_graph = e.graph;
+      fake::st.pageable = e.pageable;
+      nb_steps = 1 << 30;
+      Rig rig(cfg);
+      std::vector<float> buf(64, 0.f);
+      nb_steps = 3;  // a run of five steps ends after three
+      fake::st.calls = 0;
+      fake::st.fail_at = k;
+      fake::st.failed.clear();
+      const std::string r = e.f(*rig.s, buf.data());
+      fake::st.fail_at = -1;
+      if (fake::st.failed.empty()) break;  // every call of it has failed once
+      ++failed;
+      // a failed wait leaves what it waited for; elapsed times are not results
+      if (fake::st.failed != "cudaStreamSynchronize" && !r.empty())
+        CHECK(fake::st.stream->queue.empty(), "%s (graph %d, pageable %d): work in flight after %s failed at call %d", e.name,
+              e.graph, e.pageable, fake::st.failed.c_str(), k);
+      fake::drain(fake::st.stream);
+      // the narrowband was empty at the end: a step that still takes itself
+      // for a part of the run would do nothing
+      nb_steps = 1 << 30;
+      rig.s->s_.ctl[CTL_NB] = 0;
+      bool empty = true;
+      const std::string q = rig.s->one_step(&empty);
+      CHECK(q.empty() && !empty, "%s (graph %d, pageable %d): next step after %s failed at call %d: %s", e.name, e.graph,
+            e.pageable, fake::st.failed.c_str(), k, q.c_str());
+    }
+    CHECK(failed > 1, "%s: only %d calls", e.name, failed);
+  }
+}
+}  // namespace
+
+const KernelSet& kernels_fast() { static const KernelSet k = make_kernels(); return k; }
+const KernelSet& kernels_exact() { return kernels_fast(); }
+namespace mlp {
+__global__ void k_features(int, const int*, const int*, const int*, const int*, const float*, int, const float*, float, const float*,
+                           __nv_bfloat16*) {}
+std::string Net::forward_dev(const __nv_bfloat16*, int, const int*, int, float*, cudaStream_t) { return ""; }
+std::string Net::append_pairs(const __nv_bfloat16*, const float*, const int*, int, cudaStream_t, long long*) { return ""; }
+}  // namespace mlp
+}  // namespace lsgb
+
+int main(int argc, char** argv) {
+  for (int i = 1; i < argc; ++i) {
+    const std::string a = argv[i];
+    if (a == "errors") lsgb::errors();
+    else { std::printf("unknown check %s\n", a.c_str()); return 99; }
+  }
+  std::printf("%d failures\n", lsgb::failures);
+  return lsgb::failures ? 1 : 0;
+}

@@ -1,0 +1,35 @@
+"""The solver's host side on the CPU: ls_solver.cu over a runtime of host
+memory and queued work (tests/cpp/fake_cuda.h), with failures made by an error
+code from the faked call."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "sci-solver_level-set_gb300", "csrc")
+
+
+@pytest.fixture(scope="module")
+def program(tmp_path_factory):
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("no nvcc")
+    d = str(tmp_path_factory.mktemp("solver_host"))
+    exe = os.path.join(d, "solver_host")
+    cmd = [nvcc, "-std=c++17", "-O1", "-cudart", "none", "-gencode", "arch=compute_103a,code=sm_103a", "-I", CSRC,
+           os.path.join(ROOT, "tests", "cpp", "solver_host.cu"), os.path.join(ROOT, "tests", "cpp", "fake_cuda.cpp"), os.path.join(CSRC, "ls_solver.cu"),
+           os.path.join(CSRC, "ls_layout.cpp"), "-o", exe]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-4000:]
+    return exe
+
+
+def _check(program, name):
+    r = subprocess.run([program, name], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout[-4000:]
+
+
+def test_nothing_in_flight_after_an_error(program):
+    _check(program, "errors")
