@@ -2314,6 +2314,21 @@ cudaError_t launch_fim_persistent(const DevMesh& m, const DevState& s, const Ste
   return cudaLaunchKernelEx(&cfg, k_fim_persist<3, 384, false, 2, false>, m, s, sp);
 }
 
+// Lets fn's launches have `smem` bytes of dynamic shared memory.  The limit
+// belongs to the function, for every handle of the process: it is set to all
+// that the device has, so that no mesh's setup lowers it under another's
+// launches (cudaErrorInvalidValue, as ever, where `smem` is more).
+inline cudaError_t allow_smem(const void* fn, int smem) {
+  cudaFuncAttributes a;
+  int dev = 0, optin = 0;
+  cudaError_t e = cudaFuncGetAttributes(&a, fn);
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              std::max(smem, optin - (int)a.sharedSizeBytes));
+}
+
 // Resident CTAs of the persistent kernel launch_fim_persistent picks (0
 // where there is no persistent form).
 cudaError_t configure_persistent(const DevMesh& m, const StepParams& sp, Launch& L) {
@@ -2324,7 +2339,7 @@ cudaError_t configure_persistent(const DevMesh& m, const StepParams& sp, Launch&
   int occ = 0;
   cudaError_t e = cudaSuccess;
   auto query = [&](const void* fn, int block, int smem) {
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    e = allow_smem(fn, smem);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, block, smem);
   };
   if (use_pair(m, sp, L)) {
@@ -2409,33 +2424,33 @@ cudaError_t configure_launch(const DevMesh& m, const StepParams& sp, Launch& L) 
       // 7: one copy per thread, lep threads)
       L.pair_block = sp.ctas == 7 ? L.fim_block : ((sp.lep + 1) / 2 + 31) / 32 * 32;
       const int ps = pair_smem(sp, sp.lep);
-      e = cudaFuncSetAttribute(LS_PAIR_KERNEL(sp), cudaFuncAttributeMaxDynamicSharedMemorySize, ps);
+      e = allow_smem(LS_PAIR_KERNEL(sp), ps);
       if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, LS_PAIR_KERNEL(sp), L.pair_block, ps);
     } else if (L.fim_block <= 384 && sp.ctas == 2) {
-      e = cudaFuncSetAttribute(k_fim_compact<384, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs);
+      e = allow_smem((const void*)k_fim_compact<384, 2, false>, cs);
       if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fim_compact<384, 2, false>, L.fim_block, cs);
     } else if (L.fim_block <= 384 && sp.ctas == 4) {
-      e = cudaFuncSetAttribute(k_fim_compact<384, 4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs);
+      e = allow_smem((const void*)k_fim_compact<384, 4, false>, cs);
       if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fim_compact<384, 4, false>, L.fim_block, cs);
     } else if (L.fim_block <= 384) {
-      e = cudaFuncSetAttribute(k_fim_compact<384, 3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs);
+      e = allow_smem((const void*)k_fim_compact<384, 3, false>, cs);
       if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fim_compact<384, 3, false>, L.fim_block, cs);
     } else if (L.fim_block <= 512) {
-      e = cudaFuncSetAttribute(k_fim_compact<512, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs);
+      e = allow_smem((const void*)k_fim_compact<512, 1, false>, cs);
       if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fim_compact<512, 1, false>, L.fim_block, cs);
     } else {
-      e = cudaFuncSetAttribute(k_fim_compact<1024, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs);
+      e = allow_smem((const void*)k_fim_compact<1024, 1, false>, cs);
       if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fim_compact<1024, 1, false>, L.fim_block, cs);
     }
     // precision-form variants (selected at launch when tau > 0)
     if (e == cudaSuccess) {
       if (L.fim_block <= 384)
-        e = cudaFuncSetAttribute(k_fim_compact<384, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs);
+        e = allow_smem((const void*)k_fim_compact<384, 2, true>, cs);
       else if (L.fim_block <= 512)
-        e = cudaFuncSetAttribute(k_fim_compact<512, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs);
+        e = allow_smem((const void*)k_fim_compact<512, 1, true>, cs);
       else
-        e = cudaFuncSetAttribute(k_fim_compact<1024, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs);
+        e = allow_smem((const void*)k_fim_compact<1024, 1, true>, cs);
     }
   } else if (m.dim == 3) {
     if (!m.capped && L.fim_block <= 384 && sp.ctas >= 5 && sp.ctas <= 7) {
@@ -2443,7 +2458,7 @@ cudaError_t configure_launch(const DevMesh& m, const StepParams& sp, Launch& L) 
       // (the precision form keeps the one-copy kernel)
       L.pair_block = sp.ctas == 7 ? L.fim_block : ((sp.lep + 1) / 2 + 31) / 32 * 32;
       const int ps = pair_smem(sp, sp.lep);
-      e = cudaFuncSetAttribute(LS_PAIR_KERNEL(sp), cudaFuncAttributeMaxDynamicSharedMemorySize, ps);
+      e = allow_smem(LS_PAIR_KERNEL(sp), ps);
       if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, LS_PAIR_KERNEL(sp), L.pair_block, ps);
     } else if (L.fim_block <= 384 && sp.ctas == 2)
@@ -2471,8 +2486,7 @@ cudaError_t configure_launch(const DevMesh& m, const StepParams& sp, Launch& L) 
   L.seed_grid = std::min(L.sms * 16, m.nparts);
   L.seed_smem = (int)sizeof(float) * (sp.lvp + sp.lgp);
   if (L.seed_smem > 48 * 1024) {
-    e = cudaFuncSetAttribute(m.dim == 3 ? (const void*)k_seed<4> : (const void*)k_seed<3>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, L.seed_smem);
+    e = allow_smem(m.dim == 3 ? (const void*)k_seed<4> : (const void*)k_seed<3>, L.seed_smem);
     if (e != cudaSuccess) return e;
   }
   L.upd_block = kUpdBlock;
@@ -2481,7 +2495,7 @@ cudaError_t configure_launch(const DevMesh& m, const StepParams& sp, Launch& L) 
   {
     const void* fn = update_kernel(m, sp);
     if (L.upd_smem > 48 * 1024) {
-      e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, L.upd_smem);
+      e = allow_smem(fn, L.upd_smem);
       if (e != cudaSuccess) return e;
     }
     occ = 0;
