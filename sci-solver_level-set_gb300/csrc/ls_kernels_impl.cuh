@@ -91,7 +91,8 @@ __device__ __forceinline__ FimIter fim_iter(const DevMesh& m, const DevState& s,
   const int cur = f.t % 3, nxt = cur == 2 ? 0 : cur + 1;
   f.base = s_ctl[CTL_BASE];
   f.nvis = s_ctl[CTL_VISITS + cur];
-  f.count = s_ctl[CTL_STOP] ? 0 : f.nvis + s_ctl[CTL_CANDS + cur];
+  // (nor does an iteration behind one that was abandoned run on what it left)
+  f.count = s_ctl[CTL_STOP] || s_ctl[CTL_ERR] ? 0 : f.nvis + s_ctl[CTL_CANDS + cur];
   f.list = s.lists + (size_t)cur * m.nparts;
   f.next = s.lists + (size_t)nxt * m.nparts;
   f.next_n = s.ctl + CTL_VISITS + nxt;
@@ -1541,9 +1542,11 @@ __global__ void __launch_bounds__(MAXT, MINB) k_fim_persist(DevMesh m, DevState 
 // count: one warp per patch over every patch.  The redistanced phi goes to
 // phi_rd; outside the narrowband (or with no update, last != 0) it is the
 // step's result and goes to phi too.  The update then reads phi_rd and
-// writes phi, so that no copy pass follows it.
+// writes phi, so that no copy pass follows it.  Behind an abandoned FIM loop
+// nothing is written (and the narrowband is empty for the update): phi stays
+// what it was before the step.
 __global__ void k_narrowband(DevMesh m, DevState s, StepParams sp, int last) {
-  if (s.ctl[CTL_STOP]) return;
+  if (s.ctl[CTL_STOP] || s.ctl[CTL_ERR]) return;
   __shared__ unsigned long long s_cnt, s_pv, s_np;
   if (threadIdx.x == 0) { s_cnt = 0; s_pv = 0; s_np = 0; }
   __syncthreads();
