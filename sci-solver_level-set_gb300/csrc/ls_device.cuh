@@ -98,12 +98,12 @@ enum {
   CTL_ITER = 12,    // stamp of the first iteration of the next loop body
   CTL_BASE = 13,    // base stamp of the step
   CTL_ITERS = 14,   // iterations of this step that visited a patch
-  CTL_LAST = 15,    // stamp of the last iteration that visited a patch
   // a run enqueues a step before it knows how the previous one ended (host-set
   // CTL_CHAIN, 0 outside a run's later steps): if that one ran out of
   // narrowband or failed, the step finds CTL_STOP set and does nothing
-  CTL_CHAIN = 16,
-  CTL_STOP = 17,
+  CTL_CHAIN = 15,
+  CTL_STOP = 16,
+  CTL_VISITED = 17,  // [3] iteration t visited a patch (word t % 3)
   CTL_WORDS = 32
 };
 // Stamps restart (every stamped array cleared) between steps once they pass
@@ -131,12 +131,20 @@ struct DevState {
 };
 constexpr int kGridBarrierWords = 2 + 1024;
 
-// Counts iteration t of this step if it visited a patch (one thread, once for
-// each iteration: when the next one starts, or at the end of a loop body).
-__device__ __forceinline__ void count_iteration(int* ctl, unsigned long long* stats, int t) {
-  if (*reinterpret_cast<volatile int*>(ctl + CTL_LAST) != t) return;
+// An iteration counts if it visited a patch: its CTAs mark the iteration's own
+// word, which one thread takes when the next iteration starts or at the end of
+// a loop body.  The next iteration's CTAs, some done before that thread has
+// looked, mark another word.
+__host__ __device__ __forceinline__ void mark_iteration(int* ctl, int t) { ctl[CTL_VISITED + t % 3] = 1; }
+__host__ __device__ __forceinline__ bool take_iteration(int* ctl, int t) {
+  volatile int* w = ctl + CTL_VISITED + t % 3;
+  if (!*w) return false;
+  *w = 0;
   ctl[CTL_ITERS] += 1;
-  atomicAdd(&stats[5], 1ull);
+  return true;
+}
+__device__ __forceinline__ void count_iteration(int* ctl, unsigned long long* stats, int t) {
+  if (take_iteration(ctl, t)) atomicAdd(&stats[5], 1ull);
 }
 
 // Learned warm start / training-pair collection buffers (null when off).

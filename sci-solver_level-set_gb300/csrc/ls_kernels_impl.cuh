@@ -52,7 +52,7 @@ __global__ void k_begin(DevState s, int restart) {
   if (threadIdx.x == 0) {
     c[CTL_STOP] = c[CTL_CHAIN] && (c[CTL_NB] == 0 || c[CTL_CAP] || c[CTL_ERR]) ? 1 : 0;
     if (c[CTL_STOP]) return;
-    for (int i = 0; i < 3; ++i) c[CTL_VISITS + i] = c[CTL_CANDS + i] = 0;
+    for (int i = 0; i < 3; ++i) c[CTL_VISITS + i] = c[CTL_CANDS + i] = c[CTL_VISITED + i] = 0;
     if (!restart) {
       c[CTL_NB_PREV] = c[CTL_NB_VALID] ? c[CTL_NB] : 0;
       c[CTL_NB_VALID] = 1;
@@ -60,7 +60,7 @@ __global__ void k_begin(DevState s, int restart) {
     c[CTL_NB] = 0;
     c[CTL_BODIES] = c[CTL_CAP] = c[CTL_ERR] = c[CTL_ITERS] = 0;
     const int u = c[CTL_ITER];
-    c[CTL_BASE] = c[CTL_LAST] = u;  // u: seeds, u + 1: warm-start values
+    c[CTL_BASE] = u;  // u: seeds, u + 1: warm-start values
     c[CTL_ITER] = u + 2;
     s.sched[0] = 0;
   }
@@ -178,7 +178,7 @@ struct FimCount {
 __device__ __forceinline__ void fim_count_flush(const DevState& s, const FimIter& f, const FimCount& n) {
   if (n.visits) {
     atomicAdd(&s.stats[0], (unsigned long long)n.visits);
-    s.ctl[CTL_LAST] = f.t;  // counted as an iteration by count_iteration
+    mark_iteration(s.ctl, f.t);
   }
   if (n.checks) atomicAdd(&s.stats[1], (unsigned long long)n.checks);
   if (n.early) atomicAdd(&s.stats[8], (unsigned long long)n.early);

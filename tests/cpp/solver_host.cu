@@ -162,6 +162,30 @@ void errors() {
     CHECK(failed > 1, "%s: only %d calls", e.name, failed);
   }
 }
+// Counted iterations, whatever the order of CTA 0 (which counts the previous
+// iteration when it starts) and of the other CTAs' ends in a launch: every
+// pattern of eight iterations that visit a patch or not, with CTA 0 first or
+// last in each launch, and the count at body ends of four.
+void iterations() {
+  for (int visits = 0; visits < 256; ++visits)
+    for (int late = 0; late < 256; ++late)
+      for (int persistent = 0; persistent < 2; ++persistent) {
+        int ctl[CTL_WORDS] = {}, want = 0;
+        const int t0 = 2;
+        for (int i = 0; i < 8; ++i) {
+          const int t = t0 + i;
+          const bool v = (visits >> i) & 1, last = (late >> i) & 1, first = !persistent && i % 4 == 0;
+          want += v;
+          if (last && v) mark_iteration(ctl, t);
+          if (!first) take_iteration(ctl, t - 1);
+          if (!last && v) mark_iteration(ctl, t);
+          if (persistent ? i == 7 : i % 4 == 3) take_iteration(ctl, t);
+        }
+        CHECK(ctl[CTL_ITERS] == want, "visits %02x, late %02x, persistent %d: %d iterations instead of %d", visits, late,
+              persistent, ctl[CTL_ITERS], want);
+        if (failures > 5) return;
+      }
+}
 }  // namespace
 
 const KernelSet& kernels_fast() { static const KernelSet k = make_kernels(); return k; }
@@ -178,6 +202,7 @@ int main(int argc, char** argv) {
   for (int i = 1; i < argc; ++i) {
     const std::string a = argv[i];
     if (a == "errors") lsgb::errors();
+    else if (a == "iterations") lsgb::iterations();
     else { std::printf("unknown check %s\n", a.c_str()); return 99; }
   }
   std::printf("%d failures\n", lsgb::failures);

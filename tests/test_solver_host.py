@@ -33,3 +33,7 @@ def _check(program, name):
 
 def test_nothing_in_flight_after_an_error(program):
     _check(program, "errors")
+
+
+def test_iterations_counted_in_any_order(program):
+    _check(program, "iterations")
