@@ -879,8 +879,16 @@ std::string Solver::enqueue_chain(int nsteps, float* history, int* done) {
     return e;
   };
   int s = 0;
+  bool pending = false;  // step s - 1 has not been settled
   for (; s < nsteps && r.empty() && !empty; ++s) {
-    if (h_ctl_[CTL_ITER] > kStampLimit) LS_TRY(restart_stamps(0), "stamps");
+    if (h_ctl_[CTL_ITER] > kStampLimit) {
+      // behind a step whose end is known: the distances of a run's last step
+      // stay readable
+      if (pending) r = settle(s - 1);
+      pending = false;
+      if (!r.empty() || empty) break;
+      LS_TRY(restart_stamps(0), "stamps");
+    }
     LS_TRY(cudaGraphLaunch(graph_exec_, stream_), "graph launch");
     if (history)
       LS_TRY(K_->unpermute(m_, s_.phi, 0, m_.nv, history + (size_t)(s + 1) * m_.nv, s_.ctl, L_, stream_), "unpermute");
@@ -891,10 +899,11 @@ std::string Solver::enqueue_chain(int nsteps, float* history, int* done) {
       chained_ = true;
       LS_TRY(cudaMemsetAsync(s_.ctl + CTL_CHAIN, 1, sizeof(int), stream_), "memset");
     }
-    if (s > 0) r = settle(s - 1);
+    if (pending) r = settle(s - 1);
+    pending = true;
   }
   // the last enqueued step, unless the one before it ended the run
-  if (r.empty() && !empty && s > 0) r = settle(s - 1);
+  if (r.empty() && !empty && pending) r = settle(s - 1);
   return r;
 }
 

@@ -82,21 +82,13 @@ cudaError_t CUDARTAPI cudaEventDestroy(cudaEvent_t e) { delete reinterpret_cast<
 cudaError_t CUDARTAPI cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
   FAKE_CALL("cudaEventRecord");
   *reinterpret_cast<fake::Stream**>(e) = fake::of(s);
-  // what is recorded behind the event stays in flight
-  fake::enqueue(fake::of(s), nullptr);
+  fake::enqueue(fake::of(s), [] {}, e);
   return cudaSuccess;
 }
 cudaError_t CUDARTAPI cudaEventSynchronize(cudaEvent_t e) {
   FAKE_CALL("cudaEventSynchronize");
   fake::Stream* s = *reinterpret_cast<fake::Stream**>(e);
-  // up to the last event mark but none behind it (each mark is waited for in turn)
-  if (!s) return cudaSuccess;
-  size_t n = 0;
-  for (size_t i = 0; i < s->queue.size(); ++i)
-    if (!s->queue[i]) { n = i + 1; break; }
-  for (size_t i = 0; i < n; ++i)
-    if (s->queue[i]) s->queue[i]();
-  s->queue.erase(s->queue.begin(), s->queue.begin() + n);
+  if (s) fake::drain(s, e);
   return cudaSuccess;
 }
 cudaError_t CUDARTAPI cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 1.f; return fake::call("cudaEventElapsedTime"); }

@@ -14,8 +14,12 @@
 
 namespace fake {
 using Work = std::function<void()>;
+struct Item {
+  Work work;
+  void* event;  // recorded here
+};
 struct Stream {
-  std::vector<Work> queue;
+  std::vector<Item> queue;
 };
 struct Graph {
   std::vector<Work> work;  // what was captured into it, in order
@@ -38,14 +42,16 @@ inline cudaError_t call(const char* name) {
   }
   return cudaSuccess;
 }
-inline void enqueue(Stream* s, Work w) {
+inline void enqueue(Stream* s, Work w, void* event = nullptr) {
   if (st.capture) st.capture->push_back(std::move(w));
-  else s->queue.push_back(std::move(w));
+  else s->queue.push_back({std::move(w), event});
 }
-inline void drain(Stream* s) {
-  for (size_t i = 0; i < s->queue.size(); ++i)
-    if (s->queue[i]) s->queue[i]();
-  s->queue.clear();
+// runs a stream's work, up to the last place where `event` was recorded when given
+inline void drain(Stream* s, void* event = nullptr) {
+  size_t n = s->queue.size();
+  while (event && n > 0 && s->queue[n - 1].event != event) --n;
+  for (size_t i = 0; i < n; ++i) s->queue[i].work();
+  s->queue.erase(s->queue.begin(), s->queue.begin() + n);
 }
 inline Stream* of(cudaStream_t s) { return reinterpret_cast<Stream*>(s); }
 }  // namespace fake

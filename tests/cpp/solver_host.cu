@@ -42,6 +42,7 @@ void step_words(const DevState& s, int nv) {
   if (c[CTL_STOP]) return;
   c[CTL_ITER] += 12;
   c[CTL_BODIES] = 1;
+  s.cell[0] = make_int4(0, c[CTL_BASE], 0, -1);
   c[CTL_NB] = nb_steps-- > 0 ? 1 : 0;
   if (c[CTL_NB])
     for (int v = 0; v < nv; ++v) s.phi[v] += 1.f;
@@ -186,6 +187,22 @@ void iterations() {
         if (failures > 5) return;
       }
 }
+// The distances of a run's last step stay readable, wherever the stamps
+// restart within the run (a new handle's do after a few steps).
+void restarts() {
+  for (int n = 1; n < 9; ++n)
+    for (int extra = 0; extra < 4; ++extra) {
+      fake::st.pageable = 1;
+      nb_steps = 1 << 30;
+      Rig rig(SolverConfig{});
+      nb_steps = n;
+      int done = -1;
+      const std::string r = rig.s->run(n + extra, nullptr, &done);
+      CHECK(r.empty() && done == n, "run of %d of %d steps: %d done, %s", n, n + extra, done, r.c_str());
+      const DevState& d = rig.s->s_;
+      CHECK(d.cell[0].y == d.ctl[CTL_BASE], "run of %d of %d steps: distances cleared", n, n + extra);
+    }
+}
 }  // namespace
 
 const KernelSet& kernels_fast() { static const KernelSet k = make_kernels(); return k; }
@@ -203,6 +220,7 @@ int main(int argc, char** argv) {
     const std::string a = argv[i];
     if (a == "errors") lsgb::errors();
     else if (a == "iterations") lsgb::iterations();
+    else if (a == "restarts") lsgb::restarts();
     else { std::printf("unknown check %s\n", a.c_str()); return 99; }
   }
   std::printf("%d failures\n", lsgb::failures);

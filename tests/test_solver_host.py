@@ -37,3 +37,7 @@ def test_nothing_in_flight_after_an_error(program):
 
 def test_iterations_counted_in_any_order(program):
     _check(program, "iterations")
+
+
+def test_distances_stay_where_a_run_ends(program):
+    _check(program, "restarts")
