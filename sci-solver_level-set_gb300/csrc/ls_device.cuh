@@ -103,7 +103,7 @@ enum {
   // narrowband or failed, the step finds CTL_STOP set and does nothing
   CTL_CHAIN = 15,
   CTL_STOP = 16,
-  CTL_VISITED = 17,  // [3] iteration t visited a patch (word t % 3)
+  CTL_VISITED = 17,  // [3] an iteration visited a patch (visited_word)
   CTL_WORDS = 32
 };
 // Stamps restart (every stamped array cleared) between steps once they pass
@@ -134,10 +134,12 @@ constexpr int kGridBarrierWords = 2 + 1024;
 // An iteration counts if it visited a patch: its CTAs mark the iteration's own
 // word, which one thread takes when the next iteration starts or at the end of
 // a loop body.  The next iteration's CTAs, some done before that thread has
-// looked, mark another word.
-__host__ __device__ __forceinline__ void mark_iteration(int* ctl, int t) { ctl[CTL_VISITED + t % 3] = 1; }
+// looked, mark another word.  (The word goes with the list that the iteration
+// makes, whose counters the sweep kernels have at hand: kept for t % 3, the
+// stamp cost the 56-register kernels two spills.)
+__host__ __device__ __forceinline__ int* visited_word(int* ctl, int t) { return ctl + CTL_VISITED + (t + 1) % 3; }
 __host__ __device__ __forceinline__ bool take_iteration(int* ctl, int t) {
-  volatile int* w = ctl + CTL_VISITED + t % 3;
+  volatile int* w = visited_word(ctl, t);
   if (!*w) return false;
   *w = 0;
   ctl[CTL_ITERS] += 1;

@@ -178,7 +178,7 @@ struct FimCount {
 __device__ __forceinline__ void fim_count_flush(const DevState& s, const FimIter& f, const FimCount& n) {
   if (n.visits) {
     atomicAdd(&s.stats[0], (unsigned long long)n.visits);
-    mark_iteration(s.ctl, f.t);
+    f.next_n[CTL_VISITED - CTL_VISITS] = 1;  // visited_word
   }
   if (n.checks) atomicAdd(&s.stats[1], (unsigned long long)n.checks);
   if (n.early) atomicAdd(&s.stats[8], (unsigned long long)n.early);

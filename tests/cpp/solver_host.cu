@@ -177,9 +177,9 @@ void iterations() {
           const int t = t0 + i;
           const bool v = (visits >> i) & 1, last = (late >> i) & 1, first = !persistent && i % 4 == 0;
           want += v;
-          if (last && v) mark_iteration(ctl, t);
+          if (last && v) *visited_word(ctl, t) = 1;
           if (!first) take_iteration(ctl, t - 1);
-          if (!last && v) mark_iteration(ctl, t);
+          if (!last && v) *visited_word(ctl, t) = 1;
           if (persistent ? i == 7 : i % 4 == 3) take_iteration(ctl, t);
         }
         CHECK(ctl[CTL_ITERS] == want, "visits %02x, late %02x, persistent %d: %d iterations instead of %d", visits, late,
