@@ -614,9 +614,9 @@ def main():
     step_ms_prof = (ps["ms_sweep"] + ps["ms_check"] + ps["ms_schedule"] + ps["ms_seed"] + ps["ms_narrowband"]
                     + ps["ms_update"])
     kernel_ms = {k: ps["ms_" + k] / prof_steps for k in ("sweep", "check", "schedule", "seed", "narrowband", "update")}
-    # the FIM kernel the run used: k_fim_pair at the settings 5 to 7 (patches
+    # the FIM kernel the run used: k_fim_pair at the settings 0 and 5 to 7 (patches
     # of up to 384 copies), one copy per thread otherwise
-    sweep_kernel = "k_fim_pair" if ls.get_params().fim_ctas_per_sm in (5, 6, 7) else "k_fim_compact"
+    sweep_kernel = "k_fim_pair" if ls.get_params().fim_ctas_per_sm in (0, 5, 6, 7) else "k_fim_compact"
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": profile_traffic(bytes_per_launch),
                 "kernel": sweep_kernel + " (FIM iterations: checks, visits and the next list)",

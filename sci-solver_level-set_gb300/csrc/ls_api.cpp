@@ -142,7 +142,7 @@ lsgb::SolverConfig solver_config(const ls_params& p) {
   cfg.inside_niter = p.inside_iterations > 0 ? p.inside_iterations : 1;
   cfg.max_fim_iters = p.max_fim_iters > 0 ? p.max_fim_iters : 100000;
   cfg.graph_chunk = p.graph_chunk > 0 ? p.graph_chunk : 4;
-  cfg.fim_ctas = p.fim_ctas_per_sm > 0 ? p.fim_ctas_per_sm : 5;
+  cfg.fim_ctas = p.fim_ctas_per_sm > 0 ? p.fim_ctas_per_sm : 0;
   cfg.dt = p.time_step;
   cfg.bandwidth = p.bandwidth;
   cfg.curv_coeff = p.curv_coeff;
@@ -180,7 +180,7 @@ ls_status ls_default_params(ls_params* p) {
   p->length_scale = 0.0;
   p->fp64_threshold = 3.814697265625e-06;
   p->graph_chunk = 4;
-  p->fim_ctas_per_sm = 5;
+  p->fim_ctas_per_sm = 0;
   p->barrier_wait_limit = 0;
   return LS_OK;
 }

@@ -2484,6 +2484,7 @@ cudaError_t configure_launch(const DevMesh& m, const StepParams& sp, Launch& L) 
   }
   if (e != cudaSuccess) return e;
   if (occ < 1) occ = 1;
+  L.fim_ctas = occ;
   // no more CTAs than patches: a small mesh's launches are short
   L.fim_grid = std::min(L.sms * occ, m.nparts);
   L.seed_grid = std::min(L.sms * 16, m.nparts);

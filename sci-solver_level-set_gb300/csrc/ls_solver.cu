@@ -306,20 +306,6 @@ std::string Solver::init(const Layout& L, const SolverConfig& cfg, const float* 
   sp_.tau = (cfg.fp64_flagged && L.dim == 3) ? (float)cfg.fp64_tau : 0.f;
   sp_.xdiv = (cfg.bit_exact && ref) ? 1 : 0;
   sp_.ctas = (cfg.fim_ctas >= 2 && cfg.fim_ctas <= 7) ? cfg.fim_ctas : 5;
-  if (sp_.ctas == 5 && !cfg.bit_exact && L.dim == 3) {
-    // The default's tet sweep on large meshes: its six-CTA form (56 instead of
-    // 64 registers, a few spilled), where the lists are long enough for the
-    // sixth CTA to hide more than the spills cost.  Step times with 64 / 56
-    // registers: 32^3 (1,331 patches) 229 / 232 us, 48^3 (4,913) 323 / 319,
-    // 64^3 (10,648) 436 / 431, 80^3 (19,683) 605 / 590, 112^3 (54,872) 1009 /
-    // 958, 128^3 (79,507) 1108 / 1070; graph patches of 16 vertices, 64^3
-    // (17,165) 791 / 778, 80^3 (33,000) 966 / 987.  The bit-exact build's
-    // solver spills more: 48^3 726 / 783 us.  Same results.
-    int dev = 0, sms = 0;
-    LS_TRY(cudaGetDevice(&dev), "device");
-    LS_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "device");
-    if (np >= 100 * sms) sp_.ctas = 6;
-  }
   sp_.tol = (float)cfg.smallnum;
   sp_.eps_h64 = cfg.smallnum;
   sp_.eps_h = (float)sp_.eps_h64;
@@ -335,6 +321,28 @@ std::string Solver::init(const Layout& L, const SolverConfig& cfg, const float* 
   sp_.spin_limit = cfg.spin_limit != 0 ? cfg.spin_limit : (1 << 22);
   (void)d1;
   LS_TRY(K_->configure(m_, sp_, L_), "configure");
+  if (cfg.fim_ctas == 0 && !cfg.bit_exact && !cfg.persistent && !(sp_.tau > 0.f) && L_.pair_block > 0 &&
+      np >= 100 * L_.sms) {
+    // The default's tet sweep on large meshes: setting 6's registers (56
+    // instead of 64), where they let one more CTA reside -- blocks of 192
+    // threads whose shared memory fits six times, of 160 threads where it fits
+    // seven times -- and the lists are long.  Step times, 64 / 56 registers,
+    // with the further CTA: 27-vertex blocks (324 copies) 32^3 (9 patches per
+    // SM) 240 / 248 us, 40^3 (18) 280 / 283, 64^3 (70) 463 / 460, 80^3 (129)
+    // 613 / 607, 128^3 (523) 1248 / 1206; 16-vertex graph patches (271) 64^3
+    // (113) 794 / 779, 96^3 (375) 1494 / 1439; without it: the same at 80^3
+    // (284 copies, 118 ghosts, 219) 1126 / 1166, 12-vertex graph patches 64^3
+    // (151) 759 / 778, 8-vertex blocks 128^3 (1807) 1436 / 1471.  The bit-exact
+    // build's solver spills more: 48^3 726 / 783 us.  Same results.
+    StepParams six = sp_;
+    Launch l6{};
+    six.ctas = 6;
+    LS_TRY(K_->configure(m_, six, l6), "configure");
+    if (l6.fim_ctas > L_.fim_ctas) {
+      sp_ = six;
+      L_ = l6;
+    }
+  }
   if (L_.pair_block > 0) {
     // the two-copies-per-thread sweep stages precomputed per-copy geometry
     // (metric terms and heights, 64 bytes a copy) instead of the 24 bytes of

@@ -15,6 +15,7 @@ namespace lsgb {
 struct Launch {
   int sms;
   int fim_grid, fim_block, fim_smem;
+  int fim_ctas;    // resident CTAs of the sweep kernel per SM
   int pair_block;  // threads of the two-copies-per-thread sweep kernel (0: not used)
   int persist_grid;  // CTAs of the persistent FIM kernel (all resident; 0: no persistent form here)
   int upd_grid, upd_block, upd_smem;
@@ -69,7 +70,7 @@ struct SolverConfig {
   int inside_niter = 1;
   int max_fim_iters = 100000;
   int graph_chunk = 4;
-  int fim_ctas = 3;
+  int fim_ctas = 0;  // FIM setting (ls_params::fim_ctas_per_sm); 0: chosen by the mesh
   double dt = 1.0;
   double bandwidth = 16.0;
   double curv_coeff = 1.0;

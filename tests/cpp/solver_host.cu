@@ -27,7 +27,8 @@ int failures = 0;
 
 // Steps with a narrowband that the fake kernels still have to give.
 int nb_steps = 1 << 30;
-int fim_captured = 0;  // FIM launches captured or enqueued since it was cleared
+int sms = 152;
+int ctas[8] = {};  // resident CTAs of each FIM setting; 0: no two-copies kernel
 
 void begin_words(int* c) {
   c[CTL_STOP] = c[CTL_CHAIN] && (c[CTL_NB] == 0 || c[CTL_CAP] || c[CTL_ERR]) ? 1 : 0;
@@ -56,16 +57,17 @@ cudaError_t put(cudaStream_t st, fake::Work w) {
 
 KernelSet make_kernels() {
   KernelSet k{};
-  k.configure = [](const DevMesh&, const StepParams&, Launch& L) {
+  k.configure = [](const DevMesh&, const StepParams& sp, Launch& L) {
     L = Launch{};
-    L.sms = 152;
+    L.sms = sms;
+    L.fim_ctas = ctas[sp.ctas];
+    L.pair_block = L.fim_ctas ? 192 : 0;
     L.warp_grid = L.flat_grid = 1;
     return cudaSuccess;
   };
   k.begin = [](const DevState& s, int, cudaStream_t st) { return put(st, [=] { begin_words(s.ctl); }); };
   k.seed = [](const DevMesh&, const DevState&, const StepParams&, const Launch&, cudaStream_t st) { return put(st, [] {}); };
   k.fim = [](const DevMesh&, const DevState& s, const StepParams&, int off, const Launch&, cudaStream_t st) {
-    ++fim_captured;
     return put(st, [=] { if (off == 0 && !s.ctl[CTL_STOP]) s.ctl[CTL_ITER] += 4; });
   };
   k.narrowband = [](const DevMesh& m, const DevState& s, const StepParams&, const Launch&, cudaStream_t st) {
@@ -88,12 +90,19 @@ KernelSet make_kernels() {
   return k;
 }
 
-// A strip of two triangles (dim 2) or one tetrahedron in one patch.
-Layout make_layout(int dim) {
+// Pairs of triangles (dim 2) or tetrahedra, one patch each.
+Layout make_layout(int dim, int n) {
   Layout L;
-  const float xyz[12] = {0, 0, 0, 1, 0, 0, 0, 1, 0, dim == 2 ? 1.f : 0.f, dim == 2 ? 1.f : 0.f, dim == 2 ? 0.f : 1.f};
-  const int tri[6] = {0, 1, 2, 1, 3, 2}, tet[4] = {0, 1, 2, 3}, npart[4] = {0, 0, 0, 0};
-  const std::string r = build_layout(dim, 4, xyz, dim == 2 ? 2 : 1, dim == 2 ? tri : tet, npart, 1, L);
+  std::vector<float> xyz;
+  std::vector<int> elems, npart;
+  for (int k = 0; k < n; ++k) {
+    const float x = 2.f * k;
+    const float p[12] = {x, 0, 0, x + 1, 0, 0, x, 1, 0, dim == 2 ? x + 1 : x, dim == 2 ? 1.f : 0.f, dim == 2 ? 0.f : 1.f};
+    xyz.insert(xyz.end(), p, p + 12);
+    for (int v : dim == 2 ? std::vector<int>{0, 1, 2, 1, 3, 2} : std::vector<int>{0, 1, 2, 3}) elems.push_back(4 * k + v);
+    npart.insert(npart.end(), 4, k);
+  }
+  const std::string r = build_layout(dim, 4 * n, xyz.data(), dim == 2 ? 2 * n : n, elems.data(), npart.data(), n, L);
   CHECK(r.empty(), "layout: %s", r.c_str());
   return L;
 }
@@ -101,8 +110,8 @@ Layout make_layout(int dim) {
 struct Rig {
   Layout L;
   std::unique_ptr<Solver> s{new Solver()};
-  std::vector<float> phi{1.f, 2.f, 3.f, 4.f};
-  explicit Rig(const SolverConfig& cfg, int dim = 3) : L(make_layout(dim)) {
+  std::vector<float> phi;
+  explicit Rig(const SolverConfig& cfg, int dim = 3, int n = 1) : L(make_layout(dim, n)), phi(4 * n, 1.f) {
     fake::st.fail_at = -1;
     const std::string r = s->init(L, cfg, nullptr);
     CHECK(r.empty(), "init: %s", r.c_str());
@@ -203,6 +212,34 @@ void restarts() {
       CHECK(d.cell[0].y == d.ctl[CTL_BASE], "run of %d of %d steps: distances cleared", n, n + extra);
     }
 }
+// The FIM setting: a caller's own stays; the default is 5, or 6 where that lets
+// one more CTA reside on a mesh of at least 100 patches per SM.
+void settings() {
+  struct Case { int setting, dim, patches, five, six, exact, persistent, prec, want; } cases[] = {
+      {0, 3, 100, 5, 6, 0, 0, 0, 6}, {0, 3, 100, 6, 7, 0, 0, 0, 6}, {0, 3, 100, 5, 5, 0, 0, 0, 5},
+      {0, 3, 100, 6, 6, 0, 0, 0, 5}, {0, 3, 99, 5, 6, 0, 0, 0, 5},  {0, 3, 100, 5, 6, 1, 0, 0, 5},
+      {0, 3, 100, 5, 6, 0, 1, 0, 5}, {0, 3, 100, 5, 6, 0, 0, 1, 5}, {0, 3, 100, 0, 0, 0, 0, 0, 5},
+      {5, 3, 100, 5, 6, 0, 0, 0, 5}, {6, 3, 100, 5, 5, 0, 0, 0, 6}, {7, 3, 100, 5, 6, 0, 0, 0, 7},
+      {2, 3, 100, 5, 6, 0, 0, 0, 2}, {9, 3, 100, 5, 6, 0, 0, 0, 5}, {0, 2, 100, 0, 0, 0, 0, 0, 5},
+  };
+  sms = 1;
+  for (const Case& c : cases) {
+    std::fill(ctas, ctas + 8, 0);
+    ctas[5] = c.five;
+    ctas[6] = c.six;
+    SolverConfig cfg;
+    cfg.fim_ctas = c.setting;
+    cfg.bit_exact = c.exact;
+    cfg.persistent = c.persistent;
+    cfg.fp64_flagged = c.prec;
+    Rig rig(cfg, c.dim, c.patches);
+    CHECK(rig.s->sp_.ctas == c.want && rig.s->L_.fim_ctas == ctas[c.want],
+          "setting %d, dim %d, %d patches, %d and %d CTAs, exact %d, persistent %d, precision %d: %d instead of %d", c.setting,
+          c.dim, c.patches, c.five, c.six, c.exact, c.persistent, c.prec, rig.s->sp_.ctas, c.want);
+  }
+  std::fill(ctas, ctas + 8, 0);
+  sms = 152;
+}
 }  // namespace
 
 const KernelSet& kernels_fast() { static const KernelSet k = make_kernels(); return k; }
@@ -221,6 +258,7 @@ int main(int argc, char** argv) {
     if (a == "errors") lsgb::errors();
     else if (a == "iterations") lsgb::iterations();
     else if (a == "restarts") lsgb::restarts();
+    else if (a == "settings") lsgb::settings();
     else { std::printf("unknown check %s\n", a.c_str()); return 99; }
   }
   std::printf("%d failures\n", lsgb::failures);

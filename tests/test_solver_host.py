@@ -7,6 +7,8 @@ import subprocess
 
 import pytest
 
+import lsgb300
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "sci-solver_level-set_gb300", "csrc")
 
@@ -41,3 +43,12 @@ def test_iterations_counted_in_any_order(program):
 
 def test_distances_stay_where_a_run_ends(program):
     _check(program, "restarts")
+
+
+def test_fim_setting_is_the_callers_or_chosen_by_residency(program):
+    _check(program, "settings")
+
+
+def test_default_setting_is_the_librarys_choice():
+    # an explicit 5 must be told apart from the default
+    assert lsgb300.default_params().fim_ctas_per_sm == 0
