@@ -441,7 +441,7 @@ int Solver::iter_cap() const {
 // The first iterations stand in a row because a body's boundary (its end
 // kernel and the while node's turn) costs about 8 us, an iteration that finds
 // its list empty about 3.  Steps of triangle meshes take 7 to 11 iterations,
-// of tet meshes 10 to 13: eight and twelve in a row.  Measured with 8 / 12 /
+// of tet meshes 10 to 13: eight and twelve in a row (whole bodies' worth).  Measured with 8 / 12 /
 // 16: 2D 64^2, 20 steps 2042 / 2088 / 2217 us; 3D 32^3, 10 steps 2345 / 2291 /
 // 2348 us, 16^3 step 181 / 175 / 181 us (in the loop from the start 2345,
 // 2500, 214 us).

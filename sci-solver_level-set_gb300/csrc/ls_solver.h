@@ -158,7 +158,8 @@ class Solver {
   std::string learn_buffers();
   std::string fim_loop(const StepParams& sp);
   std::string build_graph();
-  int first_bodies() const { return m_.dim == 3 ? 3 : 2; }  // loop bodies' worth of iterations before the loop
+  // loop bodies' worth of iterations before the loop: at least 12 (tetrahedra) or 8 iterations
+  int first_bodies() const { return ((m_.dim == 3 ? 12 : 8) + cfg_.graph_chunk - 1) / cfg_.graph_chunk; }
   bool build_persistent_graph(std::string* err);
   std::string emit_phi(float* row);
   // the calls above, with work on the caller's arrays still in flight on an error

@@ -28,6 +28,7 @@ int failures = 0;
 // Steps with a narrowband that the fake kernels still have to give.
 int nb_steps = 1 << 30;
 int sms = 152;
+int fim_launches = 0;  // captured or enqueued
 int ctas[8] = {};  // resident CTAs of each FIM setting; 0: no two-copies kernel
 
 void begin_words(int* c) {
@@ -68,6 +69,7 @@ KernelSet make_kernels() {
   k.begin = [](const DevState& s, int, cudaStream_t st) { return put(st, [=] { begin_words(s.ctl); }); };
   k.seed = [](const DevMesh&, const DevState&, const StepParams&, const Launch&, cudaStream_t st) { return put(st, [] {}); };
   k.fim = [](const DevMesh&, const DevState& s, const StepParams&, int off, const Launch&, cudaStream_t st) {
+    ++fim_launches;
     return put(st, [=] { if (off == 0 && !s.ctl[CTL_STOP]) s.ctl[CTL_ITER] += 4; });
   };
   k.narrowband = [](const DevMesh& m, const DevState& s, const StepParams&, const Launch&, cudaStream_t st) {
@@ -240,6 +242,21 @@ void settings() {
   std::fill(ctas, ctas + 8, 0);
   sms = 152;
 }
+// The step graph's iterations before its loop: the body's length decides their
+// number only up to the next whole body.
+void first_iterations() {
+  for (int dim : {2, 3})
+    for (int chunk : {0, 1, 2, 3, 4, 6, 8, 10, 16, 32, 100}) {
+      SolverConfig cfg;
+      cfg.graph_chunk = chunk;
+      fim_launches = 0;
+      Rig rig(cfg, dim);
+      const int body = std::max(chunk + (chunk & 1), 2), least = dim == 3 ? 12 : 8;
+      const int want = (least + body - 1) / body * body;
+      CHECK(fim_launches == want + body, "dim %d, graph_chunk %d: %d launches before the loop instead of %d", dim, chunk,
+            fim_launches - body, want);
+    }
+}
 }  // namespace
 
 const KernelSet& kernels_fast() { static const KernelSet k = make_kernels(); return k; }
@@ -259,6 +276,7 @@ int main(int argc, char** argv) {
     else if (a == "iterations") lsgb::iterations();
     else if (a == "restarts") lsgb::restarts();
     else if (a == "settings") lsgb::settings();
+    else if (a == "first_iterations") lsgb::first_iterations();
     else { std::printf("unknown check %s\n", a.c_str()); return 99; }
   }
   std::printf("%d failures\n", lsgb::failures);

@@ -49,6 +49,10 @@ def test_fim_setting_is_the_callers_or_chosen_by_residency(program):
     _check(program, "settings")
 
 
+def test_iterations_before_the_loop_do_not_grow_with_its_body(program):
+    _check(program, "first_iterations")
+
+
 def test_default_setting_is_the_librarys_choice():
     # an explicit 5 must be told apart from the default
     assert lsgb300.default_params().fim_ctas_per_sm == 0
