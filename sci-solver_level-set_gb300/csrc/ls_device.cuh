@@ -166,7 +166,7 @@ struct StepParams {
   float scale;       // FIM frame length unit (1 with the reference's semantics)
   float tau;         // precision form: discriminant cancellation threshold
   int xdiv;          // interior division in double (bit-exact build, reference semantics)
-  int ctas;          // FIM CTAs per SM for patches of up to 384 copies (2, 3, 4; 5: two copies per thread)
+  int ctas;          // FIM CTAs per SM for patches of up to 384 copies (2, 3, 4; 5, 6: two copies per thread, 7: the same kernel with one)
   float tol;       // convergence threshold on oldT - newT
   float eps_h;     // denominator offset of the interior tet update
   double eps_h64;
@@ -180,6 +180,7 @@ struct StepParams {
   int spin_limit;     // polls of one grid-barrier wait of the persistent FIM kernel before it gives up;
                       // < 0: every wait of the FIM kernels (grid barrier, geometry slab copy) gives up
                       // at its first check (the setting that tests the timeout paths)
+  int wide;           // fast build, tetrahedra: the mesh has edges below 1e-7 FIM lengths (tet_solve_wave's WIDE)
 };
 
 __device__ __forceinline__ PatchPar patch_par(const DevMesh& m, const StepParams& sp, int p) {
@@ -532,34 +533,44 @@ __device__ __forceinline__ bool in_unit(float a, float b, float c) {
 // the products, without signs.)  Not all of TP, TQ, TR are LARGENUM (the
 // listings leave those solves out).
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
-// The approximate square root, its reciprocal and the reciprocal as the bare
-// hardware operations: with denormals kept, each of the solver's 17 carries
-// a test and a rescaling of its argument.  The arguments here are squared
-// lengths and products of two of them; one below 1.2e-38 stands for a
-// length under 1e-19 (or a face area under 1e-19 of a square unit, whose
-// reciprocal overflows FP32 either way).
+// The approximate square root, its reciprocal and the reciprocal.  WIDE keeps
+// denormals; without it they are the bare hardware operations: with denormals
+// kept, each of the solver's 17 carries a test and a rescaling of its argument
+// (same bits for normal arguments and results).  The arguments are squared
+// lengths, products of two of them (squared face areas, whose square roots
+// are distances: flushed to zero they put vertices on the front that they are
+// a length away from) and differences of such products, so the bare form is
+// for meshes whose shortest edge is at least 1e-7 in the FIM frame
+// (StepParams::wide).
+template <bool WIDE>
 __device__ __forceinline__ float fast_sqrt(float x) {
   float r;
-  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  if constexpr (WIDE) asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  else asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
+template <bool WIDE>
 __device__ __forceinline__ float fast_rsqrt(float x) {
   float r;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  if constexpr (WIDE) asm("rsqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  else asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
+template <bool WIDE>
 __device__ __forceinline__ float fast_rcp(float x) {
   float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  if constexpr (WIDE) asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  else asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
 
+template <bool WIDE>
 __device__ __forceinline__ float tet_solve_wave(float TP, float TQ, float TR, float PP, float PQ, float PX, float QQ,
                                                 float QX, float XX, float hX, float eps_h) {
   // edges PX, QX (lanes x, y) and RX
   const float2 d2 = f2((PP - PX) + (XX - PX), (QQ - QX) + (XX - QX));
-  const float2 ed = __fadd2_rn(f2(TP, TQ), f2(fast_sqrt(d2.x), fast_sqrt(d2.y)));
-  float best = fminf(fminf(ed.x, ed.y), TR + fast_sqrt(XX));
+  const float2 ed = __fadd2_rn(f2(TP, TQ), f2(fast_sqrt<WIDE>(d2.x), fast_sqrt<WIDE>(d2.y)));
+  float best = fminf(fminf(ed.x, ed.y), TR + fast_sqrt<WIDE>(XX));
   const float up = TP - TR, uq = TQ - TR;
   // sides: y = lam F + (1 - lam) B with |F - B|^2 = ff, (F - B).(X - B) = fw,
   // |X - B|^2 = ww and u = T_F - T_B.  At the stationary point of
@@ -569,8 +580,8 @@ __device__ __forceinline__ float tet_solve_wave(float TP, float TQ, float TR, fl
   {  // sides RQ (lane x) and RP (lane y), both from R
     const float2 G = f2(fmaf(QQ, XX, -__fmul_rn(QX, QX)), fmaf(PP, XX, -__fmul_rn(PX, PX)));  // ff ww - fw^2
     const float2 q = f2(fmaf(-uq, uq, QQ), fmaf(-up, up, PP));                                // ff - u^2
-    const float2 r = __fmul2_rn(f2(fast_sqrt(G.x), fast_sqrt(G.y)), f2(fast_rsqrt(q.x), fast_rsqrt(q.y)));
-    const float lx = __fmul_rn(fmaf(-uq, r.x, QX), fast_rcp(QQ)), ly = __fmul_rn(fmaf(-up, r.y, PX), fast_rcp(PP));
+    const float2 r = __fmul2_rn(f2(fast_sqrt<WIDE>(G.x), fast_sqrt<WIDE>(G.y)), f2(fast_rsqrt<WIDE>(q.x), fast_rsqrt<WIDE>(q.y)));
+    const float lx = __fmul_rn(fmaf(-uq, r.x, QX), fast_rcp<WIDE>(QQ)), ly = __fmul_rn(fmaf(-up, r.y, PX), fast_rcp<WIDE>(PP));
     const float2 c = __fadd2_rn(__ffma2_rn(f2(lx, ly), f2(uq, up), f2(TR, TR)), r);
     if (in_unit(lx)) best = fminf(best, c.x);
     if (in_unit(ly)) best = fminf(best, c.y);
@@ -578,12 +589,12 @@ __device__ __forceinline__ float tet_solve_wave(float TP, float TQ, float TR, fl
   {  // side QP, from Q
     const float u = TP - TQ;
     const float ff = (QQ - PQ) + (PP - PQ), fw = (QQ - QX) - (PQ - PX);
-    const float r = __fmul_rn(fast_sqrt(fmaf(ff, d2.y, -__fmul_rn(fw, fw))), fast_rsqrt(fmaf(-u, u, ff)));
-    const float lam = __fmul_rn(fmaf(-u, r, fw), fast_rcp(ff));
+    const float r = __fmul_rn(fast_sqrt<WIDE>(fmaf(ff, d2.y, -__fmul_rn(fw, fw))), fast_rsqrt<WIDE>(fmaf(-u, u, ff)));
+    const float lam = __fmul_rn(fmaf(-u, r, fw), fast_rcp<WIDE>(ff));
     if (in_unit(lam)) best = fminf(best, __fadd_rn(fmaf(lam, u, TQ), r));
   }
   {  // interior: y = l1 P + l2 Q + l3 R
-    const float idet = fast_rcp(fmaf(PP, QQ, -__fmul_rn(PQ, PQ)));
+    const float idet = fast_rcp<WIDE>(fmaf(PP, QQ, -__fmul_rn(PQ, PQ)));
     // the reference's h (also the numerator of g1), s and t
     const float h = fmaf(QQ, up, -__fmul_rn(PQ, uq));
     const float s = fmaf(-up, PQ, __fmul_rn(uq, PP)), t = fmaf(up, QX, -__fmul_rn(uq, PX));
@@ -594,8 +605,8 @@ __device__ __forceinline__ float tet_solve_wave(float TP, float TQ, float TR, fl
     // (lane y): the reference's SMALLNUM offset in l2 = (s l1 + t) / (h +
     // eps_h) can move the first point out of the face where h is small, and
     // the mirror's point is then the better one, as in the reference
-    const float dl = __fmul_rn(__fmul_rn(hX, fast_rsqrt(__fsub_rn(1.f, fmaf(g1, up, __fmul_rn(g2, uq))))), g1);
-    const float ih = fast_rcp(h + eps_h);
+    const float dl = __fmul_rn(__fmul_rn(hX, fast_rsqrt<WIDE>(__fsub_rn(1.f, fmaf(g1, up, __fmul_rn(g2, uq))))), g1);
+    const float ih = fast_rcp<WIDE>(h + eps_h);
     const float2 l1 = f2(foot1 - dl, foot1 + dl);
     const float2 l2 = __fmul2_rn(__ffma2_rn(f2(s, s), l1, f2(t, t)), f2(ih, ih));
     const float2 l3 = f2((1.f - l1.x) - l2.x, (1.f - l1.y) - l2.y);
@@ -605,7 +616,7 @@ __device__ __forceinline__ float tet_solve_wave(float TP, float TQ, float TR, fl
     const float2 a3 = __ffma2_rn(l1, f2(-PX, -PX), __ffma2_rn(l2, f2(-QX, -QX), f2(XX, XX)));
     const float2 Q = __ffma2_rn(a1, l1, __ffma2_rn(a2, l2, a3));
     const float2 lin = __ffma2_rn(f2(TP, TP), l1, __ffma2_rn(f2(TQ, TQ), l2, __fmul2_rn(f2(TR, TR), l3)));
-    const float2 c = __fadd2_rn(lin, f2(fast_sqrt(Q.x), fast_sqrt(Q.y)));
+    const float2 c = __fadd2_rn(lin, f2(fast_sqrt<WIDE>(Q.x), fast_sqrt<WIDE>(Q.y)));
     if (in_unit(l1.x, l2.x, l3.x)) best = fminf(best, c.x);
     if (in_unit(l1.y, l2.y, l3.y)) best = fminf(best, c.y);
   }
@@ -676,11 +687,12 @@ template <int K>
 __device__ __forceinline__ float tri_solve_wave(const TriGeo& g, const float* T) {
   constexpr int P = (K + 1) % 3, Q = (K + 2) % 3;
   const float u = T[Q] - T[P];
-  // none when ff <= u^2: the rsqrt is NaN or inf and the range test fails.
+  // none when ff <= u^2: the rsqrt is NaN or inf and the range test fails
+  // (denormals only where an edge is below 1e-19: its square is one).
   // Rounded down: a front stops up to the tolerance too high.  196 eikonal
   // runs (40^2 to 300^2) are 1.47e-7 from 64 bits in the mean (the quadratic
   // form 1.53e-7, this one rounded to nearest 1.57e-7).
-  const float r = __fmul_rd(g.area2, fast_rsqrt(fmaf(-u, u, g.ff[K])));
+  const float r = __fmul_rd(g.area2, fast_rsqrt<false>(fmaf(-u, u, g.ff[K])));
   const float lam = __fmul_rn(fmaf(-u, r, g.fw[K]), g.inv[K]);
   // |X - P| is the side opposite Q, |X - Q| the one opposite P
   const float best = fminf(T[P] + g.len[Q], T[Q] + g.len[P]);

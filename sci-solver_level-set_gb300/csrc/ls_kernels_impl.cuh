@@ -643,7 +643,7 @@ __device__ __forceinline__ int draw_patch(int* next, int count) {
 // values at the sweep start [4], ghost results [4], connectivity, list.
 // A candidate found unconverged by its check runs its visit from the start
 // (the check's sweep left out the ghost targets).
-template <int MAXT, int MINB, bool PREC>
+template <int MAXT, int MINB, bool PREC, bool WIDE>
 __global__ void __launch_bounds__(MAXT, MINB) k_fim_compact(DevMesh m, DevState s, StepParams sp, int off) {
   extern __shared__ float smem[];
   float* sT = smem;                       // owned + ghost values
@@ -789,7 +789,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_fim_compact(DevMesh m, DevState 
         if constexpr (PREC)
           r = tet_solve_pred<true>(a0, a1, a2, g0, g1, g2, g3, g4, g5, sp.eps_h, sp.largenum, sp.tau, &ill);
         else
-          r = tet_solve_wave(a0, a1, a2, g0, g1, -g2, g3, -g4, g5, sH[k * MAXT + cc], sp.eps_h);
+          r = tet_solve_wave<WIDE>(a0, a1, a2, g0, g1, -g2, g3, -g4, g5, sH[k * MAXT + cc], sp.eps_h);
         if (PREC && ill) {
           // discriminant cancelled: repeat in FP64 after this pass, densely
           sRep[atomicAdd(&s_rep, 1)] = code;
@@ -883,11 +883,13 @@ __global__ void __launch_bounds__(MAXT, MINB) k_fim_compact(DevMesh m, DevState 
 }
 
 // Local solver of the two-copies-per-thread sweep: the fast build's
-// planar-wave solver with the lower-bound skip (kPairWave), or the
+// planar-wave solver with the lower-bound skip (kPairWave; kPairWaveWide with
+// denormals kept), or the
 // reference's solver in its operand order (the
 // bit-exact build; kPairRefXdiv with the interior division in double, as
 // the reference semantics there).
-constexpr int kPairWave = 0, kPairRef = 1, kPairRefXdiv = 2;
+constexpr int kPairWave = 0, kPairRef = 1, kPairRefXdiv = 2, kPairWaveWide = 3;
+__host__ __device__ constexpr bool pair_wave(int solver) { return solver == kPairWave || solver == kPairWaveWide; }
 
 // The solves (bit k: target k) of a copy with values tv and heights hv that
 // can lower their target T_k.  One cannot when the three other values are
@@ -909,7 +911,7 @@ template <int SOLVER>
 __device__ __forceinline__ unsigned pair_may_lower(const float4& tv, const float4& hv, float LN) {
   const float m01 = fminf(tv.x, tv.y), m23 = fminf(tv.z, tv.w);
   const float n0 = fminf(tv.y, m23), n1 = fminf(tv.x, m23), n2 = fminf(m01, tv.w), n3 = fminf(m01, tv.z);
-  if constexpr (SOLVER == kPairWave)
+  if constexpr (pair_wave(SOLVER))
     return (n0 + 0.999f * hv.x < tv.x ? 1u : 0u) | (n1 + 0.999f * hv.y < tv.y ? 2u : 0u) |
            (n2 + 0.999f * hv.z < tv.z ? 4u : 0u) | (n3 + 0.999f * hv.w < tv.w ? 8u : 0u);
   constexpr float lo = 1.f - 1e-6f;
@@ -937,10 +939,10 @@ __device__ __forceinline__ void pair_solve(int code, const float4* sTc, const fl
   const float PP = k0 ? bb : aa, PQ = k0 ? bd : k1 ? ad : ab, PX = lo ? ab : ad;
   const float QQ = lo ? dd : bb, QX = k0 ? ad : bd, XX = k0 ? aa : k1 ? bb : dd;
   float r;
-  if constexpr (SOLVER == kPairWave) {
+  if constexpr (pair_wave(SOLVER)) {
     // the target's height: component k of the copy's record, loaded alone
     const float hX = reinterpret_cast<const float*>(sH)[4 * cc + k];
-    r = tet_solve_wave(tp, tq, tr, PP, PQ, PX, QQ, QX, XX, hX, sp.eps_h);
+    r = tet_solve_wave<SOLVER == kPairWaveWide>(tp, tq, tr, PP, PQ, PX, QQ, QX, XX, hX, sp.eps_h);
   } else {
     bool d = false;
     r = tet_solve<float, SOLVER == kPairRefXdiv, false, false>(tp, tq, tr, PP, PQ, -PX, QQ, -QX, XX, sp.eps_h,
@@ -2195,7 +2197,7 @@ inline int pair_smem(const StepParams& sp, int ncap) {
 #ifdef LS_KERNELS_EXACT
 #define LS_PAIR_SOLVERS(K, n, sp) ((sp).xdiv ? (const void*)K<n, kPairRefXdiv> : (const void*)K<n, kPairRef>)
 #else
-#define LS_PAIR_SOLVERS(K, n, sp) ((const void*)K<n, kPairWave>)
+#define LS_PAIR_SOLVERS(K, n, sp) ((sp).wide ? (const void*)K<n, kPairWaveWide> : (const void*)K<n, kPairWave>)
 #endif
 #define LS_PAIR_PICK(K, sp)                                            \
   ((sp).ctas == 7   ? LS_PAIR_SOLVERS(K, 7, sp)                      \
@@ -2208,6 +2210,22 @@ inline int pair_smem(const StepParams& sp, int ncap) {
 // 384 copies, FIM setting 5: the two-copies-per-thread sweep (L.pair_block).
 __host__ __device__ inline bool use_pair(const DevMesh& m, const StepParams& sp, const Launch& L) {
   return m.dim == 3 && !m.capped && !(sp.tau > 0.f) && L.pair_block > 0;
+}
+
+// k_fim_compact of a block size and setting.
+template <bool WIDE>
+inline const void* compact_plain(int block, int ctas) {
+  if (block > 512) return (const void*)k_fim_compact<1024, 1, false, WIDE>;
+  if (block > 384) return (const void*)k_fim_compact<512, 1, false, WIDE>;
+  return ctas == 2   ? (const void*)k_fim_compact<384, 2, false, WIDE>
+         : ctas == 4 ? (const void*)k_fim_compact<384, 4, false, WIDE>
+                     : (const void*)k_fim_compact<384, 3, false, WIDE>;
+}
+inline const void* compact_kernel(const StepParams& sp, const Launch& L, bool prec) {
+  if (!prec) return sp.wide ? compact_plain<true>(L.fim_block, sp.ctas) : compact_plain<false>(L.fim_block, sp.ctas);
+  return L.fim_block <= 384   ? (const void*)k_fim_compact<384, 2, true, false>
+         : L.fim_block <= 512 ? (const void*)k_fim_compact<512, 1, true, false>
+                              : (const void*)k_fim_compact<1024, 1, true, false>;
 }
 
 cudaError_t launch_pair(const DevMesh& m, const DevState& s, const StepParams& sp, int off, const Launch& L,
@@ -2239,25 +2257,13 @@ cudaError_t launch_fim(const DevMesh& m, const DevState& s, const StepParams& sp
   if (use_pair(m, sp, L)) {
     // tetrahedra: compacted solves, two copies per thread
     return launch_pair(m, s, sp, off, L, st);
-  } else if (compact && pr) {
-    // fast build, tetrahedra, precision form: compacted solves, FP64 repeats
-    // run densely after each sweep's FP32 pass
-    const int cs = compact_smem(sp, L.fim_block <= 384 ? 384 : L.fim_block <= 512 ? 512 : 1024);
-    if (L.fim_block <= 384) k_fim_compact<384, 2, true><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, off);
-    else if (L.fim_block <= 512) k_fim_compact<512, 1, true><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, off);
-    else k_fim_compact<1024, 1, true><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, off);
   } else if (compact) {
-    // fast build, tetrahedra: compacted solves
+    // fast build, tetrahedra: compacted solves (precision form: FP64 repeats
+    // run densely after each sweep's FP32 pass)
     const int cs = compact_smem(sp, L.fim_block <= 384 ? 384 : L.fim_block <= 512 ? 512 : 1024);
-    if (L.fim_block <= 384) {
-      if (sp.ctas == 2) k_fim_compact<384, 2, false><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, off);
-      else if (sp.ctas == 4) k_fim_compact<384, 4, false><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, off);
-      else k_fim_compact<384, 3, false><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, off);
-    } else if (L.fim_block <= 512) {
-      k_fim_compact<512, 1, false><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, off);
-    } else {
-      k_fim_compact<1024, 1, false><<<L.fim_grid, L.fim_block, cs, st>>>(m, s, sp, off);
-    }
+    void* args[] = {(void*)&m, (void*)&s, (void*)&sp, (void*)&off};
+    return cudaLaunchKernel(compact_kernel(sp, L, pr), dim3((unsigned)L.fim_grid), dim3((unsigned)L.fim_block), args,
+                            (size_t)cs, st);
   } else if (m.dim == 3) {
     if (L.fim_block <= 384) {
       if (sp.ctas == 2) LS_FIM3(384, 2);
@@ -2430,31 +2436,13 @@ cudaError_t configure_launch(const DevMesh& m, const StepParams& sp, Launch& L) 
       e = allow_smem(LS_PAIR_KERNEL(sp), ps);
       if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, LS_PAIR_KERNEL(sp), L.pair_block, ps);
-    } else if (L.fim_block <= 384 && sp.ctas == 2) {
-      e = allow_smem((const void*)k_fim_compact<384, 2, false>, cs);
-      if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fim_compact<384, 2, false>, L.fim_block, cs);
-    } else if (L.fim_block <= 384 && sp.ctas == 4) {
-      e = allow_smem((const void*)k_fim_compact<384, 4, false>, cs);
-      if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fim_compact<384, 4, false>, L.fim_block, cs);
-    } else if (L.fim_block <= 384) {
-      e = allow_smem((const void*)k_fim_compact<384, 3, false>, cs);
-      if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fim_compact<384, 3, false>, L.fim_block, cs);
-    } else if (L.fim_block <= 512) {
-      e = allow_smem((const void*)k_fim_compact<512, 1, false>, cs);
-      if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fim_compact<512, 1, false>, L.fim_block, cs);
     } else {
-      e = allow_smem((const void*)k_fim_compact<1024, 1, false>, cs);
-      if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fim_compact<1024, 1, false>, L.fim_block, cs);
+      const void* fn = compact_kernel(sp, L, false);
+      e = allow_smem(fn, cs);
+      if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, L.fim_block, cs);
     }
     // precision-form variants (selected at launch when tau > 0)
-    if (e == cudaSuccess) {
-      if (L.fim_block <= 384)
-        e = allow_smem((const void*)k_fim_compact<384, 2, true>, cs);
-      else if (L.fim_block <= 512)
-        e = allow_smem((const void*)k_fim_compact<512, 1, true>, cs);
-      else
-        e = allow_smem((const void*)k_fim_compact<1024, 1, true>, cs);
-    }
+    if (e == cudaSuccess) e = allow_smem(compact_kernel(sp, L, true), cs);
   } else if (m.dim == 3) {
     if (!m.capped && L.fim_block <= 384 && sp.ctas >= 5 && sp.ctas <= 7) {
       // bit-exact build: two copies per thread with the reference's solver

@@ -130,10 +130,10 @@ std::string build_layout(int dim, int nv, const float* xyz, int ne, const int* e
   L.xyz_p.resize((size_t)3 * nv);
   for (int v = 0; v < nv; ++v)
     for (int j = 0; j < 3; ++j) L.xyz_p[(size_t)j * nv + v] = xyz[(size_t)L.vert_permute[v] * 3 + j];
-  // LIM and mean edge length
+  // LIM, mean and shortest edge length
   {
     std::vector<int> adj(nv, 0);
-    double esum = 0;
+    double esum = 0, emin = HUGE_VAL;
     long long ecount = 0;
     for (int e = 0; e < ne; ++e) {
       const int* ev = elems + (size_t)e * d1;
@@ -143,12 +143,15 @@ std::string build_layout(int dim, int nv, const float* xyz, int ne, const int* e
           double dx = (double)xyz[(size_t)ev[a] * 3] - xyz[(size_t)ev[b] * 3];
           double dy = (double)xyz[(size_t)ev[a] * 3 + 1] - xyz[(size_t)ev[b] * 3 + 1];
           double dz = (double)xyz[(size_t)ev[a] * 3 + 2] - xyz[(size_t)ev[b] * 3 + 2];
-          esum += std::sqrt(dx * dx + dy * dy + dz * dz);
+          const double len = std::sqrt(dx * dx + dy * dy + dz * dz);
+          esum += len;
+          if (len > 0 && len < emin) emin = len;
           ecount++;
         }
     }
     L.lim = *std::max_element(adj.begin(), adj.end());
     L.mean_edge = esum / (double)ecount;
+    L.min_edge = emin < HUGE_VAL ? emin : 0.0;
   }
   // ghosts per patch and slab-local connectivity
   L.ghost_offsets.assign(nparts + 1, 0);
@@ -293,6 +296,7 @@ std::string merge_layouts(const std::vector<const Layout*>& parts, Layout& out) 
     out.lim = std::max(out.lim, P.lim);
     out.has_internal_edge = out.has_internal_edge || P.has_internal_edge;
     out.mesh_edge.push_back(P.mean_edge);
+    out.mesh_min_edge.push_back(P.min_edge);
     vb += P.nv; eb += P.ne; pb += P.nparts; cb += (int)P.full;
     gb += (int)P.ghost_ids.size(); sb += (int)P.vslot.size(); ab += (int)P.padj.size();
   }

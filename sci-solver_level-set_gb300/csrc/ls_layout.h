@@ -25,6 +25,7 @@ struct Layout {
   int lgp = 0;          // largest number of ghost vertices in a patch
   int lim = 0;          // largest number of elements at one vertex
   double mean_edge = 0; // mean element edge length
+  double min_edge = 0;  // shortest edge of positive length (0: none)
 
   // vertex order: new id -> old id and inverse; patch ranges of new ids
   std::vector<int> vert_permute, vert_ipermute, vert_offsets;
@@ -55,9 +56,9 @@ struct Layout {
   // permuted coordinates, SoA [3][nv]
   std::vector<float> xyz_p;
   // batches of independent meshes (merge_layouts): mesh of each patch and
-  // the mean edge length of each mesh; empty for a single mesh
+  // the mean and shortest edge length of each mesh; empty for a single mesh
   std::vector<int> patch_mesh;
-  std::vector<double> mesh_edge;
+  std::vector<double> mesh_edge, mesh_min_edge;
 };
 
 // Build the layout.  Returns an empty string on success, else the reason.

@@ -305,6 +305,14 @@ std::string Solver::init(const Layout& L, const SolverConfig& cfg, const float* 
   sp_.scale = (float)scale;
   sp_.tau = (cfg.fp64_flagged && L.dim == 3) ? (float)cfg.fp64_tau : 0.f;
   sp_.xdiv = (cfg.bit_exact && ref) ? 1 : 0;
+  // the planar-wave solver's denormal-keeping form where an edge is so short
+  // that products of four lengths, or differences of such products, can be
+  // denormal (lengths in the FIM frame: 1e-28 and their last bits)
+  sp_.wide = 0;
+  for (int k = 0; k < nmesh; ++k) {
+    const double e = (batch ? L.mesh_min_edge[k] : L.min_edge) / mscale[k];
+    if (e > 0 && e < 1e-7) sp_.wide = 1;
+  }
   sp_.ctas = (cfg.fim_ctas >= 2 && cfg.fim_ctas <= 7) ? cfg.fim_ctas : 5;
   sp_.tol = (float)cfg.smallnum;
   sp_.eps_h64 = cfg.smallnum;
@@ -321,7 +329,7 @@ std::string Solver::init(const Layout& L, const SolverConfig& cfg, const float* 
   sp_.spin_limit = cfg.spin_limit != 0 ? cfg.spin_limit : (1 << 22);
   (void)d1;
   LS_TRY(K_->configure(m_, sp_, L_), "configure");
-  if (cfg.fim_ctas == 0 && !cfg.bit_exact && !cfg.persistent && !(sp_.tau > 0.f) && L_.pair_block > 0 &&
+  if (cfg.fim_ctas == 0 && !cfg.bit_exact && !cfg.persistent && !(sp_.tau > 0.f) && !sp_.wide && L_.pair_block > 0 &&
       np >= 100 * L_.sms) {
     // The default's tet sweep on large meshes: setting 6's registers (56
     // instead of 64), where they let one more CTA reside -- blocks of 192
