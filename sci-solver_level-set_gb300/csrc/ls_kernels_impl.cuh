@@ -563,11 +563,7 @@ __device__ __forceinline__ void fim_copy_pass(const DevMesh& m, const DevState& 
         if (__syncthreads_and(c0)) break;
         visit = true;
         niter = sp.niter;
-        nflag *= 2;  // the visit's own repeats of this sweep, counted as run again
-        if (tid == 0) {
-          cnt.visits++;
-          cnt.bytes += (unsigned long long)(__ldg(m.patch_bytes + p) - 4 * nvp);
-        }
+        if (tid == 0) cnt.visits++;
       } else if (PREC) {
         __syncthreads();  // the queue's reset and results, before the next sweep fills it
       } else if (!any) {
