@@ -73,8 +73,9 @@ enum {
    * operation individually rounded in the reference's order).  Slower;
    * reproduces the CPU restatement of the reference bit for bit. */
   LS_BITEXACT = 1u << 4,
-  /* ls_step_host: stage host arrays through pinned buffers even where the
-   * GPU can access pageable host memory directly (the default there). */
+  /* Host arrays (phi in and out, histories, eikonal distances) go through a
+   * pinned buffer even where the GPU can access pageable host memory directly
+   * (the default there).  Same results. */
   LS_HOST_STAGING = 1u << 5,
   /* Run every FIM iteration of a time step in one cooperative (all CTAs
    * resident) launch, the iterations separated by grid-wide barriers,
@@ -384,6 +385,10 @@ ls_status ls_mlp_create(ls_mlp** m, unsigned long long seed);
 ls_status ls_mlp_destroy(ls_mlp* m);
 const char* ls_mlp_last_error(ls_mlp* m);
 int ls_mlp_num_params(void);
+/* on: the caller's rows are copied to the device before they are converted,
+ * even where the GPU can read pageable host memory directly (the default
+ * there).  Same results. */
+ls_status ls_mlp_set_host_staging(ls_mlp* m, int on);
 ls_status ls_mlp_set_params(ls_mlp* m, const float* params);
 ls_status ls_mlp_get_params(ls_mlp* m, float* params);
 /* x: n x 128 floats (rounded to BF16), y: n outputs */

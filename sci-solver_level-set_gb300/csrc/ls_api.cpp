@@ -930,6 +930,11 @@ const char* ls_mlp_last_error(ls_mlp* m) { return m ? m->err.c_str() : "null net
 
 int ls_mlp_num_params(void) { return lsgb::mlp::Net::num_params(); }
 
+ls_status ls_mlp_set_host_staging(ls_mlp* m, int on) {
+  if (!m) return LS_BAD_INPUT;
+  return mfail(m, m->net.set_host_staging(on != 0));
+}
+
 ls_status ls_mlp_set_params(ls_mlp* m, const float* p) {
   if (!m || !p) return LS_BAD_INPUT;
   return mfail(m, m->net.set_params(p));

@@ -807,8 +807,8 @@ std::string Net::init(unsigned long long seed) {
     MLP_TRY(cudaGetDevice(&dev), "device");
     MLP_TRY(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev), "device");
     if (sms_ < 1) sms_ = 1;
-    if (cudaDeviceGetAttribute(&pageable_, cudaDevAttrPageableMemoryAccess, dev) != cudaSuccess) pageable_ = 0;
   }
+  set_host_staging(false);
   // one partial-gradient row per backward CTA (at most one CTA per SM)
   MLP_TRY(alloc((void**)&Gp_, sizeof(float) * (size_t)NG_STRIDE * sms_), "alloc");
   MLP_TRY(cudaMemsetAsync(M1_, 0, sizeof(float) * NP, stream_), "memset");
@@ -825,6 +825,17 @@ std::string Net::init(unsigned long long seed) {
   std::uniform_real_distribution<float> U4(-std::sqrt(3.f / F), std::sqrt(3.f / F));
   for (int i = 0; i < F; ++i) p[3 * F * F + 3 * F + i] = U4(rng);
   return set_params(p.data());
+}
+
+// Host rows through a device copy (on), or read by the GPU where they are if
+// it can access pageable memory.
+std::string Net::set_host_staging(bool on) {
+  int dev = 0;
+  pageable_ = 0;
+  if (on) return "";
+  MLP_TRY(cudaGetDevice(&dev), "device");
+  if (cudaDeviceGetAttribute(&pageable_, cudaDevAttrPageableMemoryAccess, dev) != cudaSuccess) pageable_ = 0;
+  return "";
 }
 
 std::string Net::set_params(const float* host) {

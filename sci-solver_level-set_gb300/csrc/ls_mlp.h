@@ -23,6 +23,7 @@ class Net {
   // master parameters [W1 W2 W3 (128x128 each, [out][in]) | b1 b2 b3 | w4 | b4]
   std::string set_params(const float* host);
   std::string get_params(float* host);
+  std::string set_host_staging(bool on);
   // host-buffer entry points (features rounded to BF16 on the way in)
   std::string predict(const float* X, int n, float* y);
   std::string gradients(const float* X, const float* t, int n, float* g, float* loss);
@@ -57,7 +58,7 @@ class Net {
   char* ws_ = nullptr;  // workspace of the host-buffer entry points
   size_t ws_bytes_ = 0;
   int* h_end_ = nullptr;  // pinned mirror of the error word and the loss
-  int pageable_ = 0;      // the GPU can access pageable host memory directly
+  int pageable_ = 0;      // host rows are read by the GPU where they are
   cudaStream_t stream_ = nullptr;
   std::vector<void*> allocs_;
   float *P_ = nullptr, *G_ = nullptr, *M1_ = nullptr, *M2_ = nullptr;

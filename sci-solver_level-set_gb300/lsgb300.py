@@ -71,7 +71,7 @@ EXPORTS = [
     "ls_batch_last_error", "ls_batch_add", "ls_batch_setup", "ls_batch_solve", "ls_batch_get_phi",
     "ls_batch_get_stats", "ls_batch_reset_stats", "ls_batch_set_profile", "ls_batch_get_layout_info",
     "ls_batch_get_layout", "ls_autotune", "ls_mlp_create", "ls_mlp_destroy", "ls_mlp_last_error",
-    "ls_mlp_num_params", "ls_mlp_set_params", "ls_mlp_get_params", "ls_mlp_predict", "ls_mlp_gradients",
+    "ls_mlp_num_params", "ls_mlp_set_host_staging", "ls_mlp_set_params", "ls_mlp_get_params", "ls_mlp_predict", "ls_mlp_gradients",
     "ls_mlp_train", "ls_mlp_reserve_pairs", "ls_mlp_clear_pairs", "ls_mlp_num_pairs", "ls_mlp_train_pairs",
     "ls_learn_collect", "ls_set_learned", "ls_batch_set_learned", "ls_mlp_eval_pairs", "ls_batch_autotune",
     "ls_partition_graph", "ls_edge_cut",
@@ -129,6 +129,7 @@ def lib():
     L.ls_mlp_last_error.argtypes = [P]
     L.ls_mlp_last_error.restype = ctypes.c_char_p
     L.ls_mlp_num_params.argtypes = []
+    L.ls_mlp_set_host_staging.argtypes = [P, I]
     L.ls_mlp_set_params.argtypes = [P, V]
     L.ls_mlp_get_params.argtypes = [P, V]
     L.ls_mlp_predict.argtypes = [P, V, I, V]
@@ -551,6 +552,11 @@ class MLP:
     def _check(self, rc, what):
         if rc != LS_OK:
             raise LevelSetError(rc, "%s: %s" % (what, lib().ls_mlp_last_error(self._m).decode()))
+
+    def set_host_staging(self, on):
+        """Copy host rows to the device before their conversion even where the
+        GPU can read them directly (same results)."""
+        self._check(lib().ls_mlp_set_host_staging(self._m, 1 if on else 0), "mlp set_host_staging")
 
     def set_params(self, p):
         a = np.ascontiguousarray(p, np.float32)
