@@ -1498,7 +1498,8 @@ __device__ __forceinline__ int spread_index(const DevState& s, const StepParams&
 
 // The loop: iterations until the list is empty.  The cap is hit when an
 // iteration beyond the first sp.max_fim_iters visits a patch (its list may
-// hold candidates only, all found converged): seen when a list follows it.
+// hold candidates only, all found converged), whether a list follows it or
+// not, as in the step graph.
 template <class Pass>
 __device__ __forceinline__ void fim_loop_persistent(const DevMesh& m, const DevState& s, const StepParams& sp,
                                                     Pass&& pass) {
@@ -1513,8 +1514,8 @@ __device__ __forceinline__ void fim_loop_persistent(const DevMesh& m, const DevS
     const bool done = n[0] + n[CTL_CANDS - CTL_VISITS] == 0 || ld_relaxed(s.ctl + CTL_STOP);
     if (done || it > sp.max_fim_iters) {
       if (blockIdx.x == 0 && threadIdx.x == 0) {
-        if (!done) s.ctl[CTL_CAP] = 1;
         if (it > 0) count_iteration(s.ctl, s.stats, t - 1);
+        if (ld_relaxed(s.ctl + CTL_ITERS) > sp.max_fim_iters) s.ctl[CTL_CAP] = 1;
       }
       return;
     }
