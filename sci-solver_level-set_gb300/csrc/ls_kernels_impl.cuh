@@ -2029,7 +2029,8 @@ __global__ void k_warm_apply(DevState s, DevLearn lr, float LN, float margin) {
 // Support check after the FIM from a warm start: an owned non-seed vertex
 // whose value lies more than tol below every local solve of its elements
 // (its support) was set by the warm start, not by the wavefront; it is
-// reset to LARGENUM and its patch joins the list of another FIM loop.  One
+// reset to LARGENUM and its patch joins the list of another FIM loop, which
+// has the whole iteration cap.  One
 // CTA per patch over all patches; patches without a reached vertex skip.
 template <int D1, bool XDIV>
 __global__ void __launch_bounds__(384) k_support(DevMesh m, DevState s, StepParams sp, DevLearn lr, float tol,
@@ -2039,6 +2040,8 @@ __global__ void __launch_bounds__(384) k_support(DevMesh m, DevState s, StepPara
   float* sC = smem + sp.lvp + sp.lgp;  // owned candidates
   const int tid = threadIdx.x;
   const int base = s.ctl[CTL_BASE], t0 = s.ctl[CTL_ITER];
+  // the iteration cap is that of each FIM loop of the step
+  if (blockIdx.x == 0 && tid == 0) s.ctl[CTL_ITERS] = 0;
   // LARGENUM over the newest value of vertex v
   auto drop = [&](int v) {
     const DtCell c = s.cell[v];
