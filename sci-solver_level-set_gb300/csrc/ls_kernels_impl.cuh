@@ -887,6 +887,13 @@ __global__ void __launch_bounds__(MAXT, MINB) k_fim_compact(DevMesh m, DevState 
 constexpr int kPairWave = 0, kPairRef = 1, kPairRefXdiv = 2, kPairWaveWide = 3;
 __host__ __device__ constexpr bool pair_wave(int solver) { return solver == kPairWave || solver == kPairWaveWide; }
 
+// The least of two, NaN if one is.
+__device__ __forceinline__ float min_nan(float a, float b) {
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
 // The solves (bit k: target k) of a copy with values tv and heights hv that
 // can lower their target T_k.  One cannot when the three other values are
 // all LARGENUM (the solver returns LARGENUM), nor when min of them plus the
@@ -905,14 +912,18 @@ __host__ __device__ constexpr bool pair_wave(int solver) { return solver == kPai
 // 1077 -> 683 us.
 template <int SOLVER>
 __device__ __forceinline__ unsigned pair_may_lower(const float4& tv, const float4& hv, float LN) {
-  const float m01 = fminf(tv.x, tv.y), m23 = fminf(tv.z, tv.w);
-  const float n0 = fminf(tv.y, m23), n1 = fminf(tv.x, m23), n2 = fminf(m01, tv.w), n3 = fminf(m01, tv.z);
-  if constexpr (pair_wave(SOLVER))
+  if constexpr (pair_wave(SOLVER)) {
+    const float m01 = fminf(tv.x, tv.y), m23 = fminf(tv.z, tv.w);
+    const float n0 = fminf(tv.y, m23), n1 = fminf(tv.x, m23), n2 = fminf(m01, tv.w), n3 = fminf(m01, tv.z);
     return (n0 + 0.999f * hv.x < tv.x ? 1u : 0u) | (n1 + 0.999f * hv.y < tv.y ? 2u : 0u) |
            (n2 + 0.999f * hv.z < tv.z ? 4u : 0u) | (n3 + 0.999f * hv.w < tv.w ? 8u : 0u);
+  }
+  // (a minimum with a NaN is one: that solve is run)
   constexpr float lo = 1.f - 1e-6f;
-  return (n0 < LN && n0 * lo + hv.x < tv.x ? 1u : 0u) | (n1 < LN && n1 * lo + hv.y < tv.y ? 2u : 0u) |
-         (n2 < LN && n2 * lo + hv.z < tv.z ? 4u : 0u) | (n3 < LN && n3 * lo + hv.w < tv.w ? 8u : 0u);
+  const float m01 = min_nan(tv.x, tv.y), m23 = min_nan(tv.z, tv.w);
+  auto bound = [&](float n, float h) { return n >= LN ? LN : n * lo + h; };
+  return (bound(min_nan(tv.y, m23), hv.x) >= tv.x ? 0u : 1u) | (bound(min_nan(tv.x, m23), hv.y) >= tv.y ? 0u : 2u) |
+         (bound(min_nan(m01, tv.w), hv.z) >= tv.z ? 0u : 4u) | (bound(min_nan(m01, tv.z), hv.w) >= tv.w ? 0u : 8u);
 }
 
 // One listed solve of k_fim_pair: solve k of copy cc from the copy values
