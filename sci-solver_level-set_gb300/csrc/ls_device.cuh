@@ -104,6 +104,7 @@ enum {
   CTL_CHAIN = 15,
   CTL_STOP = 16,
   CTL_VISITED = 17,  // [3] an iteration visited a patch (visited_word)
+  CTL_ABOVE = 20,    // a seed of this step lies above LARGENUM
   CTL_WORDS = 32
 };
 // Stamps restart (every stamped array cleared) between steps once they pass

@@ -58,7 +58,7 @@ __global__ void k_begin(DevState s, int restart) {
       c[CTL_NB_VALID] = 1;
     }
     c[CTL_NB] = 0;
-    c[CTL_BODIES] = c[CTL_CAP] = c[CTL_ERR] = c[CTL_ITERS] = 0;
+    c[CTL_BODIES] = c[CTL_CAP] = c[CTL_ERR] = c[CTL_ITERS] = c[CTL_ABOVE] = 0;
     const int u = c[CTL_ITER];
     c[CTL_BASE] = u;  // u: seeds, u + 1: warm-start values
     c[CTL_ITER] = u + 2;
@@ -72,6 +72,7 @@ __device__ __forceinline__ int ld_relaxed(const int* p) { return *reinterpret_ca
 // the sizes of its list (visits, then candidates).
 struct FimIter {
   int t, base, nvis, count;
+  bool above;       // values above LARGENUM (pair_may_lower)
   const int* list;  // visits from the front, candidates from the back
   int* next;        // the next iteration's list
   int* next_n;      // and its sizes: [0] visits, [CTL_CANDS - CTL_VISITS] candidates
@@ -90,6 +91,7 @@ __device__ __forceinline__ FimIter fim_iter(const DevMesh& m, const DevState& s,
   f.t = rel ? s_ctl[CTL_ITER] + t : t;
   const int cur = f.t % 3, nxt = cur == 2 ? 0 : cur + 1;
   f.base = s_ctl[CTL_BASE];
+  f.above = s_ctl[CTL_ABOVE] != 0;
   f.nvis = s_ctl[CTL_VISITS + cur];
   // (nor does an iteration behind one that was abandoned run on what it left)
   f.count = s_ctl[CTL_STOP] || s_ctl[CTL_ERR] ? 0 : f.nvis + s_ctl[CTL_CANDS + cur];
@@ -234,7 +236,9 @@ __global__ void __launch_bounds__(kSeedBlock) k_seed(DevMesh m, DevState s, Step
         for (int k = 0; k < D1; ++k) {
           if (cross || val[k] == 0.f) {
             const int gv = idx[k] < nvp ? vs + idx[k] : m.ghost_ids[gs + idx[k] - nvp];
-            *reinterpret_cast<int2*>(s.cell + gv) = make_int2(__float_as_int(fabsf(val[k]) / sc), base);
+            const float d = fabsf(val[k]) / sc;
+            *reinterpret_cast<int2*>(s.cell + gv) = make_int2(__float_as_int(d), base);
+            if (d > sp.largenum) s.ctl[CTL_ABOVE] = 1;
             found = 1;
           }
         }
@@ -899,8 +903,10 @@ __device__ __forceinline__ float min_nan(float a, float b) {
 // all LARGENUM (the solver returns LARGENUM), nor when min of them plus the
 // target's height over their face is at least T_k: every candidate is a value
 // T_lin(y) + |y - X| at a point y of the face.
-// Planar-wave solver: 0.999 x the height (with three LARGENUMs the sum is no
-// less than T_k either).
+// Planar-wave solver: 0.999 x the height.  With three LARGENUMs the sum is no
+// less than T_k either, unless T_k is above LARGENUM, as only a seed can be:
+// fim_pair_pass takes those out of the listing where a step has such seeds
+// (pair_below, 0.8 % of a step for the branch; tested here it is 2-3 %).
 // Reference solver (bit-exact build): what its FP32 candidates satisfy
 // whatever their rounding.  With weights in [0, 1], T_lin rounds to at least
 // min (1 - 4e-7).  The squared distance is the quadratic form of the solve's
@@ -925,6 +931,13 @@ __device__ __forceinline__ unsigned pair_may_lower(const float4& tv, const float
   return (bound(min_nan(tv.y, m23), hv.x) >= tv.x ? 0u : 1u) | (bound(min_nan(tv.x, m23), hv.y) >= tv.y ? 0u : 2u) |
          (bound(min_nan(m01, tv.w), hv.z) >= tv.z ? 0u : 4u) | (bound(min_nan(m01, tv.z), hv.w) >= tv.w ? 0u : 8u);
 }
+
+// The solves of a copy with an input below LARGENUM.
+__device__ __forceinline__ unsigned pair_below(const float4& tv, float LN) {
+  const unsigned b = (tv.x < LN ? 1u : 0u) | (tv.y < LN ? 2u : 0u) | (tv.z < LN ? 4u : 0u) | (tv.w < LN ? 8u : 0u);
+  return (b & (b - 1u)) ? 0xFu : ~b & (b ? 0xFu : 0u);
+}
+constexpr unsigned kAbove = 1u << 8;  // in a copy's flags: the step has seeds above LARGENUM
 
 // One listed solve of k_fim_pair: solve k of copy cc from the copy values
 // at the sweep start; the result lowers the owned target's shared value or
@@ -1114,6 +1127,7 @@ __device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& 
   __shared__ unsigned s_min[2];  // patch minimum, by parity of the CTA's patches
   __shared__ int s_n[2];  // listed solves, by sweep parity (reset one sweep ahead)
   __shared__ int s_li;    // list entry of the next patch
+  __shared__ unsigned s_above;  // kAbove or 0
   __shared__ int s_ng;    // ghost-target solves listed when a check becomes a visit
   __shared__ unsigned s_seed[kSeedMaskWords];  // seed flags of the owned vertices (bit i = vertex i)
   __shared__ __align__(8) unsigned long long s_bar;  // geometry slab copies of the current patch
@@ -1136,6 +1150,7 @@ __device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& 
   const bool seed_mask = sp.lvp <= 32 * kSeedMaskWords;
   if (tid == 0) {
     s_n[0] = s_n[1] = 0;
+    s_above = f.above ? kAbove : 0u;
     s_li = vb;
     s_err = 0;
     s_cnt = FimCount{};
@@ -1182,7 +1197,7 @@ __device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& 
     // the copies' connectivity (the previous patch's last reads of sC came
     // before its final barrier) and flags, which only this thread reads:
     // bits 0 .. 3 the vertices of copy j that changed in the previous
-    // sweep (all on the first), bits 4 .. 7 its ghost vertices
+    // sweep (all on the first), bits 4 .. 7 its ghost vertices, kAbove
     unsigned flags[2] = {0u, 0u};
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
@@ -1192,7 +1207,7 @@ __device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& 
         sC[c] = cv;
         const unsigned ghost = (cv.x >= nvp ? 1u : 0u) | (cv.y >= nvp ? 2u : 0u) | (cv.z >= nvp ? 4u : 0u) |
                                (cv.w >= nvp ? 8u : 0u);
-        flags[j] = 0xFu | (ghost << 4);
+        flags[j] = 0xFu | (ghost << 4) | (pair_wave(SOLVER) ? s_above : 0u);
       }
     }
     if (tid == 0) {
@@ -1251,6 +1266,11 @@ __device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& 
           need[j] = pair_may_lower<SOLVER>(sTc[c], sH[c], sp.largenum) & cand & (~(flags[j] >> 4) | allow_ghost) & 0xFu;
         }
       }
+      if (pair_wave(SOLVER) && (flags[0] & kAbove)) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          if (need[j]) need[j] &= pair_below(sTc[tid + j * blockDim.x], sp.largenum);
+      }
       {
         // list positions: one shared atomic per thread for both copies
         const int nt = __popc(need[0]) + __popc(need[1]);
@@ -1295,7 +1315,8 @@ __device__ __forceinline__ void fim_pair_pass(const DevMesh& m, const DevState& 
             const int c = tid + j * blockDim.x;
             if (c < nep) {
               // (all four inputs count as changed)
-              const unsigned nd = pair_may_lower<SOLVER>(sTc[c], sH[c], sp.largenum) & (flags[j] >> 4);
+              unsigned nd = pair_may_lower<SOLVER>(sTc[c], sH[c], sp.largenum) & (flags[j] >> 4);
+              if (pair_wave(SOLVER)) nd &= pair_below(sTc[c], sp.largenum);
               need[j] |= nd;
               const int n = __popc(nd);
               if (n) {

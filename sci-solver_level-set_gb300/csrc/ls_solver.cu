@@ -999,6 +999,7 @@ __global__ void k_eik_seed(DevMesh m, DevState s, const int* seeds, const float*
   const int v = __ldg(m.ipermute + seeds[i]);
   if (order[v] != i) return;
   const float a = values[i] >= LN ? LN : values[i] / scale;
+  if (a > LN) s.ctl[CTL_ABOVE] = 1;
   *reinterpret_cast<int2*>(s.cell + v) = make_int2(__float_as_int(a), s.ctl[CTL_BASE]);
 }
 // The patches one of whose element copies holds a seed (the list the seed

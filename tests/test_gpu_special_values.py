@@ -45,7 +45,7 @@ KINDS = ["plain", "collapsed", "nan", "inf", "beyond", "scattered"]
 @pytest.mark.parametrize("kind", KINDS)
 @pytest.mark.parametrize("name,n", [("c2", 8), ("c2", 5), ("c3", 7)])
 @pytest.mark.parametrize("kw", [dict(), dict(largenum=0.3), dict(length_scale=7.0), dict(ref_compat=True)])
-@pytest.mark.parametrize("bit_exact", [True])
+@pytest.mark.parametrize("bit_exact", [False, True])
 def test_kernels_agree(kind, name, n, kw, bit_exact):
     for seed in (0, 1, 2, 3, 7):
         w = _workload(name, n, seed, kind)
