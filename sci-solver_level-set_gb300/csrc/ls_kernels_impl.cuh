@@ -914,7 +914,8 @@ __device__ __forceinline__ float min_nan(float a, float b) {
 // S of their magnitudes: where h^2 >= 1e-4 S its root is at least 0.997 h.
 // So min (1 - 1e-6) + 0.99 h (hv, 0 for flat tets: ref_height) bounds them,
 // with room for the rounding of the test itself, and the solves left out
-// change no bit.  48^3 step: 525 M -> 288 M warp instructions, its FIM launches
+// change no bit.  (No result is above LARGENUM, though its candidates are: a
+// target above it, a seed, is lowered to it.)  48^3 step: 525 M -> 288 M warp instructions, its FIM launches
 // 1077 -> 683 us.
 template <int SOLVER>
 __device__ __forceinline__ unsigned pair_may_lower(const float4& tv, const float4& hv, float LN) {
@@ -927,7 +928,7 @@ __device__ __forceinline__ unsigned pair_may_lower(const float4& tv, const float
   // (a minimum with a NaN is one: that solve is run)
   constexpr float lo = 1.f - 1e-6f;
   const float m01 = min_nan(tv.x, tv.y), m23 = min_nan(tv.z, tv.w);
-  auto bound = [&](float n, float h) { return n >= LN ? LN : n * lo + h; };
+  auto bound = [&](float n, float h) { return n >= LN ? LN : min_nan(n * lo + h, LN); };
   return (bound(min_nan(tv.y, m23), hv.x) >= tv.x ? 0u : 1u) | (bound(min_nan(tv.x, m23), hv.y) >= tv.y ? 0u : 2u) |
          (bound(min_nan(m01, tv.w), hv.z) >= tv.z ? 0u : 4u) | (bound(min_nan(m01, tv.z), hv.w) >= tv.w ? 0u : 8u);
 }

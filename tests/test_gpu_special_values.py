@@ -60,3 +60,17 @@ def test_kernels_agree(kind, name, n, kw, bit_exact):
         for done, hist in out[1:]:
             assert done == out[0][0]
             assert np.array_equal(hist, out[0][1], equal_nan=True)
+
+
+@pytest.mark.parametrize("stretch", [1, 2, 5, 50])
+@pytest.mark.parametrize("largenum", [0.05, 0.1, 0.3])
+def test_exact_kernels_agree_where_candidates_pass_largenum(stretch, largenum):
+    # interface values between LARGENUM and the heights of their tets: the
+    # solver's result is capped at LARGENUM, though its candidates lie above
+    for seed in range(12):
+        w = dict(_workload("c2", 8, seed, "plain"), update="none")
+        w["xyz"] = w["xyz"] * np.array([stretch, 1, 1], np.float32)
+        w["phi0"] = np.random.default_rng(seed).normal(size=len(w["phi0"])).astype(np.float32) * np.float32(w["h"])
+        hist = [lsgb300.from_workload(w, bit_exact=True, fim_ctas_per_sm=c, largenum=largenum, max_fim_iters=150).solve(2)[0]
+                for c in (3, 5, 7)]
+        assert np.array_equal(hist[0], hist[1], equal_nan=True) and np.array_equal(hist[0], hist[2], equal_nan=True)
