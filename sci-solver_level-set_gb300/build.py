@@ -20,7 +20,8 @@ SOURCES = ["ls_layout.cpp", "ls_meshio.cpp", "ls_partition.cpp", "ls_api.cpp", "
 # translation units compiled without FMA contraction
 NO_FMA = {"ls_kernels_exact.cu"}
 # the fast kernel build: hardware-approximate division and square root
-# (denormals kept); the bit-exact build keeps IEEE-rounded operations
+# (denormals kept, but for the planar-wave solvers' bare operations:
+# fast_sqrt); the bit-exact build keeps IEEE-rounded operations
 FAST_DIV_SQRT = {"ls_kernels.cu"}
 
 

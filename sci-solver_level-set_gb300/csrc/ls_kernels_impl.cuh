@@ -263,8 +263,9 @@ __global__ void __launch_bounds__(kSeedBlock) k_seed(DevMesh m, DevState s, Step
 // Fast build: a tet solve whose candidates provably cannot fall below the
 // target's current value (min(TA, TB, TC) + 0.999 x D's height over the
 // base plane >= T_D) is skipped -- in exact arithmetic it cannot change
-// min(T_D, r).  The bit-exact build keeps every solve (the reference's
-// arithmetic, including FP32 candidates that fall below that bound).
+// min(T_D, r).  The bit-exact build keeps every solve here (the reference's
+// arithmetic, including FP32 candidates that fall below that bound); its
+// k_fim_pair leaves out those that provably change no bit (pair_may_lower).
 #ifdef LS_KERNELS_EXACT
 constexpr bool kLbSkip = false;
 #else
@@ -1103,7 +1104,7 @@ __device__ __forceinline__ bool slab_wait(unsigned bar, unsigned parity, bool gi
 // (k_geometry) by two bulk asynchronous copies that thread 0 issues at the
 // start of each patch; they land while the threads gather the values and
 // load the connectivity, and thread 0 waits for them (bounded) before the
-// setup barrier.  A wait that runs out sets ctl[3] = 2, waits once more for
+// setup barrier.  A wait that runs out sets CTL_ERR, waits once more for
 // the copies in flight and ends the CTA's pass; the host then reports
 // LS_DEVICE_TIMEOUT.
 // Patches: the list entry of the CTA's index first, later ones from
